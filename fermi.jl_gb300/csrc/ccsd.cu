@@ -625,12 +625,12 @@ void residual(fcc_ctx* c) {
       ps.rd2 = 1; ps.rd3 = v; ps.rs1 = n; ps.rs2 = 0; ps.rs3 = 1;
       ps.kd2 = 1; ps.kd3 = Q; ps.ks1 = 0; ps.ks2 = 0; ps.ks3 = n * n;
       if (tc->exact) {
-        const int S = tc->oz_groups - 1;
+        const int S = tc->oz.S;
         Wk = S * oz_kpad(Q);
         ps.Kp = Wk;
         if ((int64_t)c->bvvA.n < R * Wk) c->bvvA.alloc(R * Wk);
         if ((int64_t)c->bvvEx.n < R) c->bvvEx.alloc(R);
-        pack_oz(Btvv.p, ps, S, c->bvvA.p, c->bvvEx.p, s);
+        pack_oz(Btvv.p, ps, S, tc->oz.bits, c->bvvA.p, c->bvvEx.p, s);
       } else {
         Wk = packed_kp(Q, tc->scheme.P);
         ps.Kp = Wk;
@@ -656,10 +656,9 @@ void residual(fcc_ctx* c) {
         ep.alpha = 1.0; ep.beta = 0.0; ep.C = c->Wslab.p; ep.mode = EPI_F64;
         const int64_t r0 = a0 * v;
         if (tc->exact) {
-          const int G = tc->oz_groups;
-          ep.work = 2.0 * (double)ep.M * (double)ep.N * (double)Q * ((double)(G - 1) * (double)G / 2.0);
-          gemm_oz(c->bvvA.p + r0 * Wk, ep.M, c->bvvEx.p + r0, c->bvvA.p + r0 * Wk, ep.N, c->bvvEx.p + r0, Wk / (G - 1),
-                  G, ep, tc->err, s);
+          ep.work = 2.0 * (double)ep.M * (double)ep.N * (double)Q * oz_pairs(tc->oz);
+          gemm_oz(c->bvvA.p + r0 * Wk, ep.M, c->bvvEx.p + r0, c->bvvA.p + r0 * Wk, ep.N, c->bvvEx.p + r0,
+                  Wk / tc->oz.S, tc->oz, ep, tc->ozws, tc->err, s);
         } else {
           ep.work = 2.0 * (double)ep.M * (double)ep.N * (double)Q * tc->scheme.P;
           ep.no_loads = tc->no_loads_once;
@@ -934,7 +933,7 @@ int ccsd_run(fcc_ctx* c, const fcc_opts* opt, fcc_iter_stats* log, int32_t log_c
       TcScope scope(kind == K_F64 ? nullptr : &c->tc);
       c->tc.enabled = kind != K_F64;
       c->tc.exact = kind == K_EXACT || kind == K_EXACT9;
-      if (kind == K_EXACT9) c->tc.oz_groups = OZ_G_FINISH;
+      if (kind == K_EXACT9) c->tc.oz = oz_level(OZ_G_FINISH);
       // exact-slice width by the size of the step: 6 weight groups (15 slice
       // pairs; noise floor in the Jacobi step ~1e-8 at (H2O)8) while the step
       // is above 100 max_rms, then 7 groups (21 pairs, floor ~1e-10, two
@@ -945,7 +944,7 @@ int ccsd_run(fcc_ctx* c, const fcc_opts* opt, fcc_iter_stats* log, int32_t log_c
         const int groups = std::max(exact_groups, want);
         if (groups != exact_groups) { best_rms = 1e300; stalled = 0; }
         exact_groups = groups;
-        c->tc.oz_groups = groups;
+        c->tc.oz = oz_level(groups);
       }
       c->tc.scheme = SPLIT3;
       if (c->test_fault == FCC_TEST_FAULT_NO_LOADS && kind == K_MIX) {

@@ -441,7 +441,8 @@ void run_tc(TcEngine* tc, double alpha, const TView& A, const TView& B, double b
   const int64_t M = gdim(gm), N = gdim(gn), K = gdim(gk);
   if (tc->exact) {
     // exact-slice products: S digit slices of each operand, FP64 output
-    const int G = tc->oz_groups, S = G - 1;
+    const OzLevel lv = tc->oz;
+    const int S = lv.S;
     const int64_t Kpad = oz_kpad(K), W = S * Kpad;
     if ((int64_t)tc->bufA.n < M * W) tc->bufA.alloc(M * W);
     if ((int64_t)tc->bufB.n < N * W) tc->bufB.alloc(N * W);
@@ -452,29 +453,28 @@ void run_tc(TcEngine* tc, double alpha, const TView& A, const TView& B, double b
     PackSpec pb{N, K, W, gn[1].dim, gn[2].dim, gn[0].s[1], gn[1].s[1], gn[2].s[1],
                 gk[1].dim, gk[2].dim, gk[0].s[1], gk[1].s[1], gk[2].s[1], S, 0};
     bool fresh;
-    TcEngine::KeptPack* ka = kept_a(tc, A.p, pa, S, fresh);
+    TcEngine::KeptPack* ka = kept_a(tc, A.p, pa, 10 * lv.bits + S, fresh);
     __nv_bfloat16* pA = tc->bufA.p;
     int* eA = tc->exA.p;
     if (ka) {
       if (fresh) {
         if ((int64_t)ka->buf.n < M * W) ka->buf.alloc(M * W);
         if ((int64_t)ka->ex.n < M) ka->ex.alloc(M);
-        pack_oz(A.p, pa, S, ka->buf.p, ka->ex.p, s);
+        pack_oz(A.p, pa, S, lv.bits, ka->buf.p, ka->ex.p, s);
       }
       pA = ka->buf.p;
       eA = ka->ex.p;
     } else {
-      pack_oz(A.p, pa, S, pA, eA, s);
+      pack_oz(A.p, pa, S, lv.bits, pA, eA, s);
     }
-    pack_oz(B.p, pb, S, tc->bufB.p, tc->exB.p, s);
+    pack_oz(B.p, pb, S, lv.bits, tc->bufB.p, tc->exB.p, s);
     EpiMap ep;
     ep.M = M; ep.N = N;
     ep.md2 = gm[1].dim; ep.md3 = gm[2].dim; ep.ms1 = gm[0].s[2]; ep.ms2 = gm[1].s[2]; ep.ms3 = gm[2].s[2];
     ep.nd2 = gn[1].dim; ep.nd3 = gn[2].dim; ep.ns1 = gn[0].s[2]; ep.ns2 = gn[1].s[2]; ep.ns3 = gn[2].s[2];
     ep.alpha = alpha; ep.beta = beta; ep.C = C.p; ep.mode = EPI_F64;
-    const double npairs = (double)(G - 1) * (double)G / 2.0;
-    ep.work = 2.0 * (double)M * (double)N * (double)K * npairs;
-    gemm_oz(pA, M, eA, tc->bufB.p, N, tc->exB.p, Kpad, G, ep, tc->err, s);
+    ep.work = 2.0 * (double)M * (double)N * (double)K * oz_pairs(lv);
+    gemm_oz(pA, M, eA, tc->bufB.p, N, tc->exB.p, Kpad, lv, ep, tc->ozws, tc->err, s);
     tc->tc_calls++;
     tc->tc_flops += ep.work;
     return;

@@ -78,6 +78,11 @@ __device__ __forceinline__ void pack_load4(const double* __restrict__ src, const
                                            int64_t k0, int cnt, double (&x)[4]) {
   if (k1) {
     const double* sp = src + ro + k0 * ps.ks3;
+    if (ps.ks3 == 1 && cnt == 4 && (reinterpret_cast<uintptr_t>(sp) & 15) == 0) {
+      const double2 a = *reinterpret_cast<const double2*>(sp), b = *reinterpret_cast<const double2*>(sp + 2);
+      x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
+      return;
+    }
 #pragma unroll
     for (int q = 0; q < 4; ++q) x[q] = q < cnt ? sp[q * ps.ks3] : 0.0;
   } else {
@@ -136,6 +141,19 @@ struct EpiMap {
   int no_loads = 0;    // test hook: the producer issues no TMA loads, so the bounded waits give up
 };
 
+// Offsets of row m and column n in C (32-bit divisions: M, N < 2^31; a 64-bit
+// one costs a thread about a microsecond on this part).
+__device__ __forceinline__ int64_t epi_row_off(const EpiMap& ep, uint32_t m) {
+  const uint32_t d3 = (uint32_t)ep.md3, d2 = (uint32_t)ep.md2;
+  const uint32_t m3 = m % d3, r = m / d3;
+  return (int64_t)(r / d2) * ep.ms1 + (int64_t)(r % d2) * ep.ms2 + (int64_t)m3 * ep.ms3;
+}
+__device__ __forceinline__ int64_t epi_col_off(const EpiMap& ep, uint32_t n) {
+  const uint32_t d3 = (uint32_t)ep.nd3, d2 = (uint32_t)ep.nd2;
+  const uint32_t n3 = n % d3, r = n / d3;
+  return (int64_t)(r / d2) * ep.ns1 + (int64_t)(r % d2) * ep.ns2 + (int64_t)n3 * ep.ns3;
+}
+
 int64_t packed_kp(int64_t K, int P = 3);
 void pack_split(const double* src, const PackSpec& ps, __nv_bfloat16* dst, cudaStream_t s);
 // D = A' B'^T over Kp packed columns; rows a_row0.. of A' (a_rows total) and
@@ -152,22 +170,43 @@ void scale_output(const EpiMap& ep, double beta, cudaStream_t s);
 // Exact-slice products (the Ozaki scheme: Ozaki, Ogita, Oishi & Rump, Numer.
 // Algorithms 59, 95 (2012); on tensor cores: Mukunoki et al., ISC 2020).
 // Each row r of an operand is scaled by 2^e_r (|x| < 2^e_r over the row) and
-// cut into S = G-1 signed 6-bit digit slices, x = 2^e_r sum_s d_s 2^(-6(s+1)),
-// |d| <= 64, stored exactly in BF16.  A.B^T is the sum over slice pairs
-// (s, t) with s + t + 2 <= G of the digit products; pairs of one weight
-// 2^(-6(s+t+2)) are summed on the tensor cores in FP32 over chunks of 2048
-// products (|sum| <= 2^23, so every partial sum is an exact integer) and the
-// chunks are added in double-FP32 (~2^-48 relative) in TMEM.  The result
-// carries the slice truncation error, ~2^(-6(G-1)) of max|A_r| max|B_c| per
-// term (G = 8: ~1e-12 of max|C| for Gaussian operands).
+// cut into S balanced digit slices of b bits, x = 2^e_r sum_s d_s 2^(-b s),
+// |d_1| <= 2^b, |d_s| <= 2^(b-1), stored exactly in BF16 (8-bit significand).
+// A.B^T is the sum over slice pairs (s, t) with s + t <= G of the digit
+// products; pairs of one weight 2^(-b (s+t)) are summed on the tensor cores in
+// FP32 while |sum| <= 2^24, so every partial sum is an exact integer, and
+// those are added in double-FP32 (~2^-48 relative).  BF16 carries 8-bit digits
+// exactly, and fewer, wider digits need fewer products for the same bits: 48
+// bits take S = 6 and 21 products instead of the 36 of eight 6-bit digits.
+// The reduced levels of the mixed form stay at 6-bit digits: its iterates, and
+// so its converged amplitudes, depend on what those levels drop.
+// `cut` > 0: the first `cut` bands of groups get a running sum of their own
+// (the FP64 level, see gemm_oz.cu).
+struct OzLevel {
+  int S, G, cut, bits;
+};
+constexpr int OZ_MAXS = 7;
 constexpr int OZ_G_DEFAULT = 8;
+// the level of `groups` weight groups of 6-bit digits, the unit the phases of
+// the mixed form are counted in: those digits themselves up to 7 groups, 8-bit
+// digits with at least their 6 (groups - 1) bits above
+OzLevel oz_level(int groups);
+// slice pairs (BF16 products) of a level
+inline double oz_pairs(OzLevel lv) {
+  int n = 0;
+  for (int a = 1; a <= lv.S; ++a) n += std::max(0, std::min(lv.S, lv.G - a));
+  return n;
+}
 // packed layout: row r holds slice s at columns [s*Kpad, s*Kpad + K), zero up
-// to (s+1)*Kpad; ex[r] = biased FP64 exponent of max_k |x_rk| (0: all zero)
+// to (s+1)*Kpad; ex[r] = biased FP64 exponent of max_k |x_rk| (0: all zero,
+// 2047: the row holds an infinity or NaN, and so will its products)
 int64_t oz_kpad(int64_t K);
-void pack_oz(const double* src, const PackSpec& ps, int S, __nv_bfloat16* dst, int* ex, cudaStream_t s);
-// FP64 epilogue (EPI_F64) of the exact-slice product over packed operands
+// (S up to 8 with 6-bit digits, 7 with 8-bit digits)
+void pack_oz(const double* src, const PackSpec& ps, int S, int bits, __nv_bfloat16* dst, int* ex, cudaStream_t s);
+// FP64 epilogue (EPI_F64) of the exact-slice product over packed operands;
+// ws holds the partial results of products cut into several jobs
 void gemm_oz(const __nv_bfloat16* A, int64_t a_rows, const int* exA, const __nv_bfloat16* B, int64_t b_rows,
-             const int* exB, int64_t Kpad, int G, const EpiMap& ep, int* err, cudaStream_t s);
+             const int* exB, int64_t Kpad, OzLevel lv, const EpiMap& ep, DBuf<double>& ws, int* err, cudaStream_t s);
 
 // Engine state for einsum calls that run on the tensor cores: scratch for
 // the packed operands, the device error flag, the routing threshold and
@@ -176,8 +215,9 @@ struct TcEngine {
   bool enabled = false;
   SplitScheme scheme = SPLIT3;
   bool exact = false;      // exact-slice products instead of the split scheme
-  int oz_groups = OZ_G_DEFAULT;
+  OzLevel oz = oz_level(OZ_G_DEFAULT);
   DBuf<int> exA, exB;
+  DBuf<double> ozws;       // partial results of exact-slice products cut into jobs
   double min_flops = 1e6;
   int64_t min_dim = 16;   // smallest M and N routed to the tensor cores
   DBuf<__nv_bfloat16> bufA, bufB;

@@ -10,21 +10,18 @@
 namespace fcc {
 namespace tc5 {
 
-constexpr uint64_t WAIT_NS = 2000000000ull;  // every mbarrier wait gives up after 2 s
+constexpr long long WAIT_CLK = 4000000000ll;  // every mbarrier wait gives up after about 2 s of SM clocks
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-__device__ __forceinline__ uint64_t globaltimer() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-// Bounded wait on an mbarrier phase; false after WAIT_NS.
+// Bounded wait on an mbarrier phase; false after WAIT_CLK.  The limit is
+// counted on the SM clock: a wait that is not satisfied at once is the normal
+// case in every pipeline here, and reading %globaltimer in it costs more than
+// the wait itself.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-  uint64_t t0 = 0;
+  long long t0 = 0;
   for (uint32_t it = 0;; ++it) {
     uint32_t ok;
     asm volatile(
@@ -33,9 +30,30 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
         : "r"(bar), "r"(parity)
         : "memory");
     if (ok) return true;
-    if (it == 0) t0 = globaltimer();
-    else if ((it & 63) == 0 && globaltimer() - t0 > WAIT_NS) return false;
+    if (it == 0) t0 = clock64();
+    else if ((it & 15) == 0 && clock64() - t0 > WAIT_CLK) return false;
   }
+}
+
+// True in one lane of a converged warp.  Roles that issue TMA loads or MMAs
+// are entered through this and not through a comparison of the lane number:
+// their operands sit in uniform registers, and only here does the compiler
+// know that one thread runs the code.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(ok));
+  return ok != 0;
+}
+
+// Whether an mbarrier phase has completed, without waiting.
+__device__ __forceinline__ uint32_t mbar_test(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok;
 }
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
@@ -79,6 +97,15 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
+// One MMA (K = 16) of the calling CTA; acc = 0 overwrites the accumulator.
+__device__ __forceinline__ void mma_bf16(uint32_t d, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+      "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
+      : "memory");
+}
+
 // (double)f * 2^e (negated if neg) by integer exponent arithmetic; FP32
 // subnormals and results below the FP64 normal range give 0
 __device__ __forceinline__ double f32_to_f64_scaled(float f, int e, bool neg) {
@@ -96,13 +123,14 @@ __device__ __forceinline__ double f32_to_f64_scaled(float f, int e, bool neg) {
 // Output tile of linear block index lin on a tm x tn tile grid, walked in
 // groups of 8 tile rows (row fastest inside a group) so that the CTAs resident
 // at the same time share A and B panels in L2.
-__device__ __forceinline__ void grouped_tile(int64_t lin, int64_t tm, int64_t tn, int64_t& mt, int64_t& nt) {
-  constexpr int64_t GM = 8;
-  const int64_t per_group = GM * tn;
-  const int64_t g = lin / per_group;
-  const int64_t first = g * GM;
-  const int64_t gm = tm - first < GM ? tm - first : GM;
-  const int64_t r = lin - g * per_group;
+// (32-bit arithmetic: a 64-bit division takes the FP64 pipe, at 1/64 rate here)
+__device__ __forceinline__ void grouped_tile(uint32_t lin, uint32_t tm, uint32_t tn, uint32_t& mt, uint32_t& nt) {
+  constexpr uint32_t GM = 8;
+  const uint32_t per_group = GM * tn;
+  const uint32_t g = lin / per_group;
+  const uint32_t first = g * GM;
+  const uint32_t gm = tm - first < GM ? tm - first : GM;
+  const uint32_t r = lin - g * per_group;
   mt = first + r % gm;
   nt = r / gm;
 }

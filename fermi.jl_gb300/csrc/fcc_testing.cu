@@ -101,7 +101,7 @@ extern "C" int fcc_test_contract(int32_t precision, const char* spec, const doub
     if (precision == 2) eng.scheme = fcc::SPLIT6;
     if (precision == 3 || (precision >= 12 && precision <= 19)) {
       eng.exact = true;
-      eng.oz_groups = precision == 3 ? fcc::OZ_G_DEFAULT : precision - 10;
+      eng.oz = fcc::oz_level(precision == 3 ? fcc::OZ_G_DEFAULT : precision - 10);
     } else if (precision < 0 || precision > 3) {
       return FCC_ERR_BAD_ARG;
     }
@@ -166,7 +166,9 @@ extern "C" int fcc_test_split3(const double* x, int64_t R, int64_t K, int32_t ro
 extern "C" int fcc_test_pack_oz(const double* x, int64_t R, int64_t K, int32_t row_fastest, int32_t S, uint16_t* out,
                                 int32_t* ex) {
   try {
-    if (!x || !out || !ex || R < 1 || K < 1 || S < 1 || S > 8) return FCC_ERR_BAD_ARG;
+    const bool wide = S > 10;   // 10 + S: the products' 8-bit digits
+    if (wide) S -= 10;
+    if (!x || !out || !ex || R < 1 || K < 1 || S < 1 || S > (wide ? fcc::OZ_MAXS : 8)) return FCC_ERR_BAD_ARG;
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev < 1) return FCC_ERR_NO_DEVICE;
     FCC_CUDA(cudaSetDevice(0));
@@ -187,7 +189,7 @@ extern "C" int fcc_test_pack_oz(const double* x, int64_t R, int64_t K, int32_t r
     dy.alloc(n);
     dex.alloc(R);
     FCC_CUDA(cudaMemcpyAsync(dx.p, x, sizeof(double) * R * K, cudaMemcpyHostToDevice, s));
-    fcc::pack_oz(dx.p, ps, S, dy.p, dex.p, s);
+    fcc::pack_oz(dx.p, ps, S, wide ? 8 : 6, dy.p, dex.p, s);
     FCC_CUDA(cudaMemcpyAsync(out, dy.p, sizeof(uint16_t) * n, cudaMemcpyDeviceToHost, s));
     FCC_CUDA(cudaMemcpyAsync(ex, dex.p, sizeof(int32_t) * R, cudaMemcpyDeviceToHost, s));
     FCC_CUDA(cudaStreamSynchronize(s));

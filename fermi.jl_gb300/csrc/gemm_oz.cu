@@ -1,24 +1,43 @@
 // Exact-slice BF16 tensor-core contraction (the Ozaki scheme) for GB300.
 //
-// C = alpha * A.B^T + beta * C for FP64 operands, evaluated from signed 6-bit
-// digit slices of A and B (see fcc_tc.cuh).  Every digit is an integer
-// |d| <= 64, exact in BF16; every product of two digits is an integer of at
-// most 2^12, so a run of 2048 products accumulated by tcgen05.mma in FP32
-// stays an exact integer (|sum| <= 2^23).  The kernel therefore closes an
-// accumulation chunk every 32 k-blocks (or at the end of a weight group), and
-// the epilogue warps add the chunk, times its weight 2^(-6g) (exact), into a
-// double-FP32 (hi + lo, ~2^-48 relative) running sum held in TMEM.  Two TMEM
-// accumulators alternate, so the MMA thread fills one while the epilogue
-// drains the other.  The final epilogue converts hi and lo to FP64 with the
-// row and column scales applied by integer exponent arithmetic (the FP64 pipe
-// is 1/64 rate) and stores or reduces (red.add) into C.
+// C = alpha * A.B^T + beta * C for FP64 operands, evaluated from signed digit
+// slices of A and B (pack_oz.cu, fcc_tc.cuh).  Every digit is an integer,
+// |d| <= 2^bits (the first digit) or 2^(bits-1) (the others), exact in BF16,
+// and tcgen05.mma accumulates products of such digits exactly in FP32 while
+// |sum| <= 2^24.
 //
-// TMEM columns (128 x 512 x 32-bit): [0,128) and [128,256) chunk
-// accumulators, [256,384) hi and [384,512) lo words of the running sums.
+// Slice pairs of one weight 2^(-bits g) (g = sa + sb, slices counted from 1)
+// share an accumulator.  Two neighbouring groups g, g + 1 form a band and run
+// together, because their pairs can be ordered so that each step shares one
+// operand tile with the step before: the tiles
+//   B_g, A_1, B_(g-1), A_2, ..., B_1, A_g
+// arrive as one stream and step i multiplies tiles i and i + 1.  A step then
+// moves 16 KB into shared memory instead of 32 KB.  What bounds long products
+// is shared-memory bandwidth (128 B/clk per SM): the MMAs of a 128 x 128 x 64
+// step read 32 KB in 256 clk while the incoming tile is written, 384 clk with
+// one new tile (two thirds of the tensor rate), 512 with two.  Measured at M =
+// N = K = 4864: 1330 TFLOP/s executed (21 products of 6-bit digits, 3.6 ms;
+// 6.0 ms and 802 TFLOP/s with two tiles a step and single threads the compiler
+// could not tell from warps, fcc_tcgen05.cuh elect_one).
+//
+// When an accumulator could reach 2^24 (a chunk: 1-4 k-blocks of 8-bit digits,
+// 25-64 of 6-bit ones) the eight epilogue warps add it, times its weight (a
+// power of two), into a running double-FP32 sum (hi + lo, ~2^-48 relative)
+// held in registers, 64 columns per thread.  Registers instead of TMEM leave
+// TMEM for two sets of two chunk accumulators, so the MMA thread fills one set
+// while the other is drained, and a drain reads 4 bytes per element from TMEM
+// instead of moving 20.  The additions run two per instruction (fma.rn.f32x2).
+// With 8-bit digits the chunks are short and the drains show: 1200 TFLOP/s at
+// 4864, 4.0 ms for the 48 bits that took 10.2 ms with 36 products of 6-bit
+// digits.
+//
+// `cut`: the first band (groups 2 and 3) and the rest get separate running
+// sums ("parts"), each converted and added to C in FP64.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <mutex>
 
@@ -31,75 +50,103 @@ namespace {
 
 using namespace tc5;
 
-constexpr int OZ_BM = 128;
-constexpr int OZ_BN = 128;
-constexpr int OZ_BK = 64;
-constexpr int OZ_STAGES = 6;
-constexpr int OZ_THREADS = 192;      // warp 0 TMA, warp 1 MMA, warps 2-5 epilogue
-constexpr int OZ_BITS = 6;           // bits per digit slice
-constexpr int OZ_CH = 32;            // k-blocks per exact FP32 chunk: 2048 products of at most 64*64, |sum| <= 2^23
-constexpr int OZ_MAXPAIRS = 40;
-constexpr int OZ_A_BYTES = OZ_BM * OZ_BK * 2;
-constexpr int OZ_B_BYTES = OZ_BN * OZ_BK * 2;
-constexpr int OZ_STAGE_BYTES = OZ_A_BYTES + OZ_B_BYTES;
-// the final epilogue's 32 x 32 FP64 transpose tile per epilogue warp, beside
-// the operand ring (a persistent CTA is already loading its next unit)
-constexpr int OZ_TILE_BYTES = 4 * 32 * 33 * 8;
-constexpr int OZ_SMEM = OZ_STAGES * OZ_STAGE_BYTES + OZ_TILE_BYTES + 1024;
-constexpr int OZ_COL_LO = 256, OZ_COL_HI = 384;
+constexpr int OZ_BM = 128, OZ_BN = 128, OZ_BK = 64;
+constexpr int OZ_SLOTS = 11;                     // tile ring
+constexpr int OZ_TILE_BYTES = 128 * OZ_BK * 2;   // one operand tile, A or B
+constexpr int OZ_EPI_WARPS = 8;
+constexpr int OZ_THREADS = 128 + 32 * OZ_EPI_WARPS;   // warp 0 TMA, 1 MMA, 2-3 idle, 4-11 epilogue
+constexpr int OZ_XP_LD = 17;                     // FP64 transpose tile of an epilogue warp: 32 rows x 16 columns
+constexpr int OZ_XP_BYTES = OZ_EPI_WARPS * 32 * OZ_XP_LD * 8;
+constexpr int OZ_SMEM = OZ_SLOTS * OZ_TILE_BYTES + OZ_XP_BYTES + 1024;
+constexpr int OZ_MAXBANDS = 5, OZ_MAXJOBS = 152;
 
-// Slice pairs in the order of the k loop: by weight group g = sa + sb + 2,
-// then by sa; next[p] = first pair of the following group.
-struct OzPairs {
-  int n;
-  int8_t sa[OZ_MAXPAIRS], sb[OZ_MAXPAIRS], g[OZ_MAXPAIRS];
-  int16_t next[OZ_MAXPAIRS];
+// One band: groups g (and g + 1 when ngrp = 2), ntile operand tiles per
+// k-block, alternating B and A (bfirst) or A and B; the A tiles are slices 0,
+// 1, ..., the B tiles btop, btop - 1, ...; ck k-blocks per chunk.  Step j
+// multiplies tiles j and j + 1, and successive steps alternate between the
+// two groups.
+struct OzBand {
+  int16_t ntile, ck, g, ngrp, bfirst, btop;
+};
+// One piece of an output tile's work: bands [b0, b1) over k-blocks [k0, k1).
+struct OzJob {
+  int16_t b0, b1;
+  int32_t k0, k1;
+};
+struct OzParams {
+  OzBand band[OZ_MAXBANDS];
+  OzJob job[OZ_MAXJOBS];
+  int njobs, cut;              // cut: bands of the first part (0: one part)
+  int bits;                    // digit width
+  int kper, kpad;              // k-blocks per L2 block; padded columns per slice
+  uint32_t tm, tn, units;
+  double* part;                // partial results [job][M][N] (nullptr: C itself)
 };
 
-OzPairs make_pairs(int G) {
-  OzPairs p;
-  std::memset(&p, 0, sizeof(p));
-  const int S = G - 1;
-  for (int g = 2; g <= G; ++g) {
-    const int first = p.n;
-    for (int a = 1; a < g; ++a) {
-      const int b = g - a;
-      if (a > S || b > S) continue;
-      p.sa[p.n] = (int8_t)(a - 1);
-      p.sb[p.n] = (int8_t)(b - 1);
-      p.g[p.n] = (int8_t)g;
-      ++p.n;
+// The bands of groups 2..G over S slices (G <= S + 2): {.., (G-3, G-2),
+// (G-1, G)}, group 2 on its own when their number is odd.
+int make_bands(int S, int G, int bits, OzBand* out) {
+  int n = 0;
+  for (int g = 2; g <= G;) {
+    OzBand b;
+    b.g = (int16_t)g;
+    b.ngrp = (int16_t)(((G - 1) % 2 == 1 && g == 2) ? 1 : 2);
+    b.bfirst = b.ngrp == 2 && g <= S;        // B_g, A_1, B_(g-1), A_2, ..., B_1, A_g
+    b.btop = (int16_t)(b.ngrp == 1 ? 0 : (b.bfirst ? g - 1 : S - 1));
+    b.ntile = (int16_t)(2 * (b.btop + 1));
+    // units of 64 2^(2 bits - 2) (64 products of two digits after the first)
+    // that one k-block adds to a group: 4 for (1,1), 2 for a pair with one
+    // first digit, 1 otherwise; the sum may reach 2^24
+    int worst = 0;
+    for (int q = 0; q < b.ngrp; ++q) {
+      int u = 0;
+      for (int a = 1; a < g + q; ++a) {
+        const int c = g + q - a;
+        if (a <= S && c <= S) u += (a == 1 ? 2 : 1) * (c == 1 ? 2 : 1);
+      }
+      worst = std::max(worst, u);
     }
-    for (int q = first; q < p.n; ++q) p.next[q] = (int16_t)p.n;
+    b.ck = (int16_t)std::max(1, (1 << (20 - 2 * bits)) / worst);
+    out[n++] = b;
+    g += b.ngrp;
   }
-  return p;
-}
-
-// end of the chunk that starts at step st (steps pair-major, nkb k-blocks per
-// pair): at most OZ_CH steps, never across a weight group or the end st1
-__device__ __forceinline__ int oz_chunk_end(const OzPairs& pr, int nkb, int st, int st1) {
-  const int gend = (int)pr.next[st / nkb] * nkb;
-  return min(min(st + OZ_CH, gend), st1);
-}
-
-// 2^e as a double (0 below the normal range)
-__device__ __forceinline__ double oz_pow2(int e) {
-  if (e < -1022) return 0.0;
-  if (e > 1023) e = 1023;
-  return __longlong_as_double((long long)(e + 1023) << 52);
+  return n;
 }
 
 // frexp-style exponent of the row scale from the stored biased exponent
-__device__ __forceinline__ int oz_row_exp(int be) { return be ? be - 1022 : 0; }
+// (2^21 for a row with infinities or NaN)
+__device__ __forceinline__ int oz_scale_exp(int be) { return be == 2047 ? (1 << 21) : (be ? be - 1022 : 0); }
 
-// hi + lo += v in double-FP32 (TwoSum, then renormalisation)
-__device__ __forceinline__ void ff_add(float& hi, float& lo, float v) {
-  const float s = __fadd_rn(hi, v);
-  const float bb = __fsub_rn(s, hi);
-  const float err = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, bb)), __fsub_rn(v, bb));
-  const float l = __fadd_rn(lo, err);
-  const float h = __fadd_rn(s, l);
-  lo = __fsub_rn(l, __fsub_rn(h, s));
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t pack2(uint32_t x, uint32_t y) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(x), "r"(y));
+  return d;
+}
+__device__ __forceinline__ void unpack2(uint64_t d, uint32_t& x, uint32_t& y) {
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(x), "=r"(y) : "l"(d));
+}
+
+// two independent (hi + lo) += v * w in double-FP32: TwoSum of hi and v * w
+// (the product by a power of two is exact inside the fma), the error into lo,
+// renormalised
+__device__ __forceinline__ void ff_add2(uint64_t& hi, uint64_t& lo, uint64_t v, uint64_t w, uint64_t m1) {
+  const uint64_t s = fma2(v, w, hi);
+  const uint64_t nbb = fma2(s, m1, hi);       // -(s - hi)
+  const uint64_t t = add2(s, nbb);
+  const uint64_t err = add2(fma2(t, m1, hi), fma2(v, w, nbb));
+  const uint64_t l = add2(lo, err);
+  const uint64_t h = add2(s, l);
+  lo = fma2(fma2(s, m1, h), m1, l);
   hi = h;
 }
 
@@ -114,71 +161,61 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
       : "r"(taddr));
 }
 
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
-      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
-      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]),
-      "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]),
-      "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-      : "memory");
+// (hi + lo) * 2^e as one FP64 number, rounded once, by integer arithmetic: lo
+// is turned into units of the 53-bit last place of hi (at most 2^29, one
+// float-to-integer conversion) and added to the bit pattern of hi.  The FP64
+// pipe (1/64 rate) would take two conversions and an addition per element.
+// |lo| <= ulp(hi) / 2, as ff_add2 leaves it; |hi| is 0 or at least 2^-72, the
+// smallest weight.  e >= 2^20 marks a row or column with infinities or NaN.
+__device__ __forceinline__ double ff_to_f64(uint32_t h, uint32_t l, int e, bool neg) {
+  const int eh = (int)((h >> 23) & 0xFF);
+  const uint32_t m = h & 0x7FFFFFu;
+  const int down = (m == 0 && (int)(h ^ l) < 0) ? 1 : 0;    // hi a power of two, |hi + lo| in the binade below
+  const float scale = __uint_as_float((uint32_t)(306 - eh + down) << 23);   // 1 / last place, 2^(179 - eh)
+  int t = __float2int_rn(__fmul_rn(__uint_as_float(l), scale));
+  if ((int)h < 0) t = -t;
+  const int ne = eh + 896 + e;                              // biased FP64 exponent of hi
+  const uint32_t sign = (h & 0x80000000u) ^ (neg ? 0x80000000u : 0u);
+  const uint64_t mag = ((uint64_t)(((uint32_t)ne << 20) | (m >> 3)) << 32 | (uint64_t)(m << 29)) + (uint64_t)(int64_t)t;
+  uint32_t w1 = (uint32_t)(mag >> 32), w0 = (uint32_t)mag;
+  if (eh == 0 || ne <= 0) w1 = w0 = 0;
+  if (ne > 2046) { w1 = 0x7FF00000u; w0 = 0; }
+  if (e >= (1 << 20)) w1 = 0x7FF80000u;
+  return __longlong_as_double((long long)((uint64_t)(w1 | sign) << 32 | w0));
 }
 
-// Work unit u of the persistent grid: output tile grouped_tile(u % tiles)
-// over the K range u / tiles (k-blocks [kb0, kb0 + nku)), all slice pairs;
-// the unit's steps are pair-major, st = p * nku + (kb - kb0).  Units running
-// at the same time share one K range, so the operand panels they stream stay
-// in L2 across the slice pairs that reuse them.
-struct OzUnit {
-  int64_t m0, n0;
-  int kb0, nku;
-};
-__device__ __forceinline__ OzUnit oz_unit(int64_t u, int64_t tm, int64_t tn, int nkb, int kper) {
-  const int64_t tiles = tm * tn;
-  int64_t mt, nt;
-  grouped_tile(u % tiles, tm, tn, mt, nt);
-  const int z = (int)(u / tiles);
-  OzUnit r;
-  r.m0 = mt * OZ_BM;
-  r.n0 = nt * OZ_BN;
-  r.kb0 = z * kper;
-  r.nku = min(nkb, r.kb0 + kper) - r.kb0;
-  return r;
-}
-
-// Persistent: CTA b processes units b, b + gridDim.x, ...  The TMA ring and
-// the two chunk accumulators run on across units, so the loads and the MMAs
-// of a unit's first chunks overlap the previous unit's final epilogue (which
-// reads the running sums; only the epilogue warps touch those, in order).
+// Persistent: CTA b processes units b, b + gridDim.x, ...; unit u is job
+// u / tiles of output tile u % tiles.  The tile ring and the accumulator sets
+// run on across units, so the loads and MMAs of a unit's first chunks overlap
+// the previous unit's stores.  Every role walks the same sequence: parts,
+// L2 blocks of kper k-blocks (units running at the same time share one, so
+// the slices they stream stay in L2), bands, chunks of ck k-blocks.
 __global__ void __launch_bounds__(OZ_THREADS, 1)
-    gemm_oz_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int nkb,
-                   int kpad, const __grid_constant__ OzPairs pr, int kper, int64_t tm, int64_t tn,
-                   int64_t units, const int* __restrict__ exA, const int* __restrict__ exB, int G, EpiMap ep,
-                   int* err) {
+    gemm_oz_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                   const __grid_constant__ OzParams P, const int* __restrict__ exA, const int* __restrict__ exB,
+                   const __grid_constant__ EpiMap ep, int* err) {
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t full_bar[OZ_STAGES];
-  __shared__ __align__(8) uint64_t empty_bar[OZ_STAGES];
-  __shared__ __align__(8) uint64_t accf_bar[2];   // chunk accumulator b is complete
-  __shared__ __align__(8) uint64_t acce_bar[2];   // chunk accumulator b is drained
+  __shared__ __align__(8) uint64_t full_bar[OZ_SLOTS];
+  __shared__ __align__(8) uint64_t empty_bar[OZ_SLOTS];
+  __shared__ __align__(8) uint64_t accf_bar[2];   // accumulator set b is complete
+  __shared__ __align__(8) uint64_t acce_bar[2];   // accumulator set b is drained
   __shared__ __align__(8) uint64_t done_bar;      // every issued MMA has completed
   __shared__ uint32_t tmem_holder;
   __shared__ int abort_flag;
 
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sA = smem;
-  uint8_t* sB = smem + OZ_STAGES * OZ_A_BYTES;
-  double* stile = reinterpret_cast<double*>(smem + OZ_STAGES * OZ_STAGE_BYTES);
+  double* xp = reinterpret_cast<double*>(smem + OZ_SLOTS * OZ_TILE_BYTES);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t tiles = P.tm * P.tn;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < OZ_STAGES; ++s) {
+    for (int s = 0; s < OZ_SLOTS; ++s) {
       mbar_init(smem_u32(&full_bar[s]), 1);
       mbar_init(smem_u32(&empty_bar[s]), 1);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&accf_bar[b]), 1);
-      mbar_init(smem_u32(&acce_bar[b]), 4);   // one arrival per epilogue warp
+      mbar_init(smem_u32(&acce_bar[b]), OZ_EPI_WARPS);
     }
     mbar_init(smem_u32(&done_bar), 1);
     abort_flag = 0;
@@ -195,178 +232,293 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_holder;
 
-  if (warp == 0 && lane == 0) {
-    // ---------------- TMA producer
-    int it = 0;
-    bool stop = false;
-    for (int64_t u = blockIdx.x; u < units && !stop; u += gridDim.x) {
-      const OzUnit un = oz_unit(u, tm, tn, nkb, kper);
-      const int nst = pr.n * un.nku;
-      for (int st = 0; st < nst; ++st, ++it) {
-        const int s = it % OZ_STAGES;
-        const uint32_t ph = (it / OZ_STAGES) & 1;
-        if (!mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1)) { atomicExch(&abort_flag, 1); stop = true; break; }
-        if (*(volatile int*)&abort_flag) { stop = true; break; }
-        const int p = st / un.nku, kb = un.kb0 + (st - p * un.nku);
-        const uint32_t fb = smem_u32(&full_bar[s]);
-        mbar_expect_tx(fb, OZ_STAGE_BYTES);
-        tma_load_2d(smem_u32(sA + s * OZ_A_BYTES), &tmA, (int)pr.sa[p] * kpad + kb * OZ_BK, (int32_t)un.m0, fb);
-        tma_load_2d(smem_u32(sB + s * OZ_B_BYTES), &tmB, (int)pr.sb[p] * kpad + kb * OZ_BK, (int32_t)un.n0, fb);
-      }
-    }
-    // on an abort, wait (bounded) for the loads still in flight before the
-    // shared memory can be released
-    if (*(volatile int*)&abort_flag) {
-      for (int j = max(0, it - OZ_STAGES); j < it; ++j)
-        (void)mbar_wait(smem_u32(&full_bar[j % OZ_STAGES]), (j / OZ_STAGES) & 1);
-    }
-  } else if (warp == 1 && lane == 0) {
-    // ---------------- MMA issuer
-    constexpr uint32_t idesc = idesc_bf16(OZ_BM, OZ_BN);
-    int it = 0, chunk = 0;
-    bool ok = true;
-    for (int64_t u = blockIdx.x; u < units && ok; u += gridDim.x) {
-      const OzUnit un = oz_unit(u, tm, tn, nkb, kper);
-      const int nst = pr.n * un.nku;
-      for (int st = 0; st < nst && ok;) {
-        const int ce = oz_chunk_end(pr, un.nku, st, nst);
-        const int b = chunk & 1;
-        if (!mbar_wait(smem_u32(&acce_bar[b]), ((chunk >> 1) & 1) ^ 1)) { atomicExch(&abort_flag, 1); ok = false; break; }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t dcol = tmem + (uint32_t)(b * OZ_BN);
-        for (int x = st; x < ce; ++x, ++it) {
-          const int s = it % OZ_STAGES;
-          const uint32_t ph = (it / OZ_STAGES) & 1;
-          if (!mbar_wait(smem_u32(&full_bar[s]), ph)) { atomicExch(&abort_flag, 1); ok = false; break; }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint64_t ad = sw128_desc(smem_u32(sA + s * OZ_A_BYTES));
-          const uint64_t bd = sw128_desc(smem_u32(sB + s * OZ_B_BYTES));
-#pragma unroll
-          for (int kk = 0; kk < OZ_BK / 16; ++kk) {
-            const uint32_t acc = (x > st || kk > 0) ? 1u : 0u;
-            asm volatile(
-                "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(dcol),
-                "l"(ad + (uint64_t)(2 * kk)), "l"(bd + (uint64_t)(2 * kk)), "r"(idesc), "r"(acc)
-                : "memory");
+  if (warp < 4) {
+    // 384 threads x 168 registers at launch; the epilogue warps take 216
+    // (128 x 56 + 256 x 216 = 62464 <= 64512)
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    if (warp == 0 || warp == 2) {
+     if (elect_one()) {
+      // ---------------- TMA producers: warp 0 streams the A tiles, warp 2 the
+      // B tiles.  One load costs its thread ~300 clk of issue, more than the
+      // 256 clk of a step's MMAs, so one thread could not feed both.
+      const bool isB = warp == 2;
+      const CUtensorMap* tm = isB ? &tmB : &tmA;
+      int s = 0;                   // ring slot of the chain's first tile, and its phase
+      uint32_t ph = 0;
+      uint32_t issued = 0, parity = 0;   // slots loaded by this thread, phase parity of the last load of each
+      bool stop = false;
+      for (uint32_t u = blockIdx.x; u < P.units && !stop; u += gridDim.x) {
+        uint32_t mt, nt;
+        grouped_tile(u % tiles, P.tm, P.tn, mt, nt);
+        const OzJob jb = P.job[u / tiles];
+        const int row = (int)(isB ? nt * OZ_BN : mt * OZ_BM);
+        int bb = jb.b0;
+        while (bb < jb.b1 && !stop) {
+          const int be = (bb < P.cut) ? min(P.cut, (int)jb.b1) : (int)jb.b1;   // this part's bands
+          for (int zb = jb.k0; zb < jb.k1 && !stop; zb += P.kper) {
+            const int ze = min(zb + P.kper, jb.k1);
+            for (int b = bb; b < be && !stop; ++b) {
+              const OzBand bd = P.band[b];
+              const int off = (bd.bfirst != 0) == isB ? 0 : 1, np = bd.ntile >> 1;
+              const int x0 = (isB ? (int)bd.btop : 0) * P.kpad, dx = isB ? -P.kpad : P.kpad;
+              for (int kb = zb; kb < ze; ++kb) {
+                int cs = s + off;
+                uint32_t cp = ph;
+                if (cs >= OZ_SLOTS) { cs -= OZ_SLOTS; cp ^= 1; }
+                int x = x0 + kb * OZ_BK;
+                for (int i = 0; i < np; ++i, x += dx) {
+                  if (!mbar_wait(smem_u32(&empty_bar[cs]), cp ^ 1)) { atomicExch(&abort_flag, 1); stop = true; break; }
+                  const uint32_t fb = smem_u32(&full_bar[cs]);
+                  mbar_expect_tx(fb, OZ_TILE_BYTES);
+                  tma_load_2d(smem_u32(smem + cs * OZ_TILE_BYTES), tm, x, row, fb);
+                  issued |= 1u << cs;
+                  parity = (parity & ~(1u << cs)) | (cp << cs);
+                  cs += 2;
+                  if (cs >= OZ_SLOTS) { cs -= OZ_SLOTS; cp ^= 1; }
+                }
+                if (stop || *(volatile int*)&abort_flag) { stop = true; break; }
+                s += bd.ntile;
+                while (s >= OZ_SLOTS) { s -= OZ_SLOTS; ph ^= 1; }
+              }
+            }
           }
-          tc_commit(smem_u32(&empty_bar[s]));
+          bb = be;
         }
-        if (!ok) break;
-        tc_commit(smem_u32(&accf_bar[b]));
-        st = ce;
-        ++chunk;
       }
+      // on an abort, wait (bounded) for the loads still in flight before the
+      // shared memory can be released
+      if (*(volatile int*)&abort_flag) {
+        for (int c = 0; c < OZ_SLOTS; ++c)
+          if ((issued >> c) & 1) (void)mbar_wait(smem_u32(&full_bar[c]), (parity >> c) & 1);
+      }
+     }
+    } else if (warp == 1) {
+     if (elect_one()) {
+      // ---------------- MMA issuer.  An MMA's issue waits until the one before
+      // it has started, so whatever the thread does between two steps leaves
+      // the tensor pipe idle unless it runs behind an issued MMA: the next
+      // tile's barrier is read between the MMAs of a step, and a step's
+      // descriptors need one addition each.
+      constexpr uint32_t idesc = idesc_bf16(OZ_BM, OZ_BN);
+      const uint64_t desc0 = sw128_desc(smem_u32(smem));
+      const uint32_t full0 = smem_u32(&full_bar[0]), empty0 = smem_u32(&empty_bar[0]);
+      uint32_t s = 0, ph = 0;      // ring slot of the next tile, and its phase
+      uint32_t chunk = 0;
+      bool ok = true;
+      for (uint32_t u = blockIdx.x; u < P.units && ok; u += gridDim.x) {
+        const OzJob jb = P.job[u / tiles];
+        int bb = jb.b0;
+        while (bb < jb.b1 && ok) {
+          const int be = (bb < P.cut) ? min(P.cut, (int)jb.b1) : (int)jb.b1;
+          for (int zb = jb.k0; zb < jb.k1 && ok; zb += P.kper) {
+            const int ze = min(zb + P.kper, jb.k1);
+            for (int b = bb; b < be && ok; ++b) {
+              const OzBand bd = P.band[b];
+              const int nt_ = bd.ntile;
+              const uint32_t par0 = (uint32_t)(bd.g + bd.bfirst) & 1u;
+              for (int kc = zb; kc < ze && ok; kc += bd.ck, ++chunk) {
+                const int set = chunk & 1;
+                const int ntot = (min(kc + (int)bd.ck, ze) - kc) * nt_;
+                if (!mbar_wait(smem_u32(&acce_bar[set]), ((chunk >> 1) & 1) ^ 1)) {
+                  atomicExch(&abort_flag, 1);
+                  ok = false;
+                  break;
+                }
+                const uint32_t dset = tmem + (uint32_t)(set * 2 * OZ_BN);
+                uint32_t started = 0;        // bit q: the accumulator of parity q holds a sum
+                uint32_t pslot = 0, par = par0, peek = 0;
+                uint32_t curB = (uint32_t)bd.bfirst;   // the tile at s is a B tile
+                int t = 0;
+                for (int x = 0; x < ntot; ++x) {
+                  if (!peek && !mbar_wait(full0 + 8 * s, ph)) { atomicExch(&abort_flag, 1); ok = false; break; }
+                  uint32_t s2 = s + 1, ph2 = ph;
+                  if (s2 == OZ_SLOTS) { s2 = 0; ph2 ^= 1; }
+                  if (t > 0) {
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint64_t ad = desc0 + (uint64_t)((curB ? pslot : s) * (OZ_TILE_BYTES >> 4));
+                    const uint64_t bdsc = desc0 + (uint64_t)((curB ? s : pslot) * (OZ_TILE_BYTES >> 4));
+                    const uint32_t dcol = dset + par * OZ_BN;
+                    const uint32_t acc = (started >> par) & 1u;
+                    mma_bf16(dcol, ad, bdsc, idesc, acc);
+                    peek = mbar_test(full0 + 8 * s2, ph2);
+                    mma_bf16(dcol, ad + 2, bdsc + 2, idesc, 1u);
+                    started |= 1u << par;
+                    par ^= 1u;
+                    mma_bf16(dcol, ad + 4, bdsc + 4, idesc, 1u);
+                    mma_bf16(dcol, ad + 6, bdsc + 6, idesc, 1u);
+                    tc_commit(empty0 + 8 * pslot);                     // its last use
+                  } else {
+                    peek = 0;
+                  }
+                  pslot = s;
+                  s = s2;
+                  ph = ph2;
+                  curB ^= 1u;
+                  if (++t == nt_) {
+                    tc_commit(empty0 + 8 * pslot);
+                    t = 0;
+                    par = par0;
+                  }
+                }
+                if (!ok) break;
+                tc_commit(smem_u32(&accf_bar[set]));
+              }
+            }
+          }
+          bb = be;
+        }
+      }
+      tc_commit(smem_u32(&done_bar));
+     }
     }
-    tc_commit(smem_u32(&done_bar));
-  } else if (warp >= 2) {
-    // ---------------- epilogue warps: rows q*32 .. q*32+31 of each tile
-    const int q = warp & 3;
-    const uint32_t lanebase = tmem + ((uint32_t)(q * 32) << 16);
-    double (*tile)[33] = reinterpret_cast<double (*)[33]>(stile + q * 32 * 33);
+  } else {
+    // ---------------- epilogue warps: rows q*32 .. q*32+31, columns half*64 .. half*64+63 of each tile
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
+    const int q = warp & 3, half = (warp - 4) >> 2;
+    const uint32_t lanebase = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(half * 64);
+    double* tile = xp + (warp - 4) * 32 * OZ_XP_LD;
+    const uint64_t m1 = pack2(0xBF800000u, 0xBF800000u);   // -1, -1
     bool ok = true;
-    int chunk = 0;   // over all units: the accumulator and its barrier phase
+    uint32_t chunk = 0;
     // alpha = +-2^ka folds into the exponent arithmetic; otherwise one FP64 multiply
-    const unsigned long long ab = (unsigned long long)__double_as_longlong(ep.alpha);
+    const double alpha = P.part ? 1.0 : ep.alpha;
+    const unsigned long long ab = (unsigned long long)__double_as_longlong(alpha);
     const bool apow2 = (ab & ((1ull << 52) - 1)) == 0 && ((ab >> 52) & 0x7FF) != 0;
     const int ka = apow2 ? (int)((ab >> 52) & 0x7FF) - 1023 : 0;
     const bool aneg = apow2 && (ab >> 63);
-    for (int64_t u = blockIdx.x; u < units && ok; u += gridDim.x) {
-      const OzUnit un = oz_unit(u, tm, tn, nkb, kper);
-      const int nst = pr.n * un.nku;
-      int uchunk = 0;  // chunks of this unit: the first one starts the running sums
-      for (int st = 0; st < nst;) {
-        const int ce = oz_chunk_end(pr, un.nku, st, nst);
-        const int g = pr.g[st / un.nku];
-        const int b = chunk & 1;
-        ok = mbar_wait(smem_u32(&accf_bar[b]), (chunk >> 1) & 1);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok || __any_sync(0xffffffffu, *(volatile int*)&abort_flag != 0)) { atomicExch(&abort_flag, 1); ok = false; break; }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        // weight of the group, 2^(-6g), exact in FP32
-        const float wg = __int_as_float((127 - OZ_BITS * g) << 23);
+    for (uint32_t u = blockIdx.x; u < P.units && ok; u += gridDim.x) {
+      uint32_t mt, nt;
+      grouped_tile(u % tiles, P.tm, P.tn, mt, nt);
+      const int job = (int)(u / tiles);
+      const OzJob jb = P.job[job];
+      int bb = jb.b0;
+      while (bb < jb.b1 && ok) {
+        const int be = (bb < P.cut) ? min(P.cut, (int)jb.b1) : (int)jb.b1;
+        uint64_t hi[32], lo[32];
+#pragma unroll
+        for (int c = 0; c < 32; ++c) hi[c] = lo[c] = 0ull;
+        for (int zb = jb.k0; zb < jb.k1 && ok; zb += P.kper) {
+          const int ze = min(zb + P.kper, jb.k1);
+          for (int b = bb; b < be && ok; ++b) {
+            const int ck = P.band[b].ck, g0 = P.band[b].g, ng = P.band[b].ngrp;
+            for (int kc = zb; kc < ze; kc += ck, ++chunk) {
+              const int set = chunk & 1;
+              ok = mbar_wait(smem_u32(&accf_bar[set]), (chunk >> 1) & 1);
+              ok = __all_sync(0xffffffffu, ok);
+              if (!ok || __any_sync(0xffffffffu, *(volatile int*)&abort_flag != 0)) {
+                atomicExch(&abort_flag, 1);
+                ok = false;
+                break;
+              }
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+              // weight of the group, 2^(-bits g), exact in FP32; the
+              // accumulators hold exact integers of at most 2^24
 #pragma unroll 1
-        for (int c0 = 0; c0 < OZ_BN; c0 += 32) {
-          uint32_t acc[32], hi[32], lo[32];
-          tmem_ld32(lanebase + (uint32_t)(b * OZ_BN + c0), acc);
-          if (uchunk > 0) {
-            tmem_ld32(lanebase + (uint32_t)(OZ_COL_HI + c0), hi);
-            tmem_ld32(lanebase + (uint32_t)(OZ_COL_LO + c0), lo);
-          }
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+              for (int gq = 0; gq < ng; ++gq) {
+                const int g = g0 + gq;
+                const uint32_t wb = (uint32_t)(127 - P.bits * g) << 23;
+                const uint64_t w = pack2(wb, wb);
+                const uint32_t col = lanebase + (uint32_t)(set * 2 * OZ_BN + (g & 1) * OZ_BN);
 #pragma unroll
-          for (int jj = 0; jj < 32; ++jj) {
-            // the chunk sum is an exact integer below 2^22; times 2^(-6g) exact
-            const float v = __fmul_rn(__uint_as_float(acc[jj]), wg);
-            float h = uchunk > 0 ? __uint_as_float(hi[jj]) : 0.0f;
-            float l = uchunk > 0 ? __uint_as_float(lo[jj]) : 0.0f;
-            ff_add(h, l, v);
-            hi[jj] = __float_as_uint(h);
-            lo[jj] = __float_as_uint(l);
+                for (int c0 = 0; c0 < 2; ++c0) {
+                  uint32_t acc[32];
+                  tmem_ld32(col + (uint32_t)(32 * c0), acc);
+                  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                  for (int j = 0; j < 16; ++j)
+                    ff_add2(hi[16 * c0 + j], lo[16 * c0 + j], pack2(acc[2 * j], acc[2 * j + 1]), w, m1);
+                }
+              }
+              asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+              __syncwarp();
+              if (lane == 0) mbar_arrive(smem_u32(&acce_bar[set]));
+            }
           }
-          tmem_st32(lanebase + (uint32_t)(OZ_COL_HI + c0), hi);
-          tmem_st32(lanebase + (uint32_t)(OZ_COL_LO + c0), lo);
         }
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&acce_bar[b]));
-        st = ce;
-        ++chunk;
-        ++uchunk;
-      }
-      if (!ok || uchunk == 0) break;
-      // ---- final epilogue of the unit: the running sums, scaled, to C (the
-      // unit's last chunk barrier covered every MMA of the unit; the sums were
-      // written by this warp, whose stores have completed)
-      const int row = q * 32 + lane;
-      const int64_t m = un.m0 + row;
-      int64_t crow = 0;
-      int erow = 0;
-      if (m < ep.M) {
-        int64_t m3 = m % ep.md3, r = m / ep.md3;
-        int64_t m2 = r % ep.md2, m1 = r / ep.md2;
-        crow = m1 * ep.ms1 + m2 * ep.ms2 + m3 * ep.ms3;
-        erow = oz_row_exp(exA[m]);
-      }
+        if (!ok) break;
+        // ---- the part's sums, scaled, to the output
+        const int64_t m = (int64_t)mt * OZ_BM + q * 32 + lane;
+        int64_t crow = 0;
+        int erow = 0;
+        if (m < ep.M) {
+          crow = P.part ? ((int64_t)job * ep.M + m) * ep.N : epi_row_off(ep, (uint32_t)m);
+          erow = oz_scale_exp(exA[m]);
+        }
+        // this lane's share of the column exponents: columns lane and lane + 32
+        int ecl[2];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int64_t n = (int64_t)nt * OZ_BN + half * 64 + 32 * c + lane;
+          ecl[c] = n < ep.N ? oz_scale_exp(exB[n]) : 0;
+        }
+        const bool first = bb == jb.b0;
+        // 0: store, 1: add to the output, 2: add to beta times the output
+        const int bmode = first ? (P.part || ep.beta == 0.0 ? 0 : (ep.beta == 1.0 ? 1 : 2)) : 1;
+        const bool plain = bmode == 0 && apow2;
+        double* out = P.part ? P.part : static_cast<double*>(ep.C);
+#pragma unroll
+        for (int c0 = 0; c0 < 4; ++c0) {       // 16 columns at a time
+          const int64_t nb = (int64_t)nt * OZ_BN + half * 64 + 16 * c0;
+          if (nb >= ep.N) continue;
+          const int64_t nl = nb + (lane & 15);
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            uint32_t h0, h1, l0, l1;
+            unpack2(hi[8 * c0 + j], h0, h1);
+            unpack2(lo[8 * c0 + j], l0, l1);
+            const int src = 16 * (c0 & 1) + 2 * j;
+            const int e0 = erow + __shfl_sync(0xffffffffu, ecl[c0 >> 1], src) + ka;
+            const int e1 = erow + __shfl_sync(0xffffffffu, ecl[c0 >> 1], src + 1) + ka;
+            tile[lane * OZ_XP_LD + 2 * j] = ff_to_f64(h0, l0, e0, aneg);
+            tile[lane * OZ_XP_LD + 2 * j + 1] = ff_to_f64(h1, l1, e1, aneg);
+          }
+          __syncwarp();
+          const bool nok = nl < ep.N;
+          int64_t coff = 0;
+          if (nok) {
+            coff = P.part ? nl : epi_col_off(ep, (uint32_t)nl);
+          }
+          // Two rows of 16 columns per store.  The FP64 pipe takes 16 clk per
+          // warp instruction and SM, so the plain store issues none of it, and
+          // a branch, not a select, keeps the others out of it.
+          if (plain) {
+#pragma unroll 4
+            for (int j = 0; j < 16; ++j) {
+              const int r = 2 * j + (lane >> 4);
+              const int64_t off = __shfl_sync(0xffffffffu, crow, r) + coff;
+              if (nok && (int64_t)mt * OZ_BM + q * 32 + r < ep.M) out[off] = tile[r * OZ_XP_LD + (lane & 15)];
+            }
+          } else {
+            // what is added to is read first, four row pairs at a time
 #pragma unroll 1
-      for (int c0 = 0; c0 < OZ_BN; c0 += 32) {
-        if (un.n0 + c0 >= ep.N) break;
-        uint32_t hi[32], lo[32];
-        tmem_ld32(lanebase + (uint32_t)(OZ_COL_HI + c0), hi);
-        tmem_ld32(lanebase + (uint32_t)(OZ_COL_LO + c0), lo);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        // this lane's column exponent, broadcast per column below
-        const int64_t nl = un.n0 + c0 + lane;
-        const int ecl = nl < ep.N ? oz_row_exp(exB[nl]) : 0;
-        __syncwarp();
+            for (int j0 = 0; j0 < 16; j0 += 4) {
+              double prev[4];
+              int64_t off[4];
+              bool okr[4];
 #pragma unroll
-        for (int jj = 0; jj < 32; ++jj) {
-          const int e = erow + __shfl_sync(0xffffffffu, ecl, jj) + ka;
-          tile[lane][jj] = f32_to_f64_scaled(__uint_as_float(hi[jj]), e, aneg) +
-                           f32_to_f64_scaled(__uint_as_float(lo[jj]), e, aneg);
-        }
-        __syncwarp();
-        const int64_t n = un.n0 + c0 + lane;
-        const bool nok = n < ep.N;
-        int64_t coff = 0;
-        if (nok) {
-          int64_t n3 = n % ep.nd3, rr = n / ep.nd3;
-          int64_t n2 = rr % ep.nd2, n1 = rr / ep.nd2;
-          coff = n1 * ep.ns1 + n2 * ep.ns2 + n3 * ep.ns3;
-        }
+              for (int jj = 0; jj < 4; ++jj) {
+                const int r = 2 * (j0 + jj) + (lane >> 4);
+                off[jj] = __shfl_sync(0xffffffffu, crow, r) + coff;
+                okr[jj] = nok && (int64_t)mt * OZ_BM + q * 32 + r < ep.M;
+                prev[jj] = 0.0;
+                if (bmode != 0 && okr[jj]) prev[jj] = out[off[jj]];
+              }
+              if (bmode == 2) {
 #pragma unroll
-        for (int jr = 0; jr < 32; ++jr) {
-          const int64_t roff = __shfl_sync(0xffffffffu, crow, jr);
-          const int64_t mm = un.m0 + q * 32 + jr;
-          if (mm >= ep.M || !nok) continue;
-          double val = tile[jr][lane];
-          if (!apow2) val *= ep.alpha;
-          double* dst = static_cast<double*>(ep.C) + roff + coff;
-          if (ep.atomic) atomicAdd(dst, val);
-          else *dst = val;
+                for (int jj = 0; jj < 4; ++jj) prev[jj] *= ep.beta;
+              }
+#pragma unroll
+              for (int jj = 0; jj < 4; ++jj) {
+                if (!okr[jj]) continue;
+                const double val = tile[(2 * (j0 + jj) + (lane >> 4)) * OZ_XP_LD + (lane & 15)];
+                out[off[jj]] = apow2 ? val + prev[jj] : alpha * val + prev[jj];
+              }
+            }
+          }
+          __syncwarp();
         }
-        __syncwarp();
+        bb = be;
       }
     }
     // every MMA is complete before TMEM is freed
@@ -383,182 +535,25 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   if (threadIdx.x == 0 && abort_flag) atomicExch(err, 1);
 }
 
-// ---------------------------------------------------------------- packing
-
-__device__ __forceinline__ int biased_exp(double x) { return (int)((__double_as_longlong(x) >> 52) & 0x7FF); }
-
-// ex[r] = max over the row of the biased exponent (ex zeroed before), for
-// sources whose k index is the faster one: a warp per (row, k-slab), each
-// lane reading 4 consecutive k at a time
-__global__ void __launch_bounds__(256) oz_exp_rows_kernel(const double* __restrict__ src, PackSpec ps, int64_t kslab,
-                                                          int* __restrict__ ex) {
-  const int lane = threadIdx.x & 31;
-  const int64_t nks = (ps.K + kslab - 1) / kslab;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const bool k1 = pack_k_single(ps);
-  for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < ps.R * nks; w += nw) {
-    const int64_t r = w / nks, ka = (w % nks) * kslab, kb = min(ps.K, ka + kslab);
-    const int64_t ro = pack_row_off(ps, r);
-    int m = 0;
-    for (int64_t k0 = ka + 4 * lane; k0 < kb; k0 += 128) {
-      double xv[4];
-      pack_load4(src, ps, k1, ro, k0, (int)min((int64_t)4, kb - k0), xv);
+// C = alpha * sum_j part[j] + beta * C, the jobs summed in order.
+__global__ void __launch_bounds__(256) oz_reduce_kernel(const double* __restrict__ part, int njobs, EpiMap ep) {
+  const int64_t MN = ep.M * ep.N;
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < MN; t += (int64_t)gridDim.x * blockDim.x) {
+    double s = 0.0;
+    for (int j = 0; j < njobs; j += 8) {   // eight loads in flight, added in order
+      double x[8];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) m = max(m, biased_exp(xv[q]));
+      for (int q = 0; q < 8; ++q) x[q] = j + q < njobs ? part[(int64_t)(j + q) * MN + t] : 0.0;
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (j + q < njobs) s += x[q];
     }
-    m = __reduce_max_sync(0xffffffffu, m);
-    if (lane == 0 && m > 0) atomicMax(ex + r, m);
-  }
-}
-
-// same for sources whose row index is the faster one: 32 rows x 8 k-lanes
-// per block over one k-slab, the column offsets of each 32-column step in
-// shared memory
-__global__ void __launch_bounds__(256) oz_exp_tiles_kernel(const double* __restrict__ src, PackSpec ps, int64_t kslab,
-                                                           int* __restrict__ ex) {
-  __shared__ int red[8][32];
-  __shared__ int64_t coff[32];
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int64_t nrt = (ps.R + 31) / 32, nks = (ps.K + kslab - 1) / kslab;
-  for (int64_t tb = blockIdx.x; tb < nrt * nks; tb += gridDim.x) {
-    const int64_t r = (tb / nks) * 32 + tx;
-    const int64_t ka = (tb % nks) * kslab, kb = min(ps.K, ka + kslab);
-    const int64_t ro = r < ps.R ? pack_row_off(ps, r) : 0;
-    int m = 0;
-    for (int64_t kc = ka; kc < kb; kc += 32) {
-      __syncthreads();   // the previous offsets are consumed
-      if (ty == 0) coff[tx] = kc + tx < kb ? pack_col_off(ps, kc + tx) : 0;
-      __syncthreads();
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int kk = ty + 8 * j;
-        if (r < ps.R && kc + kk < kb) m = max(m, biased_exp(src[ro + coff[kk]]));
-      }
-    }
-    red[ty][tx] = m;
-    __syncthreads();
-    if (ty == 0) {
-      for (int j = 1; j < 8; ++j) m = max(m, red[j][tx]);
-      if (r < ps.R && m > 0) atomicMax(ex + r, m);
-    }
-    __syncthreads();
-  }
-}
-
-// bf16 bits of the integer d (|d| < 2^22; exact in bf16 for |d| <= 256): the
-// float 1.5 * 2^23 + d, less the bias, is d exactly, and its top 16 bits are
-// the bf16 of d
-__device__ __forceinline__ uint32_t oz_int_bf16(int d) {
-  return __float_as_uint(__int_as_float(0x4B400000 + d) - 12582912.0f) >> 16;
-}
-
-// The S balanced base-64 digits of y = x 2^-e (|x| < 2^e), as bf16 bits: the
-// integer Z = round(|y| 64^S) is written as d_1 64^(S-1) + ... + d_S with
-// d_S..d_2 in [-32, 32) and d_1 = the rest, 0..64, all signed like x.  The
-// low digits are the plain base-64 digits of Z + 32 (64^(S-2) + ... + 1),
-// less 32 (a digit of Z at or above 32 carries one into the next, as in the
-// sequential cut).  Integer arithmetic only; |y - sum_s d_s 64^-s| <= 64^-S / 2.
-template <int S>
-__device__ __forceinline__ void oz_digits(double x, int e, uint32_t (&d)[S]) {
-  const unsigned long long bits = (unsigned long long)__double_as_longlong(x);
-  const int be = (int)((bits >> 52) & 0x7FF);
-  unsigned long long Z = 0;
-  if (be != 0) {
-    const unsigned long long m = (bits & ((1ull << 52) - 1)) | (1ull << 52);   // |x| = m 2^(be - 1075)
-    const int sh = 1075 + e - 6 * S - be;                                      // Z = m 2^-sh, sh > 0
-    if (sh <= 0) Z = m << (-sh);
-    else if (sh < 64) Z = (m >> sh) + ((m >> (sh - 1)) & 1ull);
-  }
-  constexpr unsigned long long C = 32ull * (((1ull << (6 * (S - 1))) - 1) / 63);
-  const unsigned long long Zc = Z + C;
-  const int neg = (int)(bits >> 63);
-#pragma unroll
-  for (int s = 1; s < S; ++s) {
-    const int dv = (int)((Zc >> (6 * (S - 1 - s))) & 63ull) - 32;
-    d[s] = oz_int_bf16(neg ? -dv : dv);
-  }
-  const int top = (int)(Zc >> (6 * (S - 1)));
-  d[0] = oz_int_bf16(neg ? -top : top);
-}
-
-constexpr int OZ_MAXS = 8;
-
-// dst[r][s*Kpad + k]: row walk (k the faster source index), 2^lg threads per
-// row, each cutting 4 consecutive k and writing one 8-byte word per slice
-// (zeros over the padding [K, Kpad))
-template <int S>
-__global__ void __launch_bounds__(256) oz_pack_rows_kernel(const double* __restrict__ src, PackSpec ps, int64_t Kpad,
-                                                           const int* __restrict__ ex, __nv_bfloat16* __restrict__ dst,
-                                                           PackWalk pw) {
-  const int tpr = 1 << pw.lg, lane = threadIdx.x & (tpr - 1), rpb = 256 >> pw.lg;
-  const int64_t ng = Kpad >> 2;
-  const bool k1 = pack_k_single(ps);
-  const int64_t units = ps.R * pw.nseg;
-  for (int64_t u = (int64_t)blockIdx.x * rpb + (threadIdx.x >> pw.lg); u < units; u += (int64_t)gridDim.x * rpb) {
-    const int64_t r = pw.nseg == 1 ? u : u / pw.nseg;
-    const int64_t g0 = (u - r * pw.nseg) * pw.gseg, g1 = min(ng, g0 + pw.gseg);
-    const int e = oz_row_exp(ex[r]);
-    const int64_t ro = pack_row_off(ps, r);
-    __nv_bfloat16* drow = dst + r * (S * Kpad);
-    for (int64_t g = g0 + lane; g < g1; g += tpr) {
-      const int64_t k0 = g << 2;
-      uint2 w[S];
-      if (k0 < ps.K) {
-        double xv[4];
-        pack_load4(src, ps, k1, ro, k0, (int)min((int64_t)4, ps.K - k0), xv);
-        uint32_t dg[4][S];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) oz_digits<S>(xv[q], e, dg[q]);
-#pragma unroll
-        for (int s = 0; s < S; ++s) w[s] = make_uint2(dg[0][s] | (dg[1][s] << 16), dg[2][s] | (dg[3][s] << 16));
-      } else {
-#pragma unroll
-        for (int s = 0; s < S; ++s) w[s] = make_uint2(0u, 0u);
-      }
-#pragma unroll
-      for (int s = 0; s < S; ++s) *reinterpret_cast<uint2*>(drow + s * Kpad + k0) = w[s];
-    }
-  }
-}
-
-// transposing walk through 32 x 32 tiles (row index faster in the source):
-// source offsets of the tile's rows and columns in shared memory, coalesced
-// reads along rows, and each thread cuts two consecutive k of one row and
-// writes one 4-byte word per slice (the tiles cover [0, Kpad), zeros past K)
-template <int S>
-__global__ void __launch_bounds__(256) oz_pack_tiles_kernel(const double* __restrict__ src, PackSpec ps, int64_t Kpad,
-                                                            const int* __restrict__ ex,
-                                                            __nv_bfloat16* __restrict__ dst) {
-  __shared__ double tile[32][33];
-  __shared__ int64_t roff[32], coff[32];
-  const int64_t ntr = (ps.R + 31) / 32, ntk = Kpad / 32;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int kp = threadIdx.x & 15, rw = threadIdx.x >> 4;   // write phase: k pair, row
-  for (int64_t tb = blockIdx.x; tb < ntr * ntk; tb += gridDim.x) {
-    const int64_t r0 = (tb / ntk) * 32, k0 = (tb % ntk) * 32;
-    __syncthreads();   // the previous tile is consumed
-    if (ty == 0) roff[tx] = r0 + tx < ps.R ? pack_row_off(ps, r0 + tx) : 0;
-    else if (ty == 1) coff[tx] = k0 + tx < ps.K ? pack_col_off(ps, k0 + tx) : 0;
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int kk = ty + 8 * j;
-      tile[kk][tx] = (r0 + tx < ps.R && k0 + kk < ps.K) ? src[roff[tx] + coff[kk]] : 0.0;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const int rr = rw + 16 * j;
-      const int64_t r = r0 + rr;
-      if (r >= ps.R) continue;
-      const int e = oz_row_exp(ex[r]);
-      uint32_t da[S], db[S];
-      oz_digits<S>(tile[2 * kp][rr], e, da);
-      oz_digits<S>(tile[2 * kp + 1][rr], e, db);
-      uint32_t* d = reinterpret_cast<uint32_t*>(dst + r * (S * Kpad) + k0 + 2 * kp);
-#pragma unroll
-      for (int s = 0; s < S; ++s) d[(s * Kpad) >> 1] = da[s] | (db[s] << 16);
-    }
+    const uint32_t m = (uint32_t)t / (uint32_t)ep.N, n = (uint32_t)t - m * (uint32_t)ep.N;
+    double* dst = static_cast<double*>(ep.C) + epi_row_off(ep, m) + epi_col_off(ep, n);
+    if (ep.alpha != 1.0) s *= ep.alpha;
+    if (ep.beta == 1.0) s += *dst;
+    else if (ep.beta != 0.0) s += ep.beta * *dst;
+    *dst = s;
   }
 }
 
@@ -566,112 +561,124 @@ std::once_flag g_oz_attr;
 
 }  // namespace
 
-int64_t oz_kpad(int64_t K) { return ((K + OZ_BK - 1) / OZ_BK) * OZ_BK; }
-
-void pack_oz(const double* src, const PackSpec& ps, int S, __nv_bfloat16* dst, int* ex, cudaStream_t s) {
-  if (ps.R <= 0 || ps.K <= 0) return;
-  if (S < 1 || S > OZ_MAXS) fail(FCC_ERR_BAD_ARG, "bad slice count");
-  if (ps.R >= (int64_t(1) << 31) || ps.K >= (int64_t(1) << 31)) fail(FCC_ERR_BAD_ARG, "pack extent too large");
-  const int64_t Kpad = oz_kpad(ps.K);
-  const int pidx = prof_begin(s);
-  struct End { cudaStream_t s; int i; double b; ~End() { prof_end(s, i, PROF_PACK, b); } } pend{s, pidx,
-      2.0 * (double)ps.R * (double)ps.K * 8.0 + (double)ps.R * (double)(S * Kpad) * 2.0};
-  FCC_CUDA(cudaMemsetAsync(ex, 0, sizeof(int) * ps.R, s));
-  const int64_t kfast = std::llabs(ps.kd3 > 1 ? ps.ks3 : (ps.kd2 > 1 ? ps.ks2 : ps.ks1));
-  const int64_t rfast = std::llabs(ps.rd3 > 1 ? ps.rs3 : (ps.rd2 > 1 ? ps.rs2 : ps.rs1));
-  const bool tiles = rfast < kfast && ps.R >= 32;
-  // k-slabs so that the exponent pass has enough independent work
-  const int64_t want = 152 * 64;
-  const int64_t units = tiles ? (ps.R + 31) / 32 : ps.R;
-  int64_t kslab = ps.K;
-  if (units < want) kslab = std::max<int64_t>(256, (ps.K * units + want - 1) / want);
-  const int64_t nks = (ps.K + kslab - 1) / kslab;
-  const PackWalk pw = pack_walk(ps.R, Kpad / 4);
-  const unsigned rgrid = pack_walk_grid(pw, ps.R);
-  const unsigned tgrid = (unsigned)std::min<int64_t>(((ps.R + 31) / 32) * (Kpad / 32), 152 * 16);
-#define FCC_OZ_PACK(SS)                                                                       \
-  case SS:                                                                                    \
-    if (tiles) oz_pack_tiles_kernel<SS><<<tgrid, 256, 0, s>>>(src, ps, Kpad, ex, dst);         \
-    else oz_pack_rows_kernel<SS><<<rgrid, 256, 0, s>>>(src, ps, Kpad, ex, dst, pw);            \
-    break;
-  if (tiles) {
-    oz_exp_tiles_kernel<<<(unsigned)std::min<int64_t>(units * nks, 152 * 32), 256, 0, s>>>(src, ps, kslab, ex);
-  } else {
-    const int64_t warps = units * nks;
-    oz_exp_rows_kernel<<<(unsigned)std::min<int64_t>((warps + 7) / 8, 152 * 32), 256, 0, s>>>(src, ps, kslab, ex);
-  }
-  FCC_CHECK_LAUNCH();
-  switch (S) {
-    FCC_OZ_PACK(1)
-    FCC_OZ_PACK(2)
-    FCC_OZ_PACK(3)
-    FCC_OZ_PACK(4)
-    FCC_OZ_PACK(5)
-    FCC_OZ_PACK(6)
-    FCC_OZ_PACK(7)
-    FCC_OZ_PACK(8)
-    default: fail(FCC_ERR_BAD_ARG, "bad slice count");
-  }
-#undef FCC_OZ_PACK
-  FCC_CHECK_LAUNCH();
+OzLevel oz_level(int groups) {
+  // up to 7 groups: 6-bit digits; above: the same 6 (groups - 1) bits or more
+  // in 8-bit digits
+  if (groups <= 7) return OzLevel{groups - 1, groups, 0, 6};
+  const int S = (6 * (groups - 1) + 7) / 8;
+  return OzLevel{S, S + 1, 0, 8};
 }
 
 void gemm_oz(const __nv_bfloat16* A, int64_t a_rows, const int* exA, const __nv_bfloat16* B, int64_t b_rows,
-             const int* exB, int64_t Kpad, int G, const EpiMap& ep, int* err, cudaStream_t s) {
+             const int* exB, int64_t Kpad, OzLevel lv, const EpiMap& ep, DBuf<double>& ws, int* err, cudaStream_t s) {
   if (ep.M <= 0 || ep.N <= 0) return;
   if (ep.mode != EPI_F64) fail(FCC_ERR_BAD_ARG, "exact-slice products write FP64 only");
-  if (G < 2 || G > OZ_MAXS + 1) fail(FCC_ERR_BAD_ARG, "bad exact-slice group count");
-  if (Kpad <= 0 || Kpad % OZ_BK) fail(FCC_ERR_BAD_ARG, "bad padded K");
+  if (lv.S < 1 || lv.S > OZ_MAXS || lv.G < 2 || lv.G > lv.S + 2 || (lv.bits != 6 && lv.bits != 8)) fail(FCC_ERR_BAD_ARG, "bad exact-slice level");
+  if (Kpad <= 0 || Kpad % OZ_BK || Kpad > (1 << 27)) fail(FCC_ERR_BAD_ARG, "bad padded K");
   if (a_rows < ep.M || b_rows < ep.N) fail(FCC_ERR_BAD_ARG, "packed operands smaller than the output");
-  const int S = G - 1;
-  const int nkb = (int)(Kpad / OZ_BK);
+  if (ep.M >= (int64_t(1) << 31) || ep.N >= (int64_t(1) << 31)) fail(FCC_ERR_BAD_ARG, "output extent too large");
   std::call_once(g_oz_attr, []() {
     cudaFuncSetAttribute(gemm_oz_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM);
   });
-  const OzPairs pr = make_pairs(G);
-  CUtensorMap ta = tma_map_bf16(A, a_rows, S * Kpad, OZ_BM);
-  CUtensorMap tb = tma_map_bf16(B, b_rows, S * Kpad, OZ_BN);
+  OzParams P;
+  std::memset(&P, 0, sizeof(P));
+  const int nb = make_bands(lv.S, lv.G, lv.bits, P.band);
+  P.bits = lv.bits;
+  P.cut = lv.cut;
+  P.kpad = (int)Kpad;
+  const int nkb = (int)(Kpad / OZ_BK);
   const int64_t tm = (ep.M + OZ_BM - 1) / OZ_BM, tn = (ep.N + OZ_BN - 1) / OZ_BN;
   const int64_t tiles = tm * tn;
-  // K ranges per tile.  (1) The units that run at the same time (one per SM,
-  // about 8 tile rows x 19 tile columns in the grouped order) share one K
-  // range; their operand panels (all S slices of a 128-row block over the
-  // range) must fit in L2 together, or every slice is fetched again from HBM
-  // for each slice pair that uses it (a full-K ring launch at (H2O)8 read
-  // 17 GB for 0.76 GB of packed operands).  (2) More ranges also fill the GPU
-  // when the output has few tiles; a unit pays a fixed cost (its final
-  // epilogue and the reduction into C) of about 48 k-block steps.
-  const double panel = (double)OZ_BM * S * (double)Kpad * 2.0;
+  if (tiles * OZ_MAXJOBS >= (int64_t(1) << 31)) fail(FCC_ERR_BAD_ARG, "tensor-core grid too large");
+  P.tm = (uint32_t)tm;
+  P.tn = (uint32_t)tn;
+  // L2 blocks: the units that run at the same time (one per SM, about 8 tile
+  // rows x 19 tile columns in the grouped order) stream the same k-blocks;
+  // their panels (all S slices of a 128-row block) must fit in L2 together,
+  // or every slice is fetched again from HBM for each pair that uses it (a
+  // full-K ring launch at (H2O)8 read 17 GB for 0.76 GB of packed operands)
+  const double panel = (double)OZ_BM * lv.S * OZ_BK * 2.0;   // bytes per k-block
   const int64_t conc = std::min<int64_t>(tiles, 152);
   const int64_t rblk = std::min<int64_t>(tm, 8);
   const int64_t cblk = std::min<int64_t>(tn, (conc + rblk - 1) / rblk);
   constexpr double L2_BUDGET = 48.0 * (1 << 20);
-  int zl2 = (int)std::ceil((double)(rblk + cblk) * panel / L2_BUDGET);
-  const int total = pr.n * nkb;
-  int zw = 1;
-  double best = 1e300;
-  constexpr double CTA_FIXED_STEPS = 48.0;
-  for (int sp = 1; sp <= 64 && sp * OZ_CH <= total; ++sp) {
-    const double waves = std::ceil((double)(tiles * sp) / 152.0);
-    const double t = waves * ((double)total / sp + CTA_FIXED_STEPS);
-    if (t < best * 0.97) { best = t; zw = sp; }
+  P.kper = (int)std::max(4.0, L2_BUDGET / ((double)(rblk + cblk) * panel));
+  P.kper = std::min(P.kper & ~3, std::max(4, nkb));          // whole chunks of every band
+  // Jobs: one per output tile when there are enough tiles; otherwise each
+  // band's k-blocks are cut into pieces of about `target` steps whose partial
+  // results are summed in order by oz_reduce_kernel (one more launch).  A unit
+  // costs about FIXED steps besides its own (ramp-up, the last drain, its
+  // stores); a step is ~0.2 us.
+  int steps_kb = 0;
+  for (int b = 0; b < nb; ++b) steps_kb += P.band[b].ntile - 1;
+  const double total = (double)steps_kb * nkb;
+  constexpr double FIXED = 24.0, REDUCE = 16.0;
+  auto build = [&](double target) {
+    int n = 0;
+    if (target <= 0) {
+      P.job[n++] = OzJob{0, (int16_t)nb, 0, nkb};
+      return n;
+    }
+    for (int b = 0; b < nb;) {
+      // join bands while they stay within the target (never across the cut)
+      int e = b + 1;
+      double st = (double)(P.band[b].ntile - 1) * nkb;
+      while (e < nb && e != lv.cut && st + (double)(P.band[e].ntile - 1) * nkb <= target) {
+        st += (double)(P.band[e].ntile - 1) * nkb;
+        ++e;
+      }
+      int pieces = std::max(1, std::min(nkb, (int)std::ceil(st / target)));
+      const int len = (nkb + pieces - 1) / pieces;
+      for (int k = 0; k < nkb; k += len) {
+        if (n == OZ_MAXJOBS) return -1;
+        P.job[n++] = OzJob{(int16_t)b, (int16_t)e, k, std::min(nkb, k + len)};
+      }
+      b = e;
+    }
+    return n;
+  };
+  double best = 1e300, best_target = 0;
+  for (int q = 0; q < 12; ++q) {
+    const double target = q == 0 ? 0.0 : total / (double)(q < 5 ? q + 1 : (q < 9 ? 4 * (q - 3) : 36 << (q - 9)));
+    const int n = build(target);
+    if (n < 1 || (q > 0 && (n == 1 || (double)n * ep.M * ep.N > (double)(32 << 20)))) continue;
+    // longest CTA under the static assignment of units to CTAs
+    const int64_t units = tiles * n;
+    double t = 0;
+    for (int c = 0; c < std::min<int64_t>(units, 4); ++c) {
+      const int64_t cta = c == 0 ? 0 : (c == 1 ? std::min<int64_t>(units, 152) - 1 : (c == 2 ? 75 : 110));
+      double l = 0;
+      for (int64_t u = cta; u < units; u += 152) {
+        const OzJob& j = P.job[u / tiles];
+        double st = 0;
+        for (int b = j.b0; b < j.b1; ++b) st += P.band[b].ntile - 1;
+        l += st * (j.k1 - j.k0) + FIXED;
+        if (units > 152 * 64) { l *= (double)((units + 151) / 152); break; }
+      }
+      t = std::max(t, l);
+    }
+    if (n > 1) t += REDUCE + (double)(n + 2) * ep.M * ep.N * 8.0 / 1e6;   // ~1 MB a step
+    if (t < best * 0.97) { best = t; best_target = target; }
   }
-  int splits = std::max(zl2, zw);
-  splits = std::max(1, std::min({splits, 64, std::max(1, nkb / 4)}));
-  const int kper = (nkb + splits - 1) / splits;
-  splits = (nkb + kper - 1) / kper;
-  // no loads of C in the kernel: beta = 0 and one K range store, otherwise C
-  // is scaled by beta first (not for beta = 1) and the kernel reduces into it
-  EpiMap e2 = ep;
-  e2.atomic = (splits > 1 || ep.beta != 0.0) ? 1 : 0;
-  if (e2.atomic && ep.beta != 1.0) scale_output(ep, ep.beta, s);
-  const int64_t units = tiles * splits;
-  const int64_t grid = std::min<int64_t>(units, 152);   // one persistent CTA per SM
+  P.njobs = build(best_target);
+  P.units = (uint32_t)(tiles * P.njobs);
+  if (P.njobs > 1) {
+    const size_t need = (size_t)P.njobs * ep.M * ep.N;
+    if (ws.n < need) ws.alloc(need);
+    P.part = ws.p;
+  }
+  CUtensorMap ta = tma_map_bf16(A, a_rows, lv.S * Kpad, OZ_BM);
+  CUtensorMap tb = tma_map_bf16(B, b_rows, lv.S * Kpad, OZ_BN);
+  const unsigned grid = (unsigned)std::min<int64_t>(P.units, 152);   // one persistent CTA per SM
   const int pidx = prof_begin(s);
-  gemm_oz_kernel<<<(unsigned)grid, OZ_THREADS, OZ_SMEM, s>>>(ta, tb, nkb, (int)Kpad, pr, kper, tm, tn, units, exA,
-                                                             exB, G, e2, err);
+  gemm_oz_kernel<<<grid, OZ_THREADS, OZ_SMEM, s>>>(ta, tb, P, exA, exB, ep, err);
   FCC_CHECK_LAUNCH();
-  prof_end(s, pidx, PROF_OZ, ep.work > 0 ? ep.work : 2.0 * (double)ep.M * (double)ep.N * (double)(Kpad * pr.n));
+  if (P.njobs > 1) {
+    const int64_t MN = ep.M * ep.N;
+    oz_reduce_kernel<<<(unsigned)std::min<int64_t>((MN + 255) / 256, 152 * 8), 256, 0, s>>>(ws.p, P.njobs, ep);
+    FCC_CHECK_LAUNCH();
+  }
+  prof_end(s, pidx, PROF_OZ, ep.work > 0 ? ep.work : 2.0 * (double)ep.M * (double)ep.N * (double)Kpad * steps_kb);
 }
 
 }  // namespace fcc

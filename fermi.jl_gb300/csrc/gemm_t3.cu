@@ -118,7 +118,8 @@ __global__ void __launch_bounds__(T3_THREADS, 1) gemm_t3_kernel(const __grid_con
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_holder;
 
-  if (warp == 0 && lane == 0) {
+  if (warp == 0) {
+   if (elect_one()) {
     // ---------------- TMA producer over the tiles' K segments
     int it = 0;
     bool stop = false;
@@ -148,7 +149,9 @@ __global__ void __launch_bounds__(T3_THREADS, 1) gemm_t3_kernel(const __grid_con
       for (int q = max(0, it - Cfg::STAGES); q < it; ++q)
         (void)mbar_wait(smem_u32(&full_bar[q % Cfg::STAGES]), (q / Cfg::STAGES) & 1);
     }
-  } else if (warp == 1 && lane == 0) {
+   }
+  } else if (warp == 1) {
+   if (elect_one()) {
     // ---------------- MMA issuer
     constexpr uint32_t idesc = idesc_bf16(T3_BM, BN);
     int it = 0, lt = 0;
@@ -185,6 +188,7 @@ __global__ void __launch_bounds__(T3_THREADS, 1) gemm_t3_kernel(const __grid_con
     // TMEM is freed only after every issued MMA has completed (also on an abort)
     tc_commit(smem_u32(&done_bar));
     if (!mbar_wait(smem_u32(&done_bar), 0)) atomicExch(&abort_flag, 1);
+   }
   } else if (warp >= 2) {
     // ---------------- epilogue: TMEM -> transposed 32 x 32 blocks -> plain FP32 stores
     const int q = warp & 3;
@@ -208,7 +212,7 @@ __global__ void __launch_bounds__(T3_THREADS, 1) gemm_t3_kernel(const __grid_con
       {
         const int64_t mr = m0 + q * 32 + lane;
         if (mr < v2) {
-          const int x = (int)(mr / v), y = (int)(mr - (int64_t)x * v);
+          const int x = (int)((uint32_t)mr / (uint32_t)P.v), y = (int)mr - x * P.v;
           myroff = t3_blk(x, y, 0, nbk);
         }
       }

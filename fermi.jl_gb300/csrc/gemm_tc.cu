@@ -212,16 +212,17 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_holder;
-  int64_t mt, nt;
-  grouped_tile(blockIdx.x, (ep.M + BM - 1) / BM, (ep.N + BN - 1) / BN, mt, nt);
-  const int64_t m0 = mt * BM;
-  const int64_t n0 = nt * BN;
+  uint32_t mt, nt;
+  grouped_tile(blockIdx.x, (uint32_t)((ep.M + BM - 1) / BM), (uint32_t)((ep.N + BN - 1) / BN), mt, nt);
+  const int64_t m0 = (int64_t)mt * BM;
+  const int64_t n0 = (int64_t)nt * BN;
   // split-K: this CTA reduces k-tiles [kb, ke); partial sums are added atomically
   const int kb = (int)blockIdx.z * k_chunk;
   const int ke = min(num_k, kb + k_chunk);
   const int nkt = max(0, ke - kb);
 
-  if (warp == 0 && lane == 0) {
+  if (warp == 0) {
+   if (elect_one()) {
     // ---------------- TMA producer (none at all under the no_loads test hook:
     // nothing is then in flight, and the MMA thread's bounded wait gives up)
     for (int kt = 0; kt < (ep.no_loads ? 0 : nkt); ++kt) {
@@ -234,7 +235,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       tma_load_2d(smem_u32(sA + s * Cfg::A_BYTES), &tmA, (kb + kt) * BK, (int32_t)(a_row0 + m0), fb);
       tma_load_2d(smem_u32(sB + s * Cfg::B_BYTES), &tmB, (kb + kt) * BK, (int32_t)(b_row0 + n0), fb);
     }
-  } else if (warp == 1 && lane == 0) {
+   }
+  } else if (warp == 1) {
+   if (elect_one()) {
     // ---------------- MMA issuer (single thread)
     constexpr uint32_t idesc = idesc_bf16(BM, BN);
     bool ok = true;
@@ -262,6 +265,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&acc_bar))
                  : "memory");
     (void)ok;
+   }
   } else if (warp >= 2) {
     // ---------------- epilogue: TMEM -> registers -> strided global stores
     bool ok = mbar_wait(smem_u32(&acc_bar), 0);
@@ -275,11 +279,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     if (ok && !abort_now && nkt > 0) {
       // this lane's row offset; rows are broadcast to the warp below
       int64_t crow = 0;
-      if (m < ep.M) {
-        int64_t m3 = m % ep.md3, r = m / ep.md3;
-        int64_t m2 = r % ep.md2, m1 = r / ep.md2;
-        crow = m1 * ep.ms1 + m2 * ep.ms2 + m3 * ep.ms3;
-      }
+      if (m < ep.M) crow = epi_row_off(ep, (uint32_t)m);
       float (*tile)[33] = epi_tile[q];
 #pragma unroll 1
       for (int c0 = 0; c0 < BN; c0 += 32) {
@@ -304,11 +304,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         const int64_t n = n0 + c0 + lane;
         const bool nok = n < ep.N;
         int64_t coff = 0;
-        if (nok) {
-          int64_t n3 = n % ep.nd3, rr = n / ep.nd3;
-          int64_t n2 = rr % ep.nd2, n1 = rr / ep.nd2;
-          coff = n1 * ep.ns1 + n2 * ep.ns2 + n3 * ep.ns3;
-        }
+        if (nok) coff = epi_col_off(ep, (uint32_t)n);
         // all loads of the block first (independent, so they overlap), then
         // the stores
         // FP64 outputs with beta = 1 are reduced into C (red.add, no load);

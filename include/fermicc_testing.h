@@ -35,7 +35,8 @@ int fcc_test_split3(const double* x, int64_t R, int64_t K, int32_t row_fastest, 
 
 /* The exact-slice operand packing on device 0: x is R x K (row-major, or
  * column-major when row_fastest != 0), cut into S (1..8) signed 6-bit digit
- * slices; out receives R rows of S * Kpad bf16 bit patterns (Kpad = K
+ * slices, or for S = 11..17 into S - 10 slices of the signed 8-bit digits that
+ * the exact-slice kernel multiplies; out receives R rows of S * Kpad bf16 bit patterns (Kpad = K
  * rounded up to 64; slice s at columns [s * Kpad, s * Kpad + K), zeros to
  * (s + 1) * Kpad) and ex the R biased FP64 exponents of the row maxima. */
 int fcc_test_pack_oz(const double* x, int64_t R, int64_t K, int32_t row_fastest, int32_t S, uint16_t* out,
