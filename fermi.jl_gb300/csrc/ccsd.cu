@@ -616,7 +616,9 @@ void residual(fcc_ctx* c) {
     // packing of Bt over all (x, y) (row x * v + y, K = Q): two row ranges of
     // the same packed array, instead of packing both slices for every block.
     TcEngine* tc = tc_engine();
-    const bool tcw = tc && tc->enabled;
+    const bool exact = tc && (tc->exact || !tc->enabled);
+    const OzLevel lv = tc && tc->enabled ? tc->oz : OZ_F64;
+    const bool tcw = tc && (tc->enabled || 2.0 * v * v * v * (double)v * Q >= tc->f64_min_flops);
     const int64_t R = v * v;
     int64_t Wk = 0;   // packed row length
     if (tcw) {
@@ -624,13 +626,13 @@ void residual(fcc_ctx* c) {
       ps.R = R; ps.K = Q;
       ps.rd2 = 1; ps.rd3 = v; ps.rs1 = n; ps.rs2 = 0; ps.rs3 = 1;
       ps.kd2 = 1; ps.kd3 = Q; ps.ks1 = 0; ps.ks2 = 0; ps.ks3 = n * n;
-      if (tc->exact) {
-        const int S = tc->oz.S;
+      if (exact) {
+        const int S = lv.S;
         Wk = S * oz_kpad(Q);
         ps.Kp = Wk;
         if ((int64_t)c->bvvA.n < R * Wk) c->bvvA.alloc(R * Wk);
         if ((int64_t)c->bvvEx.n < R) c->bvvEx.alloc(R);
-        pack_oz(Btvv.p, ps, S, tc->oz.bits, c->bvvA.p, c->bvvEx.p, s);
+        pack_oz(Btvv.p, ps, S, lv.bits, c->bvvA.p, c->bvvEx.p, s);
       } else {
         Wk = packed_kp(Q, tc->scheme.P);
         ps.Kp = Wk;
@@ -655,10 +657,10 @@ void residual(fcc_ctx* c) {
         ep.ns1 = 1;
         ep.alpha = 1.0; ep.beta = 0.0; ep.C = c->Wslab.p; ep.mode = EPI_F64;
         const int64_t r0 = a0 * v;
-        if (tc->exact) {
-          ep.work = 2.0 * (double)ep.M * (double)ep.N * (double)Q * oz_pairs(tc->oz);
+        if (exact) {
+          ep.work = 2.0 * (double)ep.M * (double)ep.N * (double)Q * oz_pairs(lv);
           gemm_oz(c->bvvA.p + r0 * Wk, ep.M, c->bvvEx.p + r0, c->bvvA.p + r0 * Wk, ep.N, c->bvvEx.p + r0,
-                  Wk / tc->oz.S, tc->oz, ep, tc->ozws, tc->err, s);
+                  Wk / lv.S, lv, ep, tc->ozws, tc->err, s);
         } else {
           ep.work = 2.0 * (double)ep.M * (double)ep.N * (double)Q * tc->scheme.P;
           ep.no_loads = tc->no_loads_once;
@@ -756,9 +758,7 @@ int ccsd_run(fcc_ctx* c, const fcc_opts* opt, fcc_iter_stats* log, int32_t log_c
   if (op.mixed_finish != FCC_FINISH_EXACT && op.mixed_finish != FCC_FINISH_FP64)
     fail(FCC_ERR_BAD_ARG, "mixed_finish must be FCC_FINISH_EXACT or FCC_FINISH_FP64");
   int phase = op.precision;  // mixed: split-BF16 contractions until the switch, then exact-slice, then the finish
-  if (!c->dev_err.p) c->dev_err.alloc(1);
-  FCC_CUDA(cudaMemsetAsync(c->dev_err.p, 0, sizeof(int), s));
-  c->tc.err = c->dev_err.p;
+  reset_device_error(c);
   double best_rms = 1e300;
   int stalled = 0;
   int exact_groups = 0;   // exact-slice width of the last exact-slice iteration
@@ -930,9 +930,10 @@ int ccsd_run(fcc_ctx* c, const fcc_opts* opt, fcc_iter_stats* log, int32_t log_c
     double oldE = Ecc;
     const int iter_kind = kind;
     {
-      TcScope scope(kind == K_F64 ? nullptr : &c->tc);
+      TcScope scope(&c->tc);
       c->tc.enabled = kind != K_F64;
       c->tc.exact = kind == K_EXACT || kind == K_EXACT9;
+      // (K_F64: the engine only takes the large FP64 contractions)
       if (kind == K_EXACT9) c->tc.oz = oz_level(OZ_G_FINISH);
       // exact-slice width by the size of the step: 6 weight groups (15 slice
       // pairs; noise floor in the Jacobi step ~1e-8 at (H2O)8) while the step
@@ -1023,11 +1024,9 @@ int ccsd_run(fcc_ctx* c, const fcc_opts* opt, fcc_iter_stats* log, int32_t log_c
     float ms = 0;
     FCC_CUDA(cudaEventElapsedTime(&ms, ev0, ev1));
     if (!std::isfinite(Ecc) || !std::isfinite(rms)) { status = FCC_ERR_NAN; }
-    if (iter_kind != K_F64) {
-      int herr = 0;
-      FCC_CUDA(cudaMemcpy(&herr, c->dev_err.p, sizeof(int), cudaMemcpyDeviceToHost));
-      if (herr) { status = FCC_ERR_TIMEOUT; }
-    }
+    int herr = 0;
+    FCC_CUDA(cudaMemcpy(&herr, c->dev_err.p, sizeof(int), cudaMemcpyDeviceToHost));
+    if (herr) { status = FCC_ERR_TIMEOUT; }
     if (c->ckpt_every > 0 && ite % c->ckpt_every == 0)
       checkpoint_write(c, c->ckpt_path, cur1, cur2, Ecc, ite, 0);
     if (log && nlog < log_cap) {

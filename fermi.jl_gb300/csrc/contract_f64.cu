@@ -29,11 +29,32 @@ __device__ __forceinline__ void dmma884(double& d0, double& d1, double a, double
                : "d"(a), "d"(b));
 }
 
-// Offsets of a 3-level index x = (x1*D2 + x2)*D3 + x3.
+// Offsets of a 3-level index x = (x1*D2 + x2)*D3 + x3.  Extents are below
+// 2^31 (contract_f64_launch checks): a 64-bit division goes through the FP64
+// pipe here (1/64 rate) and one per loaded element, as this file once had, cost
+// more than the MMAs of a tile.
 __device__ __forceinline__ int64_t off3(int64_t x, int64_t D2, int64_t D3, int64_t s1, int64_t s2, int64_t s3) {
-  const int64_t x3 = x % D3, r = x / D3;
-  const int64_t x2 = r % D2, x1 = r / D2;
-  return x1 * s1 + x2 * s2 + x3 * s3;
+  const uint32_t x3 = (uint32_t)x % (uint32_t)D3, r = (uint32_t)x / (uint32_t)D3;
+  const uint32_t x2 = r % (uint32_t)D2, x1 = r / (uint32_t)D2;
+  return (int64_t)x1 * s1 + (int64_t)x2 * s2 + (int64_t)x3 * s3;
+}
+// of a 2-level index
+__device__ __forceinline__ int64_t off2(int64_t k, int64_t D2, int64_t s1, int64_t s2) {
+  const uint32_t k1 = (uint32_t)k / (uint32_t)D2, k2 = (uint32_t)k - k1 * (uint32_t)D2;
+  return (int64_t)k1 * s1 + (int64_t)k2 * s2;
+}
+
+// alpha * x + beta * c without FP64 instructions for the usual factors (a warp's
+// FP64 instruction takes its SM's pipe for 16 clk)
+__device__ __forceinline__ double f64_axpby(double x, double c, double alpha, double beta) {
+  if (alpha == -1.0) x = -x;
+  else if (alpha != 1.0) x *= alpha;
+  if (beta == 1.0) x += c;
+  else if (beta != 0.0) x += beta * c;
+  return x;
+}
+__device__ __forceinline__ void f64_store(double* dst, double x, double alpha, double beta) {
+  *dst = f64_axpby(x, beta != 0.0 ? *dst : 0.0, alpha, beta);
 }
 
 // The k loop of one 64 x 64 output tile: stage A (BM x BK) and B (BK x BN)
@@ -66,8 +87,7 @@ __device__ __forceinline__ void f64_mainloop(const double* __restrict__ A, const
         int64_t k = k0 + kk;
         double v = 0.0;
         if (rowOK[m] && k < kend) {
-          int64_t k1 = k / d.K2, k2 = k - k1 * d.K2;
-          v = A[rowA[m] + k1 * d.a_k1 + k2 * d.a_k2];
+          v = A[rowA[m] + off2(k, d.K2, d.a_k1, d.a_k2)];
         }
         As[kk][m] = v;
       }
@@ -77,8 +97,7 @@ __device__ __forceinline__ void f64_mainloop(const double* __restrict__ A, const
       bool kok = k < kend;
       int64_t koff = 0;
       if (kok) {
-        int64_t k1 = k / d.K2, k2 = k - k1 * d.K2;
-        koff = k1 * d.a_k1 + k2 * d.a_k2;
+        koff = off2(k, d.K2, d.a_k1, d.a_k2);
       }
 #pragma unroll
       for (int r = 0; r < 8; ++r) {
@@ -94,8 +113,7 @@ __device__ __forceinline__ void f64_mainloop(const double* __restrict__ A, const
         int64_t k = k0 + kk;
         double v = 0.0;
         if (colOK[n] && k < kend) {
-          int64_t k1 = k / d.K2, k2 = k - k1 * d.K2;
-          v = B[colB[n] + k1 * d.b_k1 + k2 * d.b_k2];
+          v = B[colB[n] + off2(k, d.K2, d.b_k1, d.b_k2)];
         }
         Bs[kk][n] = v;
       }
@@ -105,8 +123,7 @@ __device__ __forceinline__ void f64_mainloop(const double* __restrict__ A, const
       bool kok = k < kend;
       int64_t koff = 0;
       if (kok) {
-        int64_t k1 = k / d.K2, k2 = k - k1 * d.K2;
-        koff = k1 * d.b_k1 + k2 * d.b_k2;
+        koff = off2(k, d.K2, d.b_k1, d.b_k2);
       }
 #pragma unroll
       for (int r = 0; r < 8; ++r) {
@@ -200,10 +217,7 @@ __global__ void __launch_bounds__(NT, 5) contract_f64_kernel(const double* __res
           partial[((int64_t)blockIdx.z * d.M + m) * d.N + n] = acc[i][j][h];
           continue;
         }
-        double* dst = C + crow + colC[nl];
-        double v = d.alpha * acc[i][j][h];
-        if (d.beta != 0.0) v += d.beta * *dst;
-        *dst = v;
+        f64_store(C + crow + colC[nl], acc[i][j][h], d.alpha, d.beta);
       }
     }
   }
@@ -215,12 +229,108 @@ __global__ void splitk_reduce_kernel(const double* __restrict__ partial, int spl
   const int64_t MN = d.M * d.N;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < MN; t += (int64_t)gridDim.x * blockDim.x) {
     double s = 0.0;
-    for (int z = 0; z < splits; ++z) s += partial[(int64_t)z * MN + t];
-    const int64_t m = t / d.N, n = t - m * d.N;
-    double* dst = C + off3(m, d.M2, d.M3, d.c_m1, d.c_m2, d.c_m3) + off3(n, d.N2, d.N3, d.c_n1, d.c_n2, d.c_n3);
-    double v = d.alpha * s;
-    if (d.beta != 0.0) v += d.beta * *dst;
-    *dst = v;
+    for (int z = 0; z < splits; z += 8) {   // eight loads in flight, added in order
+      double x[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) x[q] = z + q < splits ? partial[(int64_t)(z + q) * MN + t] : 0.0;
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (z + q < splits) s += x[q];
+    }
+    const uint32_t m = (uint32_t)((uint64_t)t >> 32 ? t / d.N : (uint32_t)t / (uint32_t)d.N);
+    const int64_t n = t - (int64_t)m * d.N;
+    f64_store(C + off3(m, d.M2, d.M3, d.c_m1, d.c_m2, d.c_m3) + off3(n, d.N2, d.N3, d.c_n1, d.c_n2, d.c_n3), s,
+              d.alpha, d.beta);
+  }
+}
+
+// Small contractions: a block of four warps per 16 x 16 output tile (and K
+// range), the k-steps of four dealt to the warps in turn, operands read
+// straight into the fragments of m8n8k4, the warps' sums added in shared
+// memory in a fixed order.  An SM does two FP64 FMAs per clk, so what counts is
+// that the work reaches all SMs: with 64 x 64 tiles the contractions of a
+// dimer ran on 1-25 SMs (a 46 x 46 x 46 product took 97 us on one; 5 here).
+constexpr int SM_T = 16, SM_WARPS = 4;
+__global__ void __launch_bounds__(32 * SM_WARPS) contract_f64_small_kernel(const double* __restrict__ A,
+                                                                           const double* __restrict__ B,
+                                                                           double* __restrict__ C, CtrDesc d,
+                                                                           int k_chunk, double* __restrict__ partial) {
+  __shared__ double part[SM_WARPS][SM_T][SM_T + 1];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int64_t m0 = (int64_t)blockIdx.x * SM_T, n0 = (int64_t)blockIdx.y * SM_T;
+  const int64_t bz = partial ? 0 : blockIdx.z;
+  const int kbeg = partial ? (int)blockIdx.z * k_chunk : 0;
+  const int kend = partial ? min((int)d.K, kbeg + k_chunk) : (int)d.K;
+  A += bz * d.a_b;
+  B += bz * d.b_b;
+  C += bz * d.c_b;
+  int64_t ra[2], cb[2];
+  bool rok[2], cok[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int64_t m = m0 + 8 * i + (lane >> 2), n = n0 + 8 * i + (lane >> 2);
+    rok[i] = m < d.M;
+    cok[i] = n < d.N;
+    ra[i] = rok[i] ? off3(m, d.M2, d.M3, d.a_m1, d.a_m2, d.a_m3) : 0;
+    cb[i] = cok[i] ? off3(n, d.N2, d.N3, d.b_n1, d.b_n2, d.b_n3) : 0;
+  }
+  double acc[2][2][2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  constexpr int U = 4;   // k-steps in flight
+  for (int k0 = kbeg + 4 * warp; k0 < kend; k0 += 4 * SM_WARPS * U) {
+    double a[U][2], b[U][2];
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      const int k = k0 + 4 * SM_WARPS * q + (lane & 3);
+      const bool kok = k < kend;
+      int64_t ka = 0, kb = 0;
+      if (kok) {
+        const uint32_t k1 = (uint32_t)k / (uint32_t)d.K2, k2 = (uint32_t)k - k1 * (uint32_t)d.K2;
+        ka = (int64_t)k1 * d.a_k1 + (int64_t)k2 * d.a_k2;
+        kb = (int64_t)k1 * d.b_k1 + (int64_t)k2 * d.b_k2;
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        a[q][i] = kok && rok[i] ? A[ra[i] + ka] : 0.0;
+        b[q][i] = kok && cok[i] ? B[cb[i] + kb] : 0.0;
+      }
+    }
+    const bool m2 = m0 + 8 < d.M, n2 = n0 + 8 < d.N;   // warp-uniform: blocks wholly outside issue no MMA
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      if (k0 + 4 * SM_WARPS * q >= kend) break;
+      dmma884(acc[0][0][0], acc[0][0][1], a[q][0], b[q][0]);
+      if (n2) dmma884(acc[0][1][0], acc[0][1][1], a[q][0], b[q][1]);
+      if (m2) dmma884(acc[1][0][0], acc[1][0][1], a[q][1], b[q][0]);
+      if (m2 && n2) dmma884(acc[1][1][0], acc[1][1][1], a[q][1], b[q][1]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) part[warp][8 * i + (lane >> 2)][8 * j + 2 * (lane & 3) + h] = acc[i][j][h];
+  __syncthreads();
+#pragma unroll
+  for (int e = tid; e < SM_T * SM_T; e += 32 * SM_WARPS) {
+    // the output's faster index along the threads
+    const bool mf = d.c_n3 != 1 && (d.N3 > 1 || d.c_n2 != 1);
+    const int r = mf ? e % SM_T : e / SM_T, c = mf ? e / SM_T : e % SM_T;
+    const int64_t m = m0 + r, n = n0 + c;
+    if (m >= d.M || n >= d.N) continue;
+    double s = part[0][r][c];
+#pragma unroll
+    for (int w = 1; w < SM_WARPS; ++w) s += part[w][r][c];
+    if (partial) {
+      partial[((int64_t)blockIdx.z * d.M + m) * d.N + n] = s;
+    } else {
+      f64_store(C + off3(m, d.M2, d.M3, d.c_m1, d.c_m2, d.c_m3) + off3(n, d.N2, d.N3, d.c_n1, d.c_n2, d.c_n3), s,
+                d.alpha, d.beta);
+    }
   }
 }
 
@@ -237,35 +347,115 @@ __global__ void gemv_f64_kernel(const double* __restrict__ A, const double* __re
   for (int64_t m = warp; m < d.M; m += nwarps) {
     const double* a = A + off3(m, d.M2, d.M3, d.a_m1, d.a_m2, d.a_m3);
     double s = 0.0;
-    for (int64_t k = lane; k < d.K; k += 32) {
-      const int64_t k1 = k / d.K2, k2 = k - k1 * d.K2;
-      s += a[k1 * d.a_k1 + k2 * d.a_k2] * B[k1 * d.b_k1 + k2 * d.b_k2];
-    }
+#pragma unroll 4
+    for (int64_t k = lane; k < d.K; k += 32) s += a[off2(k, d.K2, d.a_k1, d.a_k2)] * B[off2(k, d.K2, d.b_k1, d.b_k2)];
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (lane == 0) {
-      double* dst = C + off3(m, d.M2, d.M3, d.c_m1, d.c_m2, d.c_m3);
-      double v = d.alpha * s;
-      if (d.beta != 0.0) v += d.beta * *dst;
-      *dst = v;
+    if (lane == 0) f64_store(C + off3(m, d.M2, d.M3, d.c_m1, d.c_m2, d.c_m3), s, d.alpha, d.beta);
+  }
+}
+
+// N == 1 with the rows adjacent in memory (unit stride along m): 64 rows per
+// block, lanes along the rows so that reads coalesce, four groups of warps
+// over interleaved k, summed in a fixed order.
+__global__ void __launch_bounds__(256) gemv_cols_f64_kernel(const double* __restrict__ A, const double* __restrict__ B,
+                                                            double* __restrict__ C, CtrDesc d) {
+  __shared__ double part[4][64];
+  const int x = threadIdx.x & 63, g = threadIdx.x >> 6;
+  const int64_t m = (int64_t)blockIdx.x * 64 + x;
+  const int64_t bz = blockIdx.y;
+  A += bz * d.a_b;
+  B += bz * d.b_b;
+  C += bz * d.c_b;
+  double s = 0.0;
+  if (m < d.M) {
+    const double* a = A + off3(m, d.M2, d.M3, d.a_m1, d.a_m2, d.a_m3);
+#pragma unroll 8
+    for (int64_t k = g; k < d.K; k += 4) s += a[off2(k, d.K2, d.a_k1, d.a_k2)] * B[off2(k, d.K2, d.b_k1, d.b_k2)];
+  }
+  part[g][x] = s;
+  __syncthreads();
+  if (g == 0 && m < d.M)
+    f64_store(C + off3(m, d.M2, d.M3, d.c_m1, d.c_m2, d.c_m3), (part[0][x] + part[1][x]) + (part[2][x] + part[3][x]),
+              d.alpha, d.beta);
+}
+
+// out[i0 i1 i2 i3] = alpha in + beta out: a warp per run of up to 128 elements
+// of the last index, so the index arithmetic is per run.
+__global__ void __launch_bounds__(256) axpby4_kernel(const double* __restrict__ in, double* __restrict__ out,
+                                                     uint32_t d1, uint32_t d2, uint32_t d3, int64_t si0, int64_t si1,
+                                                     int64_t si2, int64_t si3, int64_t so0, int64_t so1, int64_t so2,
+                                                     int64_t so3, double alpha, double beta, uint32_t nseg,
+                                                     int64_t runs) {
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < runs; w += nw) {
+    uint32_t r = (uint32_t)w;
+    const uint32_t seg = r % nseg;
+    r /= nseg;
+    const uint32_t i2 = r % d2;
+    r /= d2;
+    const uint32_t i1 = r % d1, i0 = r / d1;
+    const double* src = in + (int64_t)i0 * si0 + (int64_t)i1 * si1 + (int64_t)i2 * si2;
+    double* dst = out + (int64_t)i0 * so0 + (int64_t)i1 * so1 + (int64_t)i2 * so2;
+    const uint32_t j0 = seg * 128 + lane;
+    double v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint32_t j = j0 + 32 * q;
+      v[q] = j < d3 ? src[(int64_t)j * si3] : 0.0;
+    }
+    double p[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint32_t j = j0 + 32 * q;
+      p[q] = beta != 0.0 && j < d3 ? dst[(int64_t)j * so3] : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint32_t j = j0 + 32 * q;
+      if (j < d3) dst[(int64_t)j * so3] = f64_axpby(v[q], p[q], alpha, beta);
     }
   }
 }
 
-__global__ void axpby4_kernel(const double* __restrict__ in, double* __restrict__ out, int64_t d0,
-                              int64_t d1, int64_t d2, int64_t d3, int64_t si0, int64_t si1, int64_t si2,
-                              int64_t si3, int64_t so0, int64_t so1, int64_t so2, int64_t so3,
-                              double alpha, double beta, int64_t total) {
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    int64_t r = t;
-    int64_t i3 = r % d3; r /= d3;
-    int64_t i2 = r % d2; r /= d2;
-    int64_t i1 = r % d1; r /= d1;
-    int64_t i0 = r;
-    double v = alpha * in[i0 * si0 + i1 * si1 + i2 * si2 + i3 * si3];
-    double* o = out + i0 * so0 + i1 * so1 + i2 * so2 + i3 * so3;
-    if (beta != 0.0) v += beta * *o;
-    *o = v;
+// The same where the source's fastest index is another one (tx) than the
+// output's (the last): 32 x 32 tiles through shared memory, both sides
+// coalesced.  The other two indices are (oa, ob).
+__global__ void __launch_bounds__(256) axpby4_tr_kernel(const double* __restrict__ in, double* __restrict__ out,
+                                                        uint32_t dx, uint32_t d3, uint32_t db, int64_t six,
+                                                        int64_t si3, int64_t sia, int64_t sib, int64_t sox,
+                                                        int64_t so3, int64_t soa, int64_t sob, double alpha,
+                                                        double beta, uint32_t ntx, uint32_t nt3, uint32_t tiles) {
+  __shared__ double tile[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+    uint32_t r = t;
+    const uint32_t x0 = (r % ntx) * 32;
+    r /= ntx;
+    const uint32_t j0 = (r % nt3) * 32;
+    r /= nt3;
+    const uint32_t ib = r % db, ia = r / db;
+    const double* src = in + (int64_t)ia * sia + (int64_t)ib * sib;
+    double* dst = out + (int64_t)ia * soa + (int64_t)ib * sob;
+    __syncthreads();   // the previous tile is consumed
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint32_t x = x0 + tx, j = j0 + ty + 8 * q;
+      if (x < dx && j < d3) tile[ty + 8 * q][tx] = src[(int64_t)x * six + (int64_t)j * si3];
+    }
+    __syncthreads();
+    double p[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint32_t x = x0 + ty + 8 * q, j = j0 + tx;
+      p[q] = beta != 0.0 && x < dx && j < d3 ? dst[(int64_t)x * sox + (int64_t)j * so3] : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint32_t x = x0 + ty + 8 * q, j = j0 + tx;
+      if (x < dx && j < d3)
+        dst[(int64_t)x * sox + (int64_t)j * so3] = f64_axpby(tile[tx][ty + 8 * q], p[q], alpha, beta);
+    }
   }
 }
 
@@ -273,25 +463,62 @@ __global__ void axpby4_kernel(const double* __restrict__ in, double* __restrict_
 
 void contract_f64_launch(const double* A, const double* B, double* C, const CtrDesc& d, cudaStream_t s) {
   if (d.M <= 0 || d.N <= 0 || d.batch <= 0) return;
+  if (d.M >= (int64_t(1) << 31) || d.N >= (int64_t(1) << 31) || d.K >= (int64_t(1) << 31))
+    fail(FCC_ERR_BAD_ARG, "contraction extent too large");
+  if (d.K <= 0) fail(FCC_ERR_BAD_ARG, "empty contraction index");
   int64_t gm = (d.M + BM - 1) / BM, gn = (d.N + BN - 1) / BN;
   if (gn > 65535 || d.batch > 65535) fail(FCC_ERR_BAD_ARG, "contraction grid too large");
-  if (d.K <= 0) fail(FCC_ERR_BAD_ARG, "empty contraction index");
   const int pidx = prof_begin(s);
   const double pflops = 2.0 * (double)d.M * (double)d.N * (double)d.K * (double)d.batch;
   // stage along M (N) when the fastest-moving M (N) index has unit stride
   const int a_fast = (d.M3 > 1 ? d.a_m3 : d.a_m2) == 1 ? 1 : 0;
   const int b_fast = (d.N3 > 1 ? d.b_n3 : d.b_n2) == 1 ? 1 : 0;
   if (d.N == 1) {
-    const int64_t blocks = std::min<int64_t>((d.M + 7) / 8, 152 * 16);
-    gemv_f64_kernel<<<dim3((unsigned)blocks, (unsigned)d.batch), 256, 0, s>>>(A, B, C, d);
+    if (a_fast && d.M >= 32) {
+      gemv_cols_f64_kernel<<<dim3((unsigned)((d.M + 63) / 64), (unsigned)d.batch), 256, 0, s>>>(A, B, C, d);
+    } else {
+      const int64_t blocks = std::min<int64_t>((d.M + 7) / 8, 152 * 16);
+      gemv_f64_kernel<<<dim3((unsigned)blocks, (unsigned)d.batch), 256, 0, s>>>(A, B, C, d);
+    }
+    FCC_CHECK_LAUNCH();
+    prof_end(s, pidx, PROF_F64, pflops);
+    return;
+  }
+  auto workspace = [&](DBuf<double>& local, int64_t need) -> double* {
+    DBuf<double>* ws = f64_workspace();
+    if (!ws) ws = &local;
+    if ((int64_t)ws->n < need) ws->alloc(need);
+    return ws->p;
+  };
+  DBuf<double> local;
+  const int64_t MN = d.M * d.N;
+  const unsigned rgrid = (unsigned)std::min<int64_t>((MN + 255) / 256, 152 * 8);
+  // 16 x 16 tiles while the 64 x 64 ones would leave SMs without work; K is
+  // then cut so that about two blocks per SM share it (partials reduced in a
+  // fixed order, so results stay deterministic)
+  const int64_t sm = (d.M + SM_T - 1) / SM_T, sn = (d.N + SM_T - 1) / SM_T;
+  if (gm * gn * d.batch < 3 * 152 && sn <= 65535) {
+    int64_t splits = 1;
+    if (d.batch == 1 && sm * sn < 152) splits = std::min<int64_t>((304 + sm * sn - 1) / (sm * sn), d.K / 128);
+    if (splits > 1) {
+      const int64_t chunk = ((d.K + splits - 1) / splits + 15) / 16 * 16;
+      splits = (d.K + chunk - 1) / chunk;
+      double* part = workspace(local, splits * MN);
+      contract_f64_small_kernel<<<dim3((unsigned)sm, (unsigned)sn, (unsigned)splits), 32 * SM_WARPS, 0, s>>>(
+          A, B, C, d, (int)chunk, part);
+      FCC_CHECK_LAUNCH();
+      splitk_reduce_kernel<<<rgrid, 256, 0, s>>>(part, (int)splits, C, d);
+    } else {
+      contract_f64_small_kernel<<<dim3((unsigned)sm, (unsigned)sn, (unsigned)d.batch), 32 * SM_WARPS, 0, s>>>(
+          A, B, C, d, 0, nullptr);
+    }
     FCC_CHECK_LAUNCH();
     prof_end(s, pidx, PROF_F64, pflops);
     return;
   }
   // fewer output tiles than one wave of resident CTAs (96 registers x 128
   // threads: 5 per SM) and a long K: split K so that about 8 CTAs per SM
-  // share the work (partials reduced in a fixed order, so results stay
-  // deterministic).  Under one wave the FP64 pipe idles on DMMA latency:
+  // share the work.  Under one wave the FP64 pipe idles on DMMA latency:
   // 387 CTAs ran at 0.8 TFLOP/s where 1216 reach 1.08.
   constexpr int64_t WAVE_CTAS = 5 * 152, SPLIT_CTAS = 8 * 152;
   if (d.batch == 1 && gm * gn < WAVE_CTAS && d.K >= 32 * BK) {
@@ -299,18 +526,11 @@ void contract_f64_launch(const double* A, const double* B, double* C, const CtrD
     splits = std::max<int64_t>(2, std::min<int64_t>(splits, 1024));
     const int64_t chunk = ((d.K + splits - 1) / splits + BK - 1) / BK * BK;
     splits = (d.K + chunk - 1) / chunk;
-    DBuf<double> local;
-    DBuf<double>* ws = f64_workspace();
-    if (!ws) ws = &local;
-    DBuf<double>& scratch = *ws;
-    const int64_t need = splits * d.M * d.N;
-    if ((int64_t)scratch.n < need) scratch.alloc(need);
+    double* part = workspace(local, splits * MN);
     dim3 grid((unsigned)gm, (unsigned)gn, (unsigned)splits);
-    contract_f64_kernel<<<grid, NT, 0, s>>>(A, B, C, d, a_fast, b_fast, chunk, scratch.p);
+    contract_f64_kernel<<<grid, NT, 0, s>>>(A, B, C, d, a_fast, b_fast, chunk, part);
     FCC_CHECK_LAUNCH();
-    const int64_t MN = d.M * d.N;
-    splitk_reduce_kernel<<<(unsigned)std::min<int64_t>((MN + 255) / 256, 152 * 8), 256, 0, s>>>(scratch.p, (int)splits,
-                                                                                                 C, d);
+    splitk_reduce_kernel<<<rgrid, 256, 0, s>>>(part, (int)splits, C, d);
     FCC_CHECK_LAUNCH();
     prof_end(s, pidx, PROF_F64, pflops);
     return;
@@ -322,14 +542,47 @@ void contract_f64_launch(const double* A, const double* B, double* C, const CtrD
 }
 
 void tensor_axpby_launch(const TView& in, const TView& out, double alpha, double beta, cudaStream_t s) {
-  int64_t total = out.dim[0] * out.dim[1] * out.dim[2] * out.dim[3];
+  int64_t total = 1;
+  for (int k = 0; k < 4; ++k) {
+    total *= out.dim[k];
+    if (out.dim[k] >= (int64_t(1) << 31)) fail(FCC_ERR_BAD_ARG, "tensor extent too large");
+  }
   if (total <= 0) return;
-  int threads = 256;
-  int64_t blocks = std::min<int64_t>((total + threads - 1) / threads, 152 * 32);
-  axpby4_kernel<<<(unsigned)blocks, threads, 0, s>>>(in.p, out.p, out.dim[0], out.dim[1], out.dim[2],
-                                                      out.dim[3], in.str[0], in.str[1], in.str[2],
-                                                      in.str[3], out.str[0], out.str[1], out.str[2],
-                                                      out.str[3], alpha, beta, total);
+  // Indices slowest first by their stride in the output (unit extents in
+  // front), so the last one is what the threads run along.
+  int ord[4] = {0, 1, 2, 3};
+  std::stable_sort(ord, ord + 4, [&](int a, int b) {
+    const bool ua = out.dim[a] == 1, ub = out.dim[b] == 1;
+    if (ua != ub) return ua;
+    return std::llabs(out.str[a]) > std::llabs(out.str[b]);
+  });
+  int64_t dim[4], si[4], so[4];
+  for (int k = 0; k < 4; ++k) {
+    dim[k] = out.dim[ord[k]];
+    si[k] = in.str[ord[k]];
+    so[k] = out.str[ord[k]];
+  }
+  // the source's fastest index, if it is another one than the output's
+  int x = 3;
+  for (int k = 0; k < 3; ++k)
+    if (dim[k] > 1 && std::llabs(si[k]) < std::llabs(si[x])) x = k;
+  if (x != 3 && dim[x] >= 8 && dim[3] >= 8) {
+    const int o1 = x == 0 ? 1 : 0, o2 = x == 2 ? 1 : 2;   // the other two, slower first
+    const int64_t ntx = (dim[x] + 31) / 32, nt3 = (dim[3] + 31) / 32;
+    const int64_t tiles = ntx * nt3 * dim[o1] * dim[o2];
+    if (tiles >= (int64_t(1) << 31)) fail(FCC_ERR_BAD_ARG, "tensor too large");
+    axpby4_tr_kernel<<<(unsigned)std::min<int64_t>(tiles, 152 * 16), 256, 0, s>>>(
+        in.p, out.p, (uint32_t)dim[x], (uint32_t)dim[3], (uint32_t)dim[o2], si[x], si[3], si[o1], si[o2], so[x], so[3],
+        so[o1], so[o2], alpha, beta, (uint32_t)ntx, (uint32_t)nt3, (uint32_t)tiles);
+    FCC_CHECK_LAUNCH();
+    return;
+  }
+  const int64_t nseg = (dim[3] + 127) / 128;
+  const int64_t runs = dim[0] * dim[1] * dim[2] * nseg;
+  if (runs >= (int64_t(1) << 31)) fail(FCC_ERR_BAD_ARG, "tensor too large");
+  axpby4_kernel<<<(unsigned)std::min<int64_t>((runs + 7) / 8, 152 * 16), 256, 0, s>>>(
+      in.p, out.p, (uint32_t)dim[1], (uint32_t)dim[2], (uint32_t)dim[3], si[0], si[1], si[2], si[3], so[0], so[1],
+      so[2], so[3], alpha, beta, (uint32_t)nseg, runs);
   FCC_CHECK_LAUNCH();
 }
 
@@ -427,8 +680,9 @@ TcEngine::KeptPack* kept_a(TcEngine* tc, const double* src, const PackSpec& ps, 
   return nullptr;
 }
 
-// Tensor-core evaluation of C = alpha * A.B + beta * C (no batch index).
-void run_tc(TcEngine* tc, double alpha, const TView& A, const TView& B, double beta, const TView& C,
+// Tensor-core evaluation of C = alpha * A.B + beta * C (no batch index): by
+// exact-slice products of level lv, or (lv.S = 0) by the engine's split scheme.
+void run_tc(TcEngine* tc, OzLevel lv, double alpha, const TView& A, const TView& B, double beta, const TView& C,
             std::vector<Ix> gm, std::vector<Ix> gn, std::vector<Ix> gk, cudaStream_t s) {
   // fastest-moving member last: the one with the smallest stride in the operand that is read along it
   auto order = [](std::vector<Ix>& g, int op) {
@@ -439,9 +693,8 @@ void run_tc(TcEngine* tc, double alpha, const TView& A, const TView& B, double b
   order(gk, 0);
   pad3(gm); pad3(gn); pad3(gk);
   const int64_t M = gdim(gm), N = gdim(gn), K = gdim(gk);
-  if (tc->exact) {
+  if (lv.S > 0) {
     // exact-slice products: S digit slices of each operand, FP64 output
-    const OzLevel lv = tc->oz;
     const int S = lv.S;
     const int64_t Kpad = oz_kpad(K), W = S * Kpad;
     if ((int64_t)tc->bufA.n < M * W) tc->bufA.alloc(M * W);
@@ -562,7 +815,17 @@ void einsum(double alpha, const char* spec, const TView& A, const TView& B, doub
     std::vector<Ix> m3 = gm, n3 = gn, k3 = gk;
     if (flops >= tc->min_flops && gdim(gm) >= tc->min_dim && gdim(gn) >= tc->min_dim && try_fuse(m3, 3) && try_fuse(n3, 3) &&
         try_fuse(k3, 3)) {
-      run_tc(tc, alpha, A, B, beta, C, m3, n3, k3, s);
+      run_tc(tc, tc->exact ? tc->oz : OzLevel{0, 0, 0, 0}, alpha, A, B, beta, C, m3, n3, k3, s);
+      return;
+    }
+  }
+  // FP64: exact-slice products at the FP64 level from f64_min_flops on (see
+  // TcEngine), DMMA below
+  if (tc && gb.empty()) {
+    const double flops = 2.0 * (double)gdim(gm) * (double)gdim(gn) * (double)gdim(gk);
+    std::vector<Ix> m3 = gm, n3 = gn, k3 = gk;
+    if (flops >= tc->f64_min_flops && gdim(gm) > 1 && gdim(gn) > 1 && try_fuse(m3, 3) && try_fuse(n3, 3) && try_fuse(k3, 3)) {
+      run_tc(tc, OZ_F64, alpha, A, B, beta, C, m3, n3, k3, s);
       return;
     }
   }
@@ -680,6 +943,17 @@ extern "C" int fcc_gemm_f64_noalloc(int64_t M, int64_t N, int64_t K, double alph
   int st = FCC_OK;
   double* scratch = noalloc_scratch_ptr(st);
   if (!scratch) return st;
+  // index arithmetic is 32-bit: a longer K goes in pieces added to C
+  constexpr int64_t KMAX = int64_t(1) << 30;
+  for (int64_t k0 = KMAX; k0 < K; k0 += KMAX) {
+    const int rc = fcc_gemm_f64_noalloc(M, N, std::min(KMAX, K - k0), alpha, A + k0, lda, B + k0 * ldb, ldb,
+                                        k0 == KMAX ? beta : 1.0, C, ldc, stream);
+    if (rc != FCC_OK) return rc;
+  }
+  if (K > KMAX) {
+    K = KMAX;
+    beta = 1.0;
+  }
   CtrDesc d;
   d.M = M; d.M2 = 1; d.N = N; d.N2 = N; d.K = K; d.K2 = K; d.batch = 1;
   d.a_m1 = lda; d.a_m2 = 0; d.a_k1 = 0; d.a_k2 = 1; d.a_b = 0;

@@ -23,6 +23,8 @@ int guarded(fcc_ctx* c, F&& f) {
       if (e != cudaSuccess) { c->last_error = cudaGetErrorString(e); return FCC_ERR_CUDA; }
     }
     fcc::WorkspaceScope ws(c ? &c->f64ws : nullptr);
+    fcc::TcScope tc(c ? &c->tc : nullptr);   // large FP64 contractions run on the tensor cores
+    if (c) c->tc.enabled = false;
     return f();
   } catch (const fcc::Error& e) {
     if (c) c->last_error = e.what;
@@ -79,7 +81,7 @@ void common_tail(fcc_ctx* c, const double* eps_o, const double* eps_v, double e_
   c->e_ref = e_ref;
   fcc::setup_integrals(c);
   fcc::make_mp2_guess(c);
-  FCC_CUDA(cudaStreamSynchronize(c->stream));
+  fcc::check_device_error(c, "the integral setup");
   c->have_ints = true;
   c->have_guess = false;
   c->have_ccsd = false;
@@ -172,6 +174,9 @@ int fcc_create(fcc_ctx** out, int32_t o, int32_t v, int32_t naux, int32_t device
   c->n = (int64_t)o + v;
   int rc = guarded(c, [&]() {
     FCC_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
+    c->dev_err.alloc(1);
+    c->tc.err = c->dev_err.p;
+    fcc::reset_device_error(c);
     return FCC_OK;
   });
   if (rc != FCC_OK) { delete c; return rc; }
@@ -193,6 +198,7 @@ int fcc_upload_df(fcc_ctx* c, const double* Boo, const double* Bov, const double
                   const double* eps_v, double e_ref) {
   if (!c) return FCC_ERR_BAD_ARG;
   return guarded(c, [&]() {
+    fcc::reset_device_error(c);
     if (!Boo || !Bov || !Bvv || !eps_o || !eps_v) fcc::fail(FCC_ERR_BAD_ARG, "null input");
     if (c->Q <= 0) fcc::fail(FCC_ERR_STATE, "context created with naux = 0 (conventional); use fcc_upload_conv");
     const int64_t o = c->o, v = c->v, Q = c->Q, n = c->n;
@@ -222,6 +228,7 @@ int fcc_upload_ao3_df(fcc_ctx* c, const double* Pqp, const double* Jh, const dou
                       int32_t core, int32_t ndocc, const double* eps, double e_ref) {
   if (!c) return FCC_ERR_BAD_ARG;
   return guarded(c, [&]() {
+    fcc::reset_device_error(c);
     check_ao_ranges(c, Pqp, C, eps, nbf, nmo, core, ndocc, e_ref);
     if (!Jh) fcc::fail(FCC_ERR_BAD_ARG, "null input");
     const int64_t Q = c->Q, nb = nbf;
@@ -245,6 +252,7 @@ int fcc_upload_ao_df(fcc_ctx* c, const double* Bmn, const double* C, int32_t nbf
                      int32_t ndocc, const double* eps, double e_ref) {
   if (!c) return FCC_ERR_BAD_ARG;
   return guarded(c, [&]() {
+    fcc::reset_device_error(c);
     check_ao_ranges(c, Bmn, C, eps, nbf, nmo, core, ndocc, e_ref);
     const int64_t Q = c->Q, nb = nbf;
     fcc::DBuf<double> dB;
@@ -263,6 +271,7 @@ int fcc_upload_conv(fcc_ctx* c, const double* OOOO, const double* OOOV, const do
                     const double* OVVV, const double* VVVV, const double* eps_o, const double* eps_v, double e_ref) {
   if (!c) return FCC_ERR_BAD_ARG;
   return guarded(c, [&]() {
+    fcc::reset_device_error(c);
     if (!OOOO || !OOOV || !OOVV || !OVOV || !OVVV || !VVVV || !eps_o || !eps_v) fcc::fail(FCC_ERR_BAD_ARG, "null input");
     const int64_t o = c->o, v = c->v, n = c->n;
     if (n > 64) fcc::fail(FCC_ERR_BAD_ARG, "conventional path supports at most 64 active orbitals");

@@ -49,7 +49,8 @@ struct fcc_ctx {
   fcc::DBuf<float> derr1s, derr2s;
   fcc::DBuf<double> derr1d, derr2d;
 
-  // split-BF16 tensor-core engine (mixed form) and its device error flag
+  // tensor-core engine (reduced contractions of the mixed and exact forms,
+  // large FP64 ones of every form) and its device error flag
   fcc::TcEngine tc;
   fcc::DBuf<int> dev_err;
   // the last run
@@ -70,6 +71,15 @@ struct fcc_ctx {
 };
 
 namespace fcc {
+// The flag that a tensor-core kernel sets when a bounded wait gave up: cleared
+// before a call's work, read (with a stream synchronisation) after it.
+inline void reset_device_error(fcc_ctx* c) { FCC_CUDA(cudaMemsetAsync(c->dev_err.p, 0, sizeof(int), c->stream)); }
+inline void check_device_error(fcc_ctx* c, const char* what) {
+  int herr = 0;
+  FCC_CUDA(cudaMemcpyAsync(&herr, c->dev_err.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  FCC_CUDA(cudaStreamSynchronize(c->stream));
+  if (herr) fail(FCC_ERR_TIMEOUT, std::string("a tensor-core wait gave up in ") + what);
+}
 void setup_integrals(fcc_ctx* c);
 void make_mp2_guess(fcc_ctx* c);
 double cc_energy(fcc_ctx* c, const double* t1, const double* t2);

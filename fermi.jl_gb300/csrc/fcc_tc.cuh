@@ -185,7 +185,19 @@ void scale_output(const EpiMap& ep, double beta, cudaStream_t s);
 struct OzLevel {
   int S, G, cut, bits;
 };
-constexpr int OZ_MAXS = 7;
+// FP64 level: 64 bits below the row maximum, every pair of weight 2^-72 and
+// up (36 products), the first band summed apart.  Dropped pairs and cut digits
+// are below 2^-64 of max|A_r| max|B_c| per term and the sums carry ~2^-60 of
+// the result, where an FP64 product accumulates roundings of 2^-53 of its
+// partial sums.  Error against quadruple precision on the operands of (H2O)4
+// (2-norm of the difference over that of the result), this level / seven
+// slices / FP64 pipe: DF fit over J^-1/2 1.2e-16 / 3.7e-15 / 1.8e-14, MO
+// transform 1.3e-17 / 1.6e-16 / 5.3e-16, (ia|jb) 6e-18 / 4e-17 / 2.3e-16, ring
+// 4e-18 / 5e-17 / 2.7e-16, ladder 2e-17 / 1.4e-16 / 9e-16, (T) over l 7e-18 /
+// 1.1e-16 / 1.7e-16.  Seven slices would be 5% faster; eight leave a decade for
+// rows more peaked than these.
+constexpr OzLevel OZ_F64{8, 9, 1, 8};
+constexpr int OZ_MAXS = 8;
 constexpr int OZ_G_DEFAULT = 8;
 // the level of `groups` weight groups of 6-bit digits, the unit the phases of
 // the mixed form are counted in: those digits themselves up to 7 groups, 8-bit
@@ -201,7 +213,6 @@ inline double oz_pairs(OzLevel lv) {
 // to (s+1)*Kpad; ex[r] = biased FP64 exponent of max_k |x_rk| (0: all zero,
 // 2047: the row holds an infinity or NaN, and so will its products)
 int64_t oz_kpad(int64_t K);
-// (S up to 8 with 6-bit digits, 7 with 8-bit digits)
 void pack_oz(const double* src, const PackSpec& ps, int S, int bits, __nv_bfloat16* dst, int* ex, cudaStream_t s);
 // FP64 epilogue (EPI_F64) of the exact-slice product over packed operands;
 // ws holds the partial results of products cut into several jobs
@@ -220,6 +231,9 @@ struct TcEngine {
   DBuf<double> ozws;       // partial results of exact-slice products cut into jobs
   double min_flops = 1e6;
   int64_t min_dim = 16;   // smallest M and N routed to the tensor cores
+  // FP64 contractions of this size and more run as exact-slice products at the
+  // FP64 level, whether `enabled` or not
+  double f64_min_flops = 4e7;
   DBuf<__nv_bfloat16> bufA, bufB;
   int* err = nullptr;
   int no_loads_once = 0;   // test hook: the next split-BF16 GEMM runs with EpiMap::no_loads
@@ -258,7 +272,8 @@ struct KeepPackedA {
   }
 };
 
-// Current engine of this host thread (nullptr: every contraction is FP64).
+// Current engine of this host thread (nullptr: every contraction is on the
+// FP64 pipe).
 TcEngine*& tc_engine();
 
 struct TcScope {

@@ -62,7 +62,6 @@ extern "C" int fcc_test_triples_subset(fcc_ctx* c, const int32_t* ijk, int32_t n
     }
     std::vector<double> each;
     fcc::WorkspaceScope ws(&c->f64ws);
-    fcc::TcScope fp64(nullptr);
     fcc::triples_fp64(c, &sub, &each);
     for (int32_t q = 0; q < n; ++q) e_each[q] = each[q];
     return FCC_OK;
@@ -97,12 +96,15 @@ extern "C" int fcc_test_contract(int32_t precision, const char* spec, const doub
     FCC_CUDA(cudaMemcpyAsync(dB.p, B, nb * 8, cudaMemcpyHostToDevice, s));
     FCC_CUDA(cudaMemcpyAsync(dC.p, C, nc * 8, cudaMemcpyHostToDevice, s));
     fcc::TcEngine eng;
-    eng.enabled = precision != FCC_PREC_FP64;
+    const bool fp64 = precision == FCC_PREC_FP64 || precision == 20 || precision == 21;
+    eng.enabled = !fp64;
+    if (precision == 20) eng.f64_min_flops = 0.0;
+    if (precision == 21) eng.f64_min_flops = 1e300;
     if (precision == 2) eng.scheme = fcc::SPLIT6;
     if (precision == 3 || (precision >= 12 && precision <= 19)) {
       eng.exact = true;
       eng.oz = fcc::oz_level(precision == 3 ? fcc::OZ_G_DEFAULT : precision - 10);
-    } else if (precision < 0 || precision > 3) {
+    } else if (!fp64 && (precision < 0 || precision > 3)) {
       return FCC_ERR_BAD_ARG;
     }
     eng.min_flops = 0.0;
@@ -113,7 +115,7 @@ extern "C" int fcc_test_contract(int32_t precision, const char* spec, const doub
       fcc::einsum(alpha, spec, view_of(dA.p, adims, arank), view_of(dB.p, bdims, brank), beta,
                   view_of(dC.p, cdims, crank), s);
     }
-    if (precision != FCC_PREC_FP64 && eng.tc_calls != 1) return FCC_ERR_BAD_ARG;
+    if (((!fp64 || precision == 20) && eng.tc_calls != 1) || (precision == 21 && eng.tc_calls != 0)) return FCC_ERR_BAD_ARG;
     int herr = 0;
     FCC_CUDA(cudaMemcpyAsync(C, dC.p, nc * 8, cudaMemcpyDeviceToHost, s));
     FCC_CUDA(cudaMemcpyAsync(&herr, err.p, sizeof(int), cudaMemcpyDeviceToHost, s));

@@ -535,19 +535,29 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   if (threadIdx.x == 0 && abort_flag) atomicExch(err, 1);
 }
 
-// C = alpha * sum_j part[j] + beta * C, the jobs summed in order.
-__global__ void __launch_bounds__(256) oz_reduce_kernel(const double* __restrict__ part, int njobs, EpiMap ep) {
+// C = alpha * sum_j part[j] + beta * C, the jobs summed in order.  The first
+// nhi jobs (all of them without a cut) are those of the first part: exact
+// multiples of 2^-24 of the row and column scales whose sum fits 53 bits, so it
+// is exact, and adding the sum of the others, 2^-12 of it or less, is the one
+// rounding of the result.
+__global__ void __launch_bounds__(256) oz_reduce_kernel(const double* __restrict__ part, int nhi, int njobs,
+                                                        EpiMap ep) {
   const int64_t MN = ep.M * ep.N;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < MN; t += (int64_t)gridDim.x * blockDim.x) {
+  auto sum = [&](int64_t t, int j0, int j1) {
     double s = 0.0;
-    for (int j = 0; j < njobs; j += 8) {   // eight loads in flight, added in order
+    for (int j = j0; j < j1; j += 8) {   // eight loads in flight, added in order
       double x[8];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) x[q] = j + q < njobs ? part[(int64_t)(j + q) * MN + t] : 0.0;
+      for (int q = 0; q < 8; ++q) x[q] = j + q < j1 ? part[(int64_t)(j + q) * MN + t] : 0.0;
 #pragma unroll
       for (int q = 0; q < 8; ++q)
-        if (j + q < njobs) s += x[q];
+        if (j + q < j1) s += x[q];
     }
+    return s;
+  };
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < MN; t += (int64_t)gridDim.x * blockDim.x) {
+    double s = sum(t, 0, nhi);
+    if (nhi < njobs) s += sum(t, nhi, njobs);
     const uint32_t m = (uint32_t)t / (uint32_t)ep.N, n = (uint32_t)t - m * (uint32_t)ep.N;
     double* dst = static_cast<double*>(ep.C) + epi_row_off(ep, m) + epi_col_off(ep, n);
     if (ep.alpha != 1.0) s *= ep.alpha;
@@ -675,7 +685,12 @@ void gemm_oz(const __nv_bfloat16* A, int64_t a_rows, const int* exA, const __nv_
   FCC_CHECK_LAUNCH();
   if (P.njobs > 1) {
     const int64_t MN = ep.M * ep.N;
-    oz_reduce_kernel<<<(unsigned)std::min<int64_t>((MN + 255) / 256, 152 * 8), 256, 0, s>>>(ws.p, P.njobs, ep);
+    int nhi = P.njobs;
+    if (lv.cut) {
+      nhi = 0;
+      while (nhi < P.njobs && P.job[nhi].b0 < lv.cut) ++nhi;
+    }
+    oz_reduce_kernel<<<(unsigned)std::min<int64_t>((MN + 255) / 256, 152 * 8), 256, 0, s>>>(ws.p, nhi, P.njobs, ep);
     FCC_CHECK_LAUNCH();
   }
   prof_end(s, pidx, PROF_OZ, ep.work > 0 ? ep.work : 2.0 * (double)ep.M * (double)ep.N * (double)Kpad * steps_kb);

@@ -97,7 +97,7 @@ __device__ __forceinline__ uint32_t oz_byte_bits(uint32_t w, int sel) {
 // bf16 of a and b (upper halves) as one word, a in the lower half
 __device__ __forceinline__ uint32_t oz_pair(uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x7632); }
 
-// |x| 2^-e (|x| < 2^e) times 2^bits, rounded to an integer; bits <= 56
+// |x| 2^-e (|x| < 2^e) times 2^bits, rounded to an integer; bits <= 64
 __device__ __forceinline__ unsigned long long oz_fixed(unsigned long long x, int e, int bits) {
   const int be = (int)((x >> 52) & 0x7FF);
   unsigned long long Z = 0;
@@ -117,7 +117,8 @@ __device__ __forceinline__ unsigned long long oz_fixed(unsigned long long x, int
 // low place, less that half (a digit at or above half carries one into the
 // next).  Integer arithmetic only; |y - sum_s d_s 2^(-BITS s)| <= 2^(-BITS S) / 2.
 // 8 bits: the signed Z is cut, each low digit is one byte (three instructions);
-// 6 bits: |Z| is cut and the digits take the sign.
+// otherwise (6 bits, or the 64 bits of S = 8, which leave no room for a sign)
+// |Z| is cut and the digits take the sign.
 template <int S, int BITS>
 __device__ __forceinline__ void oz_digits(double x, int e, uint32_t (&d)[S]) {
   const unsigned long long xb = (unsigned long long)__double_as_longlong(x);
@@ -125,7 +126,14 @@ __device__ __forceinline__ void oz_digits(double x, int e, uint32_t (&d)[S]) {
   const int neg = (int)(xb >> 63);
   constexpr unsigned long long HALF = 1ull << (BITS - 1);
   constexpr unsigned long long C = HALF * (((1ull << (BITS * (S - 1))) - 1) / ((1ull << BITS) - 1));
-  if (BITS == 8) {
+  if (BITS == 8 && S == 8) {
+    const unsigned long long low = (Z & ((1ull << 56) - 1)) + C;   // C < 2^56: no carry out of 57 bits
+    const uint32_t w[2] = {(uint32_t)low, (uint32_t)(low >> 32)};
+    const uint32_t flip = neg ? 0x80000000u : 0u;
+#pragma unroll
+    for (int s = 1; s < S; ++s) d[s] = oz_byte_bits(w[(S - 1 - s) >> 2], (S - 1 - s) & 3) ^ flip;
+    d[0] = oz_int_bits((int)(Z >> 56) + (int)(low >> 56)) ^ flip;
+  } else if (BITS == 8) {
     const unsigned long long Zc = (neg ? 0ull - Z : Z) + C;
     const uint32_t w[2] = {(uint32_t)Zc, (uint32_t)(Zc >> 32)};
 #pragma unroll
@@ -406,6 +414,7 @@ void pack_oz(const double* src, const PackSpec& ps, int S, int bits, __nv_bfloat
     case 85: pack<5, 8>(src, ps, dst, ex, s); break;
     case 86: pack<6, 8>(src, ps, dst, ex, s); break;
     case 87: pack<7, 8>(src, ps, dst, ex, s); break;
+    case 88: pack<8, 8>(src, ps, dst, ex, s); break;
     default: fail(FCC_ERR_BAD_ARG, "bad slice count");
   }
 }

@@ -36,6 +36,8 @@ struct fcc_scf {
   fcc::DBuf<double> H, D, F, C, Y;    // nbf^2 matrices, occupied orbitals, K intermediate
   fcc::DBuf<double> gam, gpart, red;
   fcc::DBuf<double> f64ws;            // split-K partial sums of the FP64 contractions
+  fcc::TcEngine tc;                   // exact-slice products of the large ones
+  fcc::DBuf<int> err;                 // set when a bounded wait of theirs gave up
 };
 
 namespace {
@@ -88,7 +90,7 @@ int guarded(fcc_scf* s, Fn&& f) {
       cudaError_t e = cudaSetDevice(s->device);
       if (e != cudaSuccess) { s->last_error = cudaGetErrorString(e); return FCC_ERR_CUDA; }
     }
-    fcc::TcScope fp64_only(nullptr);   // every contraction here runs in FP64
+    fcc::TcScope tc(s ? &s->tc : nullptr);   // every contraction here is FP64
     fcc::WorkspaceScope ws(s ? &s->f64ws : nullptr);
     return f();
   } catch (const fcc::Error& e) {
@@ -106,6 +108,16 @@ int guarded(fcc_scf* s, Fn&& f) {
 void check_finite(const double* p, int64_t n, const char* what) {
   for (int64_t i = 0; i < n; ++i)
     if (!std::isfinite(p[i])) fcc::fail(FCC_ERR_BAD_ARG, std::string("non-finite ") + what);
+}
+
+// Waits for the stream and reports a tensor-core wait that gave up.
+void sync_checked(fcc_scf* s) {
+  int herr = 0;
+  FCC_CUDA(cudaMemcpyAsync(&herr, s->err.p, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+  FCC_CUDA(cudaStreamSynchronize(s->stream));
+  if (!herr) return;
+  FCC_CUDA(cudaMemsetAsync(s->err.p, 0, sizeof(int), s->stream));
+  fcc::fail(FCC_ERR_TIMEOUT, "a tensor-core wait gave up");
 }
 
 // F = H + 2 J[D] (device H, D already in place); leaves F on the device.
@@ -133,7 +145,7 @@ void finish(fcc_scf* s, double* F, double* eelec) {
     FCC_CUDA(cudaMemcpyAsync(eelec, s->red.p, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
   }
   FCC_CUDA(cudaMemcpyAsync(F, s->F.p, sizeof(double) * R, cudaMemcpyDeviceToHost, s->stream));
-  FCC_CUDA(cudaStreamSynchronize(s->stream));
+  sync_checked(s);
 }
 
 }  // namespace
@@ -165,6 +177,9 @@ int fcc_scf_create(fcc_scf** out, int32_t nbf, int32_t naux, int32_t device) {
     s->F.alloc(R);
     s->gam.alloc(s->Q);
     s->red.alloc(1);
+    s->err.alloc(1);
+    FCC_CUDA(cudaMemsetAsync(s->err.p, 0, sizeof(int), s->stream));
+    s->tc.err = s->err.p;
     return FCC_OK;
   });
   if (rc != FCC_OK) {
@@ -212,7 +227,7 @@ int fcc_scf_fit(fcc_scf* s, const double* Pqp, const double* Jh) {
     FCC_CUDA(cudaMemcpyAsync(dJ.p, Jh, sizeof(double) * Q * Q, cudaMemcpyHostToDevice, s->stream));
     // AtomicIntegrals.jl:37-38: b[Q,p,q] = sum_P Pqp[p,q,P] Jh[P,Q]
     fcc::einsum(1.0, "pqP,PQ->Qpq", cm(dP.p, {n, n, Q}), cm(dJ.p, {Q, Q}), 0.0, cm(s->b.p, {Q, n, n}), s->stream);
-    FCC_CUDA(cudaStreamSynchronize(s->stream));
+    sync_checked(s);
     s->have_b = true;
     return FCC_OK;
   });

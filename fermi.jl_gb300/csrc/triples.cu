@@ -165,6 +165,9 @@ __global__ void sum_kernel(const double* part, int n, double* out) {
 
 double triples_fp64(fcc_ctx* c, const std::vector<int3>* subset, std::vector<double>* each) {
   cudaStream_t s = c->stream;
+  TcScope scope(&c->tc);
+  c->tc.enabled = false;
+  reset_device_error(c);
   const int64_t o = c->o, v = c->v, Q = c->Q, n = c->n;
   const int64_t v2 = v * v, v3 = v2 * v, ov2 = o * v2, o2v = o * o * v;
   TView B = rm(c->B.p, {Q, n, n});
@@ -265,7 +268,7 @@ double triples_fp64(fcc_ctx* c, const std::vector<int3>* subset, std::vector<dou
   FCC_CHECK_LAUNCH();
   double et = 0.0;
   FCC_CUDA(cudaMemcpyAsync(&et, out.p, sizeof(double), cudaMemcpyDeviceToHost, s));
-  FCC_CUDA(cudaStreamSynchronize(s));
+  check_device_error(c, "(T)");
   c->ovvv.release();
   c->ooov.release();
   c->Wt.release();

@@ -17,11 +17,12 @@ extern "C" {
 #endif
 
 /* C = alpha * einsum(spec, A, B) + beta * C on device 0 for row-major host
- * tensors (rank <= 4 each).  precision FCC_PREC_FP64 runs the DMMA kernel;
+ * tensors (rank <= 4 each).  precision FCC_PREC_FP64 runs the FP64 path;
  * FCC_PREC_MIXED forces the three-product split-BF16 tensor-core kernel,
  * 2 the six-product one, 3 the exact-slice (Ozaki) kernel with 8 weight
- * groups and 10 + G the exact-slice kernel with G groups (2 <= G <= 9)
- * (error if the contraction cannot be expressed for it).  Returns an fcc
+ * groups and 10 + G the exact-slice kernel with G groups (2 <= G <= 9),
+ * 20 the exact-slice kernel at the FP64 level whatever the size and 21 the
+ * FP64 pipe whatever the size (error if the contraction cannot be expressed for it).  Returns an fcc
  * status code. */
 int fcc_test_contract(int32_t precision, const char* spec, const double* A, const int64_t* adims, int32_t arank,
                       const double* B, const int64_t* bdims, int32_t brank, double* C, const int64_t* cdims,
@@ -35,7 +36,7 @@ int fcc_test_split3(const double* x, int64_t R, int64_t K, int32_t row_fastest, 
 
 /* The exact-slice operand packing on device 0: x is R x K (row-major, or
  * column-major when row_fastest != 0), cut into S (1..8) signed 6-bit digit
- * slices, or for S = 11..17 into S - 10 slices of the signed 8-bit digits that
+ * slices, or for S = 11..18 into S - 10 slices of the signed 8-bit digits that
  * the exact-slice kernel multiplies; out receives R rows of S * Kpad bf16 bit patterns (Kpad = K
  * rounded up to 64; slice s at columns [s * Kpad, s * Kpad + K), zeros to
  * (s + 1) * Kpad) and ex the R biased FP64 exponents of the row maxima. */

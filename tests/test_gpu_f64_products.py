@@ -1,0 +1,119 @@
+"""The FP64 contractions: the exact-slice products at the FP64 level and the
+small DMMA kernel against quadruple-precision references, over ragged sizes,
+index orders and wide dynamic ranges; neither may be less accurate than an
+FP64 product is."""
+import numpy as np
+import pytest
+
+from test_gpu_contract import CASES, _run
+
+pytestmark = pytest.mark.gpu
+
+TC, PIPE = 20, 21          # fcc_test_contract: tensor cores / FP64 pipe whatever the size
+
+
+def _quad(A, B):
+    """A @ B.T with ~106 bits: Dekker products accumulated by TwoSum (Ogita,
+    Rump & Oishi, SIAM J. Sci. Comput. 26, 1955 (2005))."""
+    def two_sum(a, b):
+        s = a + b
+        z = s - a
+        return s, (a - (s - z)) + (b - z)
+
+    def split(x):
+        c = 134217729.0 * x
+        h = c - (c - x)
+        return h, x - h
+    s = np.zeros((A.shape[0], B.shape[0]))
+    lo = np.zeros_like(s)
+    for k in range(A.shape[1]):
+        a, b = A[:, k][:, None], B[:, k][None, :]
+        p = a * b
+        ah, al = split(a)
+        bh, bl = split(b)
+        e = al * bl - (((p - ah * bh) - al * bh) - ah * bl)
+        s, q = two_sum(s, p)
+        lo += q + e
+    return s + lo
+
+
+@pytest.mark.parametrize("prec", [TC, PIPE])
+@pytest.mark.parametrize("spec,sa,sb,sc", CASES[:-2] + CASES[-1:])
+def test_index_orders_and_scalings(prec, spec, sa, sb, sc):
+    rng = np.random.default_rng(3)
+    A, B, C = rng.standard_normal(sa), rng.standard_normal(sb), rng.standard_normal(sc)
+    for alpha, beta in ((1.0, 0.0), (-0.5, 1.0), (0.7, -1.3)):
+        rc, out = _run(prec, spec, A, B, C, alpha, beta)
+        assert rc == 0
+        ref = alpha * np.einsum(spec, A, B) + beta * C
+        assert np.abs(out - ref).max() < 1e-13 * np.abs(ref).max()
+
+
+# a contraction of integral- or amplitude-like rows spans decades; the error of
+# an FP64 product of length K is about sqrt(K / 2) 2^-54.8 of |A_r| |B_c| / sqrt(K)
+@pytest.mark.parametrize("M,N,K", [(8, 8, 5000), (130, 17, 700), (46, 46, 46), (200, 300, 129), (64, 64, 1500)])
+@pytest.mark.parametrize("spread", [0.0, 3.0, 8.0])
+def test_no_less_accurate_than_the_fp64_pipe(M, N, K, spread):
+    rng = np.random.default_rng(M + K)
+    A = rng.standard_normal((M, K)) * 10.0 ** rng.uniform(-spread, 0, (M, K))
+    B = rng.standard_normal((N, K)) * 10.0 ** rng.uniform(-spread, 0, (N, K))
+    ref = _quad(A, B)
+    err = {}
+    for prec in (TC, PIPE):
+        rc, out = _run(prec, "mk,nk->mn", A, B, np.zeros((M, N)))
+        assert rc == 0
+        err[prec] = np.linalg.norm(out - ref) / np.linalg.norm(ref)
+    # both end with one rounding to FP64 (rms 2^-53 / sqrt(12) of an element)
+    assert err[TC] <= max(err[PIPE], 2.0 ** -53), err
+
+
+def test_peaked_rows_against_a_metric():
+    # rows with a few large entries against the inverse square root of a nearly
+    # dependent metric: the largest entries of one side meet the smallest of the
+    # other, and the sums are far below the product of the maxima
+    rng = np.random.default_rng(7)
+    n, K = 300, 500
+    x = np.linspace(0, 30, K)
+    S = np.exp(-0.5 * (x[:, None] - x[None, :]) ** 2) + 1e-9 * np.eye(K)
+    w, U = np.linalg.eigh(S)
+    J = (U / np.sqrt(w)) @ U.T
+    A = np.exp(-2.0 * (30 * rng.random(n)[:, None] - x[None, :]) ** 2) * rng.standard_normal((n, K))
+    ref = _quad(A, J)
+    err = {}
+    for prec in (TC, PIPE):
+        rc, out = _run(prec, "mk,nk->mn", A, J, np.zeros((n, K)))
+        assert rc == 0
+        err[prec] = np.linalg.norm(out - ref) / np.linalg.norm(ref)
+    assert err[TC] <= max(err[PIPE], 2.0 ** -53), err
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 5, 3), (7, 9, 1), (16, 17, 4), (33, 15, 130), (5, 5, 9000), (250, 250, 40)])
+def test_small_kernel_edges(M, N, K):
+    rng = np.random.default_rng(M * N + K)
+    A = rng.integers(-1000, 1000, (M, K)).astype(float)
+    B = rng.integers(-1000, 1000, (N, K)).astype(float)
+    C = rng.integers(-9, 9, (M, N)).astype(float)
+    rc, out = _run(PIPE, "mk,nk->mn", A, B, C, -1.0, 2.0)
+    assert rc == 0
+    assert np.array_equal(out, 2.0 * C - A @ B.T)          # integers: exact in any order
+
+
+@pytest.mark.parametrize("shape,spec,bspec", [((300, 70), "mk,k->m", "col"), ((70, 300), "km,k->m", "row"),
+                                              ((12, 25, 40), "kab,k->ab", "row"), ((31, 200), "mk,k->m", "col")])
+def test_matrix_vector_both_layouts(shape, spec, bspec):
+    rng = np.random.default_rng(1)
+    A = rng.integers(-99, 99, shape).astype(float)
+    k = shape[-1] if bspec == "col" else shape[0]
+    x = rng.integers(-99, 99, k).astype(float)
+    ref = np.einsum(spec, A, x)
+    rc, out = _run(0, spec, A, x, np.ones_like(ref), 2.0, -1.0)
+    assert rc == 0
+    assert np.array_equal(out, 2.0 * ref - 1.0)
+
+
+def test_results_repeat_bit_for_bit():
+    rng = np.random.default_rng(2)
+    for M, N, K in ((40, 30, 20000), (300, 300, 300)):
+        A, B = rng.standard_normal((M, K)), rng.standard_normal((N, K))
+        one, two = (_run(TC, "mk,nk->mn", A, B, np.zeros((M, N)))[1] for _ in range(2))
+        assert np.array_equal(one, two)
