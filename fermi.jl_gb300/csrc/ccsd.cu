@@ -27,8 +27,9 @@ namespace {
 constexpr int RED_BLOCKS = 608;  // 152 SMs x 4: fixed, so reductions are deterministic
 constexpr int RED_THREADS = 256;
 constexpr int MAX_DIIS = 8;
-// partial-sum layout per block: [0] sum dT^2, [1] energy, [2..2+MAX_DIIS) dots
-constexpr int NPART = 2 + MAX_DIIS;
+// partial-sum layout per block: [0] sum dT^2, [1] energy, [2] dot of the stored
+// error with itself, [3..3+MAX_DIIS) with the others
+constexpr int NPART = 3 + MAX_DIIS;
 
 __device__ __forceinline__ double warp_sum(double x) {
   for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
@@ -39,7 +40,9 @@ __device__ __forceinline__ double warp_sum(double x) {
 __device__ void block_reduce_store(double (&vals)[NPART], int nvals, double* part) {
   __shared__ double sm[RED_THREADS / 32][NPART];
   int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int k = 0; k < nvals; ++k) {
+#pragma unroll
+  for (int k = 0; k < NPART; ++k) {
+    if (k >= nvals) break;
     double s = warp_sum(vals[k]);
     if (lane == 0) sm[w][k] = s;
   }
@@ -51,13 +54,17 @@ __device__ void block_reduce_store(double (&vals)[NPART], int nvals, double* par
   }
 }
 
-// Sum the per-block partials (fixed order) into out[k].
+// Sum the per-block partials into out[k]: a warp per value, the lanes over the
+// blocks in turn and then the lanes, a fixed order.  (One thread per value, as
+// this was, took 50 us for the 608 dependent additions; 3 us.)
 __global__ void finish_reduce_kernel(const double* part, int nblocks, int nvals, double* out) {
-  int k = threadIdx.x;
+  const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (k >= nvals) return;
   double s = 0.0;
-  for (int b = 0; b < nblocks; ++b) s += part[b * NPART + k];
-  out[k] = s;
+#pragma unroll 4
+  for (int b = lane; b < nblocks; b += 32) s += part[b * NPART + k];
+  s = warp_sum(s);
+  if (lane == 0) out[k] = s;
 }
 
 struct ErrSlots {
@@ -73,20 +80,52 @@ struct ErrSlots {
 //   contribution Lt * (Tnew + t1new_ia t1new_jb) (T2 only).
 // rank 2: index e -> (i, a); rank 4: e -> (i, j, a, b), b fastest.  For T2
 // each warp takes whole rows (i, j, a) so the index arithmetic and
-// e_i + e_j - e_a are per row; lanes read consecutive pairs of b with 128-bit
-// loads (v even) or single elements.
-__device__ __forceinline__ void update_one(int64_t e, double t, double r, double D, double t1ab, const double* Lt,
+// e_i + e_j - e_a are per row; lanes read consecutive b.
+//
+// The FP64 pipe (two lanes per clk and SM) bounds this pass, not HBM, so it is
+// kept short: the quotient by D takes a reciprocal seed in single precision and
+// two Newton steps (Markstein, IBM J. Res. Dev. 34, 111 (1990): the remainder
+// r - q D by one fma, within the last place) instead of the compiler's division, the stored errors are widened by integer arithmetic, and the dot of
+// the error with itself comes from this pass.  (H2O)8: 0.90 + 0.19 ms with a
+// division and a second pass over the errors, see the launch list.
+// a float as a double, exactly, without the FP64 pipe (subnormals become 0)
+__device__ __forceinline__ double widen(float f) {
+  const uint32_t b = __float_as_uint(f);
+  const uint32_t hi = ((b & 0x7FFFFFFFu) >> 3) + (896u << 20);
+  if ((b & 0x7F800000u) == 0u) return 0.0;
+  if ((b & 0x7F800000u) == 0x7F800000u) return (double)f;
+  return __hiloint2double((int)(hi | (b & 0x80000000u)), (int)(b << 29));
+}
+__device__ __forceinline__ double quotient(double r, double D) {
+  // |D| is an orbital-energy difference: far inside the single-precision range
+  double y = widen(__frcp_rn((float)D));
+  y = fma(y, fma(-D, y, 1.0), y);        // 2^-24 -> 2^-47
+  const double q = r * y;
+  return fma(y, fma(-D, q, r), q);       // remainder in full precision
+}
+__device__ __forceinline__ void update_one(int64_t e, double t, double r, double D, double t1ab, bool energy, double lt,
                                            float* err_s, double* err_d, const ErrSlots& others, double& tn,
                                            double (&vals)[NPART]) {
-  const double dt = r / D;
+  const double dt = quotient(r, D);
   tn = t + dt;
-  vals[0] += dt * dt;
-  if (Lt) vals[1] += Lt[e] * (tn + t1ab);
-  double ev;
-  if (err_s) { const float f = (float)dt; err_s[e] = f; ev = (double)f; }
-  else if (err_d) { err_d[e] = dt; ev = dt; }
-  else ev = dt;
-  for (int k = 0; k < others.n; ++k) vals[2 + k] += ev * (others.s[k] ? (double)others.s[k][e] : others.d[k][e]);
+  vals[0] = fma(dt, dt, vals[0]);
+  if (energy) vals[1] = fma(lt, tn + t1ab, vals[1]);
+  double ev = dt;
+  if (err_s) {
+    const float f = (float)dt;
+    err_s[e] = f;
+    ev = widen(f);
+  } else if (err_d) {
+    err_d[e] = dt;
+  } else {
+    return;
+  }
+  vals[2] = fma(ev, ev, vals[2]);
+#pragma unroll
+  for (int k = 0; k < MAX_DIIS; ++k) {
+    if (k >= others.n) break;
+    vals[3 + k] = fma(ev, others.s[k] ? widen(others.s[k][e]) : others.d[k][e], vals[3 + k]);
+  }
 }
 
 __global__ void __launch_bounds__(RED_THREADS) update_kernel(
@@ -101,58 +140,33 @@ __global__ void __launch_bounds__(RED_THREADS) update_kernel(
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
       const int i = e / v, a = e - i * v;
       double tn;
-      update_one(e, T[e], R[e], eps[i] - eps[o + a], 0.0, nullptr, err_s, err_d, others, tn, vals);
+      update_one(e, T[e], R[e], eps[i] - eps[o + a], 0.0, false, 0.0, err_s, err_d, others, tn, vals);
       Tnew[e] = tn;
     }
   } else {
     const int lane = threadIdx.x & 31;
-    const int64_t nrows = (int64_t)o * o * v;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const bool pairs = (v & 1) == 0;
-    for (int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < nrows; row += nw) {
-      const int a = (int)(row % v);
-      const int64_t ij = row / v;
-      const int j = (int)(ij % o), i = (int)(ij / o);
+    const uint32_t nrows = (uint32_t)o * o * v;
+    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < nrows; row += nw) {
+      const int a = (int)(row % (uint32_t)v);
+      const uint32_t ij = row / (uint32_t)v;
+      const int j = (int)(ij % (uint32_t)o), i = (int)(ij / (uint32_t)o);
       const double Drow = eps[i] + eps[j] - eps[o + a];
       const double t1ia = Lt ? t1new[(int64_t)i * v + a] : 0.0;
       const double* t1j = t1new + (int64_t)j * v;
       const double* ev = eps + o;
-      const int64_t base = row * v;
-      if (pairs) {
-        for (int b = 2 * lane; b < v; b += 64) {
-          const int64_t e = base + b;
-          const double2 tv = *reinterpret_cast<const double2*>(T + e);
-          const double2 rv = *reinterpret_cast<const double2*>(R + e);
-          double2 tn;
-          update_one(e, tv.x, rv.x, Drow - ev[b], Lt ? t1ia * t1j[b] : 0.0, Lt, err_s, err_d, others, tn.x, vals);
-          update_one(e + 1, tv.y, rv.y, Drow - ev[b + 1], Lt ? t1ia * t1j[b + 1] : 0.0, Lt, err_s, err_d, others,
-                     tn.y, vals);
-          *reinterpret_cast<double2*>(Tnew + e) = tn;
-        }
-      } else {
-        for (int b = lane; b < v; b += 32) {
-          const int64_t e = base + b;
-          double tn;
-          update_one(e, T[e], R[e], Drow - ev[b], Lt ? t1ia * t1j[b] : 0.0, Lt, err_s, err_d, others, tn, vals);
-          Tnew[e] = tn;
-        }
+      const int64_t base = (int64_t)row * v;
+#pragma unroll 2
+      for (int b = lane; b < v; b += 32) {
+        const int64_t e = base + b;
+        double tn;
+        update_one(e, T[e], R[e], Drow - ev[b], Lt ? t1ia * t1j[b] : 0.0, Lt != nullptr, Lt ? Lt[e] : 0.0, err_s, err_d,
+                   others, tn, vals);
+        Tnew[e] = tn;
       }
     }
   }
-  block_reduce_store(vals, 2 + others.n, part);
-}
-
-// Self dot of the stored error (its norm^2 in the stored precision).
-__global__ void __launch_bounds__(RED_THREADS) selfdot_kernel(int64_t total, const float* es, const double* ed,
-                                                              double* part) {
-  double vals[NPART];
-#pragma unroll
-  for (int k = 0; k < NPART; ++k) vals[k] = 0.0;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-    double x = es ? (double)es[e] : ed[e];
-    vals[0] += x * x;
-  }
-  block_reduce_store(vals, 1, part);
+  block_reduce_store(vals, 3 + others.n, part);
 }
 
 // DIIS extrapolation: out = sum_k c_k (vec_k + add_res * err_k); for T2 also
@@ -177,8 +191,8 @@ __global__ void __launch_bounds__(RED_THREADS) extrapolate_kernel(int rank, int 
   auto combine = [&](int64_t e) {
     double s = 0.0;
     for (int k = 0; k < sl.n; ++k) {
-      const double ev = sl.es[k] ? (double)sl.es[k][e] : sl.ed[k][e];
-      s += c[k] * sl.vec[k][e] + c[k] * ev;
+      const double ev = sl.es[k] ? widen(sl.es[k][e]) : sl.ed[k][e];
+      s = fma(c[k], ev, fma(c[k], sl.vec[k][e], s));
     }
     out[e] = s;
     return s;
@@ -188,15 +202,15 @@ __global__ void __launch_bounds__(RED_THREADS) extrapolate_kernel(int rank, int 
   } else {
     // whole rows (i, j, a) per warp, lanes along b
     const int lane = threadIdx.x & 31;
-    const int64_t nrows = (int64_t)o * o * v;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < nrows; row += nw) {
-      const int a = (int)(row % v);
-      const int64_t ij = row / v;
-      const int j = (int)(ij % o), i = (int)(ij / o);
+    const uint32_t nrows = (uint32_t)o * o * v;
+    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < nrows; row += nw) {
+      const int a = (int)(row % (uint32_t)v);
+      const uint32_t ij = row / (uint32_t)v;
+      const int j = (int)(ij % (uint32_t)o), i = (int)(ij / (uint32_t)o);
       const double t1ia = Lt ? t1new[(int64_t)i * v + a] : 0.0;
       for (int b = lane; b < v; b += 32) {
-        const int64_t e = row * v + b;
+        const int64_t e = (int64_t)row * v + b;
         const double s = combine(e);
         if (Lt) vals[1] += Lt[e] * (s + t1ia * t1new[(int64_t)j * v + b]);
       }
@@ -213,15 +227,15 @@ __global__ void __launch_bounds__(RED_THREADS) energy_kernel(int o, int v, const
 #pragma unroll
   for (int k = 0; k < NPART; ++k) vals[k] = 0.0;
   const int lane = threadIdx.x & 31;
-  const int64_t nrows = (int64_t)o * o * v;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < nrows; row += nw) {
-    const int a = (int)(row % v);
-    const int64_t ij = row / v;
-    const int j = (int)(ij % o), i = (int)(ij / o);
+  const uint32_t nrows = (uint32_t)o * o * v;
+  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < nrows; row += nw) {
+    const int a = (int)(row % (uint32_t)v);
+    const uint32_t ij = row / (uint32_t)v;
+    const int j = (int)(ij % (uint32_t)o), i = (int)(ij / (uint32_t)o);
     const double t1ia = t1[(int64_t)i * v + a];
     for (int b = lane; b < v; b += 32) {
-      const int64_t e = row * v + b;
+      const int64_t e = (int64_t)row * v + b;
       vals[1] += Lt[e] * (t2[e] + t1ia * t1[(int64_t)j * v + b]);
     }
   }
@@ -237,18 +251,18 @@ __global__ void __launch_bounds__(RED_THREADS) mp2_energy_kernel(int o, int v, c
 #pragma unroll
   for (int k = 0; k < NPART; ++k) vals[k] = 0.0;
   const int lane = threadIdx.x & 31;
-  const int64_t nrows = (int64_t)o * o * v;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < nrows; row += nw) {
-    const int a = (int)(row % v);
-    const int64_t ij = row / v;
-    const int j = (int)(ij % o), i = (int)(ij / o);
+  const uint32_t nrows = (uint32_t)o * o * v;
+  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < nrows; row += nw) {
+    const int a = (int)(row % (uint32_t)v);
+    const uint32_t ij = row / (uint32_t)v;
+    const int j = (int)(ij % (uint32_t)o), i = (int)(ij / (uint32_t)o);
     const double Dia = eps[i] + eps[j] - eps[o + a];
     const double* iajb = ovov + (((int64_t)i * v + a) * o + j) * v;   // (ia|jb) over b
     for (int b = lane; b < v; b += 32) {
       const double x = iajb[b];
       const double y = ovov[(((int64_t)i * v + b) * o + j) * v + a];   // (ib|ja)
-      vals[1] += x * (2.0 * x - y) / (Dia - eps[o + b]);
+      vals[1] = fma(x, quotient(2.0 * x - y, Dia - eps[o + b]), vals[1]);
     }
   }
   block_reduce_store(vals, 2, part);
@@ -287,13 +301,19 @@ __global__ void diis_solve_kernel(const double* Bm, int N, double* coef, int* st
 }
 
 // t2 <- OVOV-derived MP2 numerator / D2 (RCCSDa.jl:53-89); t1 <- 0.
-__global__ void divide_d2_kernel(double* t2, const double* eps, int o, int v) {
-  int64_t total = (int64_t)o * o * v * v;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-    int64_t b = e % v, r = e / v, a = r % v;
-    r /= v;
-    int64_t j = r % o, i = r / o;
-    t2[e] /= (eps[i] + eps[j] - eps[o + a] - eps[o + b]);
+__global__ void __launch_bounds__(RED_THREADS) divide_d2_kernel(double* t2, const double* eps, int o, int v) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t nrows = (uint32_t)o * o * v;
+  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < nrows; row += nw) {
+    const int a = (int)(row % (uint32_t)v);
+    const uint32_t ij = row / (uint32_t)v;
+    const int j = (int)(ij % (uint32_t)o), i = (int)(ij / (uint32_t)o);
+    const double Drow = eps[i] + eps[j] - eps[o + a];
+    for (int b = lane; b < v; b += 32) {
+      const int64_t e = (int64_t)row * v + b;
+      t2[e] = quotient(t2[e], Drow - eps[o + b]);
+    }
   }
 }
 
@@ -332,76 +352,86 @@ __global__ void axpby_flat_kernel(double* y, const double* x, int64_t n, double 
 // X+ symmetric and X- antisymmetric under (i<->j) and under (a<->b), so only
 // i <= j, a <= b (i < j, a < b for X-) are formed.
 
+// (The three passes below walk rows per block and columns along the threads:
+// one 32-bit division per row, where a 64-bit one per element cost more than
+// the memory traffic.)
+
 // Tp[p][q] = t+ over (i<=j, c<=d), Tm[p'][q'] = t- over (i<j, c<d)
-__global__ void build_tpm_kernel(const double* __restrict__ t2, int o, int v, const int2* __restrict__ ijP,
-                                 const int2* __restrict__ ijM, const int2* __restrict__ cdP,
-                                 const int2* __restrict__ cdM, int64_t nP, int64_t nM, int64_t nij_p,
-                                 int64_t nij_m, double* __restrict__ Tp, double* __restrict__ Tm) {
-  const int64_t totP = nij_p * nP, totM = nij_m * nM;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < totP + totM; t += (int64_t)gridDim.x * blockDim.x) {
-    if (t < totP) {
-      const int64_t p = t / nP, q = t - p * nP;
-      const int2 ij = ijP[p], cd = cdP[q];
-      const double* tr = t2 + ((int64_t)ij.x * o + ij.y) * v * v;
-      Tp[t] = (cd.x == cd.y) ? tr[(int64_t)cd.x * v + cd.y]
-                             : 0.5 * (tr[(int64_t)cd.x * v + cd.y] + tr[(int64_t)cd.y * v + cd.x]);
-    } else {
-      const int64_t u = t - totP;
-      const int64_t p = u / nM, q = u - p * nM;
-      const int2 ij = ijM[p], cd = cdM[q];
-      const double* tr = t2 + ((int64_t)ij.x * o + ij.y) * v * v;
-      Tm[u] = 0.5 * (tr[(int64_t)cd.x * v + cd.y] - tr[(int64_t)cd.y * v + cd.x]);
-    }
+__global__ void __launch_bounds__(256) build_tpm_kernel(const double* __restrict__ t2, int o, int v,
+                                                        const int2* __restrict__ ijP, const int2* __restrict__ ijM,
+                                                        const int2* __restrict__ cdP, const int2* __restrict__ cdM,
+                                                        int nP, int nM, int nij_p, int nij_m, double* __restrict__ Tp,
+                                                        double* __restrict__ Tm) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  for (int p = blockIdx.y; p < nij_p + nij_m; p += gridDim.y) {
+    const bool plus = p < nij_p;
+    const int r = plus ? p : p - nij_p, n = plus ? nP : nM;
+    if (x >= n) continue;
+    const int2 ij = plus ? ijP[r] : ijM[r], cd = plus ? cdP[x] : cdM[x];
+    const double* tr = t2 + ((int64_t)ij.x * o + ij.y) * v * v;
+    const double t = tr[(int64_t)cd.x * v + cd.y], u = tr[(int64_t)cd.y * v + cd.x];
+    if (plus) Tp[(int64_t)r * nP + x] = cd.x == cd.y ? t : 0.5 * (t + u);
+    else Tm[(int64_t)r * nM + x] = 0.5 * (t - u);
   }
 }
 
 // W+- rows for the pairs (a,b) of the current block from the slab
 // W[a-a0][c][b-a0][d] = (ac|bd), b in [a0, v).
-__global__ void build_wpm_kernel(const double* __restrict__ W, int v, int a0, int64_t vb, const int2* __restrict__ abP,
-                                 const int2* __restrict__ abM, int64_t rP0, int64_t nrP, int64_t rM0, int64_t nrM,
-                                 const int2* __restrict__ cdP, const int2* __restrict__ cdM, int64_t nP, int64_t nM,
-                                 double* __restrict__ Wp, double* __restrict__ Wm) {
-  const int64_t totP = nrP * nP, totM = nrM * nM;
-  auto Wat = [&](int a, int c, int b, int d) -> double {
-    return W[(((int64_t)(a - a0) * v + c) * vb + (b - a0)) * v + d];
-  };
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < totP + totM; t += (int64_t)gridDim.x * blockDim.x) {
-    if (t < totP) {
-      const int64_t r = t / nP, q = t - r * nP;
-      const int2 ab = abP[rP0 + r], cd = cdP[q];
-      Wp[t] = (cd.x == cd.y) ? Wat(ab.x, cd.x, ab.y, cd.y) : Wat(ab.x, cd.x, ab.y, cd.y) + Wat(ab.x, cd.y, ab.y, cd.x);
-    } else {
-      const int64_t u = t - totP;
-      const int64_t r = u / nM, q = u - r * nM;
-      const int2 ab = abM[rM0 + r], cd = cdM[q];
-      Wm[u] = Wat(ab.x, cd.x, ab.y, cd.y) - Wat(ab.x, cd.y, ab.y, cd.x);
-    }
+__global__ void __launch_bounds__(256) build_wpm_kernel(const double* __restrict__ W, int v, int a0, int vb,
+                                                        const int2* __restrict__ abP, const int2* __restrict__ abM,
+                                                        int rP0, int nrP, int rM0, int nrM,
+                                                        const int2* __restrict__ cdP, const int2* __restrict__ cdM,
+                                                        int nP, int nM, double* __restrict__ Wp,
+                                                        double* __restrict__ Wm) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t cs = (int64_t)vb * v;      // slab stride of c
+  for (int p = blockIdx.y; p < nrP + nrM; p += gridDim.y) {
+    const bool plus = p < nrP;
+    const int r = plus ? p : p - nrP, n = plus ? nP : nM;
+    if (x >= n) continue;
+    const int2 ab = plus ? abP[rP0 + r] : abM[rM0 + r], cd = plus ? cdP[x] : cdM[x];
+    const double* w = W + (int64_t)(ab.x - a0) * v * cs + (int64_t)(ab.y - a0) * v;
+    const double t = w[cd.x * cs + cd.y], u = w[cd.y * cs + cd.x];
+    if (plus) Wp[(int64_t)r * nP + x] = cd.x == cd.y ? t : t + u;
+    else Wm[(int64_t)r * nM + x] = t - u;
   }
 }
 
 // R2 += L for the four index orders of every (i<=j, a<=b) of the block.
-__global__ void ladder_scatter_kernel(const double* __restrict__ Xp, const double* __restrict__ Xm, int o, int v,
-                                      const int2* __restrict__ ijP, const int2* __restrict__ abP, int64_t nij_p,
-                                      int64_t rP0, int64_t nrP, int64_t rM0, int64_t nrM, double* __restrict__ R2) {
-  const int64_t tot = nij_p * nrP;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t p = t / nrP, r = t - p * nrP;
-    const int2 ij = ijP[p], ab = abP[rP0 + r];
-    const int i = ij.x, j = ij.y, a = ab.x, b = ab.y;
-    const double xp = Xp[p * nrP + r];
+__global__ void __launch_bounds__(256) ladder_scatter_kernel(const double* __restrict__ Xp,
+                                                             const double* __restrict__ Xm, int o, int v,
+                                                             const int2* __restrict__ ijP,
+                                                             const int2* __restrict__ abP, int nij_p, int rP0, int nrP,
+                                                             int rM0, int nrM, double* __restrict__ R2) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= nrP) return;
+  const int2 ab = abP[rP0 + r];
+  const int a = ab.x, b = ab.y;
+  const int64_t vv = (int64_t)v * v, oab = (int64_t)a * v + b, oba = (int64_t)b * v + a;
+  // position in the (a<b) list, row-major
+  const int64_t rm = (int64_t)a * v - (int64_t)a * (a + 1) / 2 + (b - a - 1) - rM0;
+  for (int p = blockIdx.y; p < nij_p; p += gridDim.y) {
+    const int2 ij = ijP[p];
+    const int i = ij.x, j = ij.y;
+    const double xp = Xp[(int64_t)p * nrP + r];
     double xm = 0.0;
     if (i < j && a < b) {
-      // positions in the (i<j) and (a<b) lists, both row-major
       const int64_t pm = (int64_t)i * o - (int64_t)i * (i + 1) / 2 + (j - i - 1);
-      const int64_t rm = (int64_t)a * v - (int64_t)a * (a + 1) / 2 + (b - a - 1) - rM0;
       xm = Xm[pm * nrM + rm];
     }
-    const int64_t vv = (int64_t)v * v;
-    R2[((int64_t)i * o + j) * vv + (int64_t)a * v + b] += xp + xm;
-    if (a != b) R2[((int64_t)i * o + j) * vv + (int64_t)b * v + a] += xp - xm;
-    if (i != j) R2[((int64_t)j * o + i) * vv + (int64_t)a * v + b] += xp - xm;
-    if (i != j && a != b) R2[((int64_t)j * o + i) * vv + (int64_t)b * v + a] += xp + xm;
+    double* r1 = R2 + ((int64_t)i * o + j) * vv;
+    double* r2 = R2 + ((int64_t)j * o + i) * vv;
+    r1[oab] += xp + xm;
+    if (a != b) r1[oba] += xp - xm;
+    if (i != j) r2[oab] += xp - xm;
+    if (i != j && a != b) r2[oba] += xp + xm;
   }
+}
+
+// grid of a (columns, rows) walk by 256 threads: about 24 blocks per SM
+dim3 grid_rows(int64_t cols, int64_t rows) {
+  const int64_t x = std::max<int64_t>(1, (cols + 255) / 256);
+  return dim3((unsigned)x, (unsigned)std::max<int64_t>(1, std::min<int64_t>(rows, std::min<int64_t>(32768, (152 * 24 + x - 1) / x))));
 }
 
 int grid_for(int64_t n, int threads = 256) {
@@ -503,7 +533,7 @@ void make_mp2_guess(fcc_ctx* c) {
   const int64_t o = c->o, v = c->v;
   FCC_CUDA(cudaMemsetAsync(c->t1.p, 0, sizeof(double) * o * v, s));
   einsum1(1.0, "iajb->ijab", rm(c->ovov.p, {o, v, o, v}), 0.0, rm(c->t2.p, {o, o, v, v}), s);
-  divide_d2_kernel<<<grid_for(o * o * v * v), 256, 0, s>>>(c->t2.p, c->eps.p, (int)o, (int)v);
+  divide_d2_kernel<<<grid_for(o * o * v * 32), RED_THREADS, 0, s>>>(c->t2.p, c->eps.p, (int)o, (int)v);
   FCC_CHECK_LAUNCH();
 }
 
@@ -512,7 +542,7 @@ double cc_energy(fcc_ctx* c, const double* t1, const double* t2) {
   energy_kernel<<<RED_BLOCKS, RED_THREADS, 0, s>>>((int)c->o, (int)c->v, t2, t1, c->Lt.p, c->red.p);
   FCC_CHECK_LAUNCH();
   double* out = c->red.p + RED_BLOCKS * NPART;
-  finish_reduce_kernel<<<1, 32, 0, s>>>(c->red.p, RED_BLOCKS, 2, out);
+  finish_reduce_kernel<<<1, 32 * NPART, 0, s>>>(c->red.p, RED_BLOCKS, 2, out);
   FCC_CHECK_LAUNCH();
   double h[2];
   FCC_CUDA(cudaMemcpyAsync(h, out, sizeof(h), cudaMemcpyDeviceToHost, s));
@@ -525,7 +555,7 @@ double mp2_energy(fcc_ctx* c) {
   mp2_energy_kernel<<<RED_BLOCKS, RED_THREADS, 0, s>>>((int)c->o, (int)c->v, c->ovov.p, c->eps.p, c->red.p);
   FCC_CHECK_LAUNCH();
   double* out = c->red.p + RED_BLOCKS * NPART;
-  finish_reduce_kernel<<<1, 32, 0, s>>>(c->red.p, RED_BLOCKS, 2, out);
+  finish_reduce_kernel<<<1, 32 * NPART, 0, s>>>(c->red.p, RED_BLOCKS, 2, out);
   FCC_CHECK_LAUNCH();
   double h[2];
   FCC_CUDA(cudaMemcpyAsync(h, out, sizeof(h), cudaMemcpyDeviceToHost, s));
@@ -603,9 +633,9 @@ void residual(fcc_ctx* c) {
   {
     const int64_t nP = v * (v + 1) / 2, nM = v * (v - 1) / 2;
     const int64_t nijP = o * (o + 1) / 2, nijM = o * (o - 1) / 2;
-    build_tpm_kernel<<<grid_for(nijP * nP + nijM * nM), 256, 0, s>>>(c->t2.p, (int)o, (int)v, c->pairP_o.p,
-                                                                    c->pairM_o.p, c->pairP_v.p, c->pairM_v.p, nP, nM,
-                                                                    nijP, nijM, c->Tp.p, c->Tm.p);
+    build_tpm_kernel<<<grid_rows(nP, nijP + nijM), 256, 0, s>>>(c->t2.p, (int)o, (int)v, c->pairP_o.p, c->pairM_o.p,
+                                                                c->pairP_v.p, c->pairM_v.p, (int)nP, (int)nM,
+                                                                (int)nijP, (int)nijM, c->Tp.p, c->Tm.p);
     FCC_CHECK_LAUNCH();
     // Tp and Tm are the A operands of every block's ladder product: packed once
     KeepPackedA keep(tc_engine(), c->Tp.p, c->Tm.p);
@@ -674,15 +704,17 @@ void residual(fcc_ctx* c) {
       }
       const int64_t rP0 = startP(a0), nrP = startP(a0 + na) - rP0;
       const int64_t rM0 = startM(a0), nrM = startM(a0 + na) - rM0;
-      build_wpm_kernel<<<grid_for(nrP * nP + nrM * nM), 256, 0, s>>>(c->Wslab.p, (int)v, (int)a0, vb, c->pairP_v.p,
-                                                                    c->pairM_v.p, rP0, nrP, rM0, nrM, c->pairP_v.p,
-                                                                    c->pairM_v.p, nP, nM, c->Wp.p, c->Wm.p);
+      build_wpm_kernel<<<grid_rows(nP, nrP + nrM), 256, 0, s>>>(c->Wslab.p, (int)v, (int)a0, (int)vb, c->pairP_v.p,
+                                                                c->pairM_v.p, (int)rP0, (int)nrP, (int)rM0, (int)nrM,
+                                                                c->pairP_v.p, c->pairM_v.p, (int)nP, (int)nM, c->Wp.p,
+                                                                c->Wm.p);
       FCC_CHECK_LAUNCH();
       einsum(1.0, "pq,rq->pr", rm(c->Tp.p, {nijP, nP}), rm(c->Wp.p, {nrP, nP}), 0.0, rm(c->LXp.p, {nijP, nrP}), s);
       if (nijM > 0 && nrM > 0)
         einsum(1.0, "pq,rq->pr", rm(c->Tm.p, {nijM, nM}), rm(c->Wm.p, {nrM, nM}), 0.0, rm(c->LXm.p, {nijM, nrM}), s);
-      ladder_scatter_kernel<<<grid_for(nijP * nrP), 256, 0, s>>>(c->LXp.p, c->LXm.p, (int)o, (int)v, c->pairP_o.p,
-                                                                c->pairP_v.p, nijP, rP0, nrP, rM0, nrM, c->r2.p);
+      ladder_scatter_kernel<<<grid_rows(nrP, nijP), 256, 0, s>>>(c->LXp.p, c->LXm.p, (int)o, (int)v, c->pairP_o.p,
+                                                                 c->pairP_v.p, (int)nijP, (int)rP0, (int)nrP, (int)rM0,
+                                                                 (int)nrM, c->r2.p);
       FCC_CHECK_LAUNCH();
     }
   }
@@ -838,28 +870,20 @@ int ccsd_run(fcc_ctx* c, const fcc_opts* opt, fcc_iter_stats* log, int32_t log_c
     update_kernel<<<RED_BLOCKS, RED_THREADS, 0, s>>>(rank, T, R, c->eps.p, (int)o, (int)v, dst, errs, errd, others,
                                                      rank == 4 ? c->Lt.p : nullptr, t1new, c->red.p);
     FCC_CHECK_LAUNCH();
-    finish_reduce_kernel<<<1, 32, 0, s>>>(c->red.p, RED_BLOCKS, 2 + others.n, dout);
+    finish_reduce_kernel<<<1, 32 * NPART, 0, s>>>(c->red.p, RED_BLOCKS, 3 + others.n, dout);
     FCC_CHECK_LAUNCH();
-    int nself = 0;
-    if (diis) {
-      selfdot_kernel<<<RED_BLOCKS, RED_THREADS, 0, s>>>(len, errs, errd, c->red.p);
-      FCC_CHECK_LAUNCH();
-      finish_reduce_kernel<<<1, 32, 0, s>>>(c->red.p, RED_BLOCKS, 1, dout + 2 + MAX_DIIS);
-      FCC_CHECK_LAUNCH();
-      nself = 1;
-    }
-    FCC_CUDA(cudaMemcpyAsync(hred, dout, sizeof(double) * (2 + MAX_DIIS + nself), cudaMemcpyDeviceToHost, s));
+    FCC_CUDA(cudaMemcpyAsync(hred, dout, sizeof(double) * NPART, cudaMemcpyDeviceToHost, s));
     FCC_CUDA(cudaStreamSynchronize(s));
     *out_sumsq = hred[0];
     *out_energy = hred[1];
     if (diis) {
       ds.valid[target] = 1;
       ds.age[target] = ++ds.counter;
-      ds.norm2[target] = hred[2 + MAX_DIIS];
-      ds.dot[target][target] = hred[2 + MAX_DIIS];
+      ds.norm2[target] = hred[2];
+      ds.dot[target][target] = hred[2];
       for (size_t q = 0; q < other_ids.size(); ++q) {
-        ds.dot[target][other_ids[q]] = hred[2 + q];
-        ds.dot[other_ids[q]][target] = hred[2 + q];
+        ds.dot[target][other_ids[q]] = hred[3 + q];
+        ds.dot[other_ids[q]][target] = hred[3 + q];
       }
     }
     *cur = dst;
@@ -891,7 +915,7 @@ int ccsd_run(fcc_ctx* c, const fcc_opts* opt, fcc_iter_stats* log, int32_t log_c
     extrapolate_kernel<<<RED_BLOCKS, RED_THREADS, 0, s>>>(rank, (int)o, (int)v, sl, dcoef.p, outbuf.p,
                                                           rank == 4 ? c->Lt.p : nullptr, t1new, c->red.p);
     FCC_CHECK_LAUNCH();
-    finish_reduce_kernel<<<1, 32, 0, s>>>(c->red.p, RED_BLOCKS, 2, dout);
+    finish_reduce_kernel<<<1, 32 * NPART, 0, s>>>(c->red.p, RED_BLOCKS, 2, dout);
     FCC_CHECK_LAUNCH();
     int st = 0;
     FCC_CUDA(cudaMemcpyAsync(hred, dout, sizeof(double) * 2, cudaMemcpyDeviceToHost, s));

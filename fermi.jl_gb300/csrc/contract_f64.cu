@@ -244,6 +244,28 @@ __global__ void splitk_reduce_kernel(const double* __restrict__ partial, int spl
   }
 }
 
+// The same for few outputs and many slices: 32 outputs per block, eight warps
+// over interleaved slices, added in a fixed order.
+__global__ void __launch_bounds__(256) splitk_reduce_few_kernel(const double* __restrict__ partial, int splits,
+                                                                double* __restrict__ C, CtrDesc d) {
+  __shared__ double part[8][32];
+  const int x = threadIdx.x & 31, g = threadIdx.x >> 5;
+  const int64_t MN = d.M * d.N, t = (int64_t)blockIdx.x * 32 + x;
+  double s = 0.0;
+  if (t < MN) {
+#pragma unroll 4
+    for (int z = g; z < splits; z += 8) s += partial[(int64_t)z * MN + t];
+  }
+  part[g][x] = s;
+  __syncthreads();
+  if (g != 0 || t >= MN) return;
+#pragma unroll
+  for (int q = 1; q < 8; ++q) s += part[q][x];
+  const uint32_t m = (uint32_t)t / (uint32_t)d.N, n = (uint32_t)t - m * (uint32_t)d.N;
+  f64_store(C + off3(m, d.M2, d.M3, d.c_m1, d.c_m2, d.c_m3) + off3(n, d.N2, d.N3, d.c_n1, d.c_n2, d.c_n3), s,
+            d.alpha, d.beta);
+}
+
 // Small contractions: a block of four warps per 16 x 16 output tile (and K
 // range), the k-steps of four dealt to the warps in turn, operands read
 // straight into the fragments of m8n8k4, the warps' sums added in shared
@@ -354,14 +376,14 @@ __global__ void gemv_f64_kernel(const double* __restrict__ A, const double* __re
   }
 }
 
-// N == 1 with the rows adjacent in memory (unit stride along m): 64 rows per
-// block, lanes along the rows so that reads coalesce, four groups of warps
-// over interleaved k, summed in a fixed order.
+// N == 1 with the rows adjacent in memory (unit stride along m): 32 rows per
+// block, lanes along the rows so that reads coalesce, eight warps over
+// interleaved k, summed in a fixed order.
 __global__ void __launch_bounds__(256) gemv_cols_f64_kernel(const double* __restrict__ A, const double* __restrict__ B,
                                                             double* __restrict__ C, CtrDesc d) {
-  __shared__ double part[4][64];
-  const int x = threadIdx.x & 63, g = threadIdx.x >> 6;
-  const int64_t m = (int64_t)blockIdx.x * 64 + x;
+  __shared__ double part[8][32];
+  const int x = threadIdx.x & 31, g = threadIdx.x >> 5;
+  const int64_t m = (int64_t)blockIdx.x * 32 + x;
   const int64_t bz = blockIdx.y;
   A += bz * d.a_b;
   B += bz * d.b_b;
@@ -369,14 +391,21 @@ __global__ void __launch_bounds__(256) gemv_cols_f64_kernel(const double* __rest
   double s = 0.0;
   if (m < d.M) {
     const double* a = A + off3(m, d.M2, d.M3, d.a_m1, d.a_m2, d.a_m3);
+    if (d.K2 >= d.K) {
 #pragma unroll 8
-    for (int64_t k = g; k < d.K; k += 4) s += a[off2(k, d.K2, d.a_k1, d.a_k2)] * B[off2(k, d.K2, d.b_k1, d.b_k2)];
+      for (int64_t k = g; k < d.K; k += 8) s = fma(a[k * d.a_k2], B[k * d.b_k2], s);
+    } else {
+#pragma unroll 4
+      for (int64_t k = g; k < d.K; k += 8)
+        s = fma(a[off2(k, d.K2, d.a_k1, d.a_k2)], B[off2(k, d.K2, d.b_k1, d.b_k2)], s);
+    }
   }
   part[g][x] = s;
   __syncthreads();
-  if (g == 0 && m < d.M)
-    f64_store(C + off3(m, d.M2, d.M3, d.c_m1, d.c_m2, d.c_m3), (part[0][x] + part[1][x]) + (part[2][x] + part[3][x]),
-              d.alpha, d.beta);
+  if (g != 0 || m >= d.M) return;
+#pragma unroll
+  for (int q = 1; q < 8; ++q) s += part[q][x];
+  f64_store(C + off3(m, d.M2, d.M3, d.c_m1, d.c_m2, d.c_m3), s, d.alpha, d.beta);
 }
 
 // out[i0 i1 i2 i3] = alpha in + beta out: a warp per run of up to 128 elements
@@ -475,7 +504,7 @@ void contract_f64_launch(const double* A, const double* B, double* C, const CtrD
   const int b_fast = (d.N3 > 1 ? d.b_n3 : d.b_n2) == 1 ? 1 : 0;
   if (d.N == 1) {
     if (a_fast && d.M >= 32) {
-      gemv_cols_f64_kernel<<<dim3((unsigned)((d.M + 63) / 64), (unsigned)d.batch), 256, 0, s>>>(A, B, C, d);
+      gemv_cols_f64_kernel<<<dim3((unsigned)((d.M + 31) / 32), (unsigned)d.batch), 256, 0, s>>>(A, B, C, d);
     } else {
       const int64_t blocks = std::min<int64_t>((d.M + 7) / 8, 152 * 16);
       gemv_f64_kernel<<<dim3((unsigned)blocks, (unsigned)d.batch), 256, 0, s>>>(A, B, C, d);
@@ -507,7 +536,11 @@ void contract_f64_launch(const double* A, const double* B, double* C, const CtrD
       contract_f64_small_kernel<<<dim3((unsigned)sm, (unsigned)sn, (unsigned)splits), 32 * SM_WARPS, 0, s>>>(
           A, B, C, d, (int)chunk, part);
       FCC_CHECK_LAUNCH();
-      splitk_reduce_kernel<<<rgrid, 256, 0, s>>>(part, (int)splits, C, d);
+      if (MN <= 152 * 32) {
+        splitk_reduce_few_kernel<<<(unsigned)((MN + 31) / 32), 256, 0, s>>>(part, (int)splits, C, d);
+      } else {
+        splitk_reduce_kernel<<<rgrid, 256, 0, s>>>(part, (int)splits, C, d);
+      }
     } else {
       contract_f64_small_kernel<<<dim3((unsigned)sm, (unsigned)sn, (unsigned)d.batch), 32 * SM_WARPS, 0, s>>>(
           A, B, C, d, 0, nullptr);
@@ -561,6 +594,18 @@ void tensor_axpby_launch(const TView& in, const TView& out, double alpha, double
     dim[k] = out.dim[ord[k]];
     si[k] = in.str[ord[k]];
     so[k] = out.str[ord[k]];
+  }
+  // neighbouring indices that are contiguous in both tensors become one
+  for (int k = 2; k >= 0; --k) {
+    int n = k + 1;                       // the next slower non-unit index is k
+    if (dim[k] == 1) continue;
+    if (dim[n] > 1 && si[k] == dim[n] * si[n] && so[k] == dim[n] * so[n] && dim[k] * dim[n] < (int64_t(1) << 31)) {
+      dim[n] *= dim[k];
+      for (int q = k; q > 0; --q) { dim[q] = dim[q - 1]; si[q] = si[q - 1]; so[q] = so[q - 1]; }
+      dim[0] = 1;
+      si[0] = so[0] = 0;
+      ++k;                               // what moved into place k is looked at next
+    }
   }
   // the source's fastest index, if it is another one than the output's
   int x = 3;

@@ -59,11 +59,22 @@ __global__ void gamma_part_kernel(const double* __restrict__ b, const double* __
   part[(int64_t)blockIdx.y * Q + q] = s0 + s1;
 }
 
-__global__ void gamma_sum_kernel(const double* __restrict__ part, int64_t Q, int nchunks, double* __restrict__ gam) {
-  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= Q) return;
+// 32 values per block, eight warps over interleaved chunks, a fixed order
+__global__ void __launch_bounds__(256) gamma_sum_kernel(const double* __restrict__ part, int64_t Q, int nchunks,
+                                                        double* __restrict__ gam) {
+  __shared__ double sh[8][32];
+  const int x = threadIdx.x & 31, g = threadIdx.x >> 5;
+  const int64_t q = (int64_t)blockIdx.x * 32 + x;
   double s = 0.0;
-  for (int c = 0; c < nchunks; ++c) s += part[(int64_t)c * Q + q];
+  if (q < Q) {
+#pragma unroll 4
+    for (int c = g; c < nchunks; c += 8) s += part[(int64_t)c * Q + q];
+  }
+  sh[g][x] = s;
+  __syncthreads();
+  if (g != 0 || q >= Q) return;
+#pragma unroll
+  for (int w = 1; w < 8; ++w) s += sh[w][x];
   gam[q] = s;
 }
 
@@ -131,7 +142,7 @@ void coulomb(fcc_scf* s) {
   gamma_part_kernel<<<dim3((unsigned)qblocks, (unsigned)nchunks), GAMMA_THREADS, 0, s->stream>>>(
       s->b.p, s->D.p, Q, R, rows_per, s->gpart.p);
   FCC_CHECK_LAUNCH();
-  gamma_sum_kernel<<<(unsigned)qblocks, GAMMA_THREADS, 0, s->stream>>>(s->gpart.p, Q, (int)nchunks, s->gam.p);
+  gamma_sum_kernel<<<(unsigned)((Q + 31) / 32), 256, 0, s->stream>>>(s->gpart.p, Q, (int)nchunks, s->gam.p);
   FCC_CHECK_LAUNCH();
   FCC_CUDA(cudaMemcpyAsync(s->F.p, s->H.p, sizeof(double) * R, cudaMemcpyDeviceToDevice, s->stream));
   fcc::einsum(2.0, "Qr,Q->r", cm(s->b.p, {Q, R}), cm(s->gam.p, {Q}), 1.0, cm(s->F.p, {R}), s->stream);

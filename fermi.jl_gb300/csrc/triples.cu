@@ -153,12 +153,18 @@ __global__ void __launch_bounds__(EB) triples_energy_f64_kernel(const double* __
   }
 }
 
-__global__ void sum_kernel(const double* part, int n, double* out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double s = 0.0;
-    for (int b = 0; b < n; ++b) s += part[b];
-    *out = s;
-  }
+// sum of n values by one block, a fixed order
+__global__ void __launch_bounds__(1024) sum_kernel(const double* part, int n, double* out) {
+  __shared__ double sh[32];
+  double s = 0.0;
+#pragma unroll 4
+  for (int b = threadIdx.x; b < n; b += 1024) s += part[b];
+  s = warp_sum(s);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  s = warp_sum(sh[threadIdx.x]);
+  if (threadIdx.x == 0) *out = s;
 }
 
 }  // namespace
@@ -249,7 +255,7 @@ double triples_fp64(fcc_ctx* c, const std::vector<int3>* subset, std::vector<dou
       part.zero(s);
       build_w(t.x, t.y, t.z, 1);
       energy(t.x, t.y, t.z, 1);
-      sum_kernel<<<1, 1, 0, s>>>(part.p, (int)(o * ntiles), out.p);
+      sum_kernel<<<1, 1024, 0, s>>>(part.p, (int)(o * ntiles), out.p);
       FCC_CHECK_LAUNCH();
       FCC_CUDA(cudaMemcpyAsync(&(*each)[q], out.p, sizeof(double), cudaMemcpyDeviceToHost, s));
     }
@@ -264,7 +270,7 @@ double triples_fp64(fcc_ctx* c, const std::vector<int3>* subset, std::vector<dou
           energy(i, j, k0, nk);
         }
   }
-  sum_kernel<<<1, 1, 0, s>>>(part.p, (int)(o * ntiles), out.p);
+  sum_kernel<<<1, 1024, 0, s>>>(part.p, (int)(o * ntiles), out.p);
   FCC_CHECK_LAUNCH();
   double et = 0.0;
   FCC_CUDA(cudaMemcpyAsync(&et, out.p, sizeof(double), cudaMemcpyDeviceToHost, s));
