@@ -685,7 +685,7 @@ void residual(fcc_ctx* c) {
         ep.N = vb * v;
         ep.ms1 = vb * v;   // W[(a, c)][(b, d)]
         ep.ns1 = 1;
-        ep.alpha = 1.0; ep.beta = 0.0; ep.C = c->Wslab.p; ep.mode = EPI_F64;
+        ep.alpha = 1.0; ep.beta = 0.0; ep.C = c->Wslab.p;
         const int64_t r0 = a0 * v;
         if (exact) {
           ep.work = 2.0 * (double)ep.M * (double)ep.N * (double)Q * oz_pairs(lv);

@@ -770,7 +770,7 @@ void run_tc(TcEngine* tc, OzLevel lv, double alpha, const TView& A, const TView&
     ep.M = M; ep.N = N;
     ep.md2 = gm[1].dim; ep.md3 = gm[2].dim; ep.ms1 = gm[0].s[2]; ep.ms2 = gm[1].s[2]; ep.ms3 = gm[2].s[2];
     ep.nd2 = gn[1].dim; ep.nd3 = gn[2].dim; ep.ns1 = gn[0].s[2]; ep.ns2 = gn[1].s[2]; ep.ns3 = gn[2].s[2];
-    ep.alpha = alpha; ep.beta = beta; ep.C = C.p; ep.mode = EPI_F64;
+    ep.alpha = alpha; ep.beta = beta; ep.C = C.p;
     ep.work = 2.0 * (double)M * (double)N * (double)K * oz_pairs(lv);
     gemm_oz(pA, M, eA, tc->bufB.p, N, tc->exB.p, Kpad, lv, ep, tc->ozws, tc->err, s);
     tc->tc_calls++;
@@ -802,7 +802,7 @@ void run_tc(TcEngine* tc, OzLevel lv, double alpha, const TView& A, const TView&
   ep.M = M; ep.N = N;
   ep.md2 = gm[1].dim; ep.md3 = gm[2].dim; ep.ms1 = gm[0].s[2]; ep.ms2 = gm[1].s[2]; ep.ms3 = gm[2].s[2];
   ep.nd2 = gn[1].dim; ep.nd3 = gn[2].dim; ep.ns1 = gn[0].s[2]; ep.ns2 = gn[1].s[2]; ep.ns3 = gn[2].s[2];
-  ep.alpha = alpha; ep.beta = beta; ep.C = C.p; ep.mode = EPI_F64;
+  ep.alpha = alpha; ep.beta = beta; ep.C = C.p;
   ep.work = 2.0 * (double)M * (double)N * (double)K * sc.P;
   ep.no_loads = tc->no_loads_once;
   tc->no_loads_once = 0;

@@ -119,24 +119,16 @@ inline unsigned pack_walk_grid(const PackWalk& w, int64_t R) {
   return (unsigned)std::max<int64_t>(1, std::min<int64_t>((R * w.nseg + upb - 1) / upb, 152 * 32));
 }
 
-// Output scatter of the GEMM: element (m, n) goes to
-// C[m1*ms1 + m2*ms2 + m3*ms3 + n1*ns1 + n2*ns2 + n3*ns3] as
-//   EPI_F64 / EPI_F32: alpha * acc + beta * C (atomic add when split over K);
-//   EPI_SPLIT: the split pieces of alpha * acc written at offsets p * piece
-//              (levels per `code`, P pieces), i.e. straight into the packed
-//              operand of a following GEMM.
-enum { EPI_F64 = 0, EPI_F32 = 1, EPI_SPLIT = 2 };
+// Output scatter of the GEMMs: element (m, n) goes to the FP64 value
+// C[m1*ms1 + m2*ms2 + m3*ms3 + n1*ns1 + n2*ns2 + n3*ns3] as alpha * acc + beta * C
+// (atomic: reduced into C by several K slices).
 struct EpiMap {
   int64_t M = 0, N = 0;
   int64_t md2 = 1, md3 = 1, ms1 = 0, ms2 = 0, ms3 = 0;
   int64_t nd2 = 1, nd3 = 1, ns1 = 0, ns2 = 0, ns3 = 0;
   double alpha = 1.0, beta = 0.0;
   void* C = nullptr;
-  int mode = EPI_F64;
   int atomic = 0;
-  int64_t piece = 0;
-  int P = 3;
-  uint32_t code = 0;
   double work = 0.0;   // algorithmic BF16 flops for the timing log (0: use the padded count)
   int no_loads = 0;    // test hook: the producer issues no TMA loads, so the bounded waits give up
 };
@@ -164,8 +156,6 @@ void gemm_bf16x3(const __nv_bfloat16* A, int64_t a_rows, int64_t a_row0, const _
 // 2-D TMA map over a row-major [rows][cols] BF16 array, boxes of 64 columns
 // (one 128-byte swizzle atom) x box_rows rows; cols must be a multiple of 64.
 CUtensorMap tma_map_bf16(const __nv_bfloat16* base, int64_t rows, int64_t cols, int box_rows);
-// C = beta * C over an epilogue map (before a GEMM adds into C atomically)
-void scale_output(const EpiMap& ep, double beta, cudaStream_t s);
 
 // Exact-slice products (the Ozaki scheme: Ozaki, Ogita, Oishi & Rump, Numer.
 // Algorithms 59, 95 (2012); on tensor cores: Mukunoki et al., ISC 2020).
@@ -214,7 +204,7 @@ inline double oz_pairs(OzLevel lv) {
 // 2047: the row holds an infinity or NaN, and so will its products)
 int64_t oz_kpad(int64_t K);
 void pack_oz(const double* src, const PackSpec& ps, int S, int bits, __nv_bfloat16* dst, int* ex, cudaStream_t s);
-// FP64 epilogue (EPI_F64) of the exact-slice product over packed operands;
+// exact-slice product over packed operands, written to ep;
 // ws holds the partial results of products cut into several jobs
 void gemm_oz(const __nv_bfloat16* A, int64_t a_rows, const int* exA, const __nv_bfloat16* B, int64_t b_rows,
              const int* exB, int64_t Kpad, OzLevel lv, const EpiMap& ep, DBuf<double>& ws, int* err, cudaStream_t s);

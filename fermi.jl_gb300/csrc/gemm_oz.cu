@@ -150,17 +150,6 @@ __device__ __forceinline__ void ff_add2(uint64_t& hi, uint64_t& lo, uint64_t v, 
   hi = h;
 }
 
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-}
-
 // (hi + lo) * 2^e as one FP64 number, rounded once, by integer arithmetic: lo
 // is turned into units of the 53-bit last place of hi (at most 2^29, one
 // float-to-integer conversion) and added to the bit pattern of hi.  The FP64
@@ -582,7 +571,6 @@ OzLevel oz_level(int groups) {
 void gemm_oz(const __nv_bfloat16* A, int64_t a_rows, const int* exA, const __nv_bfloat16* B, int64_t b_rows,
              const int* exB, int64_t Kpad, OzLevel lv, const EpiMap& ep, DBuf<double>& ws, int* err, cudaStream_t s) {
   if (ep.M <= 0 || ep.N <= 0) return;
-  if (ep.mode != EPI_F64) fail(FCC_ERR_BAD_ARG, "exact-slice products write FP64 only");
   if (lv.S < 1 || lv.S > OZ_MAXS || lv.G < 2 || lv.G > lv.S + 2 || (lv.bits != 6 && lv.bits != 8)) fail(FCC_ERR_BAD_ARG, "bad exact-slice level");
   if (Kpad <= 0 || Kpad % OZ_BK || Kpad > (1 << 27)) fail(FCC_ERR_BAD_ARG, "bad padded K");
   if (a_rows < ep.M || b_rows < ep.N) fail(FCC_ERR_BAD_ARG, "packed operands smaller than the output");

@@ -154,7 +154,9 @@ __global__ void __launch_bounds__(T3_THREADS, 1) gemm_t3_kernel(const __grid_con
    if (elect_one()) {
     // ---------------- MMA issuer
     constexpr uint32_t idesc = idesc_bf16(T3_BM, BN);
-    int it = 0, lt = 0;
+    const uint64_t ad0 = sw128_desc(smem_u32(sA)), bd0 = sw128_desc(smem_u32(sB));
+    uint32_t st = 0, ph = 0, peek = 0;
+    int lt = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x, ++lt) {
       const int g = t3_tile(t, tm, tn, P.nk).g;
@@ -164,23 +166,23 @@ __global__ void __launch_bounds__(T3_THREADS, 1) gemm_t3_kernel(const __grid_con
       if (!mbar_wait(smem_u32(&acce_bar[b]), ((lt >> 1) & 1) ^ 1)) { atomicExch(&abort_flag, 1); break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t dcol = tmem + (uint32_t)(b * Cfg::TMEM_COLS);
-      for (int x = 0; x < total; ++x, ++it) {
-        const int st = it % Cfg::STAGES;
-        const uint32_t ph = (it / Cfg::STAGES) & 1;
-        if (!mbar_wait(smem_u32(&full_bar[st]), ph)) { atomicExch(&abort_flag, 1); ok = false; break; }
+      for (int x = 0; x < total; ++x) {
+        // the next stage's barrier is read between the MMAs of a stage, while
+        // the tensor pipe has work queued
+        if (!peek && !mbar_wait(smem_u32(&full_bar[st]), ph)) { atomicExch(&abort_flag, 1); ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint64_t ad = sw128_desc(smem_u32(sA + st * Cfg::A_BYTES));
-        const uint64_t bd = sw128_desc(smem_u32(sB + st * Cfg::B_BYTES));
-#pragma unroll
-        for (int q = 0; q < T3_BK / 16; ++q) {
-          const uint32_t acc = (x > 0 || q > 0) ? 1u : 0u;
-          asm volatile(
-              "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-              " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(dcol),
-              "l"(ad + (uint64_t)(2 * q)), "l"(bd + (uint64_t)(2 * q)), "r"(idesc), "r"(acc)
-              : "memory");
-        }
+        const uint64_t ad = ad0 + (uint64_t)(st * (Cfg::A_BYTES >> 4));
+        const uint64_t bd = bd0 + (uint64_t)(st * (Cfg::B_BYTES >> 4));
+        uint32_t st2 = st + 1, ph2 = ph;
+        if (st2 == Cfg::STAGES) { st2 = 0; ph2 ^= 1; }
+        mma_bf16(dcol, ad, bd, idesc, x > 0 ? 1u : 0u);
+        peek = mbar_test(smem_u32(&full_bar[st2]), ph2);
+        mma_bf16(dcol, ad + 2, bd + 2, idesc, 1u);
+        mma_bf16(dcol, ad + 4, bd + 4, idesc, 1u);
+        mma_bf16(dcol, ad + 6, bd + 6, idesc, 1u);
         tc_commit(smem_u32(&empty_bar[st]));
+        st = st2;
+        ph = ph2;
       }
       if (!ok) break;
       tc_commit(smem_u32(&accf_bar[b]));
@@ -220,15 +222,7 @@ __global__ void __launch_bounds__(T3_THREADS, 1) gemm_t3_kernel(const __grid_con
       for (int c0 = 0; c0 < BN; c0 += 32) {
         if (nb0 + c0 >= v) break;
         uint32_t r[32];
-        const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * Cfg::TMEM_COLS + c0);
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-            "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-              "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-              "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-            : "r"(taddr));
+        tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * Cfg::TMEM_COLS + c0), r);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         __syncwarp();
 #pragma unroll

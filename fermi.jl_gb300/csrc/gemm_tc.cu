@@ -175,15 +175,25 @@ __device__ __forceinline__ __nv_bfloat16 piece(const __nv_bfloat16 (&lv)[3], int
   return lev == 0 ? lv[0] : (lev == 1 ? lv[1] : lv[2]);
 }
 
+// Persistent: CTA b processes units b, b + gridDim.x, ...; unit u is K slice
+// u / tiles of output tile u % tiles (grouped_tile).  Two TMEM accumulators, so
+// the loads and MMAs of a unit run while the epilogue warps store the one
+// before: with one CTA per unit the store stage (up to 60 us a tile while it
+// issued FP64 instructions, even predicated off) added to every tile.  One
+// W-build launch at (H2O)8 (2888 x 23104, K = 672) 1.05 -> 0.28 ms, a ring
+// product (4864^3) 0.72 -> 0.43 ms.
 template <int BN>
 __global__ void __launch_bounds__(TC_THREADS, 1)
-    gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int64_t a_row0,
-                        int64_t b_row0, int num_k, int k_chunk, EpiMap ep, int* err) {
+    gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int a_row0,
+                        int b_row0, int num_k, int k_chunk, uint32_t tm, uint32_t tn, uint32_t units,
+                        const __grid_constant__ EpiMap ep, int* err) {
   using Cfg = TcCfg<BN>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[Cfg::STAGES];
   __shared__ __align__(8) uint64_t empty_bar[Cfg::STAGES];
-  __shared__ __align__(8) uint64_t acc_bar;
+  __shared__ __align__(8) uint64_t accf_bar[2];   // accumulator b holds a finished unit
+  __shared__ __align__(8) uint64_t acce_bar[2];   // accumulator b has been read out
+  __shared__ __align__(8) uint64_t done_bar;      // every issued MMA has completed
   __shared__ uint32_t tmem_holder;
   __shared__ int abort_flag;
   __shared__ float epi_tile[4][32][33];   // per epilogue warp: 32 x 32 transpose
@@ -192,19 +202,24 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   uint8_t* sA = smem;
   uint8_t* sB = smem + Cfg::STAGES * Cfg::A_BYTES;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t tiles = tm * tn;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < Cfg::STAGES; ++s) {
       mbar_init(smem_u32(&full_bar[s]), 1);
       mbar_init(smem_u32(&empty_bar[s]), 1);
     }
-    mbar_init(smem_u32(&acc_bar), 1);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(smem_u32(&accf_bar[b]), 1);
+      mbar_init(smem_u32(&acce_bar[b]), 4);   // one arrival per epilogue warp
+    }
+    mbar_init(smem_u32(&done_bar), 1);
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_holder)),
-                 "r"(BN)
+                 "r"(2 * BN)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -212,88 +227,97 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_holder;
-  uint32_t mt, nt;
-  grouped_tile(blockIdx.x, (uint32_t)((ep.M + BM - 1) / BM), (uint32_t)((ep.N + BN - 1) / BN), mt, nt);
-  const int64_t m0 = (int64_t)mt * BM;
-  const int64_t n0 = (int64_t)nt * BN;
-  // split-K: this CTA reduces k-tiles [kb, ke); partial sums are added atomically
-  const int kb = (int)blockIdx.z * k_chunk;
-  const int ke = min(num_k, kb + k_chunk);
-  const int nkt = max(0, ke - kb);
 
   if (warp == 0) {
-   if (elect_one()) {
-    // ---------------- TMA producer (none at all under the no_loads test hook:
-    // nothing is then in flight, and the MMA thread's bounded wait gives up)
-    for (int kt = 0; kt < (ep.no_loads ? 0 : nkt); ++kt) {
-      const int s = kt % Cfg::STAGES;
-      const uint32_t ph = (kt / Cfg::STAGES) & 1;
-      if (!mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1)) { atomicExch(&abort_flag, 1); break; }
-      if (*(volatile int*)&abort_flag) break;
-      const uint32_t fb = smem_u32(&full_bar[s]);
-      mbar_expect_tx(fb, Cfg::STAGE_BYTES);
-      tma_load_2d(smem_u32(sA + s * Cfg::A_BYTES), &tmA, (kb + kt) * BK, (int32_t)(a_row0 + m0), fb);
-      tma_load_2d(smem_u32(sB + s * Cfg::B_BYTES), &tmB, (kb + kt) * BK, (int32_t)(b_row0 + n0), fb);
-    }
-   }
-  } else if (warp == 1) {
-   if (elect_one()) {
-    // ---------------- MMA issuer (single thread)
-    constexpr uint32_t idesc = idesc_bf16(BM, BN);
-    bool ok = true;
-    for (int kt = 0; kt < nkt; ++kt) {
-      const int s = kt % Cfg::STAGES;
-      const uint32_t ph = (kt / Cfg::STAGES) & 1;
-      if (!mbar_wait(smem_u32(&full_bar[s]), ph)) { atomicExch(&abort_flag, 1); ok = false; break; }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint64_t ad = sw128_desc(smem_u32(sA + s * Cfg::A_BYTES));
-      const uint64_t bd = sw128_desc(smem_u32(sB + s * Cfg::B_BYTES));
-#pragma unroll
-      for (int kk = 0; kk < BK / 16; ++kk) {
-        const uint32_t acc = (kt > 0 || kk > 0) ? 1u : 0u;
-        asm volatile(
-            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-            " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
-            "l"(ad + (uint64_t)(2 * kk)), "l"(bd + (uint64_t)(2 * kk)), "r"(idesc), "r"(acc)
-            : "memory");
+    if (elect_one()) {
+      // ---------------- TMA producer (none at all under the no_loads test hook:
+      // nothing is then in flight, and the MMA thread's bounded wait gives up)
+      int it = 0, s = 0;
+      uint32_t ph = 0;
+      bool stop = ep.no_loads != 0;
+      for (uint32_t u = blockIdx.x; u < units && !stop; u += gridDim.x) {
+        uint32_t mt, nt;
+        grouped_tile(u % tiles, tm, tn, mt, nt);
+        const int kb = (int)(u / tiles) * k_chunk, ke = min(num_k, kb + k_chunk);
+        const int am = a_row0 + (int)mt * BM, bn = b_row0 + (int)nt * BN;
+        for (int k = kb; k < ke; ++k, ++it) {
+          if (!mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1)) { atomicExch(&abort_flag, 1); stop = true; break; }
+          const uint32_t fb = smem_u32(&full_bar[s]);
+          mbar_expect_tx(fb, Cfg::STAGE_BYTES);
+          tma_load_2d(smem_u32(sA + s * Cfg::A_BYTES), &tmA, k * BK, am, fb);
+          tma_load_2d(smem_u32(sB + s * Cfg::B_BYTES), &tmB, k * BK, bn, fb);
+          if (++s == Cfg::STAGES) { s = 0; ph ^= 1; }
+        }
+        if (*(volatile int*)&abort_flag) break;
       }
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                       smem_u32(&empty_bar[s]))
-                   : "memory");
+      // on an abort, wait (bounded) for the loads still in flight before the
+      // shared memory can be released
+      if (*(volatile int*)&abort_flag && !ep.no_loads) {
+        for (int q = max(0, it - Cfg::STAGES); q < it; ++q)
+          (void)mbar_wait(smem_u32(&full_bar[q % Cfg::STAGES]), (q / Cfg::STAGES) & 1);
+      }
     }
-    // signals the epilogue once every issued MMA has completed (also on abort)
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&acc_bar))
-                 : "memory");
-    (void)ok;
-   }
-  } else if (warp >= 2) {
-    // ---------------- epilogue: TMEM -> registers -> strided global stores
-    bool ok = mbar_wait(smem_u32(&acc_bar), 0);
-    ok = __all_sync(0xffffffffu, ok);
-    if (!ok) atomicExch(&abort_flag, 1);
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  } else if (warp == 1) {
+    if (elect_one()) {
+      // ---------------- MMA issuer: the next stage's barrier is read between
+      // the MMAs of a stage, while the tensor pipe has work queued
+      constexpr uint32_t idesc = idesc_bf16(BM, BN);
+      const uint64_t ad0 = sw128_desc(smem_u32(sA)), bd0 = sw128_desc(smem_u32(sB));
+      uint32_t s = 0, ph = 0, lt = 0, peek = 0;
+      bool ok = true;
+      for (uint32_t u = blockIdx.x; u < units && ok; u += gridDim.x, ++lt) {
+        const int kb = (int)(u / tiles) * k_chunk, nkt = min(num_k, kb + k_chunk) - kb;
+        const uint32_t b = lt & 1;
+        if (!mbar_wait(smem_u32(&acce_bar[b]), ((lt >> 1) & 1) ^ 1)) { atomicExch(&abort_flag, 1); break; }
+        const uint32_t dcol = tmem + b * BN;
+        for (int x = 0; x < nkt; ++x) {
+          if (!peek && !mbar_wait(smem_u32(&full_bar[s]), ph)) { atomicExch(&abort_flag, 1); ok = false; break; }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint64_t ad = ad0 + (uint64_t)(s * (Cfg::A_BYTES >> 4));
+          const uint64_t bd = bd0 + (uint64_t)(s * (Cfg::B_BYTES >> 4));
+          uint32_t s2 = s + 1, ph2 = ph;
+          if (s2 == Cfg::STAGES) { s2 = 0; ph2 ^= 1; }
+          mma_bf16(dcol, ad, bd, idesc, x > 0 ? 1u : 0u);
+          peek = mbar_test(smem_u32(&full_bar[s2]), ph2);
+          mma_bf16(dcol, ad + 2, bd + 2, idesc, 1u);
+          mma_bf16(dcol, ad + 4, bd + 4, idesc, 1u);
+          mma_bf16(dcol, ad + 6, bd + 6, idesc, 1u);
+          tc_commit(smem_u32(&empty_bar[s]));
+          s = s2;
+          ph = ph2;
+        }
+        if (!ok) break;
+        tc_commit(smem_u32(&accf_bar[b]));
+      }
+      // TMEM is freed only after every issued MMA has completed (also on an abort)
+      tc_commit(smem_u32(&done_bar));
+      if (!mbar_wait(smem_u32(&done_bar), 0)) atomicExch(&abort_flag, 1);
+    }
+  } else {
+    // ---------------- epilogue: TMEM -> transposed 32 x 32 blocks -> strided global stores
     const int q = warp & 3;              // TMEM lane quadrant this warp may access
-    const int row = q * 32 + lane;
-    const int64_t m = m0 + row;
-    const bool abort_now = __any_sync(0xffffffffu, *(volatile int*)&abort_flag != 0);
-    if (ok && !abort_now && nkt > 0) {
+    float (*tile)[33] = epi_tile[q];
+    const float alpha = (float)ep.alpha;
+    // 0: store; 1: reduce into C (no load; beta = 1 or several K slices); 2: add to beta C
+    const int mode = ep.atomic || ep.beta == 1.0 ? 1 : (ep.beta == 0.0 ? 0 : 2);
+    uint32_t lt = 0;
+    for (uint32_t u = blockIdx.x; u < units; u += gridDim.x, ++lt) {
+      uint32_t mt, nt;
+      grouped_tile(u % tiles, tm, tn, mt, nt);
+      const uint32_t b = lt & 1;
+      bool ok = mbar_wait(smem_u32(&accf_bar[b]), (lt >> 1) & 1);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok || __any_sync(0xffffffffu, *(volatile int*)&abort_flag != 0)) { atomicExch(&abort_flag, 1); break; }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const int64_t m0 = (int64_t)mt * BM + q * 32, n0 = (int64_t)nt * BN;
+      const int rows = (int)min((int64_t)32, ep.M - m0);
       // this lane's row offset; rows are broadcast to the warp below
-      int64_t crow = 0;
-      if (m < ep.M) crow = epi_row_off(ep, (uint32_t)m);
-      float (*tile)[33] = epi_tile[q];
+      const int64_t crow = lane < rows ? epi_row_off(ep, (uint32_t)(m0 + lane)) : 0;
 #pragma unroll 1
       for (int c0 = 0; c0 < BN; c0 += 32) {
         if (n0 + c0 >= ep.N) break;
         uint32_t r[32];
-        const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0;
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-            "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-              "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-              "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-            : "r"(taddr));
+        tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + b * BN + (uint32_t)c0, r);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         // transpose the warp's 32 x 32 block through shared memory so each
         // store instruction writes 32 consecutive columns of one row
@@ -303,79 +327,50 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         __syncwarp();
         const int64_t n = n0 + c0 + lane;
         const bool nok = n < ep.N;
-        int64_t coff = 0;
-        if (nok) coff = epi_col_off(ep, (uint32_t)n);
-        // all loads of the block first (independent, so they overlap), then
-        // the stores
-        // FP64 outputs with beta = 1 are reduced into C (red.add, no load);
-        // only other betas read C
-        const bool rmw = ep.beta != 0.0 && !ep.atomic && ep.mode != EPI_SPLIT &&
-                         !(ep.mode == EPI_F64 && ep.beta == 1.0);
-        double prev[32];
-        float prevf[32];
-        if (rmw) {
-#pragma unroll
+        double* dst = static_cast<double*>(ep.C) + (nok ? epi_col_off(ep, (uint32_t)n) : 0);
+        // The FP32 product becomes FP64 by integer arithmetic: an FP64
+        // instruction takes its pipe for 16 clk per warp.
+        if (mode == 0) {
+#pragma unroll 8
           for (int jr = 0; jr < 32; ++jr) {
             const int64_t roff = __shfl_sync(0xffffffffu, crow, jr);
-            const bool ok2 = nok && (m0 + q * 32 + jr) < ep.M;
-            prev[jr] = 0.0;
-            prevf[jr] = 0.0f;
-            if (ok2) {
-              if (ep.mode == EPI_F32) prevf[jr] = static_cast<const float*>(ep.C)[roff + coff];
-              else prev[jr] = static_cast<const double*>(ep.C)[roff + coff];
+            if (jr < rows && nok) dst[roff] = f32_to_f64_scaled(alpha * tile[jr][lane], 0, false);
+          }
+        } else if (mode == 1) {
+#pragma unroll 8
+          for (int jr = 0; jr < 32; ++jr) {
+            const int64_t roff = __shfl_sync(0xffffffffu, crow, jr);
+            if (jr < rows && nok) atomicAdd(dst + roff, f32_to_f64_scaled(alpha * tile[jr][lane], 0, false));
+          }
+        } else {
+#pragma unroll 1
+          for (int j0 = 0; j0 < 32; j0 += 8) {
+            double prev[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const int64_t roff = __shfl_sync(0xffffffffu, crow, j0 + j);
+              prev[j] = j0 + j < rows && nok ? dst[roff] : 0.0;
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const int64_t roff = __shfl_sync(0xffffffffu, crow, j0 + j);
+              if (j0 + j < rows && nok)
+                dst[roff] = f32_to_f64_scaled(alpha * tile[j0 + j][lane], 0, false) + ep.beta * prev[j];
             }
           }
         }
-#pragma unroll
-        for (int jr = 0; jr < 32; ++jr) {
-          const int64_t roff = __shfl_sync(0xffffffffu, crow, jr);
-          const int64_t mm = m0 + q * 32 + jr;
-          if (mm >= ep.M || !nok) continue;
-          const int64_t off = roff + coff;
-          if (ep.mode == EPI_F32) {
-            // FP32 output: FP32 arithmetic (the FP64 pipe is 1/64 rate on GB300)
-            float* dst = static_cast<float*>(ep.C) + off;
-            float fv = (float)ep.alpha * tile[jr][lane];
-            if (rmw) fv += (float)ep.beta * prevf[jr];
-            if (ep.atomic) atomicAdd(dst, fv);
-            else *dst = fv;
-            continue;
-          }
-          if (ep.mode == EPI_F64) {
-            // FP32 product, converted to FP64 by integer arithmetic (the FP64
-            // pipe, which F2F conversions use, is 1/64 rate on GB300)
-            double val = f32_to_f64_scaled((float)ep.alpha * tile[jr][lane], 0, false);
-            double* dst = static_cast<double*>(ep.C) + off;
-            if (ep.atomic || ep.beta == 1.0) atomicAdd(dst, val);
-            else if (rmw) *dst = val + ep.beta * prev[jr];
-            else *dst = val;
-            continue;
-          }
-          double val = (double)((float)ep.alpha * tile[jr][lane]);
-          if (rmw) val = (ep.beta == 1.0) ? prev[jr] + val : val + ep.beta * prev[jr];
-          if (ep.mode == EPI_SPLIT) {
-            __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(ep.C) + off;
-            __nv_bfloat16 lv[3];
-            split3(val, lv);
-            for (int p = 0; p < ep.P; ++p) dst[p * ep.piece] = piece(lv, (ep.code >> (2 * p)) & 3);
-          } else if (ep.mode == EPI_F32) {
-            float* dst = static_cast<float*>(ep.C) + off;
-            if (ep.atomic) atomicAdd(dst, (float)val);
-            else *dst = (float)val;
-          } else {
-            double* dst = static_cast<double*>(ep.C) + off;
-            if (ep.atomic) atomicAdd(dst, val);
-            else *dst = val;
-          }
-        }
       }
+      // the accumulator is free for the unit after next
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&acce_bar[b]));
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(BN) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * BN) : "memory");
   }
   if (threadIdx.x == 0 && abort_flag) atomicExch(err, 1);
 }
@@ -505,19 +500,13 @@ __global__ void pack_pad_kernel(PackSpec ps, __nv_bfloat16* __restrict__ dst) {
   }
 }
 
-// C = beta * C over an epilogue map (before split-K atomics).
-__global__ void scale_out_kernel(EpiMap ep, double beta) {
-  const int64_t total = ep.M * ep.N;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t m = t / ep.N, n = t - m * ep.N;
-    const int64_t m3 = m % ep.md3, qm = m / ep.md3, n3 = n % ep.nd3, qn = n / ep.nd3;
-    const int64_t off = (qm / ep.md2) * ep.ms1 + (qm % ep.md2) * ep.ms2 + m3 * ep.ms3 + (qn / ep.nd2) * ep.ns1 +
-                        (qn % ep.nd2) * ep.ns2 + n3 * ep.ns3;
-    if (ep.mode == EPI_F32) {
-      float* d = static_cast<float*>(ep.C) + off;
-      *d = beta == 0.0 ? 0.0f : (float)(beta * *d);
-    } else {
-      double* d = static_cast<double*>(ep.C) + off;
+// C = beta * C over an epilogue map (before split-K atomics): a row per block
+// in turn, columns along the threads.
+__global__ void __launch_bounds__(256) scale_out_kernel(EpiMap ep, double beta) {
+  for (int64_t n = (int64_t)blockIdx.x * 256 + threadIdx.x; n < ep.N; n += (int64_t)gridDim.x * 256) {
+    double* dst = static_cast<double*>(ep.C) + epi_col_off(ep, (uint32_t)n);
+    for (int64_t m = blockIdx.y; m < ep.M; m += gridDim.y) {
+      double* d = dst + epi_row_off(ep, (uint32_t)m);
       *d = beta == 0.0 ? 0.0 : beta * *d;
     }
   }
@@ -569,7 +558,7 @@ void launch_tc(const __nv_bfloat16* A, int64_t a_rows, int64_t a_row0, const __n
   const int num_k = (int)(Kp / BK);
   // split K across CTAs when the output has too few tiles to fill the GPU
   int splits = 1;
-  if (ep.mode != EPI_SPLIT && tm * tn < 152 && num_k >= 16)
+  if (tm * tn < 152 && num_k >= 16)
     splits = (int)std::min<int64_t>((152 + tm * tn - 1) / (tm * tn), num_k / 8);
   splits = std::max(1, std::min(splits, 64));
   const int chunk = (num_k + splits - 1) / splits;
@@ -577,16 +566,18 @@ void launch_tc(const __nv_bfloat16* A, int64_t a_rows, int64_t a_row0, const __n
   EpiMap e2 = ep;
   if (splits > 1) {
     if (ep.beta != 1.0) {   // C = beta * C before the partial sums are added
-      const int64_t tot = ep.M * ep.N;
-      scale_out_kernel<<<(unsigned)std::min<int64_t>((tot + 255) / 256, 152 * 16), 256, 0, s>>>(ep, ep.beta);
+      const int64_t x = std::min<int64_t>((ep.N + 255) / 256, 152 * 16);
+      const int64_t y = std::max<int64_t>(1, std::min<int64_t>(ep.M, 152 * 16 / x));
+      scale_out_kernel<<<dim3((unsigned)x, (unsigned)y), 256, 0, s>>>(ep, ep.beta);
       FCC_CHECK_LAUNCH();
     }
     e2.atomic = 1;
   }
-  if (tm * tn > 2147483647ll) fail(FCC_ERR_BAD_ARG, "tensor-core grid too large");
-  dim3 grid((unsigned)(tm * tn), 1u, (unsigned)splits);
+  const int64_t units = tm * tn * splits;
+  if (units >= (int64_t(1) << 31)) fail(FCC_ERR_BAD_ARG, "tensor-core grid too large");
   const int pidx = prof_begin(s);
-  gemm_bf16_tc_kernel<BN><<<grid, TC_THREADS, Cfg::SMEM, s>>>(ta, tb, a_row0, b_row0, num_k, chunk, e2, err);
+  gemm_bf16_tc_kernel<BN><<<(unsigned)std::min<int64_t>(units, 152), TC_THREADS, Cfg::SMEM, s>>>(
+      ta, tb, (int)a_row0, (int)b_row0, num_k, chunk, (uint32_t)tm, (uint32_t)tn, (uint32_t)units, e2, err);
   FCC_CHECK_LAUNCH();
   // executed BF16 flops (padded K included)
   prof_end(s, pidx, PROF_TC, ep.work > 0 ? ep.work : 2.0 * (double)ep.M * (double)ep.N * (double)Kp);
@@ -598,13 +589,6 @@ int64_t packed_kp(int64_t K, int P) { return ((P * K + BK - 1) / BK) * BK; }
 
 CUtensorMap tma_map_bf16(const __nv_bfloat16* base, int64_t rows, int64_t cols, int box_rows) {
   return make_map(base, rows, cols, box_rows);
-}
-
-void scale_output(const EpiMap& ep, double beta, cudaStream_t s) {
-  const int64_t tot = ep.M * ep.N;
-  if (tot <= 0) return;
-  scale_out_kernel<<<(unsigned)std::min<int64_t>((tot + 255) / 256, 152 * 16), 256, 0, s>>>(ep, beta);
-  FCC_CHECK_LAUNCH();
 }
 
 void pack_split(const double* src, const PackSpec& ps, __nv_bfloat16* dst, cudaStream_t s) {
@@ -642,7 +626,8 @@ void pack_split(const double* src, const PackSpec& ps, __nv_bfloat16* dst, cudaS
 void gemm_bf16x3(const __nv_bfloat16* A, int64_t a_rows, int64_t a_row0, const __nv_bfloat16* B, int64_t b_rows,
                  int64_t b_row0, int64_t Kp, const EpiMap& ep, int* err, cudaStream_t s) {
   if (ep.M <= 0 || ep.N <= 0) return;
-  if (Kp <= 0 || Kp % BK) fail(FCC_ERR_BAD_ARG, "bad packed K");
+  if (Kp <= 0 || Kp % BK || Kp >= (int64_t(1) << 31)) fail(FCC_ERR_BAD_ARG, "bad packed K");
+  if (a_rows >= (int64_t(1) << 31) || b_rows >= (int64_t(1) << 31)) fail(FCC_ERR_BAD_ARG, "packed operand too large");
   if (ep.N >= 256) launch_tc<256>(A, a_rows, a_row0, B, b_rows, b_row0, Kp, ep, err, s);
   else launch_tc<128>(A, a_rows, a_row0, B, b_rows, b_row0, Kp, ep, err, s);
 }
