@@ -6,13 +6,13 @@
 //
 // Weights are BF16 for the forward/backward products with FP32 master copies
 // updated by Adam.  Everything here is hand-written: the feature kernel, a
-// BF16 tensor-core GEMM (mma.sync m16n8k16, FP32 accumulation, deterministic
-// split-K) for the five layer products, an FP32 SIMT GEMM for the one-row
-// output-layer gradient, bias+GELU forward and backward,
-// the loss, bias-gradient reductions, Adam, and the inference kernel that
-// writes the guess into a context.
+// BF16 tensor-core GEMM (mma.sync m16n8k16, FP32 accumulation) for the layer
+// products, a split one for the weight gradients, bias+GELU forward, backward
+// passes that carry the output-layer and bias gradients along, the loss, Adam,
+// and the inference kernel that writes the guess into a context.
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <new>
@@ -36,74 +36,8 @@ __device__ __forceinline__ float gelu_grad(float x) {
   return 0.5f * (1.0f + erff(x * 0.70710678118654752f)) + x * 0.39894228040143268f * expf(-0.5f * x * x);
 }
 
-template <class T>
-__device__ __forceinline__ float ld(const T* p, int64_t i);
-template <>
-__device__ __forceinline__ float ld<float>(const float* p, int64_t i) { return p[i]; }
-template <>
-__device__ __forceinline__ float ld<__nv_bfloat16>(const __nv_bfloat16* p, int64_t i) { return __bfloat162float(p[i]); }
-
-// C[m][n] = alpha * sum_k A(m,k) B(k,n) + beta * C[m][n]; A(m,k) = A[m*sam + k*sak],
-// B(k,n) = B[k*sbk + n*sbn], C row-major with ldc.  64 x 64 tile, 16-deep K.
-template <class TA, class TB>
-__global__ void __launch_bounds__(256) sgemm_kernel(int M, int N, int K, float alpha, const TA* __restrict__ A,
-                                                    int64_t sam, int64_t sak, const TB* __restrict__ B, int64_t sbk,
-                                                    int64_t sbn, float beta, float* __restrict__ C, int64_t ldc) {
-  __shared__ float As[16][64 + 1], Bs[16][64 + 1];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < K; k0 += 16) {
-    for (int e = threadIdx.x; e < 64 * 16; e += 256) {
-      int mm = e / 16, kk = e % 16;
-      int m = m0 + mm, k = k0 + kk;
-      As[kk][mm] = (m < M && k < K) ? ld(A, (int64_t)m * sam + (int64_t)k * sak) : 0.0f;
-      int nn = e % 64, kb = e / 64;
-      int n = n0 + nn, k2 = k0 + kb;
-      Bs[kb][nn] = (n < N && k2 < K) ? ld(B, (int64_t)k2 * sbk + (int64_t)n * sbn) : 0.0f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < 16; ++kk) {
-      float a[4], b[4];
-#pragma unroll
-      for (int r = 0; r < 4; ++r) a[r] = As[kk][ty * 4 + r];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) b[c] = Bs[kk][tx * 4 + c];
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c] += a[r] * b[c];
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int r = 0; r < 4; ++r)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      int m = m0 + ty * 4 + r, n = n0 + tx * 4 + c;
-      if (m < M && n < N) {
-        float v = alpha * acc[r][c];
-        if (beta != 0.0f) v += beta * C[(int64_t)m * ldc + n];
-        C[(int64_t)m * ldc + n] = v;
-      }
-    }
-}
-
-template <class TA, class TB>
-void sgemm(int M, int N, int K, float alpha, const TA* A, int64_t sam, int64_t sak, const TB* B, int64_t sbk,
-           int64_t sbn, float beta, float* C, int64_t ldc, cudaStream_t s) {
-  dim3 grid((N + 63) / 64, (M + 63) / 64);
-  sgemm_kernel<TA, TB><<<grid, 256, 0, s>>>(M, N, K, alpha, A, sam, sak, B, sbk, sbn, beta, C, ldc);
-  FCC_CHECK_LAUNCH();
-}
-
-// ---- tensor-core GEMM of the network's products: operands rounded to BF16
-// (nearest, ties to even) when staged, mma.sync m16n8k16 with FP32
-// accumulation.  64 x 64 output tile, 32-deep K slab, four warps of 32 x 32.
-// With `splits` > 1 the K range is cut into slices whose FP32 partial tiles
-// are summed in slice order by hgemm_reduce_kernel (the gradient products
-// reduce over the whole batch, K = 65536, into a 128 x 128 output).
+// ---- tensor-core products of the network: operands rounded to BF16 (nearest,
+// ties to even) when staged, mma.sync m16n8k16 with FP32 accumulation.
 constexpr int HT = 64, HK = 32, HLD = HK + 8;   // smem rows padded by 16 bytes
 
 __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
@@ -113,37 +47,44 @@ __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], const uint32_t (&a
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-template <class T>
-__device__ __forceinline__ __nv_bfloat16 to_bf(const T* p, int64_t i);
-template <>
-__device__ __forceinline__ __nv_bfloat16 to_bf<float>(const float* p, int64_t i) { return __float2bfloat16_rn(p[i]); }
-template <>
-__device__ __forceinline__ __nv_bfloat16 to_bf<__nv_bfloat16>(const __nv_bfloat16* p, int64_t i) { return p[i]; }
+__device__ __forceinline__ uint2 bf16x4(float4 x) {
+  __nv_bfloat162 lo = __floats2bfloat162_rn(x.x, x.y), hi = __floats2bfloat162_rn(x.z, x.w);
+  return make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+}
 
-// C[m][n] = alpha * sum_k A(m,k) B(k,n) + beta * C (part == nullptr), or the
-// raw partial of K slice blockIdx.z into part[z][m][n].
-template <class TA, class TB>
-__global__ void __launch_bounds__(128) hgemm_kernel(int M, int N, int K, int kchunk, float alpha,
-                                                    const TA* __restrict__ A, int64_t sam, int64_t sak,
-                                                    const TB* __restrict__ B, int64_t sbk, int64_t sbn, float beta,
-                                                    float* __restrict__ C, int64_t ldc, float* __restrict__ part) {
+// One layer over the batch: acc[b][n] = sum_k A[b][k] W(k, n), W(k, n) =
+// W[k * swk + n * swn] in BF16, A rows of K (a multiple of 4) floats, N = H.
+//   Zin == nullptr: Z = acc + bias, Y = GELU(Z)                       (forward)
+//   Zin != nullptr: Y = acc * GELU'(Zin), column sums of Y over this
+//                   block's rows into colpart[blockIdx.y][n] (FP64)   (backward)
+// 64 x 64 tile per block, 32-deep K slabs, four warps of 32 x 32; HBM bound
+// (65536 x 128 outputs: 67 MB written and 33 or 67 read), so the activation and
+// the bias gradient ride along instead of being passes of their own.
+__global__ void __launch_bounds__(128) layer_kernel(int M, int K, const float* __restrict__ A,
+                                                    const __nv_bfloat16* __restrict__ W, int swk, int swn,
+                                                    const float* __restrict__ bias, float* __restrict__ Z,
+                                                    const float* __restrict__ Zin, float* __restrict__ Y,
+                                                    double* __restrict__ colpart) {
   __shared__ __align__(16) __nv_bfloat16 As[HT][HLD];   // [m][k]
   __shared__ __align__(16) __nv_bfloat16 Bs[HT][HLD];   // [n][k]
+  __shared__ double cs[2][HT];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m0 = blockIdx.y * HT, n0 = blockIdx.x * HT;
-  const int kb = blockIdx.z * kchunk, ke = min(K, kb + kchunk);
   const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
   const int g = lane >> 2, t4 = lane & 3;
   float acc[2][4][4] = {};
-  for (int k0 = kb; k0 < ke; k0 += HK) {
-    // stage with the stride-1 index of each operand along the threads
+  for (int k0 = 0; k0 < K; k0 += HK) {
+#pragma unroll
+    for (int q = 0; q < HT * HK / 4 / 128; ++q) {
+      const int e = tid + 128 * q, mm = e / (HK / 4), kk = 4 * (e % (HK / 4)), m = m0 + mm, k = k0 + kk;
+      const float4 x = (m < M && k < K) ? *reinterpret_cast<const float4*>(A + (int64_t)m * K + k)
+                                        : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      *reinterpret_cast<uint2*>(&As[mm][kk]) = bf16x4(x);
+    }
+#pragma unroll 4
     for (int e = tid; e < HT * HK; e += 128) {
-      const int mm = sak == 1 ? e / HK : e % HT, kk = sak == 1 ? e % HK : e / HT;
-      const int m = m0 + mm, k = k0 + kk;
-      As[mm][kk] = (m < M && k < ke) ? to_bf(A, (int64_t)m * sam + (int64_t)k * sak) : __float2bfloat16_rn(0.0f);
-      const int nn = sbk == 1 ? e / HK : e % HT, k2 = sbk == 1 ? e % HK : e / HT;
-      const int n = n0 + nn, kk2 = k0 + k2;
-      Bs[nn][k2] = (n < N && kk2 < ke) ? to_bf(B, (int64_t)kk2 * sbk + (int64_t)n * sbn) : __float2bfloat16_rn(0.0f);
+      const int nn = swk == 1 ? e / HK : e % HT, kk = swk == 1 ? e % HK : e / HT, k = k0 + kk;
+      Bs[nn][kk] = k < K ? W[k * swk + (n0 + nn) * swn] : __float2bfloat16_rn(0.0f);
     }
     __syncthreads();
 #pragma unroll
@@ -171,122 +112,227 @@ __global__ void __launch_bounds__(128) hgemm_kernel(int M, int N, int K, int kch
     __syncthreads();
   }
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+  for (int j = 0; j < 4; ++j) {
+    const int n = n0 + wn + 8 * j + 2 * t4;
+    const float b0 = Zin ? 0.0f : bias[n], b1 = Zin ? 0.0f : bias[n + 1];
+    double c0 = 0.0, c1 = 0.0;
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int m = m0 + wm + 16 * i + g + 8 * h;
+        if (m >= M) continue;
+        const int64_t at = (int64_t)m * H + n;
+        if (Zin) {
+          const float2 z = *reinterpret_cast<const float2*>(Zin + at);
+          const float2 y = make_float2(acc[i][j][2 * h] * gelu_grad(z.x), acc[i][j][2 * h + 1] * gelu_grad(z.y));
+          *reinterpret_cast<float2*>(Y + at) = y;
+          c0 += (double)y.x;
+          c1 += (double)y.y;
+        } else {
+          const float2 z = make_float2(acc[i][j][2 * h] + b0, acc[i][j][2 * h + 1] + b1);
+          *reinterpret_cast<float2*>(Z + at) = z;
+          *reinterpret_cast<float2*>(Y + at) = make_float2(gelu(z.x), gelu(z.y));
+        }
+      }
+    if (Zin) {
+#pragma unroll
+      for (int off = 4; off < 32; off <<= 1) {   // over the eight rows g of the warp
+        c0 += __shfl_xor_sync(0xffffffffu, c0, off);
+        c1 += __shfl_xor_sync(0xffffffffu, c1, off);
+      }
+      if (g == 0) {
+        cs[warp >> 1][wn + 8 * j + 2 * t4] = c0;
+        cs[warp >> 1][wn + 8 * j + 2 * t4 + 1] = c1;
+      }
+    }
+  }
+  if (Zin) {
+    __syncthreads();
+    if (tid < HT) colpart[(int64_t)blockIdx.y * H + n0 + tid] = cs[0][tid] + cs[1][tid];
+  }
+}
+
+// part[z][h][n] = sum over the rows b of slice z of D[b][h] X[b][n]: a weight
+// gradient, K = the batch.  32 rows at a time in shared memory as they lie in
+// memory (BF16), read into the fragments by transposing ldmatrix; eight warps
+// over the 128 x NX output.
+template <int NX>
+__global__ void __launch_bounds__(256) wgrad_kernel(int64_t B, int64_t rows_per, const float* __restrict__ D,
+                                                    const float* __restrict__ X, float* __restrict__ part) {
+  constexpr int LDD = H + 8, LDX = NX + 8;
+  __shared__ __align__(16) __nv_bfloat16 Ds[32][LDD], Xs[32][LDX];
+  constexpr int WN = NX == 128 ? 64 : 16;        // warp tile: WM rows (h) x WN columns
+  constexpr int WM = NX == 128 ? 32 : 16;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int wm = NX == 128 ? (warp >> 1) * 32 : warp * 16, wn = NX == 128 ? (warp & 1) * 64 : 0;
+  float acc[WM / 16][WN / 8][4] = {};
+  const int64_t b0 = (int64_t)blockIdx.x * rows_per, b1 = min(B, b0 + rows_per);
+  for (int64_t b = b0; b < b1; b += 32) {
+#pragma unroll
+    for (int q = 0; q < 32 * H / 4 / 256; ++q) {
+      const int e = tid + 256 * q, r = e / (H / 4), c = 4 * (e % (H / 4));
+      const float4 x = b + r < b1 ? *reinterpret_cast<const float4*>(D + (b + r) * H + c)
+                                  : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      *reinterpret_cast<uint2*>(&Ds[r][c]) = bf16x4(x);
+    }
+#pragma unroll
+    for (int e = tid; e < 32 * NX / 4; e += 256) {
+      const int r = e / (NX / 4), c = 4 * (e % (NX / 4));
+      const float4 x = b + r < b1 ? *reinterpret_cast<const float4*>(X + (b + r) * NX + c)
+                                  : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      *reinterpret_cast<uint2*>(&Xs[r][c]) = bf16x4(x);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int ks = 0; ks < 32; ks += 16) {
+      uint32_t af[WM / 16][4], bfr[WN / 8][2];
+      // matrices (k 0-7, m 0-7), (k 0-7, m 8-15), (k 8-15, m 0-7), (k 8-15, m 8-15)
+#pragma unroll
+      for (int i = 0; i < WM / 16; ++i) {
+        const uint32_t ad = (uint32_t)__cvta_generic_to_shared(
+            &Ds[ks + (lane & 7) + 8 * (lane >> 4)][wm + 16 * i + 8 * ((lane >> 3) & 1)]);
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(af[i][0]), "=r"(af[i][1]), "=r"(af[i][2]), "=r"(af[i][3])
+                     : "r"(ad));
+      }
+#pragma unroll
+      for (int j = 0; j < WN / 8; j += 2) {
+        // (k 0-7, n 0-7), (k 8-15, n 0-7), (k 0-7, n 8-15), (k 8-15, n 8-15)
+        const uint32_t bd = (uint32_t)__cvta_generic_to_shared(
+            &Xs[ks + (lane & 7) + 8 * ((lane >> 3) & 1)][wn + 8 * j + 8 * (lane >> 4)]);
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(bfr[j][0]), "=r"(bfr[j][1]), "=r"(bfr[j + 1][0]), "=r"(bfr[j + 1][1])
+                     : "r"(bd));
+      }
+#pragma unroll
+      for (int i = 0; i < WM / 16; ++i)
+#pragma unroll
+        for (int j = 0; j < WN / 8; ++j) mma_bf16_16816(acc[i][j], af[i], bfr[j]);
+    }
+    __syncthreads();
+  }
+  const int g = lane >> 2, t4 = lane & 3;
+#pragma unroll
+  for (int i = 0; i < WM / 16; ++i)
+#pragma unroll
+    for (int j = 0; j < WN / 8; ++j)
 #pragma unroll
       for (int h = 0; h < 4; ++h) {
-        const int m = m0 + wm + 16 * i + g + (h >> 1) * 8, n = n0 + wn + 8 * j + 2 * t4 + (h & 1);
-        if (m >= M || n >= N) continue;
-        if (part) {
-          part[((int64_t)blockIdx.z * M + m) * N + n] = acc[i][j][h];
-        } else {
-          float v = alpha * acc[i][j][h];
-          if (beta != 0.0f) v += beta * C[(int64_t)m * ldc + n];
-          C[(int64_t)m * ldc + n] = v;
-        }
+        const int m = wm + 16 * i + g + 8 * (h >> 1), n = wn + 8 * j + 2 * t4 + (h & 1);
+        part[((int64_t)blockIdx.x * H + m) * NX + n] = acc[i][j][h];
       }
 }
 
-__global__ void hgemm_reduce_kernel(const float* __restrict__ part, int splits, int M, int N, float alpha,
-                                    float beta, float* __restrict__ C, int64_t ldc) {
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < (int64_t)M * N; t += (int64_t)gridDim.x * blockDim.x) {
-    float s = 0.0f;
-    for (int z = 0; z < splits; ++z) s += part[(int64_t)z * M * N + t];
-    const int64_t m = t / N, n = t - m * N;
-    float v = alpha * s;
-    if (beta != 0.0f) v += beta * C[m * ldc + n];
-    C[m * ldc + n] = v;
+// out[t] = sum over the slices, in order
+__global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* __restrict__ part, int splits, int n,
+                                                           float* __restrict__ out) {
+  const int t = blockIdx.x * 256 + threadIdx.x;
+  if (t >= n) return;
+  float s = 0.0f;
+#pragma unroll 8
+  for (int z = 0; z < splits; ++z) s += part[(int64_t)z * n + t];
+  out[t] = s;
+}
+
+// out[c] = sum_p part[p][c]: 32 columns per block, eight warps over interleaved
+// rows, a fixed order
+__global__ void __launch_bounds__(256) colreduce_kernel(const double* __restrict__ part, int nparts, int ncols,
+                                                        float* __restrict__ out) {
+  __shared__ double sh[8][32];
+  const int x = threadIdx.x & 31, g = threadIdx.x >> 5, c = blockIdx.x * 32 + x;
+  double s = 0.0;
+  if (c < ncols) {
+#pragma unroll 4
+    for (int p = g; p < nparts; p += 8) s += part[(int64_t)p * ncols + c];
+  }
+  sh[g][x] = s;
+  __syncthreads();
+  if (g != 0 || c >= ncols) return;
+#pragma unroll
+  for (int w = 1; w < 8; ++w) s += sh[w][x];
+  out[c] = (float)s;
+}
+
+// dZ2[b][h] = dy[b] w3[h] GELU'(Z2[b][h]), with the sums over this block's rows
+// of dZ2 (db2), dy H2 (dw3) and dy (db3) into part[blockIdx.x][H + H + 1].
+// Eight rows at a time, four columns per thread; one pass over Z2 and H2.
+constexpr int BACK_COLS = 2 * H + 1;
+__global__ void __launch_bounds__(256) out_back_kernel(const float* __restrict__ dy, const float* __restrict__ w3,
+                                                       const float* __restrict__ Z2, const float* __restrict__ H2,
+                                                       int64_t B, int64_t rows_per, float* __restrict__ dZ2,
+                                                       double* __restrict__ part) {
+  __shared__ double sh[8][H];
+  const int c = (threadIdx.x & 31) * 4, rg = threadIdx.x >> 5;
+  const float4 w = make_float4(w3[c], w3[c + 1], w3[c + 2], w3[c + 3]);
+  const int64_t b0 = (int64_t)blockIdx.x * rows_per, b1 = min(B, b0 + rows_per);
+  double sb[4] = {}, sw[4] = {}, sd = 0.0;
+  for (int64_t b = b0 + rg; b < b1; b += 8) {
+    const float d = dy[b];
+    const float4 z = *reinterpret_cast<const float4*>(Z2 + b * H + c), h = *reinterpret_cast<const float4*>(H2 + b * H + c);
+    const float4 y = make_float4(d * w.x * gelu_grad(z.x), d * w.y * gelu_grad(z.y), d * w.z * gelu_grad(z.z),
+                                 d * w.w * gelu_grad(z.w));
+    *reinterpret_cast<float4*>(dZ2 + b * H + c) = y;
+    sb[0] += (double)y.x; sb[1] += (double)y.y; sb[2] += (double)y.z; sb[3] += (double)y.w;
+    sw[0] += (double)(d * h.x); sw[1] += (double)(d * h.y); sw[2] += (double)(d * h.z); sw[3] += (double)(d * h.w);
+    if (c == 0) sd += (double)d;
+  }
+  double* out = part + (int64_t)blockIdx.x * BACK_COLS;
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) sh[rg][c + q] = r == 0 ? sb[q] : sw[q];
+    __syncthreads();
+    if (threadIdx.x < H) {
+      double s = sh[0][threadIdx.x];
+#pragma unroll
+      for (int k = 1; k < 8; ++k) s += sh[k][threadIdx.x];
+      out[r * H + threadIdx.x] = s;
+    }
+    __syncthreads();
+  }
+  if (c == 0) sh[rg][0] = sd;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = 0.0;
+    for (int k = 0; k < 8; ++k) s += sh[k][0];
+    out[2 * H] = s;
   }
 }
 
-// Tensor-core GEMM with the sgemm argument convention; splits K when the
-// output has fewer tiles than the GPU has SMs (partials in `work`, grown as
-// needed).
-template <class TA, class TB>
-void hgemm(int M, int N, int K, float alpha, const TA* A, int64_t sam, int64_t sak, const TB* B, int64_t sbk,
-           int64_t sbn, float beta, float* C, int64_t ldc, DBuf<float>& work, cudaStream_t s) {
-  const int tiles = ((N + HT - 1) / HT) * ((M + HT - 1) / HT);
-  int splits = 1;
-  if (tiles < 152 && K >= 8 * HK) splits = std::min((2 * 152 + tiles - 1) / tiles, K / (4 * HK));
-  splits = std::max(1, std::min(splits, 256));
-  const int kchunk = ((K + splits - 1) / splits + HK - 1) / HK * HK;
-  splits = (K + kchunk - 1) / kchunk;
-  dim3 grid((N + HT - 1) / HT, (M + HT - 1) / HT, splits);
-  if (splits == 1) {
-    hgemm_kernel<TA, TB><<<grid, 128, 0, s>>>(M, N, K, kchunk, alpha, A, sam, sak, B, sbk, sbn, beta, C, ldc, nullptr);
-    FCC_CHECK_LAUNCH();
-    return;
-  }
-  const int64_t need = (int64_t)splits * M * N;
-  if ((int64_t)work.n < need) work.alloc(need);
-  hgemm_kernel<TA, TB><<<grid, 128, 0, s>>>(M, N, K, kchunk, alpha, A, sam, sak, B, sbk, sbn, beta, C, ldc, work.p);
-  FCC_CHECK_LAUNCH();
-  hgemm_reduce_kernel<<<(unsigned)std::min<int64_t>(((int64_t)M * N + 255) / 256, 152 * 4), 256, 0, s>>>(
-      work.p, splits, M, N, alpha, beta, C, ldc);
-  FCC_CHECK_LAUNCH();
-}
-
-// Z[b][h] += bias[h]; Hact = GELU(Z)
-__global__ void bias_gelu_kernel(float* Z, float* Hact, const float* bias, int64_t B, int Hn) {
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < B * Hn; t += (int64_t)gridDim.x * blockDim.x) {
-    float z = Z[t] + bias[t % Hn];
-    Z[t] = z;
-    Hact[t] = gelu(z);
-  }
-}
-
-// dZ = dH * GELU'(Z)
-__global__ void gelu_back_kernel(const float* Z, float* dH, int64_t n) {
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x)
-    dH[t] *= gelu_grad(Z[t]);
-}
-
-// y[b] = sum_h H2[b][h] w3[h] + b3; loss partials; dy = 2 (y - target) / B
-__global__ void out_loss_kernel(const float* H2, const float* w3, const float* b3, const float* target, int64_t B,
-                                float* y, float* dy, double* loss_part) {
+// y[b] = sum_h H2[b][h] w3[h] + b3; loss partials; dy = 2 (y - target) / B.
+// A warp per row, four columns per lane.
+__global__ void __launch_bounds__(256) out_loss_kernel(const float* H2, const float* w3, const float* b3,
+                                                       const float* target, int64_t B, float* y, float* dy,
+                                                       double* loss_part) {
+  __shared__ double sm[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float4 w = make_float4(w3[4 * lane], w3[4 * lane + 1], w3[4 * lane + 2], w3[4 * lane + 3]);
   double l = 0.0;
-  for (int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; b < B; b += (int64_t)gridDim.x * blockDim.x) {
-    float s = b3[0];
-    for (int h = 0; h < H; ++h) s += H2[b * H + h] * w3[h];
-    y[b] = s;
-    if (target) {
-      float d = s - target[b];
-      l += (double)d * d;
-      dy[b] = 2.0f * d / (float)B;
+#pragma unroll 2
+  for (int64_t b = (int64_t)blockIdx.x * 8 + warp; b < B; b += (int64_t)gridDim.x * 8) {
+    const float4 h = *reinterpret_cast<const float4*>(H2 + b * H + 4 * lane);
+    float s = (h.x * w.x + h.y * w.y) + (h.z * w.z + h.w * w.w);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    s += b3[0];
+    if (lane == 0) {
+      y[b] = s;
+      if (target) {
+        float d = s - target[b];
+        l += (double)d * d;
+        dy[b] = 2.0f * d / (float)B;
+      }
     }
   }
   if (loss_part) {
-    __shared__ double sm[256];
-    sm[threadIdx.x] = l;
+    if (lane == 0) sm[warp] = l;
     __syncthreads();
-    for (int w = 128; w > 0; w >>= 1) {
-      if (threadIdx.x < w) sm[threadIdx.x] += sm[threadIdx.x + w];
-      __syncthreads();
+    if (threadIdx.x == 0) {
+      double t = 0.0;
+      for (int k = 0; k < 8; ++k) t += sm[k];
+      loss_part[blockIdx.x] = t;
     }
-    if (threadIdx.x == 0) loss_part[blockIdx.x] = sm[0];
   }
-}
-
-// g[h] = sum_b X[b][h] (bias gradients), one block per h, fixed order.
-__global__ void colsum_kernel(const float* X, int64_t B, int Hn, float* g) {
-  const int h = blockIdx.x;
-  double s = 0.0;
-  for (int64_t b = threadIdx.x; b < B; b += blockDim.x) s += X[b * Hn + h];
-  __shared__ double sm[256];
-  sm[threadIdx.x] = s;
-  __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
-    if (threadIdx.x < w) sm[threadIdx.x] += sm[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) g[h] = (float)sm[0];
-}
-
-// dH2[b][h] = dy[b] * w3[h]
-__global__ void outer_kernel(const float* dy, const float* w3, int64_t B, float* dH2) {
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < B * H; t += (int64_t)gridDim.x * blockDim.x)
-    dH2[t] = dy[t / H] * w3[t % H];
 }
 
 // Adam (Kingma & Ba 2015) on the FP32 masters, then the BF16 working copy.
@@ -536,8 +582,9 @@ struct fcc_mlp {
   bool stats = false;
   // batch work buffers
   fcc::DBuf<float> Xb, Yb, Z1, H1, Z2, H2, yb, dy, dH, dH1;
-  fcc::DBuf<double> lpart;
-  fcc::DBuf<float> work;                  // split-K partials of the tensor-core products
+  fcc::DBuf<float> Xraw;                  // host samples of fcc_mlp_grad
+  fcc::DBuf<double> lpart, colpart;       // loss and column-sum partials
+  fcc::DBuf<float> work;                  // batch slices of the weight gradients
   int64_t bcap = 0;
 };
 
@@ -548,7 +595,10 @@ void ensure_batch(fcc_mlp* m, int64_t B) {
   if (B <= m->bcap) return;
   m->Xb.alloc(B * NF); m->Yb.alloc(B); m->Z1.alloc(B * H); m->H1.alloc(B * H); m->Z2.alloc(B * H);
   m->H2.alloc(B * H); m->yb.alloc(B); m->dy.alloc(B); m->dH.alloc(B * H); m->dH1.alloc(B * H);
+  m->Xraw.alloc(B * NF);
   m->lpart.alloc(304);
+  m->colpart.alloc(std::max<int64_t>((B + HT - 1) / HT * H, 304 * BACK_COLS));
+  m->work.alloc(152 * H * H);
   m->bcap = B;
 }
 
@@ -560,12 +610,11 @@ double fwd_bwd(fcc_mlp* m, int64_t B, const float* target, bool backward) {
   const __nv_bfloat16* W2 = m->pb.p + OFF_W2;
   const float* b1 = m->p.p + OFF_B1;
   const float* b2 = m->p.p + OFF_B2;
-  // layer 1: Z1 = Xb W1^T   (B x H), K = NF; tensor cores, BF16 operands
-  hgemm<float, __nv_bfloat16>((int)B, H, NF, 1.0f, m->Xb.p, NF, 1, W1, 1, NF, 0.0f, m->Z1.p, H, m->work, s);
-  bias_gelu_kernel<<<grid_of(B * H), 256, 0, s>>>(m->Z1.p, m->H1.p, b1, B, H);
+  const dim3 lgrid(H / HT, (unsigned)((B + HT - 1) / HT));
+  // Z1 = Xb W1^T + b1, H1 = GELU(Z1); Z2 = H1 W2^T + b2, H2 = GELU(Z2)
+  layer_kernel<<<lgrid, 128, 0, s>>>((int)B, NF, m->Xb.p, W1, 1, NF, b1, m->Z1.p, nullptr, m->H1.p, nullptr);
   FCC_CHECK_LAUNCH();
-  hgemm<float, __nv_bfloat16>((int)B, H, H, 1.0f, m->H1.p, H, 1, W2, 1, H, 0.0f, m->Z2.p, H, m->work, s);
-  bias_gelu_kernel<<<grid_of(B * H), 256, 0, s>>>(m->Z2.p, m->H2.p, b2, B, H);
+  layer_kernel<<<lgrid, 128, 0, s>>>((int)B, H, m->H1.p, W2, 1, H, b2, m->Z2.p, nullptr, m->H2.p, nullptr);
   FCC_CHECK_LAUNCH();
   // output layer (w3 FP32 master used directly: 128 weights)
   out_loss_kernel<<<304, 256, 0, s>>>(m->H2.p, m->p.p + OFF_W3, m->p.p + OFF_B3, target, B, m->yb.p, m->dy.p,
@@ -581,26 +630,31 @@ double fwd_bwd(fcc_mlp* m, int64_t B, const float* target, bool backward) {
   }
   if (!backward) return loss;
   float* g = m->g.p;
-  // dL/dw3[h] = sum_b dy[b] H2[b][h];  dL/db3 = sum_b dy[b]
-  sgemm<float, float>(1, H, (int)B, 1.0f, m->dy.p, 0, 1, m->H2.p, H, 1, 0.0f, g + OFF_W3, H, s);
-  colsum_kernel<<<1, 256, 0, s>>>(m->dy.p, B, 1, g + OFF_B3);
+  // dZ2 = dy w3^T * GELU'(Z2); db2, dw3 and db3 are its column sums, those of
+  // dy H2 and the sum of dy: in this order they lie in g from OFF_B2 on
+  static_assert(OFF_W3 == OFF_B2 + H && OFF_B3 == OFF_W3 + H, "b2, w3, b3 adjacent");
+  const int64_t rows = std::max<int64_t>(8, (B + 303) / 304);
+  const int nb = (int)((B + rows - 1) / rows);
+  out_back_kernel<<<nb, 256, 0, s>>>(m->dy.p, m->p.p + OFF_W3, m->Z2.p, m->H2.p, B, rows, m->dH.p, m->colpart.p);
   FCC_CHECK_LAUNCH();
-  // dH2 = dy w3^T, dZ2 = dH2 * GELU'(Z2)
-  outer_kernel<<<grid_of(B * H), 256, 0, s>>>(m->dy.p, m->p.p + OFF_W3, B, m->dH.p);
+  colreduce_kernel<<<(BACK_COLS + 31) / 32, 256, 0, s>>>(m->colpart.p, nb, BACK_COLS, g + OFF_B2);
   FCC_CHECK_LAUNCH();
-  gelu_back_kernel<<<grid_of(B * H), 256, 0, s>>>(m->Z2.p, m->dH.p, B * H);
+  // dW2 = dZ2^T H1 (H x H, K = B)
+  const int64_t wrows = std::max<int64_t>(32, (B + 151) / 152);
+  const int wb = (int)((B + wrows - 1) / wrows);
+  wgrad_kernel<H><<<wb, 256, 0, s>>>(B, wrows, m->dH.p, m->H1.p, m->work.p);
   FCC_CHECK_LAUNCH();
-  // dW2 = dZ2^T H1 (H x H, K = B), db2 = colsum(dZ2)
-  hgemm<float, float>(H, H, (int)B, 1.0f, m->dH.p, 1, H, m->H1.p, H, 1, 0.0f, g + OFF_W2, H, m->work, s);
-  colsum_kernel<<<H, 256, 0, s>>>(m->dH.p, B, H, g + OFF_B2);
+  wgrad_reduce_kernel<<<H * H / 256, 256, 0, s>>>(m->work.p, wb, H * H, g + OFF_W2);
   FCC_CHECK_LAUNCH();
-  // dH1 = dZ2 W2 (B x H), dZ1 = dH1 * GELU'(Z1)
-  hgemm<float, __nv_bfloat16>((int)B, H, H, 1.0f, m->dH.p, H, 1, W2, H, 1, 0.0f, m->dH1.p, H, m->work, s);
-  gelu_back_kernel<<<grid_of(B * H), 256, 0, s>>>(m->Z1.p, m->dH1.p, B * H);
+  // dZ1 = (dZ2 W2) * GELU'(Z1), db1 = its column sums
+  layer_kernel<<<lgrid, 128, 0, s>>>((int)B, H, m->dH.p, W2, H, 1, nullptr, nullptr, m->Z1.p, m->dH1.p, m->colpart.p);
   FCC_CHECK_LAUNCH();
-  // dW1 = dZ1^T X (H x NF), db1 = colsum(dZ1)
-  hgemm<float, float>(H, NF, (int)B, 1.0f, m->dH1.p, 1, H, m->Xb.p, NF, 1, 0.0f, g + OFF_W1, NF, m->work, s);
-  colsum_kernel<<<H, 256, 0, s>>>(m->dH1.p, B, H, g + OFF_B1);
+  colreduce_kernel<<<H / 32, 256, 0, s>>>(m->colpart.p, (int)lgrid.y, H, g + OFF_B1);
+  FCC_CHECK_LAUNCH();
+  // dW1 = dZ1^T X (H x NF)
+  wgrad_kernel<NF><<<wb, 256, 0, s>>>(B, wrows, m->dH1.p, m->Xb.p, m->work.p);
+  FCC_CHECK_LAUNCH();
+  wgrad_reduce_kernel<<<H * NF / 256, 256, 0, s>>>(m->work.p, wb, H * NF, g + OFF_W1);
   FCC_CHECK_LAUNCH();
   return loss;
 }
@@ -854,11 +908,9 @@ int fcc_mlp_grad(fcc_mlp* m, const float* X, const float* y, int32_t n, float* g
     FCC_CUDA(cudaSetDevice(m->device));
     cudaStream_t s = m->stream;
     ensure_batch(m, n);
-    DBuf<float> Xraw;
-    Xraw.alloc((int64_t)n * NF);
-    FCC_CUDA(cudaMemcpyAsync(Xraw.p, X, sizeof(float) * n * NF, cudaMemcpyHostToDevice, s));
+    FCC_CUDA(cudaMemcpyAsync(m->Xraw.p, X, sizeof(float) * n * NF, cudaMemcpyHostToDevice, s));
     FCC_CUDA(cudaMemcpyAsync(m->Yb.p, y, sizeof(float) * n, cudaMemcpyHostToDevice, s));
-    normalise_kernel<<<grid_of((int64_t)n * NF), 256, 0, s>>>(Xraw.p, n, m->p.p + OFF_MU, m->p.p + OFF_SD, m->Xb.p);
+    normalise_kernel<<<grid_of((int64_t)n * NF), 256, 0, s>>>(m->Xraw.p, n, m->p.p + OFF_MU, m->p.p + OFF_SD, m->Xb.p);
     FCC_CHECK_LAUNCH();
     double l = fwd_bwd(m, n, m->Yb.p, true);
     FCC_CUDA(cudaMemcpyAsync(grad, m->g.p, sizeof(float) * NTRAIN, cudaMemcpyDeviceToHost, s));
