@@ -662,7 +662,7 @@ void residual(fcc_ctx* c) {
         ps.Kp = Wk;
         if ((int64_t)c->bvvA.n < R * Wk) c->bvvA.alloc(R * Wk);
         if ((int64_t)c->bvvEx.n < R) c->bvvEx.alloc(R);
-        pack_oz(Btvv.p, ps, S, lv.bits, c->bvvA.p, c->bvvEx.p, s);
+        pack_oz(Btvv.p, ps, S, lv.bits, lv.guard, c->bvvA.p, c->bvvEx.p, s);
       } else {
         Wk = packed_kp(Q, tc->scheme.P);
         ps.Kp = Wk;

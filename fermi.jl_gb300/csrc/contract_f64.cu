@@ -758,14 +758,14 @@ void run_tc(TcEngine* tc, OzLevel lv, double alpha, const TView& A, const TView&
       if (fresh) {
         if ((int64_t)ka->buf.n < M * W) ka->buf.alloc(M * W);
         if ((int64_t)ka->ex.n < M) ka->ex.alloc(M);
-        pack_oz(A.p, pa, S, lv.bits, ka->buf.p, ka->ex.p, s);
+        pack_oz(A.p, pa, S, lv.bits, lv.guard, ka->buf.p, ka->ex.p, s);
       }
       pA = ka->buf.p;
       eA = ka->ex.p;
     } else {
-      pack_oz(A.p, pa, S, lv.bits, pA, eA, s);
+      pack_oz(A.p, pa, S, lv.bits, lv.guard, pA, eA, s);
     }
-    pack_oz(B.p, pb, S, lv.bits, tc->bufB.p, tc->exB.p, s);
+    pack_oz(B.p, pb, S, lv.bits, lv.guard, tc->bufB.p, tc->exB.p, s);
     EpiMap ep;
     ep.M = M; ep.N = N;
     ep.md2 = gm[1].dim; ep.md3 = gm[2].dim; ep.ms1 = gm[0].s[2]; ep.ms2 = gm[1].s[2]; ep.ms3 = gm[2].s[2];
@@ -860,7 +860,7 @@ void einsum(double alpha, const char* spec, const TView& A, const TView& B, doub
     std::vector<Ix> m3 = gm, n3 = gn, k3 = gk;
     if (flops >= tc->min_flops && gdim(gm) >= tc->min_dim && gdim(gn) >= tc->min_dim && try_fuse(m3, 3) && try_fuse(n3, 3) &&
         try_fuse(k3, 3)) {
-      run_tc(tc, tc->exact ? tc->oz : OzLevel{0, 0, 0, 0}, alpha, A, B, beta, C, m3, n3, k3, s);
+      run_tc(tc, tc->exact ? tc->oz : OzLevel{0, 0, 0, 0, 0}, alpha, A, B, beta, C, m3, n3, k3, s);
       return;
     }
   }

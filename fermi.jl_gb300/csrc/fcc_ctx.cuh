@@ -67,7 +67,7 @@ struct fcc_ctx {
   int test_fault = 0;
 
   // (T) scratch
-  fcc::DBuf<double> ovvv, ooov, Wt;
+  fcc::DBuf<double> Wt;
 };
 
 namespace fcc {

@@ -129,6 +129,10 @@ struct EpiMap {
   double alpha = 1.0, beta = 0.0;
   void* C = nullptr;
   int atomic = 0;
+  // exact-slice products only: `batch` products of the same extents, product q
+  // over the packed rows q * ba.. of A and q * bb.. of B into C + q * bc
+  int batch = 1;
+  int64_t ba = 0, bb = 0, bc = 0;
   double work = 0.0;   // algorithmic BF16 flops for the timing log (0: use the padded count)
   int no_loads = 0;    // test hook: the producer issues no TMA loads, so the bounded waits give up
 };
@@ -171,22 +175,23 @@ CUtensorMap tma_map_bf16(const __nv_bfloat16* base, int64_t rows, int64_t cols, 
 // The reduced levels of the mixed form stay at 6-bit digits: its iterates, and
 // so its converged amplitudes, depend on what those levels drop.
 // `cut` > 0: the first `cut` bands of groups get a running sum of their own
-// (the FP64 level, see gemm_oz.cu).
+// (the FP64 level, see gemm_oz.cu).  guard: the digits are cut from x 2^-guard,
+// |d_1| <= 2^(b - guard), so that sums reach 2^24 later.
 struct OzLevel {
-  int S, G, cut, bits;
+  int S, G, cut, bits, guard;
 };
-// FP64 level: 64 bits below the row maximum, every pair of weight 2^-72 and
-// up (36 products), the first band summed apart.  Dropped pairs and cut digits
-// are below 2^-64 of max|A_r| max|B_c| per term and the sums carry ~2^-60 of
-// the result, where an FP64 product accumulates roundings of 2^-53 of its
-// partial sums.  Error against quadruple precision on the operands of (H2O)4
-// (2-norm of the difference over that of the result), this level / seven
-// slices / FP64 pipe: DF fit over J^-1/2 1.2e-16 / 3.7e-15 / 1.8e-14, MO
-// transform 1.3e-17 / 1.6e-16 / 5.3e-16, (ia|jb) 6e-18 / 4e-17 / 2.3e-16, ring
-// 4e-18 / 5e-17 / 2.7e-16, ladder 2e-17 / 1.4e-16 / 9e-16, (T) over l 7e-18 /
-// 1.1e-16 / 1.7e-16.  Seven slices would be 5% faster; eight leave a decade for
-// rows more peaked than these.
-constexpr OzLevel OZ_F64{8, 9, 1, 8};
+// FP64 level: 62 bits below the row maximum (two guard bits, so that sums of
+// first digits stay below 2^24 over 16 k-blocks), the first 36 pairs, the first
+// band summed apart.  Dropped pairs and cut digits are about 2^-62 of max|A_r|
+// max|B_c| per term and the sums carry ~2^-60 of the result, where an FP64
+// product accumulates roundings of 2^-53 of its partial sums.  Error against
+// quadruple precision on the operands of (H2O)4 (2-norm of the difference over
+// that of the result), this level / FP64 pipe: DF fit over J^-1/2 1.6e-15 /
+// 1.8e-14, MO transform 5.9e-17 / 5.3e-16, (ia|jb) 2.5e-17 / 2.3e-16, (ab|cd)
+// 2e-17 / 5.3e-16, ring 1.9e-17 / 2.7e-16, ladder 1.1e-16 / 9e-16, (T) over d
+// 2.3e-17 / 3.2e-16, over l 3e-17 / 1.7e-16.  Seven slices would be 5% faster
+// and nearly as far off as the pipe on the DF fit; eight leave a decade.
+constexpr OzLevel OZ_F64{8, 9, 1, 8, 2};
 constexpr int OZ_MAXS = 8;
 constexpr int OZ_G_DEFAULT = 8;
 // the level of `groups` weight groups of 6-bit digits, the unit the phases of
@@ -203,7 +208,8 @@ inline double oz_pairs(OzLevel lv) {
 // to (s+1)*Kpad; ex[r] = biased FP64 exponent of max_k |x_rk| (0: all zero,
 // 2047: the row holds an infinity or NaN, and so will its products)
 int64_t oz_kpad(int64_t K);
-void pack_oz(const double* src, const PackSpec& ps, int S, int bits, __nv_bfloat16* dst, int* ex, cudaStream_t s);
+void pack_oz(const double* src, const PackSpec& ps, int S, int bits, int guard, __nv_bfloat16* dst, int* ex,
+             cudaStream_t s);
 // exact-slice product over packed operands, written to ep;
 // ws holds the partial results of products cut into several jobs
 void gemm_oz(const __nv_bfloat16* A, int64_t a_rows, const int* exA, const __nv_bfloat16* B, int64_t b_rows,

@@ -118,6 +118,31 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
       : "r"(taddr));
 }
 
+// 16 and 8 columns likewise.
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+}
+// Waits for the loads issued so far; the values named pass through it, so no
+// use of them can be scheduled ahead of the wait.
+template <int N>
+__device__ __forceinline__ void tmem_wait(uint32_t (&r)[N]) {
+  static_assert(N % 8 == 0, "eight registers at a time");
+#pragma unroll
+  for (int q = 0; q < N; q += 8)
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[q]), "+r"(r[q + 1]), "+r"(r[q + 2]), "+r"(r[q + 3]), "+r"(r[q + 4]), "+r"(r[q + 5]),
+                   "+r"(r[q + 6]), "+r"(r[q + 7]));
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
+}
+
 // (double)f * 2^e (negated if neg) by integer exponent arithmetic; FP32
 // subnormals and results below the FP64 normal range give 0
 __device__ __forceinline__ double f32_to_f64_scaled(float f, int e, bool neg) {

@@ -191,7 +191,7 @@ extern "C" int fcc_test_pack_oz(const double* x, int64_t R, int64_t K, int32_t r
     dy.alloc(n);
     dex.alloc(R);
     FCC_CUDA(cudaMemcpyAsync(dx.p, x, sizeof(double) * R * K, cudaMemcpyHostToDevice, s));
-    fcc::pack_oz(dx.p, ps, S, wide ? 8 : 6, dy.p, dex.p, s);
+    fcc::pack_oz(dx.p, ps, S, wide ? 8 : 6, 0, dy.p, dex.p, s);
     FCC_CUDA(cudaMemcpyAsync(out, dy.p, sizeof(uint16_t) * n, cudaMemcpyDeviceToHost, s));
     FCC_CUDA(cudaMemcpyAsync(ex, dex.p, sizeof(int32_t) * R, cudaMemcpyDeviceToHost, s));
     FCC_CUDA(cudaStreamSynchronize(s));

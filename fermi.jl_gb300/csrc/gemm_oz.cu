@@ -31,8 +31,23 @@
 // 4864, 4.0 ms for the 48 bits that took 10.2 ms with 36 products of 6-bit
 // digits.
 //
+// Batches: products of the same shape whose rows lie apart by fixed steps in A,
+// B and C run in one launch (EpiMap batch, ba, bb, bc), which fills the chip
+// where one product has a few dozen tiles.
+//
 // `cut`: the first band (groups 2 and 3) and the rest get separate running
-// sums ("parts"), each converted and added to C in FP64.
+// sums ("parts"), each converted and added to C in FP64.  At the FP64 level
+// with one chunk in the first band (K <= 1024) that band runs last and needs no sum of its own: its two accumulators
+// are added to the others' sums in the store stage (`merged`), one conversion
+// and one pass over C instead of two.
+//
+// Short products (K a few hundred, the (T) ones) are bound by that store stage:
+// a 128 x 128 tile converts 64 elements a thread.  Integer conversion of hi,
+// lo and tail, a short form where no exponent can leave the FP64 range, sums
+// handed over through shared memory so that a warp stores whole rows, and
+// red.add where C is added to (the read would wait in the warp, the addition
+// is the L2's): 5776 x 1216 x 92 at the FP64 level 137 us; 143 with the general
+// conversion only.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -51,12 +66,13 @@ namespace {
 using namespace tc5;
 
 constexpr int OZ_BM = 128, OZ_BN = 128, OZ_BK = 64;
-constexpr int OZ_SLOTS = 11;                     // tile ring
+constexpr int OZ_SLOTS = 10;                     // tile ring
 constexpr int OZ_TILE_BYTES = 128 * OZ_BK * 2;   // one operand tile, A or B
 constexpr int OZ_EPI_WARPS = 8;
-constexpr int OZ_THREADS = 128 + 32 * OZ_EPI_WARPS;   // warp 0 TMA, 1 MMA, 2-3 idle, 4-11 epilogue
-constexpr int OZ_XP_LD = 17;                     // FP64 transpose tile of an epilogue warp: 32 rows x 16 columns
-constexpr int OZ_XP_BYTES = OZ_EPI_WARPS * 32 * OZ_XP_LD * 8;
+constexpr int OZ_THREADS = 128 + 32 * OZ_EPI_WARPS;   // warp 0 TMA of A, 1 MMA, 2 TMA of B, 3 idle, 4-11 epilogue
+constexpr int OZ_XP_LD = 17;                     // transpose tile of an epilogue warp: 32 rows x 16 columns,
+constexpr int OZ_XP_PLANE = 32 * OZ_XP_LD;       // three words per element
+constexpr int OZ_XP_BYTES = OZ_EPI_WARPS * 3 * OZ_XP_PLANE * 4;
 constexpr int OZ_SMEM = OZ_SLOTS * OZ_TILE_BYTES + OZ_XP_BYTES + 1024;
 constexpr int OZ_MAXBANDS = 5, OZ_MAXJOBS = 152;
 
@@ -76,16 +92,20 @@ struct OzJob {
 struct OzParams {
   OzBand band[OZ_MAXBANDS];
   OzJob job[OZ_MAXJOBS];
-  int njobs, cut;              // cut: bands of the first part (0: one part)
-  int bits;                    // digit width
+  uint32_t njobs;
+  int cut;                     // cut: bands of the first part (0: one part)
+  int bits, guard;             // digit width, guard bits of the scales
+  int merged;                  // the last band is added to the others' sums in the store stage
   int kper, kpad;              // k-blocks per L2 block; padded columns per slice
   uint32_t tm, tn, units;
-  double* part;                // partial results [job][M][N] (nullptr: C itself)
+  double* part;                // partial results [product][job][M][N] (nullptr: C itself)
 };
 
 // The bands of groups 2..G over S slices (G <= S + 2): {.., (G-3, G-2),
 // (G-1, G)}, group 2 on its own when their number is odd.
-int make_bands(int S, int G, int bits, OzBand* out) {
+int make_bands(OzLevel lv, OzBand* out) {
+  const int S = lv.S, G = lv.G;
+  const double first = std::ldexp(1.0, 1 - lv.guard);   // largest first digit over the largest other one
   int n = 0;
   for (int g = 2; g <= G;) {
     OzBand b;
@@ -95,18 +115,17 @@ int make_bands(int S, int G, int bits, OzBand* out) {
     b.btop = (int16_t)(b.ngrp == 1 ? 0 : (b.bfirst ? g - 1 : S - 1));
     b.ntile = (int16_t)(2 * (b.btop + 1));
     // units of 64 2^(2 bits - 2) (64 products of two digits after the first)
-    // that one k-block adds to a group: 4 for (1,1), 2 for a pair with one
-    // first digit, 1 otherwise; the sum may reach 2^24
-    int worst = 0;
+    // that one k-block adds to a group; the sum may reach 2^24
+    double worst = 0;
     for (int q = 0; q < b.ngrp; ++q) {
-      int u = 0;
+      double u = 0;
       for (int a = 1; a < g + q; ++a) {
         const int c = g + q - a;
-        if (a <= S && c <= S) u += (a == 1 ? 2 : 1) * (c == 1 ? 2 : 1);
+        if (a <= S && c <= S) u += (a == 1 ? first : 1.0) * (c == 1 ? first : 1.0);
       }
       worst = std::max(worst, u);
     }
-    b.ck = (int16_t)std::max(1, (1 << (20 - 2 * bits)) / worst);
+    b.ck = (int16_t)std::max(1, (int)(std::ldexp(1.0, 20 - 2 * lv.bits) / worst));
     out[n++] = b;
     g += b.ngrp;
   }
@@ -136,49 +155,73 @@ __device__ __forceinline__ void unpack2(uint64_t d, uint32_t& x, uint32_t& y) {
   asm("mov.b64 {%0, %1}, %2;" : "=r"(x), "=r"(y) : "l"(d));
 }
 
-// two independent (hi + lo) += v * w in double-FP32: TwoSum of hi and v * w
-// (the product by a power of two is exact inside the fma), the error into lo,
-// renormalised
+// two independent (hi + lo) += v * w: TwoSum of hi and v * w (the product by a
+// power of two is exact inside the fma), the error into lo.  lo is left to grow
+// to a few last places of hi (n chunks: sqrt(n) / 2, n / 2 at most) and
+// renormalised once at the end: seven packed operations a chunk instead of ten,
+// and the FP32 pipe is what a drain takes (two clk per packed instruction).
 __device__ __forceinline__ void ff_add2(uint64_t& hi, uint64_t& lo, uint64_t v, uint64_t w, uint64_t m1) {
   const uint64_t s = fma2(v, w, hi);
   const uint64_t nbb = fma2(s, m1, hi);       // -(s - hi)
   const uint64_t t = add2(s, nbb);
-  const uint64_t err = add2(fma2(t, m1, hi), fma2(v, w, nbb));
-  const uint64_t l = add2(lo, err);
-  const uint64_t h = add2(s, l);
-  lo = fma2(fma2(s, m1, h), m1, l);
-  hi = h;
+  lo = add2(lo, add2(fma2(t, m1, hi), fma2(v, w, nbb)));
+  hi = s;
 }
 
-// (hi + lo) * 2^e as one FP64 number, rounded once, by integer arithmetic: lo
-// is turned into units of the 53-bit last place of hi (at most 2^29, one
-// float-to-integer conversion) and added to the bit pattern of hi.  The FP64
-// pipe (1/64 rate) would take two conversions and an addition per element.
-// |lo| <= ulp(hi) / 2, as ff_add2 leaves it; |hi| is 0 or at least 2^-72, the
-// smallest weight.  e >= 2^20 marks a row or column with infinities or NaN.
-__device__ __forceinline__ double ff_to_f64(uint32_t h, uint32_t l, int e, bool neg) {
+__device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
+  s = __fadd_rn(a, b);
+  const float bb = __fsub_rn(s, a);
+  e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+}
+
+// (hi + lo + tail) * 2^e as one FP64 number by integer arithmetic: lo and tail
+// are turned into units of the 53-bit last place of hi (lo at most 2^29, tail a
+// few) and added to the bit pattern of hi.  The FP64 pipe (1/64 rate) would take
+// three conversions and two additions per element.  |lo| <= ulp(hi) / 2; |hi| is
+// 0 or at least 2^-72, the smallest weight.  e >= 2^20 marks a row or column
+// with infinities or NaN.
+__device__ __forceinline__ double ff_to_f64(float hf, float lf, float tail, int e, uint32_t neg) {
+  const uint32_t h = __float_as_uint(hf);
   const int eh = (int)((h >> 23) & 0xFF);
   const uint32_t m = h & 0x7FFFFFu;
-  const int down = (m == 0 && (int)(h ^ l) < 0) ? 1 : 0;    // hi a power of two, |hi + lo| in the binade below
+  const uint32_t rest = __float_as_uint(__fadd_rn(lf, tail));
+  const int down = (m == 0 && (int)(h ^ rest) < 0) ? 1 : 0;   // hi a power of two, the sum in the binade below
   const float scale = __uint_as_float((uint32_t)(306 - eh + down) << 23);   // 1 / last place, 2^(179 - eh)
-  int t = __float2int_rn(__fmul_rn(__uint_as_float(l), scale));
+  int t = __float2int_rn(__fmul_rn(lf, scale)) + __float2int_rn(__fmul_rn(tail, scale));
   if ((int)h < 0) t = -t;
   const int ne = eh + 896 + e;                              // biased FP64 exponent of hi
-  const uint32_t sign = (h & 0x80000000u) ^ (neg ? 0x80000000u : 0u);
+  const uint32_t sign = (h ^ neg) & 0x80000000u;
   const uint64_t mag = ((uint64_t)(((uint32_t)ne << 20) | (m >> 3)) << 32 | (uint64_t)(m << 29)) + (uint64_t)(int64_t)t;
   uint32_t w1 = (uint32_t)(mag >> 32), w0 = (uint32_t)mag;
   if (eh == 0 || ne <= 0) w1 = w0 = 0;
-  if (ne > 2046) { w1 = 0x7FF00000u; w0 = 0; }
-  if (e >= (1 << 20)) w1 = 0x7FF80000u;
+  if (ne > 2046) { w1 = e >= (1 << 20) ? 0x7FF80000u : 0x7FF00000u; w0 = 0; }
+  if (eh == 0 && e >= (1 << 20)) w1 = 0x7FF80000u;
   return __longlong_as_double((long long)((uint64_t)(w1 | sign) << 32 | w0));
 }
 
-// Persistent: CTA b processes units b, b + gridDim.x, ...; unit u is job
-// u / tiles of output tile u % tiles.  The tile ring and the accumulator sets
-// run on across units, so the loads and MMAs of a unit's first chunks overlap
-// the previous unit's stores.  Every role walks the same sequence: parts,
+// The same where no exponent can leave the FP64 range (es = (e + 896) << 20,
+// |e| < 810): half the instructions.
+__device__ __forceinline__ double ff_to_f64_safe(float hf, float lf, float tail, int es, uint32_t neg) {
+  const uint32_t h = __float_as_uint(hf), a = h & 0x7FFFFFFFu, s = h ^ a;
+  const float l = __uint_as_float(__float_as_uint(lf) ^ s);      // relative to the sign of hi
+  const float x = __uint_as_float(__float_as_uint(tail) ^ s);
+  const uint32_t down = ((h & 0x7FFFFFu) == 0u && (int)__float_as_uint(__fadd_rn(l, x)) < 0) ? 1u << 23 : 0u;
+  const float scale = __uint_as_float((306u << 23) - (a & 0x7F800000u) + down);
+  const int t = __float2int_rn(__fmul_rn(l, scale)) + __float2int_rn(__fmul_rn(x, scale));
+  const uint64_t mag = ((uint64_t)((a >> 3) + (uint32_t)es) << 32 | (uint64_t)(h << 29)) + (uint64_t)(int64_t)t;
+  const uint32_t w1 = (uint32_t)(mag >> 32) | ((s ^ neg) & 0x80000000u);
+  return __hiloint2double(a ? (int)w1 : 0, a ? (int)(uint32_t)mag : 0);
+}
+
+// Persistent: CTA b processes units b, b + gridDim.x, ...; unit u is output
+// tile u % tiles of job (u / tiles) % njobs of product u / (tiles njobs).  The
+// tile ring and the accumulator sets run on across units, so the loads and MMAs
+// of a unit's first chunks overlap the previous unit's stores.  Every role walks the same sequence: parts,
 // L2 blocks of kper k-blocks (units running at the same time share one, so
 // the slices they stream stay in L2), bands, chunks of ck k-blocks.
+// F64: the FP64 level, whose store stage may take the last band's accumulators
+// along (P.merged).
+template <bool F64>
 __global__ void __launch_bounds__(OZ_THREADS, 1)
     gemm_oz_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    const __grid_constant__ OzParams P, const int* __restrict__ exA, const int* __restrict__ exB,
@@ -193,7 +236,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   __shared__ int abort_flag;
 
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  double* xp = reinterpret_cast<double*>(smem + OZ_SLOTS * OZ_TILE_BYTES);
+  float* xp = reinterpret_cast<float*>(smem + OZ_SLOTS * OZ_TILE_BYTES);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t tiles = P.tm * P.tn;
 
@@ -222,9 +265,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   const uint32_t tmem = tmem_holder;
 
   if (warp < 4) {
-    // 384 threads x 168 registers at launch; the epilogue warps take 216
-    // (128 x 56 + 256 x 216 = 62464 <= 64512)
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    // 384 threads x 168 registers at launch; the epilogue warps take 224
+    // (128 x 48 + 256 x 224 = 63488 <= 64512)
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
     if (warp == 0 || warp == 2) {
      if (elect_one()) {
       // ---------------- TMA producers: warp 0 streams the A tiles, warp 2 the
@@ -239,8 +282,10 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       for (uint32_t u = blockIdx.x; u < P.units && !stop; u += gridDim.x) {
         uint32_t mt, nt;
         grouped_tile(u % tiles, P.tm, P.tn, mt, nt);
-        const OzJob jb = P.job[u / tiles];
-        const int row = (int)(isB ? nt * OZ_BN : mt * OZ_BM);
+        const uint32_t q = u / tiles;
+        const OzJob jb = P.job[q % P.njobs];
+        const int64_t bq = q / P.njobs;
+        const int row = (int)(isB ? bq * ep.bb + nt * OZ_BN : bq * ep.ba + mt * OZ_BM);
         int bb = jb.b0;
         while (bb < jb.b1 && !stop) {
           const int be = (bb < P.cut) ? min(P.cut, (int)jb.b1) : (int)jb.b1;   // this part's bands
@@ -295,7 +340,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       uint32_t chunk = 0;
       bool ok = true;
       for (uint32_t u = blockIdx.x; u < P.units && ok; u += gridDim.x) {
-        const OzJob jb = P.job[u / tiles];
+        const OzJob jb = P.job[(u / tiles) % P.njobs];
         int bb = jb.b0;
         while (bb < jb.b1 && ok) {
           const int be = (bb < P.cut) ? min(P.cut, (int)jb.b1) : (int)jb.b1;
@@ -362,10 +407,10 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     }
   } else {
     // ---------------- epilogue warps: rows q*32 .. q*32+31, columns half*64 .. half*64+63 of each tile
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
     const int q = warp & 3, half = (warp - 4) >> 2;
     const uint32_t lanebase = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(half * 64);
-    double* tile = xp + (warp - 4) * 32 * OZ_XP_LD;
+    float* tile = xp + (warp - 4) * 3 * OZ_XP_PLANE;
     const uint64_t m1 = pack2(0xBF800000u, 0xBF800000u);   // -1, -1
     bool ok = true;
     uint32_t chunk = 0;
@@ -373,16 +418,34 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     const double alpha = P.part ? 1.0 : ep.alpha;
     const unsigned long long ab = (unsigned long long)__double_as_longlong(alpha);
     const bool apow2 = (ab & ((1ull << 52) - 1)) == 0 && ((ab >> 52) & 0x7FF) != 0;
-    const int ka = apow2 ? (int)((ab >> 52) & 0x7FF) - 1023 : 0;
-    const bool aneg = apow2 && (ab >> 63);
+    const int ka = (apow2 ? (int)((ab >> 52) & 0x7FF) - 1023 : 0) + 2 * P.guard;
+    const uint32_t aneg = apow2 && (ab >> 63) ? 0x80000000u : 0u;
+    const double alpha_left = apow2 ? 1.0 : alpha;
     for (uint32_t u = blockIdx.x; u < P.units && ok; u += gridDim.x) {
       uint32_t mt, nt;
       grouped_tile(u % tiles, P.tm, P.tn, mt, nt);
-      const int job = (int)(u / tiles);
-      const OzJob jb = P.job[job];
+      const uint32_t slot = u / tiles;           // (product, job)
+      const OzJob jb = P.job[slot % P.njobs];
+      const int64_t bq = slot / P.njobs;
       int bb = jb.b0;
       while (bb < jb.b1 && ok) {
         const int be = (bb < P.cut) ? min(P.cut, (int)jb.b1) : (int)jb.b1;
+        // what the store stage needs, read ahead of the sums
+        const int64_t m = (int64_t)mt * OZ_BM + q * 32 + lane;
+        int64_t crow = 0;
+        int erow = 0;
+        if (m < ep.M) {
+          crow = P.part ? ((int64_t)slot * ep.M + m) * ep.N : epi_row_off(ep, (uint32_t)m) + bq * ep.bc;
+          erow = oz_scale_exp(exA[bq * ep.ba + m]) + ka;
+        }
+        // this lane's share of the column exponents: columns lane and lane + 32
+        int ecl[2];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int64_t n = (int64_t)nt * OZ_BN + half * 64 + 32 * c + lane;
+          ecl[c] = n < ep.N ? oz_scale_exp(exB[bq * ep.bb + n]) : 0;
+        }
+        int last = -1;
         uint64_t hi[32], lo[32];
 #pragma unroll
         for (int c = 0; c < 32; ++c) hi[c] = lo[c] = 0ull;
@@ -400,8 +463,15 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                 break;
               }
               asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+              if (F64 && P.merged && b == jb.b1 - 1) {   // its one chunk is read in the store stage
+                last = set;
+                continue;
+              }
               // weight of the group, 2^(-bits g), exact in FP32; the
-              // accumulators hold exact integers of at most 2^24
+              // accumulators hold exact integers of at most 2^24.  16 columns
+              // at a time, each read while the ones before are added.
+              uint32_t x[2][16];
+              tmem_ld16(lanebase + (uint32_t)(set * 2 * OZ_BN + (g0 & 1) * OZ_BN), x[0]);
 #pragma unroll 1
               for (int gq = 0; gq < ng; ++gq) {
                 const int g = g0 + gq;
@@ -409,13 +479,13 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                 const uint64_t w = pack2(wb, wb);
                 const uint32_t col = lanebase + (uint32_t)(set * 2 * OZ_BN + (g & 1) * OZ_BN);
 #pragma unroll
-                for (int c0 = 0; c0 < 2; ++c0) {
-                  uint32_t acc[32];
-                  tmem_ld32(col + (uint32_t)(32 * c0), acc);
-                  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                for (int c = 0; c < 4; ++c) {
+                  tmem_wait(x[c & 1]);
+                  if (c < 3) tmem_ld16(col + 16 * (c + 1), x[(c + 1) & 1]);
+                  else if (gq + 1 < ng) tmem_ld16(lanebase + (uint32_t)(set * 2 * OZ_BN + ((g + 1) & 1) * OZ_BN), x[0]);
 #pragma unroll
-                  for (int j = 0; j < 16; ++j)
-                    ff_add2(hi[16 * c0 + j], lo[16 * c0 + j], pack2(acc[2 * j], acc[2 * j + 1]), w, m1);
+                  for (int j = 0; j < 8; ++j)
+                    ff_add2(hi[8 * c + j], lo[8 * c + j], pack2(x[c & 1][2 * j], x[c & 1][2 * j + 1]), w, m1);
                 }
               }
               asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -426,86 +496,111 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         }
         if (!ok) break;
         // ---- the part's sums, scaled, to the output
-        const int64_t m = (int64_t)mt * OZ_BM + q * 32 + lane;
-        int64_t crow = 0;
-        int erow = 0;
-        if (m < ep.M) {
-          crow = P.part ? ((int64_t)job * ep.M + m) * ep.N : epi_row_off(ep, (uint32_t)m);
-          erow = oz_scale_exp(exA[m]);
-        }
-        // this lane's share of the column exponents: columns lane and lane + 32
-        int ecl[2];
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const int64_t n = (int64_t)nt * OZ_BN + half * 64 + 32 * c + lane;
-          ecl[c] = n < ep.N ? oz_scale_exp(exB[n]) : 0;
-        }
         const bool first = bb == jb.b0;
         // 0: store, 1: add to the output, 2: add to beta times the output
         const int bmode = first ? (P.part || ep.beta == 0.0 ? 0 : (ep.beta == 1.0 ? 1 : 2)) : 1;
-        const bool plain = bmode == 0 && apow2;
         double* out = P.part ? P.part : static_cast<double*>(ep.C);
+        // rows this lane stores: 2 j + lane / 16
+        const int rows = (int)min((int64_t)32, ep.M - ((int64_t)mt * OZ_BM + q * 32));
+        // the usual case: factors of a power of two, exponents well inside the FP64 range
+        const bool plain = __all_sync(0xffffffffu, apow2 && bmode < 2 && abs(erow) < 400 && abs(ecl[0]) < 400 &&
+                                                       abs(ecl[1]) < 400);
+        const float w2 = __uint_as_float((uint32_t)(127 - P.bits * 2) << 23);
+        const float w3 = __uint_as_float((uint32_t)(127 - P.bits * 3) << 23);
 #pragma unroll
         for (int c0 = 0; c0 < 4; ++c0) {       // 16 columns at a time
           const int64_t nb = (int64_t)nt * OZ_BN + half * 64 + 16 * c0;
           if (nb >= ep.N) continue;
-          const int64_t nl = nb + (lane & 15);
           __syncwarp();
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            uint32_t h0, h1, l0, l1;
-            unpack2(hi[8 * c0 + j], h0, h1);
-            unpack2(lo[8 * c0 + j], l0, l1);
-            const int src = 16 * (c0 & 1) + 2 * j;
-            const int e0 = erow + __shfl_sync(0xffffffffu, ecl[c0 >> 1], src) + ka;
-            const int e1 = erow + __shfl_sync(0xffffffffu, ecl[c0 >> 1], src + 1) + ka;
-            tile[lane * OZ_XP_LD + 2 * j] = ff_to_f64(h0, l0, e0, aneg);
-            tile[lane * OZ_XP_LD + 2 * j + 1] = ff_to_f64(h1, l1, e1, aneg);
+          for (int c1 = 0; c1 < 2; ++c1) {
+            uint32_t a2[8], a3[8];
+            if (F64 && last >= 0) {            // groups 2 and 3, one chunk each
+              const uint32_t col = lanebase + (uint32_t)(last * 2 * OZ_BN + 16 * c0 + 8 * c1);
+              tmem_ld8(col, a2);
+              tmem_ld8(col + OZ_BN, a3);
+              tmem_wait(a2);
+              tmem_wait(a3);
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              uint32_t x[2], y[2];
+              unpack2(hi[8 * c0 + 4 * c1 + j / 2], x[0], x[1]);
+              unpack2(lo[8 * c0 + 4 * c1 + j / 2], y[0], y[1]);
+              // renormalised (|lo| is far below |hi| unless the sums cancelled,
+              // where the difference is exact)
+              const float h0 = __uint_as_float(x[j & 1]), l0 = __uint_as_float(y[j & 1]);
+              float h = __fadd_rn(h0, l0), l = __fsub_rn(l0, __fsub_rn(h, h0));
+              float* at = tile + lane * OZ_XP_LD + 8 * c1 + j;
+              if (F64 && last >= 0) {
+                // both groups are exact; their sum (f, r) and the others' (h, l)
+                // become f' + l' + tail
+                float f, r, g, d;
+                two_sum(__fmul_rn(__uint_as_float(a2[j]), w2), __fmul_rn(__uint_as_float(a3[j]), w3), f, r);
+                two_sum(r, h, g, d);
+                d = __fadd_rn(d, l);
+                two_sum(f, g, h, l);
+                // where f and g cancelled (l = 0) the tail can be as large as h
+                const bool z = l == 0.0f;
+                two_sum(h, z ? d : l, f, r);
+                h = f;
+                l = r;
+                at[2 * OZ_XP_PLANE] = z ? 0.0f : d;
+              }
+              at[0] = h;
+              at[OZ_XP_PLANE] = l;
+            }
           }
           __syncwarp();
+          // Each lane turns into FP64 what it stores: two rows of 16 columns per
+          // instruction, in a loop (unrolled over the registers of the sums, the
+          // conversion was 50 KB of code run once per tile, bound by instruction
+          // fetch).  Adding to the output is a reduction in L2 (red.add): no
+          // load to wait for, and the order is fixed all the same: within a
+          // launch one thread owns an element and its reductions reach it in
+          // program order.  Other factors go apart, because an FP64 instruction
+          // takes the pipe for 16 clk per warp even where it is predicated off.
+          const int64_t nl = nb + (lane & 15);
           const bool nok = nl < ep.N;
-          int64_t coff = 0;
-          if (nok) {
-            coff = P.part ? nl : epi_col_off(ep, (uint32_t)nl);
-          }
-          // Two rows of 16 columns per store.  The FP64 pipe takes 16 clk per
-          // warp instruction and SM, so the plain store issues none of it, and
-          // a branch, not a select, keeps the others out of it.
+          double* dst = out + (!nok ? 0 : (P.part ? nl : epi_col_off(ep, (uint32_t)nl)));
+          const int ec = __shfl_sync(0xffffffffu, ecl[c0 >> 1], 16 * (c0 & 1) + (lane & 15));
+          const float* src = tile + (lane >> 4) * OZ_XP_LD + (lane & 15);
           if (plain) {
+            const int esr = (erow + 896) << 20, esc = ec << 20;
 #pragma unroll 4
             for (int j = 0; j < 16; ++j) {
               const int r = 2 * j + (lane >> 4);
-              const int64_t off = __shfl_sync(0xffffffffu, crow, r) + coff;
-              if (nok && (int64_t)mt * OZ_BM + q * 32 + r < ep.M) out[off] = tile[r * OZ_XP_LD + (lane & 15)];
+              const int64_t off = __shfl_sync(0xffffffffu, crow, r);
+              const int es = __shfl_sync(0xffffffffu, esr, r) + esc;
+              const float* at = src + 2 * j * OZ_XP_LD;
+              const float tail = F64 && last >= 0 ? at[2 * OZ_XP_PLANE] : 0.0f;
+              const double v = F64 ? ff_to_f64_safe(at[0], at[OZ_XP_PLANE], tail, es, aneg)
+                                   : ff_to_f64_safe(at[0], at[OZ_XP_PLANE], 0.0f, es, aneg);
+              if (!nok || r >= rows) continue;
+              if (bmode == 0) dst[off] = v;
+              else atomicAdd(dst + off, v);
             }
           } else {
-            // what is added to is read first, four row pairs at a time
 #pragma unroll 1
-            for (int j0 = 0; j0 < 16; j0 += 4) {
-              double prev[4];
-              int64_t off[4];
-              bool okr[4];
-#pragma unroll
-              for (int jj = 0; jj < 4; ++jj) {
-                const int r = 2 * (j0 + jj) + (lane >> 4);
-                off[jj] = __shfl_sync(0xffffffffu, crow, r) + coff;
-                okr[jj] = nok && (int64_t)mt * OZ_BM + q * 32 + r < ep.M;
-                prev[jj] = 0.0;
-                if (bmode != 0 && okr[jj]) prev[jj] = out[off[jj]];
-              }
-              if (bmode == 2) {
-#pragma unroll
-                for (int jj = 0; jj < 4; ++jj) prev[jj] *= ep.beta;
-              }
-#pragma unroll
-              for (int jj = 0; jj < 4; ++jj) {
-                if (!okr[jj]) continue;
-                const double val = tile[(2 * (j0 + jj) + (lane >> 4)) * OZ_XP_LD + (lane & 15)];
-                out[off[jj]] = apow2 ? val + prev[jj] : alpha * val + prev[jj];
-              }
+            for (int j = 0; j < 16; ++j) {
+              const int r = 2 * j + (lane >> 4);
+              const int64_t off = __shfl_sync(0xffffffffu, crow, r);
+              const int e = __shfl_sync(0xffffffffu, erow, r) + ec;
+              const float* at = src + 2 * j * OZ_XP_LD;
+              const float tail = F64 && last >= 0 ? at[2 * OZ_XP_PLANE] : 0.0f;
+              const double v = alpha_left * ff_to_f64(at[0], at[OZ_XP_PLANE], tail, e, aneg);
+              if (!nok || r >= rows) continue;
+              if (bmode == 0) dst[off] = v;
+              else if (bmode == 1) atomicAdd(dst + off, v);
+              else dst[off] = v + ep.beta * dst[off];
             }
           }
           __syncwarp();
+        }
+        if (F64 && last >= 0) {
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&acce_bar[last]));
         }
         bb = be;
       }
@@ -532,6 +627,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
 __global__ void __launch_bounds__(256) oz_reduce_kernel(const double* __restrict__ part, int nhi, int njobs,
                                                         EpiMap ep) {
   const int64_t MN = ep.M * ep.N;
+  part += (int64_t)blockIdx.y * njobs * MN;
   auto sum = [&](int64_t t, int j0, int j1) {
     double s = 0.0;
     for (int j = j0; j < j1; j += 8) {   // eight loads in flight, added in order
@@ -548,7 +644,7 @@ __global__ void __launch_bounds__(256) oz_reduce_kernel(const double* __restrict
     double s = sum(t, 0, nhi);
     if (nhi < njobs) s += sum(t, nhi, njobs);
     const uint32_t m = (uint32_t)t / (uint32_t)ep.N, n = (uint32_t)t - m * (uint32_t)ep.N;
-    double* dst = static_cast<double*>(ep.C) + epi_row_off(ep, m) + epi_col_off(ep, n);
+    double* dst = static_cast<double*>(ep.C) + blockIdx.y * ep.bc + epi_row_off(ep, m) + epi_col_off(ep, n);
     if (ep.alpha != 1.0) s *= ep.alpha;
     if (ep.beta == 1.0) s += *dst;
     else if (ep.beta != 0.0) s += ep.beta * *dst;
@@ -563,31 +659,36 @@ std::once_flag g_oz_attr;
 OzLevel oz_level(int groups) {
   // up to 7 groups: 6-bit digits; above: the same 6 (groups - 1) bits or more
   // in 8-bit digits
-  if (groups <= 7) return OzLevel{groups - 1, groups, 0, 6};
+  if (groups <= 7) return OzLevel{groups - 1, groups, 0, 6, 0};
   const int S = (6 * (groups - 1) + 7) / 8;
-  return OzLevel{S, S + 1, 0, 8};
+  return OzLevel{S, S + 1, 0, 8, 0};
 }
 
 void gemm_oz(const __nv_bfloat16* A, int64_t a_rows, const int* exA, const __nv_bfloat16* B, int64_t b_rows,
              const int* exB, int64_t Kpad, OzLevel lv, const EpiMap& ep, DBuf<double>& ws, int* err, cudaStream_t s) {
   if (ep.M <= 0 || ep.N <= 0) return;
-  if (lv.S < 1 || lv.S > OZ_MAXS || lv.G < 2 || lv.G > lv.S + 2 || (lv.bits != 6 && lv.bits != 8)) fail(FCC_ERR_BAD_ARG, "bad exact-slice level");
+  if (lv.S < 1 || lv.S > OZ_MAXS || lv.G < 2 || lv.G > lv.S + 2 || (lv.bits != 6 && lv.bits != 8) || lv.guard < 0 || lv.guard > 2)
+    fail(FCC_ERR_BAD_ARG, "bad exact-slice level");
   if (Kpad <= 0 || Kpad % OZ_BK || Kpad > (1 << 27)) fail(FCC_ERR_BAD_ARG, "bad padded K");
-  if (a_rows < ep.M || b_rows < ep.N) fail(FCC_ERR_BAD_ARG, "packed operands smaller than the output");
+  if (ep.batch < 1 || ep.batch > 65535 || a_rows < ep.M + (ep.batch - 1) * ep.ba || b_rows < ep.N + (ep.batch - 1) * ep.bb)
+    fail(FCC_ERR_BAD_ARG, "packed operands smaller than the output");
   if (ep.M >= (int64_t(1) << 31) || ep.N >= (int64_t(1) << 31)) fail(FCC_ERR_BAD_ARG, "output extent too large");
   std::call_once(g_oz_attr, []() {
-    cudaFuncSetAttribute(gemm_oz_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM);
+    cudaFuncSetAttribute(gemm_oz_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM);
+    cudaFuncSetAttribute(gemm_oz_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM);
   });
   OzParams P;
   std::memset(&P, 0, sizeof(P));
-  const int nb = make_bands(lv.S, lv.G, lv.bits, P.band);
+  const int nb = make_bands(lv, P.band);
   P.bits = lv.bits;
+  P.guard = lv.guard;
   P.cut = lv.cut;
   P.kpad = (int)Kpad;
   const int nkb = (int)(Kpad / OZ_BK);
   const int64_t tm = (ep.M + OZ_BM - 1) / OZ_BM, tn = (ep.N + OZ_BN - 1) / OZ_BN;
   const int64_t tiles = tm * tn;
-  if (tiles * OZ_MAXJOBS >= (int64_t(1) << 31)) fail(FCC_ERR_BAD_ARG, "tensor-core grid too large");
+  if (tiles * OZ_MAXJOBS * ep.batch >= (int64_t(1) << 31) || a_rows >= (int64_t(1) << 31) || b_rows >= (int64_t(1) << 31))
+    fail(FCC_ERR_BAD_ARG, "tensor-core grid too large");
   P.tm = (uint32_t)tm;
   P.tn = (uint32_t)tn;
   // L2 blocks: the units that run at the same time (one per SM, about 8 tile
@@ -639,15 +740,15 @@ void gemm_oz(const __nv_bfloat16* A, int64_t a_rows, const int* exA, const __nv_
   for (int q = 0; q < 12; ++q) {
     const double target = q == 0 ? 0.0 : total / (double)(q < 5 ? q + 1 : (q < 9 ? 4 * (q - 3) : 36 << (q - 9)));
     const int n = build(target);
-    if (n < 1 || (q > 0 && (n == 1 || (double)n * ep.M * ep.N > (double)(32 << 20)))) continue;
+    if (n < 1 || (q > 0 && (n == 1 || (double)n * ep.batch * ep.M * ep.N > (double)(32 << 20)))) continue;
     // longest CTA under the static assignment of units to CTAs
-    const int64_t units = tiles * n;
+    const int64_t units = tiles * n * ep.batch;
     double t = 0;
     for (int c = 0; c < std::min<int64_t>(units, 4); ++c) {
       const int64_t cta = c == 0 ? 0 : (c == 1 ? std::min<int64_t>(units, 152) - 1 : (c == 2 ? 75 : 110));
       double l = 0;
       for (int64_t u = cta; u < units; u += 152) {
-        const OzJob& j = P.job[u / tiles];
+        const OzJob& j = P.job[(u / tiles) % n];
         double st = 0;
         for (int b = j.b0; b < j.b1; ++b) st += P.band[b].ntile - 1;
         l += st * (j.k1 - j.k0) + FIXED;
@@ -655,33 +756,44 @@ void gemm_oz(const __nv_bfloat16* A, int64_t a_rows, const int* exA, const __nv_
       }
       t = std::max(t, l);
     }
-    if (n > 1) t += REDUCE + (double)(n + 2) * ep.M * ep.N * 8.0 / 1e6;   // ~1 MB a step
+    if (n > 1) t += REDUCE + (double)(n + 2) * ep.batch * ep.M * ep.N * 8.0 / 1e6;   // ~1 MB a step
     if (t < best * 0.97) { best = t; best_target = target; }
   }
-  P.njobs = build(best_target);
-  P.units = (uint32_t)(tiles * P.njobs);
+  P.njobs = (uint32_t)build(best_target);
+  P.units = (uint32_t)(tiles * P.njobs * ep.batch);
   if (P.njobs > 1) {
-    const size_t need = (size_t)P.njobs * ep.M * ep.N;
+    const size_t need = (size_t)P.njobs * ep.batch * ep.M * ep.N;
     if (ws.n < need) ws.alloc(need);
     P.part = ws.p;
+  }
+  // One job and one chunk in the first band: the other bands go first, and the
+  // store stage adds the first band's two accumulators to their sums, so the
+  // output is converted and written once instead of twice.
+  if (lv.cut == 1 && P.njobs == 1 && P.band[0].ngrp == 2 && nkb <= P.band[0].ck) {
+    std::reverse(P.band, P.band + nb);
+    P.cut = 0;
+    P.merged = 1;
+    P.kper = std::max(P.kper, nkb);
   }
   CUtensorMap ta = tma_map_bf16(A, a_rows, lv.S * Kpad, OZ_BM);
   CUtensorMap tb = tma_map_bf16(B, b_rows, lv.S * Kpad, OZ_BN);
   const unsigned grid = (unsigned)std::min<int64_t>(P.units, 152);   // one persistent CTA per SM
   const int pidx = prof_begin(s);
-  gemm_oz_kernel<<<grid, OZ_THREADS, OZ_SMEM, s>>>(ta, tb, P, exA, exB, ep, err);
+  if (lv.cut) gemm_oz_kernel<true><<<grid, OZ_THREADS, OZ_SMEM, s>>>(ta, tb, P, exA, exB, ep, err);
+  else gemm_oz_kernel<false><<<grid, OZ_THREADS, OZ_SMEM, s>>>(ta, tb, P, exA, exB, ep, err);
   FCC_CHECK_LAUNCH();
   if (P.njobs > 1) {
     const int64_t MN = ep.M * ep.N;
-    int nhi = P.njobs;
+    int nhi = (int)P.njobs;
     if (lv.cut) {
       nhi = 0;
-      while (nhi < P.njobs && P.job[nhi].b0 < lv.cut) ++nhi;
+      while (nhi < (int)P.njobs && P.job[nhi].b0 < lv.cut) ++nhi;
     }
-    oz_reduce_kernel<<<(unsigned)std::min<int64_t>((MN + 255) / 256, 152 * 8), 256, 0, s>>>(ws.p, nhi, P.njobs, ep);
+    oz_reduce_kernel<<<dim3((unsigned)std::min<int64_t>((MN + 255) / 256, 152 * 8), (unsigned)ep.batch), 256, 0, s>>>(
+        ws.p, nhi, (int)P.njobs, ep);
     FCC_CHECK_LAUNCH();
   }
-  prof_end(s, pidx, PROF_OZ, ep.work > 0 ? ep.work : 2.0 * (double)ep.M * (double)ep.N * (double)Kpad * steps_kb);
+  prof_end(s, pidx, PROF_OZ, ep.work > 0 ? ep.work : 2.0 * ep.batch * (double)ep.M * (double)ep.N * (double)Kpad * steps_kb);
 }
 
 }  // namespace fcc

@@ -97,7 +97,7 @@ __device__ __forceinline__ uint32_t oz_byte_bits(uint32_t w, int sel) {
 // bf16 of a and b (upper halves) as one word, a in the lower half
 __device__ __forceinline__ uint32_t oz_pair(uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x7632); }
 
-// |x| 2^-e (|x| < 2^e) times 2^bits, rounded to an integer; bits <= 64
+// |x| 2^-e (|x| < 2^e; e includes the guard bits) times 2^bits, rounded to an integer; bits <= 64
 __device__ __forceinline__ unsigned long long oz_fixed(unsigned long long x, int e, int bits) {
   const int be = (int)((x >> 52) & 0x7FF);
   unsigned long long Z = 0;
@@ -167,7 +167,7 @@ __device__ __forceinline__ void oz_store4(const double (&xv)[4], int e, __nv_bfl
 // exponent and cut it.
 template <int S, int BITS>
 __global__ void __launch_bounds__(256) oz_pack_rows_fused_kernel(const double* __restrict__ src, PackSpec ps,
-                                                                 int64_t Kpad, int* __restrict__ ex,
+                                                                 int64_t Kpad, int guard, int* __restrict__ ex,
                                                                  __nv_bfloat16* __restrict__ dst, int lg) {
   __shared__ int red[8];
   const int tpr = 1 << lg, lane = threadIdx.x & (tpr - 1), rpb = 256 >> lg, sub = threadIdx.x >> lg;
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(256) oz_pack_rows_fused_kernel(const double* _
     }
     if (!ok) continue;   // every thread of the block runs the same number of rounds
     if (lane == 0) ex[r] = m;
-    const int e = oz_row_exp(m);
+    const int e = oz_row_exp(m) + guard;
     __nv_bfloat16* drow = dst + r * (S * Kpad);
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(256) oz_pack_rows_fused_kernel(const double* _
 // reduces the row exponents and cuts from there, two consecutive k per thread.
 template <int S, int BITS>
 __global__ void __launch_bounds__(256) oz_pack_tiles_fused_kernel(const double* __restrict__ src, PackSpec ps,
-                                                                  int64_t Kpad, int* __restrict__ ex,
+                                                                  int64_t Kpad, int guard, int* __restrict__ ex,
                                                                   __nv_bfloat16* __restrict__ dst) {
   extern __shared__ double ftile[];   // [K][33]
   __shared__ int64_t coff[TILE_KMAX];
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(256) oz_pack_tiles_fused_kernel(const double* 
       const int rr = rw + 16 * j;
       const int64_t r = r0 + rr;
       if (r >= ps.R) continue;
-      const int e = oz_row_exp(red[0][rr]);
+      const int e = oz_row_exp(red[0][rr]) + guard;
       for (int k = 2 * kp; k < (int)Kpad; k += 32) {
         uint32_t da[S], db[S];
         oz_digits<S, BITS>(k < K ? ftile[k * 33 + rr] : 0.0, e, da);
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(256) oz_pack_tiles_fused_kernel(const double* 
 // row, each cutting 4 consecutive k and writing one 8-byte word per slice
 // (zeros over the padding [K, Kpad))
 template <int S, int BITS>
-__global__ void __launch_bounds__(256) oz_pack_rows_kernel(const double* __restrict__ src, PackSpec ps, int64_t Kpad,
+__global__ void __launch_bounds__(256) oz_pack_rows_kernel(const double* __restrict__ src, PackSpec ps, int64_t Kpad, int guard,
                                                            const int* __restrict__ ex, __nv_bfloat16* __restrict__ dst,
                                                            PackWalk pw) {
   const int tpr = 1 << pw.lg, lane = threadIdx.x & (tpr - 1), rpb = 256 >> pw.lg;
@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(256) oz_pack_rows_kernel(const double* __restr
   for (int64_t u = (int64_t)blockIdx.x * rpb + (threadIdx.x >> pw.lg); u < units; u += (int64_t)gridDim.x * rpb) {
     const int64_t r = pw.nseg == 1 ? u : u / pw.nseg;
     const int64_t g0 = (u - r * pw.nseg) * pw.gseg, g1 = min(ng, g0 + pw.gseg);
-    const int e = oz_row_exp(ex[r]);
+    const int e = oz_row_exp(ex[r]) + guard;
     const int64_t ro = pack_row_off(ps, r);
     __nv_bfloat16* drow = dst + r * (S * Kpad);
     for (int64_t g = g0 + lane; g < g1; g += tpr) {
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(256) oz_pack_rows_kernel(const double* __restr
 // reads along rows, and each thread cuts two consecutive k of one row and
 // writes one 4-byte word per slice (the tiles cover [0, Kpad), zeros past K)
 template <int S, int BITS>
-__global__ void __launch_bounds__(256) oz_pack_tiles_kernel(const double* __restrict__ src, PackSpec ps, int64_t Kpad,
+__global__ void __launch_bounds__(256) oz_pack_tiles_kernel(const double* __restrict__ src, PackSpec ps, int64_t Kpad, int guard,
                                                             const int* __restrict__ ex,
                                                             __nv_bfloat16* __restrict__ dst) {
   __shared__ double tile[32][33];
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(256) oz_pack_tiles_kernel(const double* __rest
       const int rr = rw + 16 * j;
       const int64_t r = r0 + rr;
       if (r >= ps.R) continue;
-      const int e = oz_row_exp(ex[r]);
+      const int e = oz_row_exp(ex[r]) + guard;
       uint32_t da[S], db[S];
       oz_digits<S, BITS>(tile[2 * kp][rr], e, da);
       oz_digits<S, BITS>(tile[2 * kp + 1][rr], e, db);
@@ -340,7 +340,8 @@ bool pack_by_tiles(const PackSpec& ps) {
 
 // exponent pass, then the cut
 template <int S, int BITS>
-void pack_two_pass(const double* src, const PackSpec& ps, __nv_bfloat16* dst, int* ex, bool tiles, cudaStream_t s) {
+void pack_two_pass(const double* src, const PackSpec& ps, int guard, __nv_bfloat16* dst, int* ex, bool tiles,
+                   cudaStream_t s) {
   const int64_t Kpad = oz_kpad(ps.K);
   FCC_CUDA(cudaMemsetAsync(ex, 0, sizeof(int) * ps.R, s));
   // k-slabs so that the exponent pass has enough independent work
@@ -353,25 +354,25 @@ void pack_two_pass(const double* src, const PackSpec& ps, __nv_bfloat16* dst, in
     oz_exp_tiles_kernel<<<(unsigned)std::min<int64_t>(units * nks, 152 * 32), 256, 0, s>>>(src, ps, kslab, ex);
     FCC_CHECK_LAUNCH();
     const unsigned tgrid = (unsigned)std::min<int64_t>(((ps.R + 31) / 32) * (Kpad / 32), 152 * 16);
-    oz_pack_tiles_kernel<S, BITS><<<tgrid, 256, 0, s>>>(src, ps, Kpad, ex, dst);
+    oz_pack_tiles_kernel<S, BITS><<<tgrid, 256, 0, s>>>(src, ps, Kpad, guard, ex, dst);
   } else {
     const int64_t warps = units * nks;
     oz_exp_rows_kernel<<<(unsigned)std::min<int64_t>((warps + 7) / 8, 152 * 32), 256, 0, s>>>(src, ps, kslab, ex);
     FCC_CHECK_LAUNCH();
     const PackWalk pw = pack_walk(ps.R, Kpad / 4);
-    oz_pack_rows_kernel<S, BITS><<<pack_walk_grid(pw, ps.R), 256, 0, s>>>(src, ps, Kpad, ex, dst, pw);
+    oz_pack_rows_kernel<S, BITS><<<pack_walk_grid(pw, ps.R), 256, 0, s>>>(src, ps, Kpad, guard, ex, dst, pw);
   }
   FCC_CHECK_LAUNCH();
 }
 
 template <int S, int BITS>
-void pack(const double* src, const PackSpec& ps, __nv_bfloat16* dst, int* ex, cudaStream_t s) {
+void pack(const double* src, const PackSpec& ps, int guard, __nv_bfloat16* dst, int* ex, cudaStream_t s) {
   const int64_t Kpad = oz_kpad(ps.K);
   const bool tiles = pack_by_tiles(ps);
   const int64_t ntr = (ps.R + 31) / 32;
   if (tiles && ps.K <= TILE_KMAX) {
     oz_pack_tiles_fused_kernel<S, BITS><<<(unsigned)std::min<int64_t>(ntr, 152 * 16), 256, (size_t)ps.K * 33 * 8, s>>>(
-        src, ps, Kpad, ex, dst);
+        src, ps, Kpad, guard, ex, dst);
     FCC_CHECK_LAUNCH();
     return;
   }
@@ -381,40 +382,41 @@ void pack(const double* src, const PackSpec& ps, __nv_bfloat16* dst, int* ex, cu
     while ((int64_t(16) << lg) < Kpad) ++lg;
     const int64_t rpb = 256 >> lg;
     oz_pack_rows_fused_kernel<S, BITS><<<(unsigned)std::min<int64_t>((ps.R + rpb - 1) / rpb, 152 * 16), 256, 0, s>>>(
-        src, ps, Kpad, ex, dst, lg);
+        src, ps, Kpad, guard, ex, dst, lg);
     FCC_CHECK_LAUNCH();
     return;
   }
-  pack_two_pass<S, BITS>(src, ps, dst, ex, tiles, s);
+  pack_two_pass<S, BITS>(src, ps, guard, dst, ex, tiles, s);
 }
 
 }  // namespace
 
 int64_t oz_kpad(int64_t K) { return ((K + OZ_BK - 1) / OZ_BK) * OZ_BK; }
 
-void pack_oz(const double* src, const PackSpec& ps, int S, int bits, __nv_bfloat16* dst, int* ex, cudaStream_t s) {
+void pack_oz(const double* src, const PackSpec& ps, int S, int bits, int guard, __nv_bfloat16* dst, int* ex,
+             cudaStream_t s) {
   if (ps.R <= 0 || ps.K <= 0) return;
   if (ps.R >= (int64_t(1) << 31) || ps.K >= (int64_t(1) << 31)) fail(FCC_ERR_BAD_ARG, "pack extent too large");
   const int pidx = prof_begin(s);
   struct End { cudaStream_t s; int i; double b; ~End() { prof_end(s, i, PROF_PACK, b); } } pend{s, pidx,
       (double)ps.R * (double)ps.K * 8.0 + (double)ps.R * (double)(S * oz_kpad(ps.K)) * 2.0};
   switch (10 * bits + S) {
-    case 61: pack<1, 6>(src, ps, dst, ex, s); break;
-    case 62: pack<2, 6>(src, ps, dst, ex, s); break;
-    case 63: pack<3, 6>(src, ps, dst, ex, s); break;
-    case 64: pack<4, 6>(src, ps, dst, ex, s); break;
-    case 65: pack<5, 6>(src, ps, dst, ex, s); break;
-    case 66: pack<6, 6>(src, ps, dst, ex, s); break;
-    case 67: pack<7, 6>(src, ps, dst, ex, s); break;
-    case 68: pack<8, 6>(src, ps, dst, ex, s); break;
-    case 81: pack<1, 8>(src, ps, dst, ex, s); break;
-    case 82: pack<2, 8>(src, ps, dst, ex, s); break;
-    case 83: pack<3, 8>(src, ps, dst, ex, s); break;
-    case 84: pack<4, 8>(src, ps, dst, ex, s); break;
-    case 85: pack<5, 8>(src, ps, dst, ex, s); break;
-    case 86: pack<6, 8>(src, ps, dst, ex, s); break;
-    case 87: pack<7, 8>(src, ps, dst, ex, s); break;
-    case 88: pack<8, 8>(src, ps, dst, ex, s); break;
+    case 61: pack<1, 6>(src, ps, guard, dst, ex, s); break;
+    case 62: pack<2, 6>(src, ps, guard, dst, ex, s); break;
+    case 63: pack<3, 6>(src, ps, guard, dst, ex, s); break;
+    case 64: pack<4, 6>(src, ps, guard, dst, ex, s); break;
+    case 65: pack<5, 6>(src, ps, guard, dst, ex, s); break;
+    case 66: pack<6, 6>(src, ps, guard, dst, ex, s); break;
+    case 67: pack<7, 6>(src, ps, guard, dst, ex, s); break;
+    case 68: pack<8, 6>(src, ps, guard, dst, ex, s); break;
+    case 81: pack<1, 8>(src, ps, guard, dst, ex, s); break;
+    case 82: pack<2, 8>(src, ps, guard, dst, ex, s); break;
+    case 83: pack<3, 8>(src, ps, guard, dst, ex, s); break;
+    case 84: pack<4, 8>(src, ps, guard, dst, ex, s); break;
+    case 85: pack<5, 8>(src, ps, guard, dst, ex, s); break;
+    case 86: pack<6, 8>(src, ps, guard, dst, ex, s); break;
+    case 87: pack<7, 8>(src, ps, guard, dst, ex, s); break;
+    case 88: pack<8, 8>(src, ps, guard, dst, ex, s); break;
     default: fail(FCC_ERR_BAD_ARG, "bad slice count");
   }
 }

@@ -8,16 +8,24 @@
 // six-fold permutation sum of ijk.jl:121-137 with weight
 // (2 - d_ij - d_jk) / (D_ijkabc (1 + d_ab + d_bc)) over a >= b >= c.
 //
-// For a pair i >= j and a run of k <= j, each of the twelve contractions is
-// ONE DMMA launch over the whole run: the occupied index k joins the rows or
-// columns of the product (k-run views of (ia|bd), (li|jb) or t2), so W[k][a]
-// [b][c] for up to 32 k is built by twelve launches per pair instead of
-// twelve per triplet, with the index permutations in the operand and output
-// strides.  The energy kernel then works on 8 x 8 x 8 sub-cubes (blocks
-// A >= B >= C): it stages the six permutations of a sub-cube of W in shared
-// memory with loads along W's stride-1 index, forms V from T1 and (ia|jb)
-// blocks staged beside them, and reduces in FP64 into per-(k, sub-cube)
-// partials that are summed in a fixed order at the end.
+// Two of the twelve terms always share the occupied index of their two-electron
+// integral over virtuals and amplitude over l, so they are one product over the
+// concatenated index [d, l] of two arrays,
+//   F[x][y][z] = [ (xy|zd) | -t(x,l,y,z) ],  H[x][y][z] = [ t(x,y,z,d) | (ly|xz) ],
+//   W_ijk(a,b,c) = F[i](a,b) H[k][j](c) + F[j](b,a) H[k][i](c) + F[k](c,a) H[j][i](b)
+//                + F[i](a,c) H[j][k](b) + F[k](c,b) H[i][j](a) + F[j](b,c) H[i][k](a),
+// and F and H are cut into digit slices once.  For one j, a run of i >= j and
+// all k <= j the six terms are six exact-slice products at the FP64 level into
+// W[i][k][a][b][c] (the runs of i and k join the rows or columns, or are a batch
+// where their rows are not adjacent), with c or its run the columns so that
+// stores coalesce.  (Twelve FP64-pipe contractions per pair and run of k took
+// 0.54 s at (H2O)4 where this takes 0.04, of which the products' store stages
+// are the larger part: K = v + o is short.)  The energy kernel then works on 8 x
+// 8 x 8 sub-cubes (blocks A >= B >= C): it stages the six permutations of a
+// sub-cube of W in shared memory with loads along W's stride-1 index, forms V
+// from T1 and (ia|jb) blocks staged beside them, and reduces in FP64 into
+// per-(i, k, sub-cube) partials that are summed in a fixed order at the end.
+#include <algorithm>
 #include <cmath>
 
 #include "fcc_ctx.cuh"
@@ -39,15 +47,16 @@ struct TileTri {
   int16_t a, b, c, pad;
 };
 
-// Energy of the triplets (i, j, k0 + blockIdx.y) on the sub-cube
-// tiles[blockIdx.x] (blocks A >= B >= C), from W[kq][a][b][c].
-// part[k * ntiles + tile] accumulates over the calls in a fixed order.
+// Energy of the triplets (i0 + blockIdx.y / nk, j, k0 + blockIdx.y % nk) on the
+// sub-cube tiles[blockIdx.x] (blocks A >= B >= C), from W[blockIdx.y][a][b][c].
+// part[(i * o + k) * ntiles + tile] accumulates over the calls in a fixed order.
 __global__ void __launch_bounds__(EB) triples_energy_f64_kernel(const double* __restrict__ W,
                                                                 const TileTri* __restrict__ tiles, int ntiles,
                                                                 const double* __restrict__ t1,
                                                                 const double* __restrict__ ovov,
-                                                                const double* __restrict__ eps, int o, int v, int i,
-                                                                int j, int k0, double* __restrict__ part) {
+                                                                const double* __restrict__ eps, int o, int v,
+                                                                int i0, int j, int k0, int nk,
+                                                                double* __restrict__ part) {
   __shared__ double Wt[6][ET][ET][ET + 1];   // W on the six permutations of the sub-cube
   __shared__ double Mjk[3][3][ET][ET + 1];   // (j y|k z) for y in block r1, z in block r2
   __shared__ double Mik[3][3][ET][ET + 1];
@@ -55,7 +64,7 @@ __global__ void __launch_bounds__(EB) triples_energy_f64_kernel(const double* __
   __shared__ double T1[3][3][ET];            // t1 of i, j, k on block r
   __shared__ double epsv[3][ET];
   __shared__ double red[EB / 32];
-  const int kq = blockIdx.y, k = k0 + kq;
+  const int kq = blockIdx.y, i = i0 + kq / nk, k = k0 + kq % nk;
   if (i == j && j == k) return;              // weight 2 - d_ij - d_jk = 0
   const TileTri tt = tiles[blockIdx.x];
   const int oa = tt.a * ET, ob = tt.b * ET, oc = tt.c * ET;
@@ -149,7 +158,7 @@ __global__ void __launch_bounds__(EB) triples_energy_f64_kernel(const double* __
   if (t == 0) {
     double s = 0.0;
     for (int q = 0; q < EB / 32; ++q) s += red[q];
-    part[(int64_t)k * ntiles + blockIdx.x] += (2.0 - (i == j) - (j == k)) * s;
+    part[((int64_t)i * o + k) * ntiles + blockIdx.x] += (2.0 - (i == j) - (j == k)) * s;
   }
 }
 
@@ -175,18 +184,55 @@ double triples_fp64(fcc_ctx* c, const std::vector<int3>* subset, std::vector<dou
   c->tc.enabled = false;
   reset_device_error(c);
   const int64_t o = c->o, v = c->v, Q = c->Q, n = c->n;
-  const int64_t v2 = v * v, v3 = v2 * v, ov2 = o * v2, o2v = o * o * v;
+  const int64_t v2 = v * v, v3 = v2 * v;
+  const int64_t Kc = v + o;
   TView B = rm(c->B.p, {Q, n, n});
   TView Boo = slice(slice(B, 1, 0, o), 2, 0, o);
   TView Bov = slice(slice(B, 1, 0, o), 2, o, v);
   TView Bvv = slice(slice(B, 1, o, v), 2, o, v);
-  c->ovvv.alloc(o * v3);
-  c->ooov.alloc(o * o2v);
-  einsum(1.0, "Qia,Qbd->iabd", Bov, Bvv, 0.0, rm(c->ovvv.p, {o, v, v, v}), s);   // (ia|bd) [i][a][b][d]
-  einsum(1.0, "Qli,Qjb->lijb", Boo, Bov, 0.0, rm(c->ooov.p, {o, o, o, v}), s);   // (li|jb) [l][i][j][b]
-  // runs of up to KC values of k: W holds KC * v^3 doubles (at most ~2 GB)
-  const int64_t KC = std::max<int64_t>(1, std::min<int64_t>(o, (int64_t)(2ll << 30) / (8 * v3)));
-  c->Wt.alloc(KC * v3);
+  TView t2v = rm(c->t2.p, {o, o, v, v});
+  // F and H in FP64, then their digit slices: F by (x, y, z) and by (x, z, y),
+  // H by (x, y, z) and by (y, x, z), so that every run below is adjacent rows
+  const OzLevel lv = OZ_F64;
+  const int64_t Kpad = oz_kpad(Kc), rowlen = lv.S * Kpad;
+  const int64_t RF = o * v2, RH = o * o * v;
+  DBuf<__nv_bfloat16> pF, pF2, pHx, pHy;
+  DBuf<int> eF, eF2, eHx, eHy;
+  auto pack = [&](DBuf<double>& src, int64_t d1, int64_t d2, int64_t d3, int64_t s1, int64_t s2, int64_t s3,
+                  DBuf<__nv_bfloat16>& dst, DBuf<int>& ex) {
+    PackSpec ps{};
+    ps.R = d1 * d2 * d3;
+    ps.K = Kc;
+    ps.Kp = rowlen;
+    ps.rd2 = d2; ps.rd3 = d3; ps.rs1 = s1 * Kc; ps.rs2 = s2 * Kc; ps.rs3 = s3 * Kc;
+    ps.kd2 = 1; ps.kd3 = Kc; ps.ks3 = 1;
+    dst.alloc(ps.R * rowlen);
+    ex.alloc(ps.R);
+    pack_oz(src.p, ps, lv.S, lv.bits, lv.guard, dst.p, ex.p, s);
+  };
+  {
+    DBuf<double> F;
+    F.alloc(RF * Kc);
+    TView Fv = rm(F.p, {o, v, v, Kc});
+    einsum(1.0, "Qia,Qbd->iabd", Bov, Bvv, 0.0, slice(Fv, 3, 0, v), s);           // (xy|zd)
+    einsum1(-1.0, "xlyz->xyzl", t2v, 0.0, slice(Fv, 3, v, o), s);
+    pack(F, o, v, v, v2, v, 1, pF, eF);
+    pack(F, o, v, v, v2, 1, v, pF2, eF2);
+    DBuf<double> H;
+    H.alloc(RH * Kc);
+    TView Hv = rm(H.p, {o, o, v, Kc});
+    einsum1(1.0, "xyzd->xyzd", t2v, 0.0, slice(Hv, 3, 0, v), s);
+    einsum(1.0, "Qly,Qxz->xyzl", Boo, Bov, 0.0, slice(Hv, 3, v, o), s);           // (ly|xz)
+    pack(H, o, o, v, o * v, v, 1, pHx, eHx);
+    pack(H, o, o, v, v, o * v, 1, pHy, eHy);
+    FCC_CUDA(cudaStreamSynchronize(s));   // F and H are freed here
+  }
+  // W for a run of i and of k: at most ~2 GB
+  const int64_t slots_max = std::max<int64_t>(1, (int64_t)(2ll << 30) / (8 * v3));
+  int64_t slots = 0;   // the largest run of any j
+  for (int64_t j = 0; j < o; ++j) slots = std::max(slots, (o - j) * (j + 1));
+  slots = subset ? 1 : std::min(slots, slots_max);
+  c->Wt.alloc(slots * v3);
   const int nt = (int)((v + ET - 1) / ET);
   std::vector<TileTri> th;
   for (int a = 0; a < nt; ++a)
@@ -197,55 +243,56 @@ double triples_fp64(fcc_ctx* c, const std::vector<int3>* subset, std::vector<dou
   tiles.alloc(ntiles);
   FCC_CUDA(cudaMemcpyAsync(tiles.p, th.data(), sizeof(TileTri) * ntiles, cudaMemcpyHostToDevice, s));
   DBuf<double> part, out;
-  part.alloc(o * ntiles);
+  part.alloc(o * o * ntiles);
   out.alloc(1);
   part.zero(s);
 
-  double* ovvv = c->ovvv.p;
-  double* ooov = c->ooov.p;
-  double* t2 = c->t2.p;
-  auto view = [](double* p, std::initializer_list<int64_t> dims, std::initializer_list<int64_t> strides) {
-    TView r;
-    r.p = p;
-    r.rank = (int)dims.size();
-    int q = 0;
-    for (auto d : dims) r.dim[q++] = d;
-    q = 0;
-    for (auto st : strides) r.str[q++] = st;
-    return r;
+  // One product: rows m of A (packed rows ar0..), columns n of B (br0..), each a
+  // three-level index with the given strides in W
+  struct Ix3 { int64_t d2, d3, s1, s2, s3; };
+  auto product = [&](const DBuf<__nv_bfloat16>& pa, const DBuf<int>& ea, int64_t ra, int64_t ar0, int64_t M, Ix3 m,
+                     const DBuf<__nv_bfloat16>& pb, const DBuf<int>& eb, int64_t rb, int64_t br0, int64_t N, Ix3 nn,
+                     double beta, int64_t batch, int64_t ba, int64_t bb, int64_t bc) {
+    EpiMap ep;
+    ep.M = M; ep.N = N;
+    ep.md2 = m.d2; ep.md3 = m.d3; ep.ms1 = m.s1; ep.ms2 = m.s2; ep.ms3 = m.s3;
+    ep.nd2 = nn.d2; ep.nd3 = nn.d3; ep.ns1 = nn.s1; ep.ns2 = nn.s2; ep.ns3 = nn.s3;
+    ep.beta = beta;
+    ep.C = c->Wt.p;
+    ep.batch = (int)batch; ep.ba = ba; ep.bb = bb; ep.bc = bc;
+    ep.work = 2.0 * (double)batch * (double)M * (double)N * (double)Kc * oz_pairs(lv);
+    gemm_oz(pa.p + ar0 * rowlen, ra - ar0, ea.p + ar0, pb.p + br0 * rowlen, rb - br0, eb.p + br0, Kpad, lv, ep,
+            c->tc.ozws, c->tc.err, s);
   };
-  // W[k][a][b][c] for k in [k0, k0 + nk) from the twelve terms of ijk.jl:109-114
-  auto build_w = [&](int64_t i, int64_t j, int64_t k0, int64_t nk) {
-    TView W = rm(c->Wt.p, {nk, v, v, v});
-    auto ov3 = [&](int64_t x) { return view(ovvv + x * v3, {v, v, v}, {v2, v, 1}); };             // (x a|b d)
-    TView ov3k = view(ovvv + k0 * v3, {nk, v, v, v}, {v3, v2, v, 1});                              // (k a|b d)
-    auto t2pair = [&](int64_t x, int64_t y) { return view(t2 + (x * o + y) * v2, {v, v}, {v, 1}); };
-    auto t2pairk = [&](int64_t y) { return view(t2 + (k0 * o + y) * v2, {nk, v, v}, {ov2, v, 1}); };   // t(k,y)
-    auto t2row = [&](int64_t x) { return view(t2 + x * ov2, {o, v, v}, {v2, v, 1}); };              // t(x, l)
-    TView t2rowk = view(t2 + k0 * ov2, {nk, o, v, v}, {ov2, v2, v, 1});                            // t(k, l)
-    auto oo = [&](int64_t x, int64_t y) { return view(ooov + (x * o + y) * v, {o, v}, {o2v, 1}); };   // (l x|y b)
-    auto oo_k_y = [&](int64_t y) { return view(ooov + (k0 * o + y) * v, {o, nk, v}, {o2v, o * v, 1}); };   // (l k|y b)
-    auto oo_x_k = [&](int64_t x) { return view(ooov + (x * o + k0) * v, {o, nk, v}, {o2v, v, 1}); };       // (l x|k b)
-    einsum(1.0, "abd,kcd->kabc", ov3(i), t2pairk(j), 0.0, W, s);     // :109
-    einsum(-1.0, "lb,klca->kabc", oo(i, j), t2rowk, 1.0, W, s);
-    einsum(1.0, "bad,kcd->kabc", ov3(j), t2pairk(i), 1.0, W, s);     // :110
-    einsum(-1.0, "la,klcb->kabc", oo(j, i), t2rowk, 1.0, W, s);
-    einsum(1.0, "kcad,bd->kabc", ov3k, t2pair(j, i), 1.0, W, s);     // :111
-    einsum(-1.0, "lka,lbc->kabc", oo_k_y(i), t2row(j), 1.0, W, s);
-    einsum(1.0, "kcbd,da->kabc", ov3k, t2pair(j, i), 1.0, W, s);     // :112
-    einsum(-1.0, "lkb,lac->kabc", oo_k_y(j), t2row(i), 1.0, W, s);
-    einsum(1.0, "acd,kdb->kabc", ov3(i), t2pairk(j), 1.0, W, s);     // :113
-    einsum(-1.0, "lkc,lba->kabc", oo_x_k(i), t2row(j), 1.0, W, s);
-    einsum(1.0, "bcd,kda->kabc", ov3(j), t2pairk(i), 1.0, W, s);     // :114
-    einsum(-1.0, "lkc,lab->kabc", oo_x_k(j), t2row(i), 1.0, W, s);
+  // W[i][k][a][b][c] for i in [i0, i0 + ni), k in [k0, k0 + nk) and one j
+  auto build_w = [&](int64_t i0, int64_t ni, int64_t j, int64_t k0, int64_t nk) {
+    const int64_t ws = nk * v3;   // stride of i
+    // F[i](a,b) H[k][j](c): rows (i,a,b), columns (k,c)
+    product(pF, eF, RF, i0 * v2, ni * v2, {v, v, ws, v2, v}, pHy, eHy, RH, (j * o + k0) * v, nk * v,
+            {nk, v, 0, v3, 1}, 0.0, 1, 0, 0, 0);
+    // F[j](b,a) H[k][i](c): rows (b,a), columns (k,c), a product per i
+    product(pF, eF, RF, j * v2, v2, {v, v, 0, v, v2}, pHy, eHy, RH, (i0 * o + k0) * v, nk * v, {nk, v, 0, v3, 1}, 1.0,
+            ni, 0, o * v, ws);
+    // H[j][i](b) F[k](c,a): rows (i,b), columns (k,a,c)
+    product(pHx, eHx, RH, (j * o + i0) * v, ni * v, {ni, v, 0, ws, v}, pF2, eF2, RF, k0 * v2, nk * v2,
+            {v, v, v3, v2, 1}, 1.0, 1, 0, 0, 0);
+    // H[j][k](b) F[i](a,c): rows (k,b), columns (i,a,c)
+    product(pHx, eHx, RH, (j * o + k0) * v, nk * v, {nk, v, 0, v3, v}, pF, eF, RF, i0 * v2, ni * v2,
+            {v, v, ws, v2, 1}, 1.0, 1, 0, 0, 0);
+    // H[i][j](a) F[k](c,b): rows (i,a), columns (k,b,c)
+    product(pHy, eHy, RH, (j * o + i0) * v, ni * v, {ni, v, 0, ws, v2}, pF2, eF2, RF, k0 * v2, nk * v2,
+            {v, v, v3, v, 1}, 1.0, 1, 0, 0, 0);
+    // H[i][k](a) F[j](b,c): rows (k,a), columns (b,c), a product per i
+    product(pHx, eHx, RH, (i0 * o + k0) * v, nk * v, {nk, v, 0, v3, v2}, pF, eF, RF, j * v2, v2, {v, v, 0, v, 1}, 1.0,
+            ni, o * v, 0, ws);
   };
-  auto energy = [&](int64_t i, int64_t j, int64_t k0, int64_t nk) {
+  auto energy = [&](int64_t i0, int64_t ni, int64_t j, int64_t k0, int64_t nk) {
     const int pe = prof_begin(s);
-    dim3 g((unsigned)ntiles, (unsigned)nk);
+    dim3 g((unsigned)ntiles, (unsigned)(ni * nk));
     triples_energy_f64_kernel<<<g, EB, 0, s>>>(c->Wt.p, tiles.p, ntiles, c->t1.p, c->ovov.p, c->eps.p, (int)o, (int)v,
-                                               (int)i, (int)j, (int)k0, part.p);
+                                               (int)i0, (int)j, (int)k0, (int)nk, part.p);
     FCC_CHECK_LAUNCH();
-    prof_end(s, pe, PROF_TRIPLES, (double)nk * (double)v * (v + 1) * (v + 2) / 6.0);
+    prof_end(s, pe, PROF_TRIPLES, (double)ni * (double)nk * (double)v * (v + 1) * (v + 2) / 6.0);
   };
   if (subset) {
     // one triplet at a time, each energy read separately
@@ -253,30 +300,31 @@ double triples_fp64(fcc_ctx* c, const std::vector<int3>* subset, std::vector<dou
     for (size_t q = 0; q < subset->size(); ++q) {
       const int3 t = (*subset)[q];
       part.zero(s);
-      build_w(t.x, t.y, t.z, 1);
-      energy(t.x, t.y, t.z, 1);
-      sum_kernel<<<1, 1024, 0, s>>>(part.p, (int)(o * ntiles), out.p);
+      build_w(t.x, 1, t.y, t.z, 1);
+      energy(t.x, 1, t.y, t.z, 1);
+      sum_kernel<<<1, 1024, 0, s>>>(part.p, (int)(o * o * ntiles), out.p);
       FCC_CHECK_LAUNCH();
       FCC_CUDA(cudaMemcpyAsync(&(*each)[q], out.p, sizeof(double), cudaMemcpyDeviceToHost, s));
     }
     FCC_CUDA(cudaStreamSynchronize(s));
   } else {
-    for (int64_t i = 0; i < o; ++i)
-      for (int64_t j = 0; j <= i; ++j)
-        for (int64_t k0 = 0; k0 <= j; k0 += KC) {
-          const int64_t nk = std::min<int64_t>(KC, j + 1 - k0);
-          if (i == j && j == k0 && nk == 1) continue;   // i = j = k only: weight 0
-          build_w(i, j, k0, nk);
-          energy(i, j, k0, nk);
+    for (int64_t j = 0; j < o; ++j) {
+      const int64_t nk = std::min<int64_t>(j + 1, slots);
+      const int64_t ni = std::min<int64_t>(std::max<int64_t>(1, slots / nk), 32768 / nk);
+      for (int64_t k0 = 0; k0 <= j; k0 += nk)
+        for (int64_t i0 = j; i0 < o; i0 += ni) {
+          const int64_t kk = std::min(nk, j + 1 - k0), ii = std::min(ni, o - i0);
+          if (ii == 1 && i0 == j && k0 == j) continue;   // i = j = k only: weight 0
+          build_w(i0, ii, j, k0, kk);
+          energy(i0, ii, j, k0, kk);
         }
+    }
   }
-  sum_kernel<<<1, 1024, 0, s>>>(part.p, (int)(o * ntiles), out.p);
+  sum_kernel<<<1, 1024, 0, s>>>(part.p, (int)(o * o * ntiles), out.p);
   FCC_CHECK_LAUNCH();
   double et = 0.0;
   FCC_CUDA(cudaMemcpyAsync(&et, out.p, sizeof(double), cudaMemcpyDeviceToHost, s));
   check_device_error(c, "(T)");
-  c->ovvv.release();
-  c->ooov.release();
   c->Wt.release();
   return subset ? 0.0 : et;
 }

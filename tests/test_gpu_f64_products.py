@@ -67,6 +67,24 @@ def test_no_less_accurate_than_the_fp64_pipe(M, N, K, spread):
     assert err[TC] <= max(err[PIPE], 2.0 ** -53), err
 
 
+# Sums far below their terms: the leading groups of the exact-slice sums cancel
+# and the rest decides.  Every operand is cut 2^-62 below its row's scale (up to
+# twice the maximum) and pairs of weight 2^-76 of it are dropped, seven of 2^14
+# at most per term: 2^-58 of the scales together, 2^-56 of the maxima.
+@pytest.mark.parametrize("M,N,K", [(130, 400, 16), (300, 257, 64), (500, 260, 336), (260, 250, 1024), (250, 260, 1088)])
+@pytest.mark.parametrize("level", [4, 13, 22, 30, 45])
+def test_sums_that_cancel(M, N, K, level):
+    rng = np.random.default_rng(K + level)
+    a, b = rng.standard_normal((M, K // 2)), rng.standard_normal((N, K // 2))
+    A = np.concatenate([a, -a * (1 + 2.0 ** -level * rng.standard_normal(a.shape))], 1)
+    B = np.concatenate([b, b], 1)
+    rc, out = _run(TC, "mk,nk->mn", A, B, np.zeros((M, N)))
+    assert rc == 0
+    ref = _quad(A, B)
+    scale = np.abs(A).max(1)[:, None] * np.abs(B).max(1)[None, :]
+    assert np.all(np.abs(out - ref) <= K * 2.0 ** -56 * scale + 2.0 ** -53 * np.abs(ref))
+
+
 def test_peaked_rows_against_a_metric():
     # rows with a few large entries against the inverse square root of a nearly
     # dependent metric: the largest entries of one side meet the smallest of the
