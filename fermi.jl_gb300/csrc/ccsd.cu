@@ -648,8 +648,9 @@ void residual(fcc_ctx* c) {
     TcEngine* tc = tc_engine();
     const bool exact = tc && (tc->exact || !tc->enabled);
     const OzLevel lv = tc && tc->enabled ? tc->oz : OZ_F64;
-    const bool tcw = tc && (tc->enabled || 2.0 * v * v * v * (double)v * Q >= tc->f64_min_flops);
     const int64_t R = v * v;
+    const bool tcw = tc && (tc->enabled || (2.0 * v * v * v * (double)v * Q >= tc->f64_min_flops &&
+                                            scratch_fits(2.0 * ((double)R * lv.S * oz_kpad(Q) - (double)c->bvvA.n))));
     int64_t Wk = 0;   // packed row length
     if (tcw) {
       PackSpec ps{};

@@ -813,6 +813,14 @@ void run_tc(TcEngine* tc, OzLevel lv, double alpha, const TView& A, const TView&
 
 }  // namespace
 
+// The slices take twice the memory of an FP64 operand.  Large ones are taken
+// only while they leave half of the free memory; the FP64 pipe needs none.
+bool scratch_fits(double bytes) {
+  if (bytes < 4e9) return true;
+  size_t f = 0, t = 0;
+  return cudaMemGetInfo(&f, &t) == cudaSuccess && bytes <= 0.5 * (double)f;
+}
+
 static std::atomic<int64_t> g_launches{0};
 void note_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 int64_t launch_count() { return g_launches.load(std::memory_order_relaxed); }
@@ -825,6 +833,12 @@ TcEngine*& tc_engine() {
 DBuf<double>*& f64_workspace() {
   thread_local DBuf<double>* w = nullptr;
   return w;
+}
+
+// bytes by which run_tc would grow the engine's buffers for a product
+static double pack_growth(const TcEngine* tc, const OzLevel& lv, int64_t M, int64_t N, int64_t K) {
+  const double w = (double)lv.S * (double)oz_kpad(K);
+  return 2.0 * (std::max(0.0, (double)M * w - (double)tc->bufA.n) + std::max(0.0, (double)N * w - (double)tc->bufB.n));
 }
 
 void einsum(double alpha, const char* spec, const TView& A, const TView& B, double beta, const TView& C,
@@ -869,7 +883,8 @@ void einsum(double alpha, const char* spec, const TView& A, const TView& B, doub
   if (tc && gb.empty()) {
     const double flops = 2.0 * (double)gdim(gm) * (double)gdim(gn) * (double)gdim(gk);
     std::vector<Ix> m3 = gm, n3 = gn, k3 = gk;
-    if (flops >= tc->f64_min_flops && gdim(gm) > 1 && gdim(gn) > 1 && try_fuse(m3, 3) && try_fuse(n3, 3) && try_fuse(k3, 3)) {
+    if (flops >= tc->f64_min_flops && gdim(gm) > 1 && gdim(gn) > 1 && try_fuse(m3, 3) && try_fuse(n3, 3) && try_fuse(k3, 3) &&
+        scratch_fits(pack_growth(tc, OZ_F64, gdim(gm), gdim(gn), gdim(gk)))) {
       run_tc(tc, OZ_F64, alpha, A, B, beta, C, m3, n3, k3, s);
       return;
     }

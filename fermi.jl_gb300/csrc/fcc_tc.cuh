@@ -161,6 +161,9 @@ void gemm_bf16x3(const __nv_bfloat16* A, int64_t a_rows, int64_t a_row0, const _
 // (one 128-byte swizzle atom) x box_rows rows; cols must be a multiple of 64.
 CUtensorMap tma_map_bf16(const __nv_bfloat16* base, int64_t rows, int64_t cols, int box_rows);
 
+// whether scratch of that many bytes is small or leaves half of the free memory
+bool scratch_fits(double bytes);
+
 // Exact-slice products (the Ozaki scheme: Ozaki, Ogita, Oishi & Rump, Numer.
 // Algorithms 59, 95 (2012); on tensor cores: Mukunoki et al., ISC 2020).
 // Each row r of an operand is scaled by 2^e_r (|x| < 2^e_r over the row) and

@@ -196,43 +196,67 @@ double triples_fp64(fcc_ctx* c, const std::vector<int3>* subset, std::vector<dou
   const OzLevel lv = OZ_F64;
   const int64_t Kpad = oz_kpad(Kc), rowlen = lv.S * Kpad;
   const int64_t RF = o * v2, RH = o * o * v;
-  DBuf<__nv_bfloat16> pF, pF2, pHx, pHy;
-  DBuf<int> eF, eF2, eHx, eHy;
-  auto pack = [&](DBuf<double>& src, int64_t d1, int64_t d2, int64_t d3, int64_t s1, int64_t s2, int64_t s3,
-                  DBuf<__nv_bfloat16>& dst, DBuf<int>& ex) {
+  // one packed operand: its rows from a first row on
+  struct Packed {
+    DBuf<__nv_bfloat16> p;
+    DBuf<int> e;
+    void alloc(int64_t rows, int64_t rowlen) { p.alloc(rows * rowlen); e.alloc(rows); }
+  };
+  struct Rows { const __nv_bfloat16* p; const int* e; int64_t n; };
+  Packed pF, pF2, pHx, pHy, pFj;
+  auto rows = [&](const Packed& x, int64_t r0) { return Rows{x.p.p + r0 * rowlen, x.e.p + r0, (int64_t)x.e.n - r0}; };
+  auto pack = [&](const double* src, int64_t d1, int64_t d2, int64_t d3, int64_t s1, int64_t s2, int64_t s3, Packed& dst) {
     PackSpec ps{};
     ps.R = d1 * d2 * d3;
     ps.K = Kc;
     ps.Kp = rowlen;
     ps.rd2 = d2; ps.rd3 = d3; ps.rs1 = s1 * Kc; ps.rs2 = s2 * Kc; ps.rs3 = s3 * Kc;
     ps.kd2 = 1; ps.kd3 = Kc; ps.ks3 = 1;
-    dst.alloc(ps.R * rowlen);
-    ex.alloc(ps.R);
-    pack_oz(src.p, ps, lv.S, lv.bits, lv.guard, dst.p, ex.p, s);
+    pack_oz(src, ps, lv.S, lv.bits, lv.guard, dst.p.p, dst.e.p, s);
   };
   {
-    DBuf<double> F;
-    F.alloc(RF * Kc);
-    TView Fv = rm(F.p, {o, v, v, Kc});
-    einsum(1.0, "Qia,Qbd->iabd", Bov, Bvv, 0.0, slice(Fv, 3, 0, v), s);           // (xy|zd)
-    einsum1(-1.0, "xlyz->xyzl", t2v, 0.0, slice(Fv, 3, v, o), s);
-    pack(F, o, v, v, v2, v, 1, pF, eF);
-    pack(F, o, v, v, v2, 1, v, pF2, eF2);
     DBuf<double> H;
     H.alloc(RH * Kc);
     TView Hv = rm(H.p, {o, o, v, Kc});
     einsum1(1.0, "xyzd->xyzd", t2v, 0.0, slice(Hv, 3, 0, v), s);
     einsum(1.0, "Qly,Qxz->xyzl", Boo, Bov, 0.0, slice(Hv, 3, v, o), s);           // (ly|xz)
-    pack(H, o, o, v, o * v, v, 1, pHx, eHx);
-    pack(H, o, o, v, v, o * v, 1, pHy, eHy);
-    FCC_CUDA(cudaStreamSynchronize(s));   // F and H are freed here
+    pHx.alloc(RH, rowlen);
+    pHy.alloc(RH, rowlen);
+    pack(H.p, o, o, v, o * v, v, 1, pHx);
+    pack(H.p, o, o, v, v, o * v, 1, pHy);
+    FCC_CUDA(cudaStreamSynchronize(s));   // H is freed here
+  }
+  DBuf<double> F;
+  F.alloc(RF * Kc);
+  TView Fv = rm(F.p, {o, v, v, Kc});
+  einsum(1.0, "Qia,Qbd->iabd", Bov, Bvv, 0.0, slice(Fv, 3, 0, v), s);             // (xy|zd)
+  einsum1(-1.0, "xlyz->xyzl", t2v, 0.0, slice(Fv, 3, v, o), s);
+  // The slices of F take four times the memory of F, twice that of the FP64
+  // array in either order.  Where they do not fit beside the rest, F stays in
+  // FP64 and the rows of a run are packed for each pair of runs (hook: t3_kc).
+  size_t mfree = 0, mtotal = 0;
+  FCC_CUDA(cudaMemGetInfo(&mfree, &mtotal));
+  const bool whole = c->t3_kc_override <= 0 && 4.0 * (double)RF * (double)rowlen + 6e9 < (double)mfree;
+  if (whole) {
+    pF.alloc(RF, rowlen);
+    pF2.alloc(RF, rowlen);
+    pack(F.p, o, v, v, v2, v, 1, pF);
+    pack(F.p, o, v, v, v2, 1, v, pF2);
+    FCC_CUDA(cudaStreamSynchronize(s));
+    F.release();
   }
   // W for a run of i and of k: at most ~2 GB
   const int64_t slots_max = std::max<int64_t>(1, (int64_t)(2ll << 30) / (8 * v3));
   int64_t slots = 0;   // the largest run of any j
   for (int64_t j = 0; j < o; ++j) slots = std::max(slots, (o - j) * (j + 1));
-  slots = subset ? 1 : std::min(slots, slots_max);
+  slots = subset ? 1 : std::min(slots, c->t3_kc_override > 0 ? (int64_t)c->t3_kc_override : slots_max);
   c->Wt.alloc(slots * v3);
+  if (!whole) {
+    const int64_t run = std::min(slots, o);
+    pF.alloc(run * v2, rowlen);
+    pFj.alloc(v2, rowlen);
+    pF2.alloc(run * v2, rowlen);
+  }
   const int nt = (int)((v + ET - 1) / ET);
   std::vector<TileTri> th;
   for (int a = 0; a < nt; ++a)
@@ -250,9 +274,8 @@ double triples_fp64(fcc_ctx* c, const std::vector<int3>* subset, std::vector<dou
   // One product: rows m of A (packed rows ar0..), columns n of B (br0..), each a
   // three-level index with the given strides in W
   struct Ix3 { int64_t d2, d3, s1, s2, s3; };
-  auto product = [&](const DBuf<__nv_bfloat16>& pa, const DBuf<int>& ea, int64_t ra, int64_t ar0, int64_t M, Ix3 m,
-                     const DBuf<__nv_bfloat16>& pb, const DBuf<int>& eb, int64_t rb, int64_t br0, int64_t N, Ix3 nn,
-                     double beta, int64_t batch, int64_t ba, int64_t bb, int64_t bc) {
+  auto product = [&](Rows a, int64_t M, Ix3 m, Rows b, int64_t N, Ix3 nn, double beta, int64_t batch, int64_t ba,
+                     int64_t bb, int64_t bc) {
     EpiMap ep;
     ep.M = M; ep.N = N;
     ep.md2 = m.d2; ep.md3 = m.d3; ep.ms1 = m.s1; ep.ms2 = m.s2; ep.ms3 = m.s3;
@@ -261,30 +284,40 @@ double triples_fp64(fcc_ctx* c, const std::vector<int3>* subset, std::vector<dou
     ep.C = c->Wt.p;
     ep.batch = (int)batch; ep.ba = ba; ep.bb = bb; ep.bc = bc;
     ep.work = 2.0 * (double)batch * (double)M * (double)N * (double)Kc * oz_pairs(lv);
-    gemm_oz(pa.p + ar0 * rowlen, ra - ar0, ea.p + ar0, pb.p + br0 * rowlen, rb - br0, eb.p + br0, Kpad, lv, ep,
-            c->tc.ozws, c->tc.err, s);
+    gemm_oz(a.p, a.n, a.e, b.p, b.n, b.e, Kpad, lv, ep, c->tc.ozws, c->tc.err, s);
   };
   // W[i][k][a][b][c] for i in [i0, i0 + ni), k in [k0, k0 + nk) and one j
   auto build_w = [&](int64_t i0, int64_t ni, int64_t j, int64_t k0, int64_t nk) {
     const int64_t ws = nk * v3;   // stride of i
+    Rows fi, fj, fk;              // F[i] and F[j] by (x, y, z), F[k] by (x, z, y)
+    if (whole) {
+      fi = rows(pF, i0 * v2);
+      fj = rows(pF, j * v2);
+      fk = rows(pF2, k0 * v2);
+    } else {
+      pack(F.p + i0 * v2 * Kc, ni, v, v, v2, v, 1, pF);
+      pack(F.p + j * v2 * Kc, 1, v, v, v2, v, 1, pFj);
+      pack(F.p + k0 * v2 * Kc, nk, v, v, v2, 1, v, pF2);
+      fi = rows(pF, 0);
+      fj = rows(pFj, 0);
+      fk = rows(pF2, 0);
+    }
+    const Rows hk = rows(pHy, (j * o + k0) * v);    // H[k..][j]
+    const Rows hki = rows(pHy, (i0 * o + k0) * v);  // H[k..][i]
+    const Rows hji = rows(pHx, (j * o + i0) * v), hjk = rows(pHx, (j * o + k0) * v);
+    const Rows hij = rows(pHy, (j * o + i0) * v), hik = rows(pHx, (i0 * o + k0) * v);
     // F[i](a,b) H[k][j](c): rows (i,a,b), columns (k,c)
-    product(pF, eF, RF, i0 * v2, ni * v2, {v, v, ws, v2, v}, pHy, eHy, RH, (j * o + k0) * v, nk * v,
-            {nk, v, 0, v3, 1}, 0.0, 1, 0, 0, 0);
+    product(fi, ni * v2, {v, v, ws, v2, v}, hk, nk * v, {nk, v, 0, v3, 1}, 0.0, 1, 0, 0, 0);
     // F[j](b,a) H[k][i](c): rows (b,a), columns (k,c), a product per i
-    product(pF, eF, RF, j * v2, v2, {v, v, 0, v, v2}, pHy, eHy, RH, (i0 * o + k0) * v, nk * v, {nk, v, 0, v3, 1}, 1.0,
-            ni, 0, o * v, ws);
+    product(fj, v2, {v, v, 0, v, v2}, hki, nk * v, {nk, v, 0, v3, 1}, 1.0, ni, 0, o * v, ws);
     // H[j][i](b) F[k](c,a): rows (i,b), columns (k,a,c)
-    product(pHx, eHx, RH, (j * o + i0) * v, ni * v, {ni, v, 0, ws, v}, pF2, eF2, RF, k0 * v2, nk * v2,
-            {v, v, v3, v2, 1}, 1.0, 1, 0, 0, 0);
+    product(hji, ni * v, {ni, v, 0, ws, v}, fk, nk * v2, {v, v, v3, v2, 1}, 1.0, 1, 0, 0, 0);
     // H[j][k](b) F[i](a,c): rows (k,b), columns (i,a,c)
-    product(pHx, eHx, RH, (j * o + k0) * v, nk * v, {nk, v, 0, v3, v}, pF, eF, RF, i0 * v2, ni * v2,
-            {v, v, ws, v2, 1}, 1.0, 1, 0, 0, 0);
+    product(hjk, nk * v, {nk, v, 0, v3, v}, fi, ni * v2, {v, v, ws, v2, 1}, 1.0, 1, 0, 0, 0);
     // H[i][j](a) F[k](c,b): rows (i,a), columns (k,b,c)
-    product(pHy, eHy, RH, (j * o + i0) * v, ni * v, {ni, v, 0, ws, v2}, pF2, eF2, RF, k0 * v2, nk * v2,
-            {v, v, v3, v, 1}, 1.0, 1, 0, 0, 0);
+    product(hij, ni * v, {ni, v, 0, ws, v2}, fk, nk * v2, {v, v, v3, v, 1}, 1.0, 1, 0, 0, 0);
     // H[i][k](a) F[j](b,c): rows (k,a), columns (b,c), a product per i
-    product(pHx, eHx, RH, (i0 * o + k0) * v, nk * v, {nk, v, 0, v3, v2}, pF, eF, RF, j * v2, v2, {v, v, 0, v, 1}, 1.0,
-            ni, o * v, 0, ws);
+    product(hik, nk * v, {nk, v, 0, v3, v2}, fj, v2, {v, v, 0, v, 1}, 1.0, ni, o * v, 0, ws);
   };
   auto energy = [&](int64_t i0, int64_t ni, int64_t j, int64_t k0, int64_t nk) {
     const int pe = prof_begin(s);
@@ -310,7 +343,7 @@ double triples_fp64(fcc_ctx* c, const std::vector<int3>* subset, std::vector<dou
   } else {
     for (int64_t j = 0; j < o; ++j) {
       const int64_t nk = std::min<int64_t>(j + 1, slots);
-      const int64_t ni = std::min<int64_t>(std::max<int64_t>(1, slots / nk), 32768 / nk);
+      const int64_t ni = std::min<int64_t>({std::max<int64_t>(1, slots / nk), 32768 / nk, o});
       for (int64_t k0 = 0; k0 <= j; k0 += nk)
         for (int64_t i0 = j; i0 < o; i0 += ni) {
           const int64_t kk = std::min(nk, j + 1 - k0), ii = std::min(ni, o - i0);

@@ -135,3 +135,24 @@ def test_results_repeat_bit_for_bit():
         A, B = rng.standard_normal((M, K)), rng.standard_normal((N, K))
         one, two = (_run(TC, "mk,nk->mn", A, B, np.zeros((M, N)))[1] for _ in range(2))
         assert np.array_equal(one, two)
+
+
+def test_triples_pack_by_runs_gives_the_same_energy():
+    # runs of three, each packed when it is used: the same products, so only the
+    # split of a product into jobs (one rounding of an element of W) can differ
+    from conftest import inputs
+    from fermicc import Options, RCCSD, _lib
+    from fermicc.rccsd import Context
+    inp = inputs(2)
+    Options.reset()
+    Options.set("cc_max_iter", 2)
+    ctx = Context(inp)
+    RCCSD.compute(inp, context=ctx)
+    lib = _lib.load()
+    whole = ctx.triples(_lib.FCC_PREC_FP64)
+    assert lib.fcc_test_set_t3_kc(ctx.h, 3) == 0
+    runs = ctx.triples(_lib.FCC_PREC_FP64)
+    assert lib.fcc_test_set_t3_kc(ctx.h, 0) == 0
+    ctx.close()
+    Options.reset()
+    assert abs(runs - whole) < 1e-13 * abs(whole), (runs, whole)
