@@ -36,35 +36,72 @@ __device__ __forceinline__ double warp_sum(double x) {
   return x;
 }
 
-// Block-reduce NPART values held per thread into part[blockIdx.x*NPART + k].
-__device__ void block_reduce_store(double (&vals)[NPART], int nvals, double* part) {
-  __shared__ double sm[RED_THREADS / 32][NPART];
-  int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+constexpr int NRED = 16;   // NPART padded to a power of two
+// scratch behind the partial sums (doubles): results of up to four launches and the block counter
+constexpr int RED_OUT = 16, RED_TAIL = 5 * RED_OUT;
+
+// blocks of a pass over the rank-2 or rank-4 amplitudes: a thread per element
+// or a warp per row, up to RED_BLOCKS
+int red_blocks(int rank, int64_t o, int64_t v) {
+  const int64_t n = rank == 2 ? (o * v + RED_THREADS - 1) / RED_THREADS : (o * o * v + RED_THREADS / 32 - 1) / (RED_THREADS / 32);
+  return (int)std::min<int64_t>(RED_BLOCKS, std::max<int64_t>(1, n));
+}
+
+// Sum nvals values held per thread over the grid into out.  Each warp halves the
+// set of values as it halves the distance between lanes: 16 FP64 additions per
+// lane instead of five for each value (the FP64 pipe takes 16 clk per warp
+// instruction: the 11 values of an update took 14 us of a launch over 608
+// blocks at (H2O)1, 3 us with this and the blocks that have elements).  The last
+// block to arrive adds the blocks' partial sums, in block order by lanes, so the
+// result does not depend on which it is and needs no second launch.
+__device__ void grid_reduce(double (&vals)[NPART], int nvals, double* part, double* out, unsigned* counter) {
+  __shared__ double sm[RED_THREADS / 32][NRED];
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (nvals <= 3) {
 #pragma unroll
-  for (int k = 0; k < NPART; ++k) {
-    if (k >= nvals) break;
-    double s = warp_sum(vals[k]);
-    if (lane == 0) sm[w][k] = s;
+    for (int k = 0; k < 3; ++k) {
+      const double s = k < nvals ? warp_sum(vals[k]) : 0.0;
+      if (lane == 0) sm[w][k] = s;
+    }
+  } else {
+    double x[NRED];
+#pragma unroll
+    for (int k = 0; k < NRED; ++k) x[k] = k < NPART ? vals[k < NPART ? k : 0] : 0.0;
+#pragma unroll
+    for (int h = NRED / 2; h >= 1; h >>= 1) {   // lanes 2h apart keep one half each
+      const bool up = (lane & (2 * h)) != 0;
+#pragma unroll
+      for (int k = 0; k < h; ++k) {
+        const double send = up ? x[k] : x[k + h], keep = up ? x[k + h] : x[k];
+        x[k] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * h);
+      }
+    }
+    x[0] += __shfl_xor_sync(0xffffffffu, x[0], 1);
+    // bit 2h of the lane chose bit h of the value's number
+    if (!(lane & 1)) sm[w][lane >> 1] = x[0];
   }
   __syncthreads();
   if (threadIdx.x < nvals) {
     double s = 0.0;
     for (int i = 0; i < RED_THREADS / 32; ++i) s += sm[i][threadIdx.x];
-    part[blockIdx.x * NPART + threadIdx.x] = s;
+    if (gridDim.x == 1) out[threadIdx.x] = s;
+    else part[blockIdx.x * NPART + threadIdx.x] = s;
   }
-}
-
-// Sum the per-block partials into out[k]: a warp per value, the lanes over the
-// blocks in turn and then the lanes, a fixed order.  (One thread per value, as
-// this was, took 50 us for the 608 dependent additions; 3 us.)
-__global__ void finish_reduce_kernel(const double* part, int nblocks, int nvals, double* out) {
-  const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (k >= nvals) return;
-  double s = 0.0;
+  if (gridDim.x == 1) return;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicInc(counter, gridDim.x - 1) == gridDim.x - 1;   // wraps to 0 for the next launch
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int k = w; k < nvals; k += RED_THREADS / 32) {
+    double s = 0.0;
 #pragma unroll 4
-  for (int b = lane; b < nblocks; b += 32) s += part[b * NPART + k];
-  s = warp_sum(s);
-  if (lane == 0) out[k] = s;
+    for (int b = lane; b < (int)gridDim.x; b += 32) s += __ldcg(part + b * NPART + k);
+    s = warp_sum(s);
+    if (lane == 0) out[k] = s;
+  }
 }
 
 struct ErrSlots {
@@ -131,7 +168,8 @@ __device__ __forceinline__ void update_one(int64_t e, double t, double r, double
 __global__ void __launch_bounds__(RED_THREADS) update_kernel(
     int rank, const double* __restrict__ T, const double* __restrict__ R, const double* __restrict__ eps,
     int o, int v, double* __restrict__ Tnew, float* __restrict__ err_s, double* __restrict__ err_d,
-    ErrSlots others, const double* __restrict__ Lt, const double* __restrict__ t1new, double* part) {
+    ErrSlots others, const double* __restrict__ Lt, const double* __restrict__ t1new, double* part, double* out,
+    unsigned* counter) {
   double vals[NPART];
 #pragma unroll
   for (int k = 0; k < NPART; ++k) vals[k] = 0.0;
@@ -166,7 +204,7 @@ __global__ void __launch_bounds__(RED_THREADS) update_kernel(
       }
     }
   }
-  block_reduce_store(vals, 3 + others.n, part);
+  grid_reduce(vals, 3 + others.n, part, out, counter);
 }
 
 // DIIS extrapolation: out = sum_k c_k (vec_k + add_res * err_k); for T2 also
@@ -182,7 +220,8 @@ __global__ void __launch_bounds__(RED_THREADS) extrapolate_kernel(int rank, int 
                                                                   const double* __restrict__ coef,
                                                                   double* __restrict__ out,
                                                                   const double* __restrict__ Lt,
-                                                                  const double* __restrict__ t1new, double* part) {
+                                                                  const double* __restrict__ t1new, double* part,
+                                                                  double* sums, unsigned* counter) {
   double vals[NPART];
 #pragma unroll
   for (int k = 0; k < NPART; ++k) vals[k] = 0.0;
@@ -216,13 +255,14 @@ __global__ void __launch_bounds__(RED_THREADS) extrapolate_kernel(int rank, int 
       }
     }
   }
-  block_reduce_store(vals, 2, part);
+  grid_reduce(vals, 2, part, sums, counter);
 }
 
 // Energy of given amplitudes: sum Lt * (t2 + t1 t1), whole rows (i, j, a) per warp.
 __global__ void __launch_bounds__(RED_THREADS) energy_kernel(int o, int v, const double* __restrict__ t2,
                                                              const double* __restrict__ t1,
-                                                             const double* __restrict__ Lt, double* part) {
+                                                             const double* __restrict__ Lt, double* part, double* out,
+                                                             unsigned* counter) {
   double vals[NPART];
 #pragma unroll
   for (int k = 0; k < NPART; ++k) vals[k] = 0.0;
@@ -239,14 +279,14 @@ __global__ void __launch_bounds__(RED_THREADS) energy_kernel(int o, int v, const
       vals[1] += Lt[e] * (t2[e] + t1ia * t1[(int64_t)j * v + b]);
     }
   }
-  block_reduce_store(vals, 2, part);
+  grid_reduce(vals, 2, part, out, counter);
 }
 
 // DF-MP2 correlation energy from (ia|jb) (RMP2a.jl:91-140 forms the same sum
 // pair by pair from the factors): sum (ia|jb) [2 (ia|jb) - (ib|ja)] / D_ijab,
 // whole rows (i, j, a) per warp, lanes along b.
 __global__ void __launch_bounds__(RED_THREADS) mp2_energy_kernel(int o, int v, const double* __restrict__ ovov,
-                                                                 const double* __restrict__ eps, double* part) {
+                                                                 const double* __restrict__ eps, double* part, double* out, unsigned* counter) {
   double vals[NPART];
 #pragma unroll
   for (int k = 0; k < NPART; ++k) vals[k] = 0.0;
@@ -265,39 +305,61 @@ __global__ void __launch_bounds__(RED_THREADS) mp2_energy_kernel(int o, int v, c
       vals[1] = fma(x, quotient(2.0 * x - y, Dia - eps[o + b]), vals[1]);
     }
   }
-  block_reduce_store(vals, 2, part);
+  grid_reduce(vals, 2, part, out, counter);
 }
 
-// Solve the bordered DIIS system B c = (0,..,0,1) in FP64 with partial
-// pivoting (DIIS.jl:66-87); one thread, N <= MAX_DIIS + 1.
-__global__ void diis_solve_kernel(const double* Bm, int N, double* coef, int* status) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double A[MAX_DIIS + 1][MAX_DIIS + 2];
-  for (int r = 0; r < N; ++r) {
-    for (int c = 0; c < N; ++c) A[r][c] = Bm[r * N + c];
-    A[r][N] = (r == N - 1) ? 1.0 : 0.0;
+// Solve the bordered DIIS systems B c = (0,..,0,1) in FP64 with partial pivoting
+// (DIIS.jl:66-87), N <= MAX_DIIS + 1, a warp for each of the two (T1, T2): the
+// lanes share the pivot search, the factors of a column and the elements below
+// it.  (One thread and local arrays took 11 us for each; 4 us for both.)
+constexpr int DIIS_N = MAX_DIIS + 1;
+__global__ void __launch_bounds__(32) diis_solve_kernel(const double* Bm, int N0, int N1, double* coef, double* status) {
+  __shared__ double A[DIIS_N][DIIS_N + 1];
+  __shared__ double f[DIIS_N];
+  const int N = blockIdx.x == 0 ? N0 : N1, lane = threadIdx.x;
+  Bm += blockIdx.x * DIIS_N * DIIS_N;
+  coef += blockIdx.x * DIIS_N;
+  for (int e = lane; e < N * (N + 1); e += 32) {
+    const int r = e / (N + 1), c = e % (N + 1);
+    A[r][c] = c < N ? Bm[r * N + c] : (r == N - 1 ? 1.0 : 0.0);
   }
+  __syncwarp();
   int st = 0;
   for (int col = 0; col < N; ++col) {
-    int piv = col;
-    for (int r = col + 1; r < N; ++r)
-      if (fabs(A[r][col]) > fabs(A[piv][col])) piv = r;
-    if (A[piv][col] == 0.0) { st = 1; break; }
-    if (piv != col)
-      for (int c = 0; c <= N; ++c) { double t = A[col][c]; A[col][c] = A[piv][c]; A[piv][c] = t; }
-    for (int r = col + 1; r < N; ++r) {
-      double f = A[r][col] / A[col][col];
-      for (int c = col; c <= N; ++c) A[r][c] -= f * A[col][c];
+    // the first row of the largest magnitude
+    unsigned long long key = lane >= col && lane < N ? (unsigned long long)__double_as_longlong(fabs(A[lane][col])) : 0ull;
+    int piv = lane >= col && lane < N ? lane : DIIS_N;
+    for (int h = 16; h > 0; h >>= 1) {
+      const unsigned long long ok = __shfl_xor_sync(0xffffffffu, key, h);
+      const int op = __shfl_xor_sync(0xffffffffu, piv, h);
+      if (ok > key || (ok == key && op < piv)) { key = ok; piv = op; }
     }
+    if (key == 0ull) { st = 1; break; }
+    if (piv != col && lane <= N) {
+      const double t = A[col][lane];
+      A[col][lane] = A[piv][lane];
+      A[piv][lane] = t;
+    }
+    __syncwarp();
+    if (lane > col && lane < N) f[lane] = A[lane][col] / A[col][col];
+    __syncwarp();
+    const int w = N - col;   // columns col + 1 .. N of the rows below
+    for (int e = lane; e < (N - 1 - col) * w; e += 32) {
+      const int r = col + 1 + e / w, c = col + 1 + e % w;
+      A[r][c] -= f[r] * A[col][c];
+    }
+    __syncwarp();
   }
+  if (lane != 0) return;
   if (!st) {
     for (int r = N - 1; r >= 0; --r) {
       double s = A[r][N];
-      for (int c = r + 1; c < N; ++c) s -= A[r][c] * coef[c];
-      coef[r] = s / A[r][r];
+      for (int c = r + 1; c < N; ++c) s -= A[r][c] * f[c];
+      f[r] = s / A[r][r];
+      coef[r] = f[r];
     }
   }
-  *status = st;
+  status[blockIdx.x] = st;
 }
 
 // t2 <- OVOV-derived MP2 numerator / D2 (RCCSDa.jl:53-89); t1 <- 0.
@@ -500,7 +562,8 @@ void setup_integrals(fcc_ctx* c) {
   c->Fvv.alloc(v * v);
   c->Foo.alloc(o * o);
   c->Bt.alloc(Q * n * n);
-  c->red.alloc(RED_BLOCKS * NPART + 64);
+  c->red.alloc(RED_BLOCKS * NPART + RED_TAIL + 1);
+  c->red.zero(c->stream);   // the block counter
   // ladder: (ac|bd) slab for a block of virtuals a (b >= block start), blocks
   // of a sized to ~512 MB; pair tables of the symmetric/antisymmetric channels
   int64_t per_a = v * v * v;
@@ -528,6 +591,9 @@ void setup_integrals(fcc_ctx* c) {
   c->LXm.alloc(std::max<int64_t>(1, nijM * rows_max));
 }
 
+static double* red_out(fcc_ctx* c, int q) { return c->red.p + RED_BLOCKS * NPART + q * RED_OUT; }
+static unsigned* red_counter(fcc_ctx* c) { return reinterpret_cast<unsigned*>(c->red.p + RED_BLOCKS * NPART + RED_TAIL); }
+
 void make_mp2_guess(fcc_ctx* c) {
   cudaStream_t s = c->stream;
   const int64_t o = c->o, v = c->v;
@@ -539,10 +605,9 @@ void make_mp2_guess(fcc_ctx* c) {
 
 double cc_energy(fcc_ctx* c, const double* t1, const double* t2) {
   cudaStream_t s = c->stream;
-  energy_kernel<<<RED_BLOCKS, RED_THREADS, 0, s>>>((int)c->o, (int)c->v, t2, t1, c->Lt.p, c->red.p);
-  FCC_CHECK_LAUNCH();
-  double* out = c->red.p + RED_BLOCKS * NPART;
-  finish_reduce_kernel<<<1, 32 * NPART, 0, s>>>(c->red.p, RED_BLOCKS, 2, out);
+  double* out = red_out(c, 0);
+  energy_kernel<<<red_blocks(4, c->o, c->v), RED_THREADS, 0, s>>>((int)c->o, (int)c->v, t2, t1, c->Lt.p, c->red.p, out,
+                                                                  red_counter(c));
   FCC_CHECK_LAUNCH();
   double h[2];
   FCC_CUDA(cudaMemcpyAsync(h, out, sizeof(h), cudaMemcpyDeviceToHost, s));
@@ -552,10 +617,9 @@ double cc_energy(fcc_ctx* c, const double* t1, const double* t2) {
 
 double mp2_energy(fcc_ctx* c) {
   cudaStream_t s = c->stream;
-  mp2_energy_kernel<<<RED_BLOCKS, RED_THREADS, 0, s>>>((int)c->o, (int)c->v, c->ovov.p, c->eps.p, c->red.p);
-  FCC_CHECK_LAUNCH();
-  double* out = c->red.p + RED_BLOCKS * NPART;
-  finish_reduce_kernel<<<1, 32 * NPART, 0, s>>>(c->red.p, RED_BLOCKS, 2, out);
+  double* out = red_out(c, 0);
+  mp2_energy_kernel<<<red_blocks(4, c->o, c->v), RED_THREADS, 0, s>>>((int)c->o, (int)c->v, c->ovov.p, c->eps.p, c->red.p,
+                                                                      out, red_counter(c));
   FCC_CHECK_LAUNCH();
   double h[2];
   FCC_CUDA(cudaMemcpyAsync(h, out, sizeof(h), cudaMemcpyDeviceToHost, s));
@@ -826,26 +890,26 @@ int ccsd_run(fcc_ctx* c, const fcc_opts* opt, fcc_iter_stats* log, int32_t log_c
   double dE = 1.0, rms = 1.0;
   int ite = 1, nlog = 0;
   double* hred = nullptr;
-  FCC_CUDA(cudaMallocHost(&hred, sizeof(double) * 64));
+  // pinned: results of the launches (RED_TAIL), the DIIS matrices, the device's error flag
+  constexpr int HB = RED_TAIL, HERR = HB + 2 * DIIS_N * DIIS_N;
+  FCC_CUDA(cudaMallocHost(&hred, sizeof(double) * (HERR + 1)));
   struct HostFree { double* p; ~HostFree() { if (p) cudaFreeHost(p); } } hf{hred};
   DBuf<double> dB, dcoef;
-  DBuf<int> dstat;
-  dB.alloc((MAX_DIIS + 1) * (MAX_DIIS + 1));
-  dcoef.alloc(MAX_DIIS + 1);
-  dstat.alloc(4);
+  dB.alloc(2 * DIIS_N * DIIS_N);
+  dcoef.alloc(2 * DIIS_N);
   cudaEvent_t ev0, ev1;
   FCC_CUDA(cudaEventCreate(&ev0));
   FCC_CUDA(cudaEventCreate(&ev1));
   struct EvFree { cudaEvent_t a, b; ~EvFree() { cudaEventDestroy(a); cudaEventDestroy(b); } } evf{ev0, ev1};
-  double* dout = c->red.p + RED_BLOCKS * NPART;
-
+  // The update of one amplitude tensor (rank 2 or 4; its sums go to red_out(c,
+  // rank / 2 - 1)) and, once the sums are here, the host's part of it: both
+  // tensors are launched before the host waits, and so are both extrapolations.
+  struct Pending { int target = -1; std::vector<int> others; };
   auto run_update = [&](int rank, DiisState& ds, DBuf<double>& vecs, DBuf<float>& es, DBuf<double>& ed,
-                        const double* T, const double* R, DBuf<double>& plain, double** cur, const double* t1new,
-                        double* out_sumsq, double* out_energy) {
+                        const double* T, const double* R, DBuf<double>& plain, double** cur, const double* t1new) {
     int64_t len = rank == 2 ? len1 : len2;
     ErrSlots others{};
-    int target = -1;
-    std::vector<int> other_ids;
+    Pending pd;
     if (diis) {
       // DIIS.jl:38-50: evict the slot with the largest error norm when full
       if (ds.count() + 1 > ds.ndiis) {
@@ -853,78 +917,65 @@ int ccsd_run(fcc_ctx* c, const fcc_opts* opt, fcc_iter_stats* log, int32_t log_c
         for (int k = 0; k < ds.ndiis; ++k)
           if (ds.valid[k] && (worst < 0 || ds.norm2[k] > ds.norm2[worst])) worst = k;
         ds.valid[worst] = 0;
-        target = worst;
+        pd.target = worst;
       } else {
-        for (int k = 0; k < ds.ndiis; ++k) if (!ds.valid[k]) { target = k; break; }
+        for (int k = 0; k < ds.ndiis; ++k) if (!ds.valid[k]) { pd.target = k; break; }
       }
       for (int k = 0; k < ds.ndiis; ++k)
         if (ds.valid[k]) {
           others.s[others.n] = ds.fp32 ? es.p + (int64_t)k * len : nullptr;
           others.d[others.n] = ds.fp32 ? nullptr : ed.p + (int64_t)k * len;
-          other_ids.push_back(k);
+          pd.others.push_back(k);
           others.n++;
         }
     }
-    double* dst = diis ? vec_slot(vecs, len, target) : plain.p;
-    float* errs = (diis && ds.fp32) ? es.p + (int64_t)target * len : nullptr;
-    double* errd = (diis && !ds.fp32) ? ed.p + (int64_t)target * len : nullptr;
-    update_kernel<<<RED_BLOCKS, RED_THREADS, 0, s>>>(rank, T, R, c->eps.p, (int)o, (int)v, dst, errs, errd, others,
-                                                     rank == 4 ? c->Lt.p : nullptr, t1new, c->red.p);
+    double* dst = diis ? vec_slot(vecs, len, pd.target) : plain.p;
+    float* errs = (diis && ds.fp32) ? es.p + (int64_t)pd.target * len : nullptr;
+    double* errd = (diis && !ds.fp32) ? ed.p + (int64_t)pd.target * len : nullptr;
+    update_kernel<<<red_blocks(rank, o, v), RED_THREADS, 0, s>>>(rank, T, R, c->eps.p, (int)o, (int)v, dst, errs, errd,
+                                                                 others, rank == 4 ? c->Lt.p : nullptr, t1new, c->red.p,
+                                                                 red_out(c, rank / 2 - 1), red_counter(c));
     FCC_CHECK_LAUNCH();
-    finish_reduce_kernel<<<1, 32 * NPART, 0, s>>>(c->red.p, RED_BLOCKS, 3 + others.n, dout);
-    FCC_CHECK_LAUNCH();
-    FCC_CUDA(cudaMemcpyAsync(hred, dout, sizeof(double) * NPART, cudaMemcpyDeviceToHost, s));
-    FCC_CUDA(cudaStreamSynchronize(s));
-    *out_sumsq = hred[0];
-    *out_energy = hred[1];
-    if (diis) {
-      ds.valid[target] = 1;
-      ds.age[target] = ++ds.counter;
-      ds.norm2[target] = hred[2];
-      ds.dot[target][target] = hred[2];
-      for (size_t q = 0; q < other_ids.size(); ++q) {
-        ds.dot[target][other_ids[q]] = hred[3 + q];
-        ds.dot[other_ids[q]][target] = hred[3 + q];
-      }
-    }
     *cur = dst;
+    return pd;
+  };
+  auto note_update = [&](DiisState& ds, const Pending& pd, const double* h) {
+    if (!diis) return;
+    ds.valid[pd.target] = 1;
+    ds.age[pd.target] = ++ds.counter;
+    ds.norm2[pd.target] = h[2];
+    ds.dot[pd.target][pd.target] = h[2];
+    for (size_t q = 0; q < pd.others.size(); ++q) {
+      ds.dot[pd.target][pd.others[q]] = h[3 + q];
+      ds.dot[pd.others[q]][pd.target] = h[3 + q];
+    }
   };
 
-  auto extrapolate = [&](int rank, DiisState& ds, DBuf<double>& vecs, DBuf<float>& es, DBuf<double>& ed,
-                         DBuf<double>& outbuf, const double* t1new, double* out_energy) -> bool {
-    int64_t len = rank == 2 ? len1 : len2;
+  // the stored vectors of one tensor, oldest first, and its DIIS matrix into hB
+  auto subspace = [&](const DiisState& ds, double* hB) {
     std::vector<int> ids;
     for (int k = 0; k < ds.ndiis; ++k) if (ds.valid[k]) ids.push_back(k);
     std::sort(ids.begin(), ids.end(), [&](int a, int b) { return ds.age[a] < ds.age[b]; });
-    int m = (int)ids.size();
+    const int m = (int)ids.size(), N = m + 1;
     if (m < 2) fail(FCC_ERR_STATE, "DIIS cannot extrapolate from one vector");
-    int N = m + 1;
-    std::vector<double> Bm(N * N, 1.0);
-    Bm[N * N - 1] = 0.0;
-    for (int a = 0; a < m; ++a)
-      for (int b = 0; b < m; ++b) Bm[a * N + b] = ds.dot[ids[a]][ids[b]];
-    FCC_CUDA(cudaMemcpyAsync(dB.p, Bm.data(), sizeof(double) * N * N, cudaMemcpyHostToDevice, s));
-    diis_solve_kernel<<<1, 1, 0, s>>>(dB.p, N, dcoef.p, dstat.p);
-    FCC_CHECK_LAUNCH();
+    for (int a = 0; a < N; ++a)
+      for (int b = 0; b < N; ++b) hB[a * N + b] = a == m ? (b == m ? 0.0 : 1.0) : (b == m ? 1.0 : ds.dot[ids[a]][ids[b]]);
+    return ids;
+  };
+  auto extrapolate = [&](int rank, DiisState& ds, const std::vector<int>& ids, DBuf<double>& vecs, DBuf<float>& es,
+                         DBuf<double>& ed, DBuf<double>& outbuf, const double* t1new) {
+    int64_t len = rank == 2 ? len1 : len2;
     VecSlots sl{};
-    for (int a = 0; a < m; ++a) {
+    sl.n = (int)ids.size();
+    for (int a = 0; a < sl.n; ++a) {
       sl.vec[a] = vec_slot(vecs, len, ids[a]);
       sl.es[a] = ds.fp32 ? es.p + (int64_t)ids[a] * len : nullptr;
       sl.ed[a] = ds.fp32 ? nullptr : ed.p + (int64_t)ids[a] * len;
     }
-    sl.n = m;
-    extrapolate_kernel<<<RED_BLOCKS, RED_THREADS, 0, s>>>(rank, (int)o, (int)v, sl, dcoef.p, outbuf.p,
-                                                          rank == 4 ? c->Lt.p : nullptr, t1new, c->red.p);
+    extrapolate_kernel<<<red_blocks(rank, o, v), RED_THREADS, 0, s>>>(
+        rank, (int)o, (int)v, sl, dcoef.p + (rank / 2 - 1) * DIIS_N, outbuf.p, rank == 4 ? c->Lt.p : nullptr, t1new,
+        c->red.p, red_out(c, rank / 2 - 1), red_counter(c));
     FCC_CHECK_LAUNCH();
-    finish_reduce_kernel<<<1, 32 * NPART, 0, s>>>(c->red.p, RED_BLOCKS, 2, dout);
-    FCC_CHECK_LAUNCH();
-    int st = 0;
-    FCC_CUDA(cudaMemcpyAsync(hred, dout, sizeof(double) * 2, cudaMemcpyDeviceToHost, s));
-    FCC_CUDA(cudaMemcpyAsync(&st, dstat.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-    FCC_CUDA(cudaStreamSynchronize(s));
-    if (st) fail(FCC_ERR_NAN, "singular DIIS matrix");
-    *out_energy = hred[1];
-    return true;
   };
 
   int status = FCC_OK;
@@ -985,15 +1036,26 @@ int ccsd_run(fcc_ctx* c, const fcc_opts* opt, fcc_iter_stats* log, int32_t log_c
         c->test_fault = 0;
       }
     }
-    double ss1, ss2, e_dummy, e_new;
-    run_update(2, D1s, c->dvec1, c->derr1s, c->derr1d, c->t1.p, c->r1.p, tn1, &cur1, nullptr, &ss1, &e_dummy);
-    run_update(4, D2s, c->dvec2, c->derr2s, c->derr2d, c->t2.p, c->r2.p, tn2, &cur2, cur1, &ss2, &e_new);
-    double r1 = std::sqrt(ss1 / (double)len1), r2 = std::sqrt(ss2 / (double)len2);   // :193-194
+    const Pending p1 = run_update(2, D1s, c->dvec1, c->derr1s, c->derr1d, c->t1.p, c->r1.p, tn1, &cur1, nullptr);
+    const Pending p2 = run_update(4, D2s, c->dvec2, c->derr2s, c->derr2d, c->t2.p, c->r2.p, tn2, &cur2, cur1);
+    FCC_CUDA(cudaMemcpyAsync(hred, red_out(c, 0), sizeof(double) * 2 * RED_OUT, cudaMemcpyDeviceToHost, s));
+    FCC_CUDA(cudaStreamSynchronize(s));
+    note_update(D1s, p1, hred);
+    note_update(D2s, p2, hred + RED_OUT);
+    double e_new = hred[RED_OUT + 1];
+    double r1 = std::sqrt(hred[0] / (double)len1), r2 = std::sqrt(hred[RED_OUT] / (double)len2);   // :193-194
     bool did = false;
     if (diis && ite >= op.diis_start && ite % op.diis_relax == 0 && D1s.count() >= 2 && D2s.count() >= 2) {   // :204
-      double e1d;
-      extrapolate(2, D1s, c->dvec1, c->derr1s, c->derr1d, tx1, nullptr, &e1d);
-      extrapolate(4, D2s, c->dvec2, c->derr2s, c->derr2d, tx2, tx1.p, &e_new);
+      const std::vector<int> id1 = subspace(D1s, hred + HB), id2 = subspace(D2s, hred + HB + DIIS_N * DIIS_N);
+      FCC_CUDA(cudaMemcpyAsync(dB.p, hred + HB, sizeof(double) * 2 * DIIS_N * DIIS_N, cudaMemcpyHostToDevice, s));
+      diis_solve_kernel<<<2, 32, 0, s>>>(dB.p, (int)id1.size() + 1, (int)id2.size() + 1, dcoef.p, red_out(c, 2));
+      FCC_CHECK_LAUNCH();
+      extrapolate(2, D1s, id1, c->dvec1, c->derr1s, c->derr1d, tx1, nullptr);
+      extrapolate(4, D2s, id2, c->dvec2, c->derr2s, c->derr2d, tx2, tx1.p);
+      FCC_CUDA(cudaMemcpyAsync(hred, red_out(c, 0), sizeof(double) * 3 * RED_OUT, cudaMemcpyDeviceToHost, s));
+      FCC_CUDA(cudaStreamSynchronize(s));
+      if (hred[2 * RED_OUT] != 0.0 || hred[2 * RED_OUT + 1] != 0.0) fail(FCC_ERR_NAN, "singular DIIS matrix");
+      e_new = hred[RED_OUT + 1];
       cur1 = tx1.p;
       cur2 = tx2.p;
       did = true;
@@ -1044,14 +1106,14 @@ int ccsd_run(fcc_ctx* c, const fcc_opts* opt, fcc_iter_stats* log, int32_t log_c
         if (ready || stalled >= 5) kind = finish;
       }
     }
+    int* const herr = reinterpret_cast<int*>(hred + HERR);
+    FCC_CUDA(cudaMemcpyAsync(herr, c->dev_err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
     FCC_CUDA(cudaEventRecord(ev1, s));
     FCC_CUDA(cudaEventSynchronize(ev1));
     float ms = 0;
     FCC_CUDA(cudaEventElapsedTime(&ms, ev0, ev1));
     if (!std::isfinite(Ecc) || !std::isfinite(rms)) { status = FCC_ERR_NAN; }
-    int herr = 0;
-    FCC_CUDA(cudaMemcpy(&herr, c->dev_err.p, sizeof(int), cudaMemcpyDeviceToHost));
-    if (herr) { status = FCC_ERR_TIMEOUT; }
+    if (*herr) { status = FCC_ERR_TIMEOUT; }
     if (c->ckpt_every > 0 && ite % c->ckpt_every == 0)
       checkpoint_write(c, c->ckpt_path, cur1, cur2, Ecc, ite, 0);
     if (log && nlog < log_cap) {

@@ -266,93 +266,100 @@ __global__ void __launch_bounds__(256) splitk_reduce_few_kernel(const double* __
             d.alpha, d.beta);
 }
 
-// Small contractions: a block of four warps per 16 x 16 output tile (and K
-// range), the k-steps of four dealt to the warps in turn, operands read
-// straight into the fragments of m8n8k4, the warps' sums added in shared
-// memory in a fixed order.  An SM does two FP64 FMAs per clk, so what counts is
-// that the work reaches all SMs: with 64 x 64 tiles the contractions of a
-// dimer ran on 1-25 SMs (a 46 x 46 x 46 product took 97 us on one; 5 here).
-constexpr int SM_T = 16, SM_WARPS = 4;
+// Small contractions: a block of four warps per 8 x 8 output tile and K range,
+// the k-steps of four dealt to the warps in turn, operands read straight into
+// the fragments of m8n8k4.  An SM does two FP64 FMAs per clk, so one m8n8k4
+// takes the SM 128 clk, its two loads are free, and what counts is that the work
+// reaches all SMs: with 64 x 64 tiles the contractions of a dimer ran on 1-25
+// SMs (a 46 x 46 x 46 product took 97 us on one), with 16 x 16 tiles a 90 x 90 x
+// 90 one ran on 36 (13 us; 6 here).  Where the tiles are fewer than the SMs a
+// cluster of up to eight blocks shares a tile's K and the first block adds the
+// sums, read from the others' shared memory, in block order: no second launch
+// and no partial sums in memory (15 x 190 x 190: 21 us with 16 x 16 tiles, 6
+// here).
+constexpr int SM_T = 8, SM_WARPS = 4;
 __global__ void __launch_bounds__(32 * SM_WARPS) contract_f64_small_kernel(const double* __restrict__ A,
                                                                            const double* __restrict__ B,
                                                                            double* __restrict__ C, CtrDesc d,
-                                                                           int k_chunk, double* __restrict__ partial) {
-  __shared__ double part[SM_WARPS][SM_T][SM_T + 1];
+                                                                           int k_chunk, int cl,
+                                                                           double* __restrict__ partial) {
+  __shared__ double part[SM_WARPS][SM_T * SM_T];
+  __shared__ double sum[SM_T * SM_T];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int64_t m0 = (int64_t)blockIdx.x * SM_T, n0 = (int64_t)blockIdx.y * SM_T;
-  const int64_t bz = partial ? 0 : blockIdx.z;
-  const int kbeg = partial ? (int)blockIdx.z * k_chunk : 0;
-  const int kend = partial ? min((int)d.K, kbeg + k_chunk) : (int)d.K;
-  A += bz * d.a_b;
-  B += bz * d.b_b;
-  C += bz * d.c_b;
-  int64_t ra[2], cb[2];
-  bool rok[2], cok[2];
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int64_t m = m0 + 8 * i + (lane >> 2), n = n0 + 8 * i + (lane >> 2);
-    rok[i] = m < d.M;
-    cok[i] = n < d.N;
-    ra[i] = rok[i] ? off3(m, d.M2, d.M3, d.a_m1, d.a_m2, d.a_m3) : 0;
-    cb[i] = cok[i] ? off3(n, d.N2, d.N3, d.b_n1, d.b_n2, d.b_n3) : 0;
-  }
-  double acc[2][2][2];
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-  constexpr int U = 4;   // k-steps in flight
+  // z: K range of a partial product, or (batch, block of the cluster)
+  const uint32_t zb = partial ? 0 : blockIdx.z / (uint32_t)cl;
+  const int zk = partial ? (int)blockIdx.z : (int)(blockIdx.z - zb * (uint32_t)cl);
+  const int kbeg = zk * k_chunk;
+  const int kend = min((int)d.K, kbeg + k_chunk);
+  A += (int64_t)zb * d.a_b;
+  B += (int64_t)zb * d.b_b;
+  C += (int64_t)zb * d.c_b;
+  const int64_t m = m0 + (lane >> 2), n = n0 + (lane >> 2);
+  const bool rok = m < d.M, cok = n < d.N;
+  const int64_t ra = rok ? off3(m, d.M2, d.M3, d.a_m1, d.a_m2, d.a_m3) : 0;
+  const int64_t cb = cok ? off3(n, d.N2, d.N3, d.b_n1, d.b_n2, d.b_n3) : 0;
+  double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+  constexpr int U = 8;   // k-steps in flight
   for (int k0 = kbeg + 4 * warp; k0 < kend; k0 += 4 * SM_WARPS * U) {
-    double a[U][2], b[U][2];
+    double a[U], b[U];
 #pragma unroll
     for (int q = 0; q < U; ++q) {
       const int k = k0 + 4 * SM_WARPS * q + (lane & 3);
-      const bool kok = k < kend;
-      int64_t ka = 0, kb = 0;
-      if (kok) {
+      a[q] = b[q] = 0.0;
+      if (k < kend) {
         const uint32_t k1 = (uint32_t)k / (uint32_t)d.K2, k2 = (uint32_t)k - k1 * (uint32_t)d.K2;
-        ka = (int64_t)k1 * d.a_k1 + (int64_t)k2 * d.a_k2;
-        kb = (int64_t)k1 * d.b_k1 + (int64_t)k2 * d.b_k2;
-      }
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        a[q][i] = kok && rok[i] ? A[ra[i] + ka] : 0.0;
-        b[q][i] = kok && cok[i] ? B[cb[i] + kb] : 0.0;
+        if (rok) a[q] = A[ra + (int64_t)k1 * d.a_k1 + (int64_t)k2 * d.a_k2];
+        if (cok) b[q] = B[cb + (int64_t)k1 * d.b_k1 + (int64_t)k2 * d.b_k2];
       }
     }
-    const bool m2 = m0 + 8 < d.M, n2 = n0 + 8 < d.N;   // warp-uniform: blocks wholly outside issue no MMA
 #pragma unroll
     for (int q = 0; q < U; ++q) {
       if (k0 + 4 * SM_WARPS * q >= kend) break;
-      dmma884(acc[0][0][0], acc[0][0][1], a[q][0], b[q][0]);
-      if (n2) dmma884(acc[0][1][0], acc[0][1][1], a[q][0], b[q][1]);
-      if (m2) dmma884(acc[1][0][0], acc[1][0][1], a[q][1], b[q][0]);
-      if (m2 && n2) dmma884(acc[1][1][0], acc[1][1][1], a[q][1], b[q][1]);
+      dmma884(acc[q & 1][0], acc[q & 1][1], a[q], b[q]);
     }
   }
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) part[warp][8 * i + (lane >> 2)][8 * j + 2 * (lane & 3) + h] = acc[i][j][h];
+  // lane: row lane / 4, columns 2 (lane % 4) and the next
+  part[warp][2 * lane] = acc[0][0] + acc[1][0];
+  part[warp][2 * lane + 1] = acc[0][1] + acc[1][1];
   __syncthreads();
+  double s = 0.0;
+  if (tid < SM_T * SM_T) {
+    s = part[0][tid];
 #pragma unroll
-  for (int e = tid; e < SM_T * SM_T; e += 32 * SM_WARPS) {
-    // the output's faster index along the threads
-    const bool mf = d.c_n3 != 1 && (d.N3 > 1 || d.c_n2 != 1);
-    const int r = mf ? e % SM_T : e / SM_T, c = mf ? e / SM_T : e % SM_T;
-    const int64_t m = m0 + r, n = n0 + c;
-    if (m >= d.M || n >= d.N) continue;
-    double s = part[0][r][c];
+    for (int w = 1; w < SM_WARPS; ++w) s += part[w][tid];
+  }
+  if (!partial && cl > 1) {
+    if (tid < SM_T * SM_T) sum[tid] = s;
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (zk == 0 && tid < SM_T * SM_T) {
+      const uint32_t own = (uint32_t)__cvta_generic_to_shared(&sum[tid]);
+      double other[7];
 #pragma unroll
-    for (int w = 1; w < SM_WARPS; ++w) s += part[w][r][c];
-    if (partial) {
-      partial[((int64_t)blockIdx.z * d.M + m) * d.N + n] = s;
-    } else {
-      f64_store(C + off3(m, d.M2, d.M3, d.c_m1, d.c_m2, d.c_m3) + off3(n, d.N2, d.N3, d.c_n1, d.c_n2, d.c_n3), s,
-                d.alpha, d.beta);
+      for (int q = 1; q < 8; ++q) {
+        other[q - 1] = 0.0;
+        if (q < cl) {
+          uint32_t addr;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(own), "r"(q));
+          asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(other[q - 1]) : "r"(addr) : "memory");
+        }
+      }
+#pragma unroll
+      for (int q = 1; q < 8; ++q)
+        if (q < cl) s += other[q - 1];
     }
+    // the other blocks' shared memory stays until it is read
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (zk != 0) return;
+  }
+  if (tid >= SM_T * SM_T) return;
+  const int64_t mo = m0 + (tid >> 3), no = n0 + (tid & 7);
+  if (mo >= d.M || no >= d.N) return;
+  if (partial) {
+    partial[((int64_t)blockIdx.z * d.M + mo) * d.N + no] = s;
+  } else {
+    f64_store(C + off3(mo, d.M2, d.M3, d.c_m1, d.c_m2, d.c_m3) + off3(no, d.N2, d.N3, d.c_n1, d.c_n2, d.c_n3), s,
+              d.alpha, d.beta);
   }
 }
 
@@ -522,19 +529,21 @@ void contract_f64_launch(const double* A, const double* B, double* C, const CtrD
   DBuf<double> local;
   const int64_t MN = d.M * d.N;
   const unsigned rgrid = (unsigned)std::min<int64_t>((MN + 255) / 256, 152 * 8);
-  // 16 x 16 tiles while the 64 x 64 ones would leave SMs without work; K is
-  // then cut so that about two blocks per SM share it (partials reduced in a
-  // fixed order, so results stay deterministic)
+  // 8 x 8 tiles while the 64 x 64 ones would leave SMs without work.  Up to
+  // eight blocks share a tile while there are fewer than two blocks per SM and
+  // each has 16 values of k; a longer K over few tiles (over 512 a block) is cut
+  // into partial sums for all SMs, reduced in a fixed order by a second launch.
   const int64_t sm = (d.M + SM_T - 1) / SM_T, sn = (d.N + SM_T - 1) / SM_T;
   if (gm * gn * d.batch < 3 * 152 && sn <= 65535) {
-    int64_t splits = 1;
-    if (d.batch == 1 && sm * sn < 152) splits = std::min<int64_t>((304 + sm * sn - 1) / (sm * sn), d.K / 128);
-    if (splits > 1) {
-      const int64_t chunk = ((d.K + splits - 1) / splits + 15) / 16 * 16;
-      splits = (d.K + chunk - 1) / chunk;
+    int64_t cl = 1;
+    while (cl < 8 && sm * sn * d.batch * cl < 152 && d.K >= 32 * cl && d.batch * cl * 2 <= 65535) cl *= 2;
+    const int64_t splits0 = (304 + sm * sn - 1) / (sm * sn);
+    if (d.batch == 1 && splits0 > 8 && d.K > 4096) {
+      const int64_t chunk = ((d.K + splits0 - 1) / splits0 + 15) / 16 * 16;
+      const int64_t splits = (d.K + chunk - 1) / chunk;
       double* part = workspace(local, splits * MN);
       contract_f64_small_kernel<<<dim3((unsigned)sm, (unsigned)sn, (unsigned)splits), 32 * SM_WARPS, 0, s>>>(
-          A, B, C, d, (int)chunk, part);
+          A, B, C, d, (int)chunk, 1, part);
       FCC_CHECK_LAUNCH();
       if (MN <= 152 * 32) {
         splitk_reduce_few_kernel<<<(unsigned)((MN + 31) / 32), 256, 0, s>>>(part, (int)splits, C, d);
@@ -542,8 +551,18 @@ void contract_f64_launch(const double* A, const double* B, double* C, const CtrD
         splitk_reduce_kernel<<<rgrid, 256, 0, s>>>(part, (int)splits, C, d);
       }
     } else {
-      contract_f64_small_kernel<<<dim3((unsigned)sm, (unsigned)sn, (unsigned)d.batch), 32 * SM_WARPS, 0, s>>>(
-          A, B, C, d, 0, nullptr);
+      const int chunk = (int)(((d.K + cl - 1) / cl + 3) / 4 * 4);
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3((unsigned)sm, (unsigned)sn, (unsigned)(d.batch * cl));
+      cfg.blockDim = dim3(32 * SM_WARPS);
+      cfg.stream = s;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = at[0].val.clusterDim.y = 1;
+      at[0].val.clusterDim.z = (unsigned)cl;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      FCC_CUDA(cudaLaunchKernelEx(&cfg, contract_f64_small_kernel, A, B, C, d, chunk, (int)cl, (double*)nullptr));
     }
     FCC_CHECK_LAUNCH();
     prof_end(s, pidx, PROF_F64, pflops);

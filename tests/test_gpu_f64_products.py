@@ -105,7 +105,7 @@ def test_peaked_rows_against_a_metric():
     assert err[TC] <= max(err[PIPE], 2.0 ** -53), err
 
 
-@pytest.mark.parametrize("M,N,K", [(1, 5, 3), (7, 9, 1), (16, 17, 4), (33, 15, 130), (5, 5, 9000), (250, 250, 40)])
+@pytest.mark.parametrize("M,N,K", [(1, 5, 3), (7, 9, 1), (16, 17, 4), (33, 15, 130), (5, 5, 9000), (250, 250, 40), (9, 8, 1701), (1, 2, 4097), (64, 8, 31)])
 def test_small_kernel_edges(M, N, K):
     rng = np.random.default_rng(M * N + K)
     A = rng.integers(-1000, 1000, (M, K)).astype(float)
