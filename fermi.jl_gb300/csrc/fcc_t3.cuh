@@ -22,18 +22,26 @@ struct T3Params {
   T3Seg seg[3][T3_NSEG];
   int i, j, k0, nk, o, v;
   int bn;      // B tile width: 128, 160, 192 or 256 (t3_bn(v) unless set for a test)
-  float* G;    // G[g][k - k0] FP32 in 8 x 8 x 8 sub-cube blocks (t3_blk)
+  float* G;    // G[g][k - k0] FP32 in 8 x 8 x 8 sub-cubes (t3_cube, t3_pos)
   int* err;    // set to 1 if a bounded wait gave up
 };
 
 // Layout of one G_g[k] slab over (pair first index x, pair second index y,
-// lone index z): 8 x 8 x 8 sub-cubes, each 512 contiguous floats, blocks
-// ordered (X, Y, Z) with nb = ceil(v / 8) per index; the energy kernel reads
-// whole sub-cubes with 2 KB loads.
+// lone index z): 8 x 8 x 8 sub-cubes of 512 contiguous floats, blocks ordered
+// (X, Y, Z) with nb = ceil(v / 8) per index.  Inside a sub-cube the 32-byte runs
+// of the lone index l are placed so that reads over eight l and four adjacent
+// values of h or m, over four l and eight h or m, or of 16-byte halves over
+// eight h or m meet 32 different banks: the energy kernel copies sub-cubes as
+// they are and reads them in any index order without bank conflicts, and the
+// GEMM still stores a run as one 32-byte sector.
 __host__ __device__ constexpr int64_t t3_nb(int64_t v) { return (v + 7) / 8; }
 __host__ __device__ constexpr int64_t t3_slab(int64_t v) { return t3_nb(v) * t3_nb(v) * t3_nb(v) * 512; }
-__device__ __forceinline__ int64_t t3_blk(int x, int y, int z, int64_t nb) {
-  return ((((int64_t)(x >> 3) * nb + (y >> 3)) * nb + (z >> 3)) << 9) + ((x & 7) << 6) + ((y & 7) << 3) + (z & 7);
+// the run of (h, m), its halves exchanged where bit 2 of h ^ m is set
+__host__ __device__ constexpr int t3_run(int h, int m) { return (((h ^ m) & 3) << 3) | ((h & 7) << 5) | ((m & 4) << 6); }
+__host__ __device__ constexpr int t3_pos(int h, int m, int l) { return t3_run(h, m) | (l ^ ((h ^ m) & 4)); }
+// first float of sub-cube (X, Y, Z)
+__host__ __device__ constexpr int64_t t3_cube(int X, int Y, int Z, int64_t nb) {
+  return (((int64_t)X * nb + Y) * nb + Z) << 9;
 }
 
 // the B tile width used for v virtuals (256 with several column tiles above 256)

@@ -86,7 +86,6 @@ __global__ void __launch_bounds__(T3_THREADS, 1) gemm_t3_kernel(const __grid_con
   __shared__ __align__(8) uint64_t done_bar;      // every issued MMA has completed
   __shared__ uint32_t tmem_holder;
   __shared__ int abort_flag;
-  __shared__ float epi_tile[4][32][33];
 
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sA = smem;
@@ -192,10 +191,14 @@ __global__ void __launch_bounds__(T3_THREADS, 1) gemm_t3_kernel(const __grid_con
     if (!mbar_wait(smem_u32(&done_bar), 0)) atomicExch(&abort_flag, 1);
    }
   } else if (warp >= 2) {
-    // ---------------- epilogue: TMEM -> transposed 32 x 32 blocks -> plain FP32 stores
+    // ---------------- epilogue: each lane has a row (x, y) and stores its columns
+    // in whole 32-byte sectors straight from the registers.  (Transposed through
+    // shared memory for 128-byte rows, an element took about eight instructions
+    // of the warp instead of one and a half, and the shared memory shared with
+    // the MMAs: 167 ms of a (T) at (H2O)8 where this takes 160, 29 and 24 ms at
+    // (H2O)6 with odd sizes.)
     const int q = warp & 3;
     const int64_t v2 = v * v;
-    float (*tile)[33] = epi_tile[q];
     int lt = 0;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++lt) {
       const T3Tile tl = t3_tile(t, tm, tn, P.nk);
@@ -208,33 +211,27 @@ __global__ void __launch_bounds__(T3_THREADS, 1) gemm_t3_kernel(const __grid_con
       const int64_t nbk = t3_nb(v);
       float* out = P.G + ((int64_t)tl.g * P.nk + tl.kq) * t3_slab(v);
       const int64_t nb0 = (int64_t)tl.nt * BN;
-      // this lane's row (pair (x, y)) offset in the blocked layout; rows are
-      // broadcast to the warp below
-      int64_t myroff = 0;
-      {
-        const int64_t mr = m0 + q * 32 + lane;
-        if (mr < v2) {
-          const int x = (int)((uint32_t)mr / (uint32_t)P.v), y = (int)mr - x * P.v;
-          myroff = t3_blk(x, y, 0, nbk);
-        }
-      }
+      const int64_t mr = m0 + q * 32 + lane;
+      const int x = (int)((uint32_t)mr / (uint32_t)P.v), y = (int)mr - x * P.v;
+      float* dst = out + t3_cube(x >> 3, y >> 3, 0, nbk) + t3_run(x & 7, y & 7);
+      const bool swap = ((x ^ y) & 4) != 0;
 #pragma unroll 1
       for (int c0 = 0; c0 < BN; c0 += 32) {
         if (nb0 + c0 >= v) break;
         uint32_t r[32];
         tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * Cfg::TMEM_COLS + c0), r);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        __syncwarp();
 #pragma unroll
-        for (int jj = 0; jj < 32; ++jj) tile[lane][jj] = __uint_as_float(r[jj]);
-        __syncwarp();
-        const int64_t n = nb0 + c0 + lane;
-        const int64_t coff = ((n >> 3) << 9) + (n & 7);   // lone index z = n within the (X, Y) block row
-#pragma unroll 4
-        for (int jr = 0; jr < 32; ++jr) {
-          const int64_t roff = __shfl_sync(0xffffffffu, myroff, jr);
-          const int64_t m = m0 + q * 32 + jr;
-          if (m < v2 && n < v) out[roff + coff] = tile[jr][lane];
+        for (int g = 0; g < 4; ++g) {
+          const int64_t n = nb0 + c0 + 8 * g;
+          if (mr < v2 && n < v) {   // columns past v in the last run are padding of the slab
+            uint32_t w[8];
+#pragma unroll
+            for (int l = 0; l < 8; ++l) w[l] = swap ? r[8 * g + (l ^ 4)] : r[8 * g + l];
+            asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst + ((n >> 3) << 9)), "r"(w[0]),
+                         "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                         : "memory");
+          }
         }
       }
       // the accumulator is free for the tile after next
