@@ -202,9 +202,18 @@ double triples_fp64(fcc_ctx* c, const std::vector<int3>* subset, std::vector<dou
     DBuf<int> e;
     void alloc(int64_t rows, int64_t rowlen) { p.alloc(rows * rowlen); e.alloc(rows); }
   };
-  struct Rows { const __nv_bfloat16* p; const int* e; int64_t n; };
+  // rows of a packed operand from one on, and the same rows in FP64: three
+  // levels of strides and that of a product of a batch, in rows
+  struct Rows { const __nv_bfloat16* p; const int* e; int64_t n; const double* f; int64_t s1, s2, s3, sb; };
   Packed pF, pF2, pHx, pHy, pFj;
-  auto rows = [&](const Packed& x, int64_t r0) { return Rows{x.p.p + r0 * rowlen, x.e.p + r0, (int64_t)x.e.n - r0}; };
+  auto rows = [&](const Packed& x, int64_t r0, const double* f, int64_t s1, int64_t s2, int64_t s3, int64_t sb) {
+    return Rows{x.p.p + r0 * rowlen, x.e.p + r0, (int64_t)x.e.n - r0, f, s1, s2, s3, sb};
+  };
+  // Small systems on the FP64 pipe: an exact-slice product takes 33 us however
+  // short, a few us on the pipe while it has little to do (at (H2O)1 1.2 ms for
+  // the 30 products, 0.2 on the pipe; at (H2O)2 the pipe would need 6 ms where
+  // the slices take 2).  The line is 0.2 ms of the pipe's time.
+  const bool pipe = (double)o * o * o * (double)v3 * Kc < 1e8;
   auto pack = [&](const double* src, int64_t d1, int64_t d2, int64_t d3, int64_t s1, int64_t s2, int64_t s3, Packed& dst) {
     PackSpec ps{};
     ps.R = d1 * d2 * d3;
@@ -214,17 +223,18 @@ double triples_fp64(fcc_ctx* c, const std::vector<int3>* subset, std::vector<dou
     ps.kd2 = 1; ps.kd3 = Kc; ps.ks3 = 1;
     pack_oz(src, ps, lv.S, lv.bits, lv.guard, dst.p.p, dst.e.p, s);
   };
-  {
-    DBuf<double> H;
-    H.alloc(RH * Kc);
-    TView Hv = rm(H.p, {o, o, v, Kc});
-    einsum1(1.0, "xyzd->xyzd", t2v, 0.0, slice(Hv, 3, 0, v), s);
-    einsum(1.0, "Qly,Qxz->xyzl", Boo, Bov, 0.0, slice(Hv, 3, v, o), s);           // (ly|xz)
+  DBuf<double> H;
+  H.alloc(RH * Kc);
+  TView Hv = rm(H.p, {o, o, v, Kc});
+  einsum1(1.0, "xyzd->xyzd", t2v, 0.0, slice(Hv, 3, 0, v), s);
+  einsum(1.0, "Qly,Qxz->xyzl", Boo, Bov, 0.0, slice(Hv, 3, v, o), s);             // (ly|xz)
+  if (!pipe) {
     pHx.alloc(RH, rowlen);
     pHy.alloc(RH, rowlen);
     pack(H.p, o, o, v, o * v, v, 1, pHx);
     pack(H.p, o, o, v, v, o * v, 1, pHy);
-    FCC_CUDA(cudaStreamSynchronize(s));   // H is freed here
+    FCC_CUDA(cudaStreamSynchronize(s));
+    H.release();
   }
   DBuf<double> F;
   F.alloc(RF * Kc);
@@ -236,7 +246,7 @@ double triples_fp64(fcc_ctx* c, const std::vector<int3>* subset, std::vector<dou
   // FP64 and the rows of a run are packed for each pair of runs (hook: t3_kc).
   size_t mfree = 0, mtotal = 0;
   FCC_CUDA(cudaMemGetInfo(&mfree, &mtotal));
-  const bool whole = c->t3_kc_override <= 0 && 4.0 * (double)RF * (double)rowlen + 6e9 < (double)mfree;
+  const bool whole = !pipe && c->t3_kc_override <= 0 && 4.0 * (double)RF * (double)rowlen + 6e9 < (double)mfree;
   if (whole) {
     pF.alloc(RF, rowlen);
     pF2.alloc(RF, rowlen);
@@ -251,7 +261,7 @@ double triples_fp64(fcc_ctx* c, const std::vector<int3>* subset, std::vector<dou
   for (int64_t j = 0; j < o; ++j) slots = std::max(slots, (o - j) * (j + 1));
   slots = subset ? 1 : std::min(slots, c->t3_kc_override > 0 ? (int64_t)c->t3_kc_override : slots_max);
   c->Wt.alloc(slots * v3);
-  if (!whole) {
+  if (!whole && !pipe) {
     const int64_t run = std::min(slots, o);
     pF.alloc(run * v2, rowlen);
     pFj.alloc(v2, rowlen);
@@ -283,29 +293,43 @@ double triples_fp64(fcc_ctx* c, const std::vector<int3>* subset, std::vector<dou
     ep.beta = beta;
     ep.C = c->Wt.p;
     ep.batch = (int)batch; ep.ba = ba; ep.bb = bb; ep.bc = bc;
+    if (pipe) {
+      CtrDesc d{};
+      d.M = M; d.M2 = m.d2; d.M3 = m.d3; d.N = N; d.N2 = nn.d2; d.N3 = nn.d3; d.K = d.K2 = Kc; d.batch = batch;
+      d.a_m1 = a.s1 * Kc; d.a_m2 = a.s2 * Kc; d.a_m3 = a.s3 * Kc; d.a_k2 = 1;
+      d.b_n1 = b.s1 * Kc; d.b_n2 = b.s2 * Kc; d.b_n3 = b.s3 * Kc; d.b_k2 = 1;
+      d.c_m1 = m.s1; d.c_m2 = m.s2; d.c_m3 = m.s3; d.c_n1 = nn.s1; d.c_n2 = nn.s2; d.c_n3 = nn.s3;
+      d.a_b = batch > 1 && ba ? a.sb * Kc : 0;
+      d.b_b = batch > 1 && bb ? b.sb * Kc : 0;
+      d.c_b = bc;
+      d.alpha = 1.0; d.beta = beta;
+      contract_f64_launch(a.f, b.f, c->Wt.p, d, s);
+      return;
+    }
     ep.work = 2.0 * (double)batch * (double)M * (double)N * (double)Kc * oz_pairs(lv);
     gemm_oz(a.p, a.n, a.e, b.p, b.n, b.e, Kpad, lv, ep, c->tc.ozws, c->tc.err, s);
   };
   // W[i][k][a][b][c] for i in [i0, i0 + ni), k in [k0, k0 + nk) and one j
   auto build_w = [&](int64_t i0, int64_t ni, int64_t j, int64_t k0, int64_t nk) {
     const int64_t ws = nk * v3;   // stride of i
-    Rows fi, fj, fk;              // F[i] and F[j] by (x, y, z), F[k] by (x, z, y)
-    if (whole) {
-      fi = rows(pF, i0 * v2);
-      fj = rows(pF, j * v2);
-      fk = rows(pF2, k0 * v2);
-    } else {
+    if (!whole && !pipe) {
       pack(F.p + i0 * v2 * Kc, ni, v, v, v2, v, 1, pF);
       pack(F.p + j * v2 * Kc, 1, v, v, v2, v, 1, pFj);
       pack(F.p + k0 * v2 * Kc, nk, v, v, v2, 1, v, pF2);
-      fi = rows(pF, 0);
-      fj = rows(pFj, 0);
-      fk = rows(pF2, 0);
     }
-    const Rows hk = rows(pHy, (j * o + k0) * v);    // H[k..][j]
-    const Rows hki = rows(pHy, (i0 * o + k0) * v);  // H[k..][i]
-    const Rows hji = rows(pHx, (j * o + i0) * v), hjk = rows(pHx, (j * o + k0) * v);
-    const Rows hij = rows(pHy, (j * o + i0) * v), hik = rows(pHx, (i0 * o + k0) * v);
+    // F[i] and F[j] by (x, y, z), F[k] by (x, z, y)
+    const double* Fp = F.p;
+    const double* Hp = H.p;
+    const Rows fi = rows(pF, whole ? i0 * v2 : 0, Fp + i0 * v2 * Kc, v2, v, 1, 0);
+    const Rows fj = rows(whole || pipe ? pF : pFj, whole ? j * v2 : 0, Fp + j * v2 * Kc, v2, v, 1, 0);
+    const Rows fk = rows(pF2, whole ? k0 * v2 : 0, Fp + k0 * v2 * Kc, v2, 1, v, 0);
+    auto h = [&](const Packed& ph, int64_t first, int64_t x, int64_t y, int64_t s2, int64_t sb) {
+      return rows(ph, first * v, Hp + (x * o + y) * v * Kc, 0, s2, 1, sb);
+    };
+    const Rows hk = h(pHy, j * o + k0, k0, j, o * v, 0);         // H[k..][j]
+    const Rows hki = h(pHy, i0 * o + k0, k0, i0, o * v, v);      // H[k..][i]
+    const Rows hji = h(pHx, j * o + i0, j, i0, v, 0), hjk = h(pHx, j * o + k0, j, k0, v, 0);
+    const Rows hij = h(pHy, j * o + i0, i0, j, o * v, 0), hik = h(pHx, i0 * o + k0, i0, k0, v, o * v);
     // F[i](a,b) H[k][j](c): rows (i,a,b), columns (k,c)
     product(fi, ni * v2, {v, v, ws, v2, v}, hk, nk * v, {nk, v, 0, v3, 1}, 0.0, 1, 0, 0, 0);
     // F[j](b,a) H[k][i](c): rows (b,a), columns (k,c), a product per i

@@ -156,3 +156,28 @@ def test_triples_pack_by_runs_gives_the_same_energy():
     ctx.close()
     Options.reset()
     assert abs(runs - whole) < 1e-13 * abs(whole), (runs, whole)
+
+
+def test_triples_small_and_sliced_forms_agree():
+    # a size on either side of the rule o^3 v^3 (v + o) < 1e8 against the oracle's
+    # sum over all triples is in test_gpu_triples.py; here the same amplitudes
+    # triple by triple against the whole
+    from conftest import inputs
+    from fermicc import Options, RCCSD, _lib
+    from fermicc.rccsd import Context
+    import ctypes
+    inp = inputs(1)
+    Options.reset()
+    Options.set("cc_max_iter", 2)
+    ctx = Context(inp)
+    RCCSD.compute(inp, context=ctx)
+    lib = _lib.load()
+    whole = ctx.triples(_lib.FCC_PREC_FP64)
+    o = inp.o
+    ijk = np.array([(i, j, k) for i in range(o) for j in range(i + 1) for k in range(j + 1) if not i == j == k], np.int32)
+    each = np.zeros(len(ijk))
+    assert lib.fcc_test_triples_subset(ctx.h, ijk.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)), len(ijk),
+                                       each.ctypes.data_as(ctypes.POINTER(ctypes.c_double))) == 0
+    ctx.close()
+    Options.reset()
+    assert abs(each.sum() - whole) < 1e-12 * abs(whole), (each.sum(), whole)
