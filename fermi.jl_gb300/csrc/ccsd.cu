@@ -379,6 +379,63 @@ __global__ void __launch_bounds__(RED_THREADS) divide_d2_kernel(double* t2, cons
   }
 }
 
+// out[i][j][:] = a x[i][j][:] - x[j][i][:] over rows of `len`, the rows (i, j)
+// and (j, i) together so that x is read once: HBM bound, 60 us at (H2O)8 (189
+// MB each way; 486 us as two passes over out).
+__global__ void __launch_bounds__(256) swap_sub_kernel(const double* __restrict__ x, double* __restrict__ out, int o,
+                                                       int64_t len, double a) {
+  const int i = blockIdx.y, j = blockIdx.z;
+  if (j < i) return;
+  constexpr int U = 8;
+  const int64_t rij = ((int64_t)i * o + j) * len, rji = ((int64_t)j * o + i) * len;
+  const int64_t e0 = (int64_t)blockIdx.x * (256 * U) + threadIdx.x;
+  double p[U], q[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int64_t e = e0 + 256 * u;
+    p[u] = e < len ? x[rij + e] : 0.0;
+    q[u] = e < len && i != j ? x[rji + e] : p[u];
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int64_t e = e0 + 256 * u;
+    if (e < len) {
+      out[rij + e] = fma(a, p[u], -q[u]);
+      if (i != j) out[rji + e] = fma(a, q[u], -p[u]);
+    }
+  }
+}
+
+// R[i][j][a][b] += P[i][j][a][b] + P[j][i][b][a], the pairs (i, j) and (j, i) of a
+// 32 x 32 tile together, so P and R are read once: 107 us at (H2O)8, 551 as two
+// passes.
+__global__ void __launch_bounds__(256) sym_add_kernel(const double* __restrict__ P, double* __restrict__ R, int o, int v) {
+  const int i = blockIdx.y, j = blockIdx.z;
+  if (j < i) return;
+  __shared__ double tij[32][33], tji[32][33];   // P[i][j] tile (a, b), P[j][i] tile (b, a)
+  const int nt = (v + 31) / 32, a0 = (blockIdx.x / nt) * 32, b0 = (blockIdx.x % nt) * 32;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int64_t rij = ((int64_t)i * o + j) * v * v, rji = ((int64_t)j * o + i) * v * v;
+  double x[4], y[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int r = ty + 8 * q;
+    const bool ij = a0 + r < v && b0 + tx < v, ji = b0 + r < v && a0 + tx < v;
+    const int64_t eij = rij + (int64_t)(a0 + r) * v + b0 + tx, eji = rji + (int64_t)(b0 + r) * v + a0 + tx;
+    tij[r][tx] = ij ? P[eij] : 0.0;
+    tji[r][tx] = ji ? P[eji] : 0.0;
+    x[q] = ij ? R[eij] : 0.0;
+    y[q] = ji && i != j ? R[eji] : 0.0;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int r = ty + 8 * q;
+    if (a0 + r < v && b0 + tx < v) R[rij + (int64_t)(a0 + r) * v + b0 + tx] = (x[q] + tij[r][tx]) + tji[tx][r];
+    if (i != j && b0 + r < v && a0 + tx < v) R[rji + (int64_t)(b0 + r) * v + a0 + tx] = (y[q] + tji[r][tx]) + tij[tx][r];
+  }
+}
+
 // X = 1 - T, Y = 1 + T^T with T[a,i] = t1[i,a] (n x n, row-major).
 __global__ void dress_mats_kernel(const double* t1, int o, int v, double* X, double* Y) {
   int n = o + v;
@@ -645,12 +702,9 @@ void residual(fcc_ctx* c) {
   TView Btoo = blk(Bt, 0, o, 0, o), Btov = blk(Bt, 0, o, o, v), Btvo = blk(Bt, o, v, 0, o), Btvv = blk(Bt, o, v, o, v);
 
   // ---- T1-dressed factors: Bt = X B Y^T blockwise
-  einsum1(1.0, "Qij->Qij", Boo, 0.0, Btoo, s);
+  FCC_CUDA(cudaMemcpyAsync(c->Bt.p, c->B.p, sizeof(double) * Q * n * n, cudaMemcpyDeviceToDevice, s));
   einsum(1.0, "Qib,jb->Qij", Bov, t1, 1.0, Btoo, s);
-  einsum1(1.0, "Qia->Qia", Bov, 0.0, Btov, s);
-  einsum1(1.0, "Qab->Qab", Bvv, 0.0, Btvv, s);
   einsum(-1.0, "ka,Qkb->Qab", t1, Bov, 1.0, Btvv, s);
-  einsum1(1.0, "Qai->Qai", Bvo, 0.0, Btvo, s);
   einsum(-1.0, "ka,Qki->Qai", t1, Boo, 1.0, Btvo, s);
   einsum(1.0, "Qac,ic->Qai", Btvv, t1, 1.0, Btvo, s);
 
@@ -686,9 +740,13 @@ void residual(fcc_ctx* c) {
   TView Di = rm(c->Dint.p, {v, o, o, v});   // [a][i][k][c]
   TView Xo = rm(c->Xo.p, {o, o, o, o});     // [k][i][l][j]
 
+  auto swap_sub = [&](const double* x, double* out, double a) {
+    const int64_t len = v * v;
+    swap_sub_kernel<<<dim3((unsigned)((len + 2047) / 2048), (unsigned)o, (unsigned)o), 256, 0, s>>>(x, out, (int)o, len, a);
+    FCC_CHECK_LAUNCH();
+  };
   // u_ijab = 2 t_ijab - t_jiab
-  einsum1(2.0, "ijab->ijab", t2, 0.0, u, s);
-  einsum1(-1.0, "jiab->ijab", t2, 1.0, u, s);
+  swap_sub(c->t2.p, c->u.p, 2.0);
 
   // ---- doubles
   einsum(1.0, "Qai,Qbj->ijab", Btvo, Btvo, 0.0, R2, s);                 // (ai|bj)
@@ -797,8 +855,7 @@ void residual(fcc_ctx* c) {
   // F_ijab = t_kj^bc C_ki^ac: one o^3 v^3 contraction instead of two
   TView Fr = rm(c->Fring.p, {o, o, v, v});
   einsum(1.0, "kjbc,kiac->ijab", t2, Ci, 0.0, Fr, s);
-  einsum1(-0.5, "ijab->ijab", Fr, 0.0, P, s);
-  einsum1(-1.0, "jiab->ijab", Fr, 1.0, P, s);
+  swap_sub(c->Fring.p, c->P.p, -0.5);
   einsum(0.5, "jkbc,aikc->ijab", u, Di, 1.0, P, s);
   // Fock-like terms
   TView Fvvp = rm(c->Fvv.p, {v, v}), Foop = rm(c->Foo.p, {o, o});
@@ -809,8 +866,11 @@ void residual(fcc_ctx* c) {
   einsum(1.0, "jlcd,klcd->kj", u, V2, 1.0, Foop, s);
   einsum(1.0, "ijac,bc->ijab", t2, Fvvp, 1.0, P, s);
   einsum(-1.0, "ikab,kj->ijab", t2, Foop, 1.0, P, s);
-  einsum1(1.0, "ijab->ijab", P, 1.0, R2, s);
-  einsum1(1.0, "jiba->ijab", P, 1.0, R2, s);
+  {
+    const int64_t nt = (v + 31) / 32;
+    sym_add_kernel<<<dim3((unsigned)(nt * nt), (unsigned)o, (unsigned)o), 256, 0, s>>>(c->P.p, c->r2.p, (int)o, (int)v);
+    FCC_CHECK_LAUNCH();
+  }
 
   // ---- singles
   einsum1(1.0, "ai->ia", Fvo, 0.0, R1, s);

@@ -416,12 +416,12 @@ __global__ void __launch_bounds__(256) gemv_cols_f64_kernel(const double* __rest
 }
 
 // out[i0 i1 i2 i3] = alpha in + beta out: a warp per run of up to 128 elements
-// of the last index, so the index arithmetic is per run.
+// of the last index (runs of equal length), so the index arithmetic is per run.
 __global__ void __launch_bounds__(256) axpby4_kernel(const double* __restrict__ in, double* __restrict__ out,
                                                      uint32_t d1, uint32_t d2, uint32_t d3, int64_t si0, int64_t si1,
                                                      int64_t si2, int64_t si3, int64_t so0, int64_t so1, int64_t so2,
                                                      int64_t so3, double alpha, double beta, uint32_t nseg,
-                                                     int64_t runs) {
+                                                     uint32_t seglen, int64_t runs) {
   const int lane = threadIdx.x & 31;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < runs; w += nw) {
@@ -433,23 +433,24 @@ __global__ void __launch_bounds__(256) axpby4_kernel(const double* __restrict__ 
     const uint32_t i1 = r % d1, i0 = r / d1;
     const double* src = in + (int64_t)i0 * si0 + (int64_t)i1 * si1 + (int64_t)i2 * si2;
     double* dst = out + (int64_t)i0 * so0 + (int64_t)i1 * so1 + (int64_t)i2 * so2;
-    const uint32_t j0 = seg * 128 + lane;
+    const uint32_t jend = min(d3, (seg + 1) * seglen), jw = seg * seglen, j0 = jw + lane;
     double v[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const uint32_t j = j0 + 32 * q;
-      v[q] = j < d3 ? src[(int64_t)j * si3] : 0.0;
+      v[q] = j < jend ? src[(int64_t)j * si3] : 0.0;
     }
     double p[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const uint32_t j = j0 + 32 * q;
-      p[q] = beta != 0.0 && j < d3 ? dst[(int64_t)j * so3] : 0.0;
+      p[q] = beta != 0.0 && j < jend ? dst[(int64_t)j * so3] : 0.0;
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const uint32_t j = j0 + 32 * q;
-      if (j < d3) dst[(int64_t)j * so3] = f64_axpby(v[q], p[q], alpha, beta);
+      if (jw + 32 * q >= jend) break;   // an FP64 instruction takes its 16 clk also where no lane needs it
+      if (j < jend) dst[(int64_t)j * so3] = f64_axpby(v[q], p[q], alpha, beta);
     }
   }
 }
@@ -641,12 +642,12 @@ void tensor_axpby_launch(const TView& in, const TView& out, double alpha, double
     FCC_CHECK_LAUNCH();
     return;
   }
-  const int64_t nseg = (dim[3] + 127) / 128;
+  const int64_t nseg = (dim[3] + 127) / 128, seglen = ((dim[3] + nseg - 1) / nseg + 31) / 32 * 32;
   const int64_t runs = dim[0] * dim[1] * dim[2] * nseg;
   if (runs >= (int64_t(1) << 31)) fail(FCC_ERR_BAD_ARG, "tensor too large");
   axpby4_kernel<<<(unsigned)std::min<int64_t>((runs + 7) / 8, 152 * 16), 256, 0, s>>>(
       in.p, out.p, (uint32_t)dim[1], (uint32_t)dim[2], (uint32_t)dim[3], si[0], si[1], si[2], si[3], so[0], so[1],
-      so[2], so[3], alpha, beta, (uint32_t)nseg, runs);
+      so[2], so[3], alpha, beta, (uint32_t)nseg, (uint32_t)seglen, runs);
   FCC_CHECK_LAUNCH();
 }
 
