@@ -12,13 +12,16 @@
 // operand tile with the step before: the tiles
 //   B_g, A_1, B_(g-1), A_2, ..., B_1, A_g
 // arrive as one stream and step i multiplies tiles i and i + 1.  A step then
-// moves 16 KB into shared memory instead of 32 KB.  What bounds long products
+// moves one tile into shared memory instead of two.  What bounds long products
 // is shared-memory bandwidth (128 B/clk per SM): the MMAs of a 128 x 128 x 64
-// step read 32 KB in 256 clk while the incoming tile is written, 384 clk with
-// one new tile (two thirds of the tensor rate), 512 with two.  Measured at M =
-// N = K = 4864: 1330 TFLOP/s executed (21 products of 6-bit digits, 3.6 ms;
-// 6.0 ms and 802 TFLOP/s with two tiles a step and single threads the compiler
-// could not tell from warps, fcc_tcgen05.cuh elect_one).
+// step read 32 KB in 256 clk while the incoming 16 KB are written, 384 clk (two
+// thirds of the tensor rate; 512 with two new tiles).  So two CTAs on
+// neighbouring SMs share a 256 x 128 tile where its rows allow (cta_group::2):
+// each keeps half of every B tile, and reads 24 KB and writes 12 a step, 288
+// clk.  Measured at M = N = K = 4864, 21 products of 6-bit digits: 3.03 ms and
+// 1596 TFLOP/s executed (3.60 with single CTAs; 6.0 with two new tiles a step
+// and roles in threads the compiler could not tell from warps, fcc_tcgen05.cuh
+// elect_one).
 //
 // When an accumulator could reach 2^24 (a chunk: 1-4 k-blocks of 8-bit digits,
 // 25-64 of 6-bit ones) the eight epilogue warps add it, times its weight (a
@@ -27,8 +30,8 @@
 // TMEM for two sets of two chunk accumulators, so the MMA thread fills one set
 // while the other is drained, and a drain reads 4 bytes per element from TMEM
 // instead of moving 20.  The additions run two per instruction (fma.rn.f32x2).
-// With 8-bit digits the chunks are short and the drains show: 1200 TFLOP/s at
-// 4864, 4.0 ms for the 48 bits that took 10.2 ms with 36 products of 6-bit
+// With 8-bit digits the chunks are short and the drains show: 1325 TFLOP/s at
+// 4864, 3.65 ms for the 48 bits that took 10.2 ms with 36 products of 6-bit
 // digits.
 //
 // Batches: products of the same shape whose rows lie apart by fixed steps in A,
@@ -46,8 +49,7 @@
 // lo and tail, a short form where no exponent can leave the FP64 range, sums
 // handed over through shared memory so that a warp stores whole rows, and
 // red.add where C is added to (the read would wait in the warp, the addition
-// is the L2's): 5776 x 1216 x 92 at the FP64 level 137 us; 143 with the general
-// conversion only.
+// is the L2's): 5776 x 1216 x 92 at the FP64 level 133 us.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -213,15 +215,19 @@ __device__ __forceinline__ double ff_to_f64_safe(float hf, float lf, float tail,
   return __hiloint2double(a ? (int)w1 : 0, a ? (int)(uint32_t)mag : 0);
 }
 
-// Persistent: CTA b processes units b, b + gridDim.x, ...; unit u is output
+// Persistent: worker b processes units b, b + workers, ...; unit u is output
 // tile u % tiles of job (u / tiles) % njobs of product u / (tiles njobs).  The
 // tile ring and the accumulator sets run on across units, so the loads and MMAs
-// of a unit's first chunks overlap the previous unit's stores.  Every role walks the same sequence: parts,
-// L2 blocks of kper k-blocks (units running at the same time share one, so
-// the slices they stream stay in L2), bands, chunks of ck k-blocks.
+// of a unit's first chunks overlap the previous unit's stores.  Every role walks
+// the same sequence: parts, L2 blocks of kper k-blocks (units running at the
+// same time share one, so the slices they stream stay in L2), bands, chunks of
+// ck k-blocks.  PAIR: a cluster of two CTAs is one worker; each loads its rows
+// of A and half of B, the loads of both count on the first CTA's barriers, which
+// issues the MMAs for both; barriers that free tiles or hand over accumulators
+// are signalled in both.
 // F64: the FP64 level, whose store stage may take the last band's accumulators
 // along (P.merged).
-template <bool F64>
+template <bool F64, bool PAIR>
 __global__ void __launch_bounds__(OZ_THREADS, 1)
     gemm_oz_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    const __grid_constant__ OzParams P, const int* __restrict__ exA, const int* __restrict__ exB,
@@ -239,6 +245,11 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   float* xp = reinterpret_cast<float*>(smem + OZ_SLOTS * OZ_TILE_BYTES);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t tiles = P.tm * P.tn;
+  // PAIR: two CTAs share a 256 x 128 tile; this one has 128 of its rows and
+  // loads half of each B tile; the first issues the MMAs
+  const uint32_t rank = PAIR ? cluster_rank() : 0u;
+  const uint32_t wid = PAIR ? blockIdx.x >> 1 : blockIdx.x, nwork = PAIR ? gridDim.x >> 1 : gridDim.x;
+  constexpr int UM = PAIR ? 2 * OZ_BM : OZ_BM;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < OZ_SLOTS; ++s) {
@@ -247,20 +258,28 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&accf_bar[b]), 1);
-      mbar_init(smem_u32(&acce_bar[b]), OZ_EPI_WARPS);
+      mbar_init(smem_u32(&acce_bar[b]), PAIR ? 2 * OZ_EPI_WARPS : OZ_EPI_WARPS);
     }
     mbar_init(smem_u32(&done_bar), 1);
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_holder)),
-                 "r"(512)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_holder)),
+                   "r"(512)
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_holder)),
+                   "r"(512)
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (PAIR) cluster_sync();     // both CTAs' barriers are there before either is signalled
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_holder;
 
@@ -279,13 +298,13 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       uint32_t ph = 0;
       uint32_t issued = 0, parity = 0;   // slots loaded by this thread, phase parity of the last load of each
       bool stop = false;
-      for (uint32_t u = blockIdx.x; u < P.units && !stop; u += gridDim.x) {
+      for (uint32_t u = wid; u < P.units && !stop; u += nwork) {
         uint32_t mt, nt;
         grouped_tile(u % tiles, P.tm, P.tn, mt, nt);
         const uint32_t q = u / tiles;
         const OzJob jb = P.job[q % P.njobs];
         const int64_t bq = q / P.njobs;
-        const int row = (int)(isB ? bq * ep.bb + nt * OZ_BN : bq * ep.ba + mt * OZ_BM);
+        const int row = (int)(isB ? bq * ep.bb + nt * OZ_BN + rank * (OZ_BN / 2) : bq * ep.ba + mt * UM + rank * OZ_BM);
         int bb = jb.b0;
         while (bb < jb.b1 && !stop) {
           const int be = (bb < P.cut) ? min(P.cut, (int)jb.b1) : (int)jb.b1;   // this part's bands
@@ -303,8 +322,14 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                 for (int i = 0; i < np; ++i, x += dx) {
                   if (!mbar_wait(smem_u32(&empty_bar[cs]), cp ^ 1)) { atomicExch(&abort_flag, 1); stop = true; break; }
                   const uint32_t fb = smem_u32(&full_bar[cs]);
-                  mbar_expect_tx(fb, OZ_TILE_BYTES);
-                  tma_load_2d(smem_u32(smem + cs * OZ_TILE_BYTES), tm, x, row, fb);
+                  if (PAIR) {
+                    // both CTAs' halves count on the first one's barrier
+                    if (rank == 0) mbar_expect_tx(fb, isB ? OZ_TILE_BYTES : 2 * OZ_TILE_BYTES);
+                    tma_load_2d_pair(smem_u32(smem + cs * OZ_TILE_BYTES), tm, x, row, cluster_addr(fb, 0));
+                  } else {
+                    mbar_expect_tx(fb, OZ_TILE_BYTES);
+                    tma_load_2d(smem_u32(smem + cs * OZ_TILE_BYTES), tm, x, row, fb);
+                  }
                   issued |= 1u << cs;
                   parity = (parity & ~(1u << cs)) | (cp << cs);
                   cs += 2;
@@ -321,25 +346,34 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       }
       // on an abort, wait (bounded) for the loads still in flight before the
       // shared memory can be released
-      if (*(volatile int*)&abort_flag) {
+      // (a pair's first CTA waits for the loads of both)
+      if (*(volatile int*)&abort_flag && rank == 0) {
         for (int c = 0; c < OZ_SLOTS; ++c)
           if ((issued >> c) & 1) (void)mbar_wait(smem_u32(&full_bar[c]), (parity >> c) & 1);
       }
      }
-    } else if (warp == 1) {
+    } else if (warp == 1 && rank == 0) {
      if (elect_one()) {
       // ---------------- MMA issuer.  An MMA's issue waits until the one before
       // it has started, so whatever the thread does between two steps leaves
       // the tensor pipe idle unless it runs behind an issued MMA: the next
       // tile's barrier is read between the MMAs of a step, and a step's
       // descriptors need one addition each.
-      constexpr uint32_t idesc = idesc_bf16(OZ_BM, OZ_BN);
+      constexpr uint32_t idesc = idesc_bf16(UM, OZ_BN);
+      auto mma = [&](uint32_t d, uint64_t ad, uint64_t bd, uint32_t acc) {
+        if (PAIR) mma_bf16_pair(d, ad, bd, idesc, acc);
+        else mma_bf16(d, ad, bd, idesc, acc);
+      };
+      auto commit = [&](uint32_t bar) {
+        if (PAIR) tc_commit_pair(bar);
+        else tc_commit(bar);
+      };
       const uint64_t desc0 = sw128_desc(smem_u32(smem));
       const uint32_t full0 = smem_u32(&full_bar[0]), empty0 = smem_u32(&empty_bar[0]);
       uint32_t s = 0, ph = 0;      // ring slot of the next tile, and its phase
       uint32_t chunk = 0;
       bool ok = true;
-      for (uint32_t u = blockIdx.x; u < P.units && ok; u += gridDim.x) {
+      for (uint32_t u = wid; u < P.units && ok; u += nwork) {
         const OzJob jb = P.job[(u / tiles) % P.njobs];
         int bb = jb.b0;
         while (bb < jb.b1 && ok) {
@@ -373,14 +407,14 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                     const uint64_t bdsc = desc0 + (uint64_t)((curB ? s : pslot) * (OZ_TILE_BYTES >> 4));
                     const uint32_t dcol = dset + par * OZ_BN;
                     const uint32_t acc = (started >> par) & 1u;
-                    mma_bf16(dcol, ad, bdsc, idesc, acc);
+                    mma(dcol, ad, bdsc, acc);
                     peek = mbar_test(full0 + 8 * s2, ph2);
-                    mma_bf16(dcol, ad + 2, bdsc + 2, idesc, 1u);
+                    mma(dcol, ad + 2, bdsc + 2, 1u);
                     started |= 1u << par;
                     par ^= 1u;
-                    mma_bf16(dcol, ad + 4, bdsc + 4, idesc, 1u);
-                    mma_bf16(dcol, ad + 6, bdsc + 6, idesc, 1u);
-                    tc_commit(empty0 + 8 * pslot);                     // its last use
+                    mma(dcol, ad + 4, bdsc + 4, 1u);
+                    mma(dcol, ad + 6, bdsc + 6, 1u);
+                    commit(empty0 + 8 * pslot);                     // its last use
                   } else {
                     peek = 0;
                   }
@@ -389,20 +423,20 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                   ph = ph2;
                   curB ^= 1u;
                   if (++t == nt_) {
-                    tc_commit(empty0 + 8 * pslot);
+                    commit(empty0 + 8 * pslot);
                     t = 0;
                     par = par0;
                   }
                 }
                 if (!ok) break;
-                tc_commit(smem_u32(&accf_bar[set]));
+                commit(smem_u32(&accf_bar[set]));
               }
             }
           }
           bb = be;
         }
       }
-      tc_commit(smem_u32(&done_bar));
+      commit(smem_u32(&done_bar));
      }
     }
   } else {
@@ -414,6 +448,11 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     const uint64_t m1 = pack2(0xBF800000u, 0xBF800000u);   // -1, -1
     bool ok = true;
     uint32_t chunk = 0;
+    auto drained = [&](int set) {   // an accumulator set is free for the MMA thread
+      const uint32_t bar = smem_u32(&acce_bar[set]);
+      if (PAIR) mbar_arrive_cluster(cluster_addr(bar, 0));
+      else mbar_arrive(bar);
+    };
     // alpha = +-2^ka folds into the exponent arithmetic; otherwise one FP64 multiply
     const double alpha = P.part ? 1.0 : ep.alpha;
     const unsigned long long ab = (unsigned long long)__double_as_longlong(alpha);
@@ -421,7 +460,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     const int ka = (apow2 ? (int)((ab >> 52) & 0x7FF) - 1023 : 0) + 2 * P.guard;
     const uint32_t aneg = apow2 && (ab >> 63) ? 0x80000000u : 0u;
     const double alpha_left = apow2 ? 1.0 : alpha;
-    for (uint32_t u = blockIdx.x; u < P.units && ok; u += gridDim.x) {
+    for (uint32_t u = wid; u < P.units && ok; u += nwork) {
       uint32_t mt, nt;
       grouped_tile(u % tiles, P.tm, P.tn, mt, nt);
       const uint32_t slot = u / tiles;           // (product, job)
@@ -431,7 +470,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       while (bb < jb.b1 && ok) {
         const int be = (bb < P.cut) ? min(P.cut, (int)jb.b1) : (int)jb.b1;
         // what the store stage needs, read ahead of the sums
-        const int64_t m = (int64_t)mt * OZ_BM + q * 32 + lane;
+        const int64_t m = (int64_t)mt * UM + rank * OZ_BM + q * 32 + lane;
         int64_t crow = 0;
         int erow = 0;
         if (m < ep.M) {
@@ -490,7 +529,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
               }
               asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
               __syncwarp();
-              if (lane == 0) mbar_arrive(smem_u32(&acce_bar[set]));
+              if (lane == 0) drained(set);
             }
           }
         }
@@ -501,7 +540,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         const int bmode = first ? (P.part || ep.beta == 0.0 ? 0 : (ep.beta == 1.0 ? 1 : 2)) : 1;
         double* out = P.part ? P.part : static_cast<double*>(ep.C);
         // rows this lane stores: 2 j + lane / 16
-        const int rows = (int)min((int64_t)32, ep.M - ((int64_t)mt * OZ_BM + q * 32));
+        const int rows = (int)min((int64_t)32, ep.M - ((int64_t)mt * UM + rank * OZ_BM + q * 32));
         // the usual case: factors of a power of two, exponents well inside the FP64 range
         const bool plain = __all_sync(0xffffffffu, apow2 && bmode < 2 && abs(erow) < 400 && abs(ecl[0]) < 400 &&
                                                        abs(ecl[1]) < 400);
@@ -600,7 +639,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         if (F64 && last >= 0) {
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(&acce_bar[last]));
+          if (lane == 0) drained(last);
         }
         bb = be;
       }
@@ -612,9 +651,11 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (PAIR) cluster_sync();     // neither CTA goes while the other may still signal it or read its tiles
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
   }
   if (threadIdx.x == 0 && abort_flag) atomicExch(err, 1);
 }
@@ -665,7 +706,8 @@ OzLevel oz_level(int groups) {
 }
 
 void gemm_oz(const __nv_bfloat16* A, int64_t a_rows, const int* exA, const __nv_bfloat16* B, int64_t b_rows,
-             const int* exB, int64_t Kpad, OzLevel lv, const EpiMap& ep, DBuf<double>& ws, int* err, cudaStream_t s) {
+             const int* exB, int64_t Kpad, OzLevel lv, const EpiMap& ep0, DBuf<double>& ws, int* err, cudaStream_t s) {
+  EpiMap ep = ep0;
   if (ep.M <= 0 || ep.N <= 0) return;
   if (lv.S < 1 || lv.S > OZ_MAXS || lv.G < 2 || lv.G > lv.S + 2 || (lv.bits != 6 && lv.bits != 8) || lv.guard < 0 || lv.guard > 2)
     fail(FCC_ERR_BAD_ARG, "bad exact-slice level");
@@ -673,9 +715,33 @@ void gemm_oz(const __nv_bfloat16* A, int64_t a_rows, const int* exA, const __nv_
   if (ep.batch < 1 || ep.batch > 65535 || a_rows < ep.M + (ep.batch - 1) * ep.ba || b_rows < ep.N + (ep.batch - 1) * ep.bb)
     fail(FCC_ERR_BAD_ARG, "packed operands smaller than the output");
   if (ep.M >= (int64_t(1) << 31) || ep.N >= (int64_t(1) << 31)) fail(FCC_ERR_BAD_ARG, "output extent too large");
+  // Pairs of CTAs on 256 x 128 tiles (4864^3 at 6 bits 3.03 ms, 3.60 with single
+  // CTAs on 128 x 128), unless the last tile would leave more than an eighth of
+  // the rows' work to padding.  A long product whose columns fit pairs and whose
+  // rows do not is turned over: its stores no longer coalesce, which 32 k-blocks
+  // outweigh (528 x 2888 x 11628: 0.79 ms as it stands, 0.67 turned over).
+  auto pairs = [](int64_t rows) {
+    const int64_t t = (rows + OZ_BM - 1) / OZ_BM;
+    return t % 2 == 0 || t >= 8;
+  };
+  if (!pairs(ep.M) && pairs(ep.N) && Kpad >= 32 * OZ_BK) {
+    std::swap(A, B);
+    std::swap(a_rows, b_rows);
+    std::swap(exA, exB);
+    std::swap(ep.M, ep.N);
+    std::swap(ep.md2, ep.nd2);
+    std::swap(ep.md3, ep.nd3);
+    std::swap(ep.ms1, ep.ns1);
+    std::swap(ep.ms2, ep.ns2);
+    std::swap(ep.ms3, ep.ns3);
+    std::swap(ep.ba, ep.bb);
+  }
+  const bool pair = pairs(ep.M);
   std::call_once(g_oz_attr, []() {
-    cudaFuncSetAttribute(gemm_oz_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM);
-    cudaFuncSetAttribute(gemm_oz_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM);
+    cudaFuncSetAttribute(gemm_oz_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM);
+    cudaFuncSetAttribute(gemm_oz_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM);
+    cudaFuncSetAttribute(gemm_oz_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM);
+    cudaFuncSetAttribute(gemm_oz_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM);
   });
   OzParams P;
   std::memset(&P, 0, sizeof(P));
@@ -685,7 +751,9 @@ void gemm_oz(const __nv_bfloat16* A, int64_t a_rows, const int* exA, const __nv_
   P.cut = lv.cut;
   P.kpad = (int)Kpad;
   const int nkb = (int)(Kpad / OZ_BK);
-  const int64_t tm = (ep.M + OZ_BM - 1) / OZ_BM, tn = (ep.N + OZ_BN - 1) / OZ_BN;
+  const int64_t rows_unit = pair ? 2 * OZ_BM : OZ_BM;
+  const int64_t tm = (ep.M + rows_unit - 1) / rows_unit, tn = (ep.N + OZ_BN - 1) / OZ_BN;
+  const int64_t workers = pair ? 76 : 152;
   const int64_t tiles = tm * tn;
   if (tiles * OZ_MAXJOBS * ep.batch >= (int64_t(1) << 31) || a_rows >= (int64_t(1) << 31) || b_rows >= (int64_t(1) << 31))
     fail(FCC_ERR_BAD_ARG, "tensor-core grid too large");
@@ -697,9 +765,9 @@ void gemm_oz(const __nv_bfloat16* A, int64_t a_rows, const int* exA, const __nv_
   // or every slice is fetched again from HBM for each pair that uses it (a
   // full-K ring launch at (H2O)8 read 17 GB for 0.76 GB of packed operands)
   const double panel = (double)OZ_BM * lv.S * OZ_BK * 2.0;   // bytes per k-block
-  const int64_t conc = std::min<int64_t>(tiles, 152);
-  const int64_t rblk = std::min<int64_t>(tm, 8);
-  const int64_t cblk = std::min<int64_t>(tn, (conc + rblk - 1) / rblk);
+  const int64_t conc = std::min<int64_t>(tiles, workers);
+  const int64_t rtile = std::min<int64_t>(tm, 8);
+  const int64_t cblk = std::min<int64_t>(tn, (conc + rtile - 1) / rtile), rblk = pair ? 2 * rtile : rtile;
   constexpr double L2_BUDGET = 48.0 * (1 << 20);
   P.kper = (int)std::max(4.0, L2_BUDGET / ((double)(rblk + cblk) * panel));
   P.kper = std::min(P.kper & ~3, std::max(4, nkb));          // whole chunks of every band
@@ -745,14 +813,14 @@ void gemm_oz(const __nv_bfloat16* A, int64_t a_rows, const int* exA, const __nv_
     const int64_t units = tiles * n * ep.batch;
     double t = 0;
     for (int c = 0; c < std::min<int64_t>(units, 4); ++c) {
-      const int64_t cta = c == 0 ? 0 : (c == 1 ? std::min<int64_t>(units, 152) - 1 : (c == 2 ? 75 : 110));
+      const int64_t cta = c == 0 ? 0 : (c == 1 ? std::min<int64_t>(units, workers) - 1 : (c == 2 ? workers / 2 : 3 * workers / 4));
       double l = 0;
-      for (int64_t u = cta; u < units; u += 152) {
+      for (int64_t u = cta; u < units; u += workers) {
         const OzJob& j = P.job[(u / tiles) % n];
         double st = 0;
         for (int b = j.b0; b < j.b1; ++b) st += P.band[b].ntile - 1;
         l += st * (j.k1 - j.k0) + FIXED;
-        if (units > 152 * 64) { l *= (double)((units + 151) / 152); break; }
+        if (units > workers * 64) { l *= (double)((units + workers - 1) / workers); break; }
       }
       t = std::max(t, l);
     }
@@ -776,11 +844,22 @@ void gemm_oz(const __nv_bfloat16* A, int64_t a_rows, const int* exA, const __nv_
     P.kper = std::max(P.kper, nkb);
   }
   CUtensorMap ta = tma_map_bf16(A, a_rows, lv.S * Kpad, OZ_BM);
-  CUtensorMap tb = tma_map_bf16(B, b_rows, lv.S * Kpad, OZ_BN);
-  const unsigned grid = (unsigned)std::min<int64_t>(P.units, 152);   // one persistent CTA per SM
+  CUtensorMap tb = tma_map_bf16(B, b_rows, lv.S * Kpad, pair ? OZ_BN / 2 : OZ_BN);
+  // persistent: one CTA per SM
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(std::min<int64_t>(P.units, workers) * (pair ? 2 : 1)));
+  cfg.blockDim = dim3(OZ_THREADS);
+  cfg.dynamicSmemBytes = OZ_SMEM;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = pair ? 2 : 1;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
   const int pidx = prof_begin(s);
-  if (lv.cut) gemm_oz_kernel<true><<<grid, OZ_THREADS, OZ_SMEM, s>>>(ta, tb, P, exA, exB, ep, err);
-  else gemm_oz_kernel<false><<<grid, OZ_THREADS, OZ_SMEM, s>>>(ta, tb, P, exA, exB, ep, err);
+  if (lv.cut) FCC_CUDA(cudaLaunchKernelEx(&cfg, pair ? gemm_oz_kernel<true, true> : gemm_oz_kernel<true, false>, ta, tb, P, exA, exB, ep, err));
+  else FCC_CUDA(cudaLaunchKernelEx(&cfg, pair ? gemm_oz_kernel<false, true> : gemm_oz_kernel<false, false>, ta, tb, P, exA, exB, ep, err));
   FCC_CHECK_LAUNCH();
   if (P.njobs > 1) {
     const int64_t MN = ep.M * ep.N;

@@ -85,6 +85,22 @@ def test_sums_that_cancel(M, N, K, level):
     assert np.all(np.abs(out - ref) <= K * 2.0 ** -56 * scale + 2.0 ** -53 * np.abs(ref))
 
 
+# tiles of pairs of CTAs (even numbers of 128 rows, or eight and more), rows that
+# leave the second CTA of a pair empty, and long products turned over; integers,
+# so every digit and sum is exact
+@pytest.mark.parametrize("M,N,K", [(256, 130, 70), (257, 129, 70), (129, 40, 64), (1025, 17, 65), (1153, 300, 130),
+                                   (100, 1030, 2100), (300, 200, 2049), (90, 250, 4100)])
+@pytest.mark.parametrize("alpha,beta", [(1.0, 0.0), (-2.0, 1.0), (3.0, -0.5)])
+def test_pair_tiles(M, N, K, alpha, beta):
+    rng = np.random.default_rng(M + N + K)
+    A = rng.integers(-1000, 1000, (M, K)).astype(float)
+    B = rng.integers(-1000, 1000, (N, K)).astype(float)
+    C = 2.0 * rng.integers(-99, 99, (M, N)).astype(float)
+    rc, out = _run(TC, "mk,nk->mn", A, B, C, alpha, beta)
+    assert rc == 0
+    assert np.array_equal(out, alpha * (A @ B.T) + beta * C)
+
+
 def test_peaked_rows_against_a_metric():
     # rows with a few large entries against the inverse square root of a nearly
     # dependent metric: the largest entries of one side meet the smallest of the
