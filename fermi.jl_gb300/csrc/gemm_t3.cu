@@ -34,9 +34,9 @@ constexpr int T3_BK = 64;
 constexpr int T3_THREADS = 192;   // warp 0 TMA, warp 1 MMA, warps 2-5 epilogue
 template <int BN>
 struct T3Cfg {
-  static constexpr int STAGES = BN > 192 ? 4 : 5;
+  static constexpr int STAGES = BN > 192 ? 6 : 7;
   static constexpr int A_BYTES = T3_BM * T3_BK * 2;
-  static constexpr int B_BYTES = BN * T3_BK * 2;
+  static constexpr int B_BYTES = BN / 2 * T3_BK * 2;   // this CTA's half
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int SMEM = STAGES * STAGE_BYTES + 1024;
   static constexpr int TMEM_COLS = BN <= 32 ? 32 : BN <= 64 ? 64 : BN <= 128 ? 128 : 256;   // per accumulator (two)
@@ -70,8 +70,11 @@ __device__ __forceinline__ T3Tile t3_tile(int t, int tm, int tn, int nk) {
   return r;
 }
 
-// Persistent: each CTA walks tiles blockIdx.x, blockIdx.x + gridDim.x, ...;
-// the TMA thread streams the K segments of its tiles through a shared-memory
+// Persistent: each pair of CTAs (cta_group::2, a 256 x BN tile: 128 rows and
+// half of every B tile each) walks tiles b, b + pairs, ...; a step of 128 x 160 x
+// 64 in a single CTA moved 36 KB in and out of shared memory, 576 clk for 320 of
+// MMAs, in a pair 26 KB (the GEMMs of a (T) at (H2O)8: 160 ms, 148 in pairs).
+// The TMA thread streams the K segments of its tiles through a shared-memory
 // ring, the MMA thread alternates two TMEM accumulators, and the epilogue
 // warps store tile t while the MMAs of tile t+1 run.
 template <int BN>
@@ -100,64 +103,68 @@ __global__ void __launch_bounds__(T3_THREADS, 1) gemm_t3_kernel(const __grid_con
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&accf_bar[b]), 1);
-      mbar_init(smem_u32(&acce_bar[b]), 4);   // one arrival per epilogue warp
+      mbar_init(smem_u32(&acce_bar[b]), 8);   // one arrival per epilogue warp of the pair
     }
     mbar_init(smem_u32(&done_bar), 1);
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_holder)),
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_holder)),
                  "r"(2 * Cfg::TMEM_COLS)
                  : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  cluster_sync();     // both CTAs' barriers are there before either is signalled
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_holder;
+  const uint32_t rank = cluster_rank();
+  const int wid = blockIdx.x >> 1, nwork = gridDim.x >> 1;
 
   if (warp == 0) {
    if (elect_one()) {
     // ---------------- TMA producer over the tiles' K segments
     int it = 0;
     bool stop = false;
-    for (int t = blockIdx.x; t < ntiles && !stop; t += gridDim.x) {
+    for (int t = wid; t < ntiles && !stop; t += nwork) {
       const T3Tile tl = t3_tile(t, tm, tn, P.nk);
       const int kk = P.k0 + tl.kq;
-      const int64_t m0 = (int64_t)tl.mt * T3_BM;
+      const int64_t m0 = (int64_t)tl.mt * (2 * T3_BM) + rank * T3_BM;
       for (int s = 0; s < T3_NSEG && !stop; ++s) {
         const T3Seg sg = P.seg[tl.g][s];
         const int32_t arow = (int32_t)(t3_sel(sg.asel, P.i, P.j, kk) * v * v + m0);
-        const int32_t brow =
-            (int32_t)((t3_sel(sg.bsel1, P.i, P.j, kk) * o + t3_sel(sg.bsel2, P.i, P.j, kk)) * v + (int64_t)tl.nt * BN);
+        const int32_t brow = (int32_t)((t3_sel(sg.bsel1, P.i, P.j, kk) * o + t3_sel(sg.bsel2, P.i, P.j, kk)) * v +
+                                       (int64_t)tl.nt * BN + rank * (BN / 2));
         for (int kb = 0; kb < sg.nkb; ++kb, ++it) {
           const int st = it % Cfg::STAGES;
           const uint32_t ph = (it / Cfg::STAGES) & 1;
           if (!mbar_wait(smem_u32(&empty_bar[st]), ph ^ 1)) { atomicExch(&abort_flag, 1); stop = true; break; }
           if (*(volatile int*)&abort_flag) { stop = true; break; }
-          const uint32_t fb = smem_u32(&full_bar[st]);
-          mbar_expect_tx(fb, Cfg::STAGE_BYTES);
-          tma_load_2d(smem_u32(sA + st * Cfg::A_BYTES), &P.maps[sg.amap], kb * T3_BK, arow, fb);
-          tma_load_2d(smem_u32(sB + st * Cfg::B_BYTES), &P.maps[sg.bmap], kb * T3_BK, brow, fb);
+          const uint32_t fb = smem_u32(&full_bar[st]), f0 = cluster_addr(fb, 0);
+          // both CTAs' loads count on the first one's barrier
+          if (rank == 0) mbar_expect_tx(fb, 2 * Cfg::STAGE_BYTES);
+          tma_load_2d_pair(smem_u32(sA + st * Cfg::A_BYTES), &P.maps[sg.amap], kb * T3_BK, arow, f0);
+          tma_load_2d_pair(smem_u32(sB + st * Cfg::B_BYTES), &P.maps[sg.bmap], kb * T3_BK, brow, f0);
         }
       }
     }
-    if (stop) {
-      // wait (bounded) for loads still in flight before shared memory is released
+    if (stop && rank == 0) {
+      // wait (bounded) for both CTAs' loads still in flight before shared memory is released
       for (int q = max(0, it - Cfg::STAGES); q < it; ++q)
         (void)mbar_wait(smem_u32(&full_bar[q % Cfg::STAGES]), (q / Cfg::STAGES) & 1);
     }
    }
   } else if (warp == 1) {
-   if (elect_one()) {
-    // ---------------- MMA issuer
-    constexpr uint32_t idesc = idesc_bf16(T3_BM, BN);
+   if (rank == 0 && elect_one()) {
+    // ---------------- MMA issuer, for both CTAs
+    constexpr uint32_t idesc = idesc_bf16(2 * T3_BM, BN);
     const uint64_t ad0 = sw128_desc(smem_u32(sA)), bd0 = sw128_desc(smem_u32(sB));
     uint32_t st = 0, ph = 0, peek = 0;
     int lt = 0;
     bool ok = true;
-    for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x, ++lt) {
+    for (int t = wid; t < ntiles && ok; t += nwork, ++lt) {
       const int g = t3_tile(t, tm, tn, P.nk).g;
       int total = 0;
       for (int s = 0; s < T3_NSEG; ++s) total += P.seg[g][s].nkb;
@@ -174,20 +181,20 @@ __global__ void __launch_bounds__(T3_THREADS, 1) gemm_t3_kernel(const __grid_con
         const uint64_t bd = bd0 + (uint64_t)(st * (Cfg::B_BYTES >> 4));
         uint32_t st2 = st + 1, ph2 = ph;
         if (st2 == Cfg::STAGES) { st2 = 0; ph2 ^= 1; }
-        mma_bf16(dcol, ad, bd, idesc, x > 0 ? 1u : 0u);
+        mma_bf16_pair(dcol, ad, bd, idesc, x > 0 ? 1u : 0u);
         peek = mbar_test(smem_u32(&full_bar[st2]), ph2);
-        mma_bf16(dcol, ad + 2, bd + 2, idesc, 1u);
-        mma_bf16(dcol, ad + 4, bd + 4, idesc, 1u);
-        mma_bf16(dcol, ad + 6, bd + 6, idesc, 1u);
-        tc_commit(smem_u32(&empty_bar[st]));
+        mma_bf16_pair(dcol, ad + 2, bd + 2, idesc, 1u);
+        mma_bf16_pair(dcol, ad + 4, bd + 4, idesc, 1u);
+        mma_bf16_pair(dcol, ad + 6, bd + 6, idesc, 1u);
+        tc_commit_pair(smem_u32(&empty_bar[st]));
         st = st2;
         ph = ph2;
       }
       if (!ok) break;
-      tc_commit(smem_u32(&accf_bar[b]));
+      tc_commit_pair(smem_u32(&accf_bar[b]));
     }
     // TMEM is freed only after every issued MMA has completed (also on an abort)
-    tc_commit(smem_u32(&done_bar));
+    tc_commit_pair(smem_u32(&done_bar));
     if (!mbar_wait(smem_u32(&done_bar), 0)) atomicExch(&abort_flag, 1);
    }
   } else if (warp >= 2) {
@@ -195,19 +202,19 @@ __global__ void __launch_bounds__(T3_THREADS, 1) gemm_t3_kernel(const __grid_con
     // in whole 32-byte sectors straight from the registers.  (Transposed through
     // shared memory for 128-byte rows, an element took about eight instructions
     // of the warp instead of one and a half, and the shared memory shared with
-    // the MMAs: 167 ms of a (T) at (H2O)8 where this takes 160, 29 and 24 ms at
+    // the MMAs: 167 ms of a (T) at (H2O)8 where this took 160, 29 and 24 ms at
     // (H2O)6 with odd sizes.)
     const int q = warp & 3;
     const int64_t v2 = v * v;
     int lt = 0;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++lt) {
+    for (int t = wid; t < ntiles; t += nwork, ++lt) {
       const T3Tile tl = t3_tile(t, tm, tn, P.nk);
       const int b = lt & 1;
       bool ok = mbar_wait(smem_u32(&accf_bar[b]), (lt >> 1) & 1);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok || __any_sync(0xffffffffu, *(volatile int*)&abort_flag != 0)) { atomicExch(&abort_flag, 1); break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int64_t m0 = (int64_t)tl.mt * T3_BM;
+      const int64_t m0 = (int64_t)tl.mt * (2 * T3_BM) + rank * T3_BM;
       const int64_t nbk = t3_nb(v);
       float* out = P.G + ((int64_t)tl.g * P.nk + tl.kq) * t3_slab(v);
       const int64_t nb0 = (int64_t)tl.nt * BN;
@@ -237,14 +244,15 @@ __global__ void __launch_bounds__(T3_THREADS, 1) gemm_t3_kernel(const __grid_con
       // the accumulator is free for the tile after next
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&acce_bar[b]));
+      if (lane == 0) mbar_arrive_cluster(cluster_addr(smem_u32(&acce_bar[b]), 0));
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  cluster_sync();     // neither CTA goes while the other may still signal it or read its tiles
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * Cfg::TMEM_COLS)
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * Cfg::TMEM_COLS)
                  : "memory");
   }
   if (threadIdx.x == 0 && abort_flag) atomicExch(P.err, 1);
@@ -257,12 +265,22 @@ void launch_t3(const T3Params& P, cudaStream_t s) {
   std::call_once(once, []() {
     cudaFuncSetAttribute(gemm_t3_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
   });
-  const int64_t tm = ((int64_t)P.v * P.v + T3_BM - 1) / T3_BM;
+  const int64_t tm = ((int64_t)P.v * P.v + 2 * T3_BM - 1) / (2 * T3_BM);
   const int64_t tn = (P.v + BN - 1) / BN;
   const int64_t ntiles = tm * tn * 3 * P.nk;
   if (ntiles > (int64_t)1 << 30) fail(FCC_ERR_BAD_ARG, "too many (T) tiles in one launch");
-  const unsigned grid = (unsigned)std::min<int64_t>(ntiles, 152);
-  gemm_t3_kernel<BN><<<grid, T3_THREADS, Cfg::SMEM, s>>>(P, (int)tm, (int)tn, (int)ntiles);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(2 * std::min<int64_t>(ntiles, 76)));   // a CTA per SM, in pairs
+  cfg.blockDim = dim3(T3_THREADS);
+  cfg.dynamicSmemBytes = Cfg::SMEM;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 2;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  FCC_CUDA(cudaLaunchKernelEx(&cfg, gemm_t3_kernel<BN>, P, (int)tm, (int)tn, (int)ntiles));
   FCC_CHECK_LAUNCH();
 }
 
