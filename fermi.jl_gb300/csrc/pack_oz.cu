@@ -6,14 +6,17 @@
 //
 // HBM bound: 8 bytes read and 2 S written per element.  The row exponent is
 // needed before the first digit, so where a row's share fits, one kernel reads
-// it once into registers (k the faster source index, up to 4096 columns) or
-// shared memory (row index faster, up to 176 columns), reduces the exponent
-// and cuts from there; longer rows take an exponent pass of their own.
+// it once into registers or shared memory (k the faster source index, up to 4096
+// and 14080 columns) or into the shared memory of a block or cluster (row index
+// faster, up to 176 and 1536 columns), reduces the exponent and cuts from there;
+// longer rows, and few long ones, take an exponent pass of their own.
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <mutex>
 
 #include "fcc_tc.cuh"
+#include "fcc_tcgen05.cuh"
 
 namespace fcc {
 
@@ -265,6 +268,133 @@ __global__ void __launch_bounds__(256) oz_pack_tiles_fused_kernel(const double* 
   }
 }
 
+// The same for K up to 8 x TILE_KW: a cluster of up to eight blocks shares 32
+// rows, each with its range of columns, and exchanges the maxima through
+// distributed shared memory, so the source is read once and by one launch
+// instead of a memset, an exponent pass and the cut.  With the rows through
+// shared memory below: packs of a mixed solve at (H2O)8 99 -> 92 ms, of an exact
+// step at (H2O)6 odd 2.08 -> 1.89.
+constexpr int TILE_KW = 192;
+template <int S, int BITS>
+__global__ void __launch_bounds__(256) oz_pack_tiles_cluster_kernel(const double* __restrict__ src, PackSpec ps,
+                                                                    int64_t Kpad, int guard, int* __restrict__ ex,
+                                                                    __nv_bfloat16* __restrict__ dst, int nc, int kw) {
+  extern __shared__ double ftile[];   // [kw][33]
+  __shared__ int64_t coff[TILE_KW];
+  __shared__ int red[8][32];
+  __shared__ int own[32], tot[32];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int kp = threadIdx.x & 15, rw = threadIdx.x >> 4;   // write phase: k pair, row
+  const int rank = (int)tc5::cluster_rank();
+  const int64_t ntr = (ps.R + 31) / 32;
+  const int ka = rank * kw, K = (int)min((int64_t)kw, ps.K - ka);   // columns here (<= 0: padding only)
+  const int kend = (int)min((int64_t)kw, Kpad - ka);
+  for (int k = threadIdx.x; k < K; k += 256) coff[k] = pack_col_off(ps, ka + k);
+  __syncthreads();
+  for (int64_t tb = blockIdx.x / nc; tb < ntr; tb += gridDim.x / nc) {
+    const int64_t r0 = tb * 32;
+    const bool rok = r0 + tx < ps.R;
+    const int64_t ro = rok ? pack_row_off(ps, r0 + tx) : 0;
+    int m = 0;
+#pragma unroll 8
+    for (int kk = ty; kk < K; kk += 8) {
+      const double x = rok ? src[ro + coff[kk]] : 0.0;
+      m = max(m, biased_exp(x));
+      ftile[kk * 33 + tx] = x;
+    }
+    red[ty][tx] = m;
+    __syncthreads();
+    if (ty == 0) {
+#pragma unroll
+      for (int j = 1; j < 8; ++j) m = max(m, red[j][tx]);
+      own[tx] = m;
+    }
+    tc5::cluster_sync();
+    if (ty == 0) {
+      const uint32_t at = tc5::smem_u32(&own[tx]);
+      int part[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        part[q] = 0;
+        if (q < nc)
+          asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(part[q]) : "r"(tc5::cluster_addr(at, q)) : "memory");
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q) m = max(m, part[q]);
+      tot[tx] = m;
+      if (rok && rank == 0) ex[r0 + tx] = m;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int rr = rw + 16 * j;
+      const int64_t r = r0 + rr;
+      if (r >= ps.R) continue;
+      const int e = oz_row_exp(tot[rr]) + guard;
+      for (int k = 2 * kp; k < kend; k += 32) {
+        uint32_t da[S], db[S];
+        oz_digits<S, BITS>(k < K ? ftile[k * 33 + rr] : 0.0, e, da);
+        oz_digits<S, BITS>(k + 1 < K ? ftile[(k + 1) * 33 + rr] : 0.0, e, db);
+        uint32_t* d = reinterpret_cast<uint32_t*>(dst + r * (S * Kpad) + ka + k);
+#pragma unroll
+        for (int s = 0; s < S; ++s) d[(s * Kpad) >> 1] = oz_pair(da[s], db[s]);
+      }
+    }
+    tc5::cluster_sync();   // the tile and the maxima are consumed
+  }
+}
+
+// Rows too long for registers, through shared memory: a block of 512 threads per
+// row, two to an SM up to ROW_KMAX columns.
+constexpr int ROW_KMAX = 14080;     // 110 KB
+template <int S, int BITS>
+__global__ void __launch_bounds__(512) oz_pack_rows_smem_kernel(const double* __restrict__ src, PackSpec ps,
+                                                                int64_t Kpad, int guard, int* __restrict__ ex,
+                                                                __nv_bfloat16* __restrict__ dst) {
+  extern __shared__ double ftile[];   // [Kpad]
+  __shared__ int red[16];
+  const int ng = (int)(Kpad >> 2), t = threadIdx.x;
+  const bool k1 = pack_k_single(ps);
+  for (int64_t r = blockIdx.x; r < ps.R; r += gridDim.x) {
+    const int64_t ro = pack_row_off(ps, r);
+    int m = 0;
+    for (int g0 = t; g0 < ng; g0 += 512 * 3) {
+      double xv[3][4];
+#pragma unroll
+      for (int u = 0; u < 3; ++u) {
+        const int64_t k0 = (int64_t)(g0 + 512 * u) << 2;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) xv[u][q] = 0.0;
+        if (k0 < ps.K) pack_load4(src, ps, k1, ro, k0, (int)min((int64_t)4, ps.K - k0), xv[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < 3; ++u) {
+        const int g = g0 + 512 * u;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) m = max(m, biased_exp(xv[u][q]));
+        if (g < ng) {
+          *reinterpret_cast<double2*>(ftile + 4 * g) = make_double2(xv[u][0], xv[u][1]);
+          *reinterpret_cast<double2*>(ftile + 4 * g + 2) = make_double2(xv[u][2], xv[u][3]);
+        }
+      }
+    }
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((t & 31) == 0) red[t >> 5] = m;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 16; ++w) m = max(m, red[w]);
+    if (t == 0) ex[r] = m;
+    const int e = oz_row_exp(m) + guard;
+    __nv_bfloat16* drow = dst + r * (S * Kpad);
+    for (int g = t; g < ng; g += 512) {
+      const double2 a = *reinterpret_cast<const double2*>(ftile + 4 * g), b = *reinterpret_cast<const double2*>(ftile + 4 * g + 2);
+      const double xv[4] = {a.x, a.y, b.x, b.y};
+      oz_store4<S, BITS>(xv, e, drow + 4 * g, Kpad);
+    }
+    __syncthreads();   // the row and the maxima are consumed
+  }
+}
+
 // dst[r][s*Kpad + k]: row walk (k the faster source index), 2^lg threads per
 // row, each cutting 4 consecutive k and writing one 8-byte word per slice
 // (zeros over the padding [K, Kpad))
@@ -383,6 +513,39 @@ void pack(const double* src, const PackSpec& ps, int guard, __nv_bfloat16* dst, 
     const int64_t rpb = 256 >> lg;
     oz_pack_rows_fused_kernel<S, BITS><<<(unsigned)std::min<int64_t>((ps.R + rpb - 1) / rpb, 152 * 16), 256, 0, s>>>(
         src, ps, Kpad, guard, ex, dst, lg);
+    FCC_CHECK_LAUNCH();
+    return;
+  }
+  if (tiles && Kpad <= 8 * TILE_KW) {
+    const int nc = (int)((Kpad + TILE_KW - 1) / TILE_KW);
+    const int kw = (int)((Kpad / 64 + nc - 1) / nc * 64);
+    static std::once_flag once;
+    std::call_once(once, []() {
+      cudaFuncSetAttribute(oz_pack_tiles_cluster_kernel<S, BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           TILE_KW * 33 * 8);
+    });
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(std::min<int64_t>(ntr, 152 * 4) * nc));
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = (size_t)kw * 33 * 8;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)nc;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    FCC_CUDA(cudaLaunchKernelEx(&cfg, oz_pack_tiles_cluster_kernel<S, BITS>, src, ps, Kpad, guard, ex, dst, nc, kw));
+    FCC_CHECK_LAUNCH();
+    return;
+  }
+  if (!tiles && Kpad > 4096 && Kpad <= ROW_KMAX && ps.R >= 304) {
+    static std::once_flag once;
+    std::call_once(once, []() {
+      cudaFuncSetAttribute(oz_pack_rows_smem_kernel<S, BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROW_KMAX * 8);
+    });
+    oz_pack_rows_smem_kernel<S, BITS><<<(unsigned)std::min<int64_t>(ps.R, 152 * 8), 512, (size_t)Kpad * 8, s>>>(
+        src, ps, Kpad, guard, ex, dst);
     FCC_CHECK_LAUNCH();
     return;
   }

@@ -36,13 +36,14 @@ def _digits(x, e, S):
 
 # K = 100 and 700: the one-pass row walk with one and several warps a row, the
 # fused and the two-pass transposing walk; 4500: the two-pass row walk
-@pytest.mark.parametrize("row_fastest,K", [(0, 100), (0, 700), (0, 4500), (1, 100), (1, 700)])
+@pytest.mark.parametrize("row_fastest,K", [(0, 100), (0, 700), (0, 4500), (0, 5000), (0, 14080), (1, 100), (1, 177),
+                                           (1, 700), (1, 1530), (1, 1600)])
 @pytest.mark.parametrize("S", [1, 4, 6, 7, 8])
 def test_device_wide_digits_are_the_integer_model(row_fastest, K, S):
     from fermicc import _lib
     lib = _lib.load()
     rng = np.random.default_rng(5 + S + 10 * row_fastest + K)
-    R = 70
+    R = 310 if K >= 5000 else 70      # long rows go through shared memory from 304 rows on
     x = rng.standard_normal((R, K)) * 10.0 ** rng.uniform(-3, 3, (R, 1))
     x[2, :] *= 10.0 ** rng.uniform(-12, 0, K)
     x[3, :] = 0.0
