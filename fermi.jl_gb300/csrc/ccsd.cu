@@ -27,9 +27,9 @@ namespace {
 constexpr int RED_BLOCKS = 608;  // 152 SMs x 4: fixed, so reductions are deterministic
 constexpr int RED_THREADS = 256;
 constexpr int MAX_DIIS = 8;
-// partial-sum layout per block: [0] sum dT^2, [1] energy, [2] dot of the stored
-// error with itself, [3..3+MAX_DIIS) with the others
-constexpr int NPART = 3 + MAX_DIIS;
+// partial-sum layout per block: [0] sum dT^2, [1] energy, [2..2+MAX_DIIS) dots of
+// the stored error with the others
+constexpr int NPART = 2 + MAX_DIIS;
 
 __device__ __forceinline__ double warp_sum(double x) {
   for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
@@ -50,10 +50,10 @@ int red_blocks(int rank, int64_t o, int64_t v) {
 // Sum nvals values held per thread over the grid into out.  Each warp halves the
 // set of values as it halves the distance between lanes: 16 FP64 additions per
 // lane instead of five for each value (the FP64 pipe takes 16 clk per warp
-// instruction: the 11 values of an update took 14 us of a launch over 608
+// instruction: the values of an update took 14 us of a launch over 608
 // blocks at (H2O)1, 3 us with this and the blocks that have elements).  The last
-// block to arrive adds the blocks' partial sums, in block order by lanes, so the
-// result does not depend on which it is and needs no second launch.
+// block to arrive adds the blocks' partial sums in block order, a lane per value,
+// so the result does not depend on which it is and needs no second launch.
 __device__ void grid_reduce(double (&vals)[NPART], int nvals, double* part, double* out, unsigned* counter) {
   __shared__ double sm[RED_THREADS / 32][NRED];
   __shared__ bool last;
@@ -95,12 +95,20 @@ __device__ void grid_reduce(double (&vals)[NPART], int nvals, double* part, doub
   __syncthreads();
   if (!last) return;
   __threadfence();
-  for (int k = w; k < nvals; k += RED_THREADS / 32) {
+  // a lane per value, the blocks in order
+  if (threadIdx.x < nvals) {
     double s = 0.0;
-#pragma unroll 4
-    for (int b = lane; b < (int)gridDim.x; b += 32) s += __ldcg(part + b * NPART + k);
-    s = warp_sum(s);
-    if (lane == 0) out[k] = s;
+    const double* p = part + threadIdx.x;
+    int b = 0;
+    for (; b + 16 <= (int)gridDim.x; b += 16) {
+      double x[16];
+#pragma unroll
+      for (int q = 0; q < 16; ++q) x[q] = __ldcg(p + (b + q) * NPART);
+#pragma unroll
+      for (int q = 0; q < 16; ++q) s += x[q];
+    }
+    for (; b < (int)gridDim.x; ++b) s += __ldcg(p + b * NPART);
+    out[threadIdx.x] = s;
   }
 }
 
@@ -121,8 +129,8 @@ struct ErrSlots {
 //
 // The FP64 pipe (two lanes per clk and SM) bounds this pass, not HBM, so it is
 // kept short: the quotient by D takes a reciprocal seed in single precision and
-// two Newton steps (Markstein, IBM J. Res. Dev. 34, 111 (1990): the remainder
-// r - q D by one fma, within the last place) instead of the compiler's division, the stored errors are widened by integer arithmetic, and the dot of
+// three Newton steps (Markstein, IBM J. Res. Dev. 34, 111 (1990): the remainder
+// r - q D by one fma, rounded as a division is) instead of the compiler's division, the stored errors are widened by integer arithmetic, and the dot of
 // the error with itself comes from this pass.  (H2O)8: 0.90 + 0.19 ms with a
 // division and a second pass over the errors, see the launch list.
 // a float as a double, exactly, without the FP64 pipe (subnormals become 0)
@@ -137,6 +145,7 @@ __device__ __forceinline__ double quotient(double r, double D) {
   // |D| is an orbital-energy difference: far inside the single-precision range
   double y = widen(__frcp_rn((float)D));
   y = fma(y, fma(-D, y, 1.0), y);        // 2^-24 -> 2^-47
+  y = fma(y, fma(-D, y, 1.0), y);        // the reciprocal, rounded
   const double q = r * y;
   return fma(y, fma(-D, q, r), q);       // remainder in full precision
 }
@@ -157,11 +166,10 @@ __device__ __forceinline__ void update_one(int64_t e, double t, double r, double
   } else {
     return;
   }
-  vals[2] = fma(ev, ev, vals[2]);
 #pragma unroll
   for (int k = 0; k < MAX_DIIS; ++k) {
     if (k >= others.n) break;
-    vals[3 + k] = fma(ev, others.s[k] ? widen(others.s[k][e]) : others.d[k][e], vals[3 + k]);
+    vals[2 + k] = fma(ev, others.s[k] ? widen(others.s[k][e]) : others.d[k][e], vals[2 + k]);
   }
 }
 
@@ -194,17 +202,45 @@ __global__ void __launch_bounds__(RED_THREADS) update_kernel(
       const double* t1j = t1new + (int64_t)j * v;
       const double* ev = eps + o;
       const int64_t base = (int64_t)row * v;
-#pragma unroll 2
-      for (int b = lane; b < v; b += 32) {
-        const int64_t e = base + b;
-        double tn;
-        update_one(e, T[e], R[e], Drow - ev[b], Lt ? t1ia * t1j[b] : 0.0, Lt != nullptr, Lt ? Lt[e] : 0.0, err_s, err_d,
-                   others, tn, vals);
-        Tnew[e] = tn;
+      const bool energy = Lt != nullptr;
+      if ((v & 1) == 0) {   // two neighbouring elements a lane
+        for (int b = 2 * lane; b < v; b += 64) {
+          const int64_t e = base + b;
+          const double2 tv = *reinterpret_cast<const double2*>(T + e);
+          const double2 rv = *reinterpret_cast<const double2*>(R + e);
+          double2 tn;
+          update_one(e, tv.x, rv.x, Drow - ev[b], energy ? t1ia * t1j[b] : 0.0, energy, energy ? Lt[e] : 0.0, err_s, err_d,
+                     others, tn.x, vals);
+          update_one(e + 1, tv.y, rv.y, Drow - ev[b + 1], energy ? t1ia * t1j[b + 1] : 0.0, energy, energy ? Lt[e + 1] : 0.0,
+                     err_s, err_d, others, tn.y, vals);
+          *reinterpret_cast<double2*>(Tnew + e) = tn;
+        }
+      } else {
+        for (int b = lane; b < v; b += 32) {
+          const int64_t e = base + b;
+          double tn;
+          update_one(e, T[e], R[e], Drow - ev[b], energy ? t1ia * t1j[b] : 0.0, energy, energy ? Lt[e] : 0.0, err_s, err_d,
+                     others, tn, vals);
+          Tnew[e] = tn;
+        }
       }
     }
   }
-  grid_reduce(vals, 3 + others.n, part, out, counter);
+  grid_reduce(vals, 2 + others.n, part, out, counter);
+}
+
+// The dot of the stored error with itself.
+__global__ void __launch_bounds__(RED_THREADS) selfdot_kernel(int64_t total, const float* es, const double* ed, double* part,
+                                                              double* out, unsigned* counter) {
+  double vals[NPART];
+#pragma unroll
+  for (int k = 0; k < NPART; ++k) vals[k] = 0.0;
+#pragma unroll 4
+  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
+    const double x = es ? widen(es[e]) : ed[e];
+    vals[0] = fma(x, x, vals[0]);
+  }
+  grid_reduce(vals, 1, part, out, counter);
 }
 
 // DIIS extrapolation: out = sum_k c_k (vec_k + add_res * err_k); for T2 also
@@ -231,7 +267,7 @@ __global__ void __launch_bounds__(RED_THREADS) extrapolate_kernel(int rank, int 
     double s = 0.0;
     for (int k = 0; k < sl.n; ++k) {
       const double ev = sl.es[k] ? widen(sl.es[k][e]) : sl.ed[k][e];
-      s = fma(c[k], ev, fma(c[k], sl.vec[k][e], s));
+      s += c[k] * sl.vec[k][e] + c[k] * ev;
     }
     out[e] = s;
     return s;
@@ -571,7 +607,19 @@ void setup_integrals(fcc_ctx* c) {
   c->Lldkc.alloc(o * v * o * v);
   c->Lt.alloc(o * o * v * v);
   TView ovov = rm(c->ovov.p, {o, v, o, v});
+  // The integrals that every form starts from stay on the FP64 pipe in one fixed
+  // order: the mixed form cuts its digits from them, and a change in their last
+  // place moves its converged amplitudes by 3e-9.  (ia|jb) is symmetric: half its
+  // tiles, the rest copied.
+  struct Wide {
+    TcEngine* e;
+    explicit Wide(TcEngine* x) : e(x) { if (e) e->f64_wide = true; }
+    void sym(bool on) { if (e) e->f64_sym = on; }
+    ~Wide() { if (e) e->f64_wide = e->f64_sym = false; }
+  } wide(tc_engine());
+  wide.sym(true);
   einsum(1.0, "Qkc,Qld->kcld", Bov, Bov, 0.0, ovov, s);
+  wide.sym(false);
   TView L = rm(c->Lldkc.p, {o, v, o, v});
   einsum1(2.0, "ldkc->ldkc", ovov, 0.0, L, s);
   einsum1(-1.0, "lckd->ldkc", ovov, 1.0, L, s);
@@ -996,18 +1044,23 @@ int ccsd_run(fcc_ctx* c, const fcc_opts* opt, fcc_iter_stats* log, int32_t log_c
                                                                  others, rank == 4 ? c->Lt.p : nullptr, t1new, c->red.p,
                                                                  red_out(c, rank / 2 - 1), red_counter(c));
     FCC_CHECK_LAUNCH();
+    if (diis) {
+      selfdot_kernel<<<(unsigned)std::min<int64_t>(RED_BLOCKS, (len + RED_THREADS - 1) / RED_THREADS), RED_THREADS, 0, s>>>(
+          len, errs, errd, c->red.p, red_out(c, 2 + rank / 2), red_counter(c));
+      FCC_CHECK_LAUNCH();
+    }
     *cur = dst;
     return pd;
   };
-  auto note_update = [&](DiisState& ds, const Pending& pd, const double* h) {
+  auto note_update = [&](DiisState& ds, const Pending& pd, const double* h, double self) {
     if (!diis) return;
     ds.valid[pd.target] = 1;
     ds.age[pd.target] = ++ds.counter;
-    ds.norm2[pd.target] = h[2];
-    ds.dot[pd.target][pd.target] = h[2];
+    ds.norm2[pd.target] = self;
+    ds.dot[pd.target][pd.target] = self;
     for (size_t q = 0; q < pd.others.size(); ++q) {
-      ds.dot[pd.target][pd.others[q]] = h[3 + q];
-      ds.dot[pd.others[q]][pd.target] = h[3 + q];
+      ds.dot[pd.target][pd.others[q]] = h[2 + q];
+      ds.dot[pd.others[q]][pd.target] = h[2 + q];
     }
   };
 
@@ -1040,7 +1093,7 @@ int ccsd_run(fcc_ctx* c, const fcc_opts* opt, fcc_iter_stats* log, int32_t log_c
 
   int status = FCC_OK;
   bool conv_final = false;
-  // Iteration kinds: FP64 residual (DMMA); split-BF16 residual with three
+  // Iteration kinds: FP64 residual; split-BF16 residual with three
   // products (mixed form, first phase); exact-slice BF16 residual at 6-8
   // weight groups (mixed form, second phase: Ozaki-scheme products whose
   // error, ~1e-11 absolute in the residual, is far below the convergence
@@ -1098,10 +1151,10 @@ int ccsd_run(fcc_ctx* c, const fcc_opts* opt, fcc_iter_stats* log, int32_t log_c
     }
     const Pending p1 = run_update(2, D1s, c->dvec1, c->derr1s, c->derr1d, c->t1.p, c->r1.p, tn1, &cur1, nullptr);
     const Pending p2 = run_update(4, D2s, c->dvec2, c->derr2s, c->derr2d, c->t2.p, c->r2.p, tn2, &cur2, cur1);
-    FCC_CUDA(cudaMemcpyAsync(hred, red_out(c, 0), sizeof(double) * 2 * RED_OUT, cudaMemcpyDeviceToHost, s));
+    FCC_CUDA(cudaMemcpyAsync(hred, red_out(c, 0), sizeof(double) * 5 * RED_OUT, cudaMemcpyDeviceToHost, s));
     FCC_CUDA(cudaStreamSynchronize(s));
-    note_update(D1s, p1, hred);
-    note_update(D2s, p2, hred + RED_OUT);
+    note_update(D1s, p1, hred, hred[3 * RED_OUT]);
+    note_update(D2s, p2, hred + RED_OUT, hred[4 * RED_OUT]);
     double e_new = hred[RED_OUT + 1];
     double r1 = std::sqrt(hred[0] / (double)len1), r2 = std::sqrt(hred[RED_OUT] / (double)len2);   // :193-194
     bool did = false;
@@ -1150,7 +1203,7 @@ int ccsd_run(fcc_ctx* c, const fcc_opts* opt, fcc_iter_stats* log, int32_t log_c
         best_rms = 1e300;
         stalled = 0;
       } else if (iter_kind == K_EXACT) {
-        // FP64 finish (one DMMA residual costs ~25 exact-slice ones): switch
+        // FP64 finish (one FP64 residual costs about two exact-slice ones): switch
         // when the criteria hold ten times over on this iteration and hold on
         // the previous one, so that the FP64 step that follows (whose energy
         // change is the next step of the same convergence) meets them at

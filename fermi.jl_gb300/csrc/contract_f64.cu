@@ -159,6 +159,7 @@ __global__ void __launch_bounds__(NT, 5) contract_f64_kernel(const double* __res
   __shared__ int64_t rowA[BM], colB[BN], rowC[BM], colC[BN];
   __shared__ int8_t rowOK[BM], colOK[BN];
 
+  if (d.sym && blockIdx.y < blockIdx.x) return;   // copied by mirror_kernel
   const int tid = threadIdx.x;
   const int64_t m0 = (int64_t)blockIdx.x * BM;
   const int64_t n0 = (int64_t)blockIdx.y * BN;
@@ -220,6 +221,28 @@ __global__ void __launch_bounds__(NT, 5) contract_f64_kernel(const double* __res
         f64_store(C + crow + colC[nl], acc[i][j][h], d.alpha, d.beta);
       }
     }
+  }
+}
+
+// C(m, n) = C(n, m) for the 64 x 64 tiles below the diagonal, 32 x 32 elements a block.
+__global__ void __launch_bounds__(256) mirror_kernel(double* __restrict__ C, CtrDesc d) {
+  if (blockIdx.x / 2 <= blockIdx.y / 2) return;
+  __shared__ double tile[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int64_t m0 = (int64_t)blockIdx.x * 32, n0 = (int64_t)blockIdx.y * 32;
+  auto at = [&](int64_t m, int64_t n) {
+    return off3(m, d.M2, d.M3, d.c_m1, d.c_m2, d.c_m3) + off3(n, d.N2, d.N3, d.c_n1, d.c_n2, d.c_n3);
+  };
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int64_t r = n0 + ty + 8 * q, c = m0 + tx;
+    if (r < d.M && c < d.N) tile[ty + 8 * q][tx] = C[at(r, c)];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int64_t m = m0 + ty + 8 * q, n = n0 + tx;
+    if (m < d.M && n < d.N) C[at(m, n)] = tile[tx][ty + 8 * q];
   }
 }
 
@@ -384,13 +407,15 @@ __global__ void gemv_f64_kernel(const double* __restrict__ A, const double* __re
 }
 
 // N == 1 with the rows adjacent in memory (unit stride along m): 32 rows per
-// block, lanes along the rows so that reads coalesce, eight warps over
-// interleaved k, summed in a fixed order.
-__global__ void __launch_bounds__(256) gemv_cols_f64_kernel(const double* __restrict__ A, const double* __restrict__ B,
-                                                            double* __restrict__ C, CtrDesc d) {
-  __shared__ double part[8][32];
+// block, lanes along the rows so that reads coalesce, a warp for each residue of
+// k modulo 32.  The sums are those of gemv_f64_kernel bit for bit (lane k mod 32,
+// then halves): the mixed form's digits are cut from what follows from them, and
+// its iterates should not depend on the memory layout of an operand.
+__global__ void __launch_bounds__(1024) gemv_cols_f64_kernel(const double* __restrict__ A, const double* __restrict__ B,
+                                                             double* __restrict__ C, CtrDesc d) {
+  __shared__ double part[32][33];
   const int x = threadIdx.x & 31, g = threadIdx.x >> 5;
-  const int64_t m = (int64_t)blockIdx.x * 32 + x;
+  const int64_t m0 = (int64_t)blockIdx.x * 32, m = m0 + x;
   const int64_t bz = blockIdx.y;
   A += bz * d.a_b;
   B += bz * d.b_b;
@@ -400,19 +425,18 @@ __global__ void __launch_bounds__(256) gemv_cols_f64_kernel(const double* __rest
     const double* a = A + off3(m, d.M2, d.M3, d.a_m1, d.a_m2, d.a_m3);
     if (d.K2 >= d.K) {
 #pragma unroll 8
-      for (int64_t k = g; k < d.K; k += 8) s = fma(a[k * d.a_k2], B[k * d.b_k2], s);
+      for (int64_t k = g; k < d.K; k += 32) s = fma(a[k * d.a_k2], B[k * d.b_k2], s);
     } else {
 #pragma unroll 4
-      for (int64_t k = g; k < d.K; k += 8)
+      for (int64_t k = g; k < d.K; k += 32)
         s = fma(a[off2(k, d.K2, d.a_k1, d.a_k2)], B[off2(k, d.K2, d.b_k1, d.b_k2)], s);
     }
   }
   part[g][x] = s;
   __syncthreads();
-  if (g != 0 || m >= d.M) return;
-#pragma unroll
-  for (int q = 1; q < 8; ++q) s += part[q][x];
-  f64_store(C + off3(m, d.M2, d.M3, d.c_m1, d.c_m2, d.c_m3), s, d.alpha, d.beta);
+  s = part[x][g];   // row m0 + g
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if (x == 0 && m0 + g < d.M) f64_store(C + off3(m0 + g, d.M2, d.M3, d.c_m1, d.c_m2, d.c_m3), s, d.alpha, d.beta);
 }
 
 // out[i0 i1 i2 i3] = alpha in + beta out: a warp per run of up to 128 elements
@@ -512,7 +536,7 @@ void contract_f64_launch(const double* A, const double* B, double* C, const CtrD
   const int b_fast = (d.N3 > 1 ? d.b_n3 : d.b_n2) == 1 ? 1 : 0;
   if (d.N == 1) {
     if (a_fast && d.M >= 32) {
-      gemv_cols_f64_kernel<<<dim3((unsigned)((d.M + 31) / 32), (unsigned)d.batch), 256, 0, s>>>(A, B, C, d);
+      gemv_cols_f64_kernel<<<dim3((unsigned)((d.M + 31) / 32), (unsigned)d.batch), 1024, 0, s>>>(A, B, C, d);
     } else {
       const int64_t blocks = std::min<int64_t>((d.M + 7) / 8, 152 * 16);
       gemv_f64_kernel<<<dim3((unsigned)blocks, (unsigned)d.batch), 256, 0, s>>>(A, B, C, d);
@@ -535,7 +559,7 @@ void contract_f64_launch(const double* A, const double* B, double* C, const CtrD
   // each has 16 values of k; a longer K over few tiles (over 512 a block) is cut
   // into partial sums for all SMs, reduced in a fixed order by a second launch.
   const int64_t sm = (d.M + SM_T - 1) / SM_T, sn = (d.N + SM_T - 1) / SM_T;
-  if (gm * gn * d.batch < 3 * 152 && sn <= 65535) {
+  if (!d.wide && gm * gn * d.batch < 3 * 152 && sn <= 65535) {
     int64_t cl = 1;
     while (cl < 8 && sm * sn * d.batch * cl < 152 && d.K >= 32 * cl && d.batch * cl * 2 <= 65535) cl *= 2;
     const int64_t splits0 = (304 + sm * sn - 1) / (sm * sn);
@@ -581,7 +605,9 @@ void contract_f64_launch(const double* A, const double* B, double* C, const CtrD
     splits = (d.K + chunk - 1) / chunk;
     double* part = workspace(local, splits * MN);
     dim3 grid((unsigned)gm, (unsigned)gn, (unsigned)splits);
-    contract_f64_kernel<<<grid, NT, 0, s>>>(A, B, C, d, a_fast, b_fast, chunk, part);
+    CtrDesc full = d;
+    full.sym = false;
+    contract_f64_kernel<<<grid, NT, 0, s>>>(A, B, C, full, a_fast, b_fast, chunk, part);
     FCC_CHECK_LAUNCH();
     splitk_reduce_kernel<<<rgrid, 256, 0, s>>>(part, (int)splits, C, d);
     FCC_CHECK_LAUNCH();
@@ -591,6 +617,11 @@ void contract_f64_launch(const double* A, const double* B, double* C, const CtrD
   dim3 grid((unsigned)gm, (unsigned)gn, (unsigned)d.batch);
   contract_f64_kernel<<<grid, NT, 0, s>>>(A, B, C, d, a_fast, b_fast, d.K, nullptr);
   FCC_CHECK_LAUNCH();
+  if (d.sym) {
+    const unsigned t = (unsigned)((d.M + 31) / 32);
+    mirror_kernel<<<dim3(t, t), 256, 0, s>>>(C, d);
+    FCC_CHECK_LAUNCH();
+  }
   prof_end(s, pidx, PROF_F64, pflops);
 }
 
@@ -900,7 +931,7 @@ void einsum(double alpha, const char* spec, const TView& A, const TView& B, doub
   }
   // FP64: exact-slice products at the FP64 level from f64_min_flops on (see
   // TcEngine), DMMA below
-  if (tc && gb.empty()) {
+  if (tc && gb.empty() && !tc->f64_wide) {
     const double flops = 2.0 * (double)gdim(gm) * (double)gdim(gn) * (double)gdim(gk);
     std::vector<Ix> m3 = gm, n3 = gn, k3 = gk;
     if (flops >= tc->f64_min_flops && gdim(gm) > 1 && gdim(gn) > 1 && try_fuse(m3, 3) && try_fuse(n3, 3) && try_fuse(k3, 3) &&
@@ -932,6 +963,8 @@ void einsum(double alpha, const char* spec, const TView& A, const TView& B, doub
   d.N = gdim(gn); d.N2 = gn[1].dim; d.N3 = gn[2].dim;
   d.K = gk[0].dim * gk[1].dim; d.K2 = gk[1].dim;
   d.batch = gb[0].dim;
+  d.sym = tc && tc->f64_sym && beta == 0.0 && d.M == d.N && d.batch == 1;
+  d.wide = tc && tc->f64_wide && 2.0 * (double)d.M * (double)d.N * (double)d.K >= 1e7;
   d.a_m1 = gm[0].s[0]; d.a_m2 = gm[1].s[0]; d.a_m3 = gm[2].s[0];
   d.a_k1 = gk[0].s[0]; d.a_k2 = gk[1].s[0]; d.a_b = gb[0].s[0];
   d.b_k1 = gk[0].s[1]; d.b_k2 = gk[1].s[1];

@@ -233,6 +233,10 @@ struct TcEngine {
   // FP64 contractions of this size and more run as exact-slice products at the
   // FP64 level, whether `enabled` or not
   double f64_min_flops = 4e7;
+  // FP64 contractions on 64 x 64 tiles of the FP64 pipe whatever their size: the
+  // integrals that every form starts from (setup_integrals)
+  bool f64_wide = false;
+  bool f64_sym = false;   // and the next ones' results are symmetric in (m, n)
   DBuf<__nv_bfloat16> bufA, bufB;
   int* err = nullptr;
   int no_loads_once = 0;   // test hook: the next split-BF16 GEMM runs with EpiMap::no_loads

@@ -300,38 +300,53 @@ __global__ void __launch_bounds__(256) out_back_kernel(const float* __restrict__
   }
 }
 
-// y[b] = sum_h H2[b][h] w3[h] + b3; loss partials; dy = 2 (y - target) / B.
-// A warp per row, four columns per lane.
+// y[b] = sum_h H2[b][h] w3[h] + b3 in the order of h; loss partials; dy = 2 (y -
+// target) / B.  A thread per row, which it reads from shared memory, where 256
+// rows of 32 columns arrive coalesced.
 __global__ void __launch_bounds__(256) out_loss_kernel(const float* H2, const float* w3, const float* b3,
                                                        const float* target, int64_t B, float* y, float* dy,
                                                        double* loss_part) {
-  __shared__ double sm[8];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const float4 w = make_float4(w3[4 * lane], w3[4 * lane + 1], w3[4 * lane + 2], w3[4 * lane + 3]);
+  __shared__ float tile[256][33];
+  __shared__ float w[H];
+  __shared__ double sm[256];
+  const int t = threadIdx.x;
+  if (t < H) w[t] = w3[t];
   double l = 0.0;
-#pragma unroll 2
-  for (int64_t b = (int64_t)blockIdx.x * 8 + warp; b < B; b += (int64_t)gridDim.x * 8) {
-    const float4 h = *reinterpret_cast<const float4*>(H2 + b * H + 4 * lane);
-    float s = (h.x * w.x + h.y * w.y) + (h.z * w.z + h.w * w.w);
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    s += b3[0];
-    if (lane == 0) {
+  for (int64_t b0 = (int64_t)blockIdx.x * 256; b0 < B; b0 += (int64_t)gridDim.x * 256) {
+    const int64_t b = b0 + t;
+    float s = b3[0];
+    for (int c = 0; c < H; c += 32) {
+      __syncthreads();
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int e = t + 256 * q, r = e >> 3, k = 4 * (e & 7);
+        const float4 x = b0 + r < B ? *reinterpret_cast<const float4*>(H2 + (b0 + r) * H + c + k) : make_float4(0, 0, 0, 0);
+        tile[r][k] = x.x;
+        tile[r][k + 1] = x.y;
+        tile[r][k + 2] = x.z;
+        tile[r][k + 3] = x.w;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < 32; ++k) s = fmaf(tile[t][k], w[c + k], s);
+    }
+    if (b < B) {
       y[b] = s;
       if (target) {
-        float d = s - target[b];
+        const float d = s - target[b];
         l += (double)d * d;
         dy[b] = 2.0f * d / (float)B;
       }
     }
   }
   if (loss_part) {
-    if (lane == 0) sm[warp] = l;
+    sm[t] = l;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      double t = 0.0;
-      for (int k = 0; k < 8; ++k) t += sm[k];
-      loss_part[blockIdx.x] = t;
+    for (int h = 128; h > 0; h >>= 1) {
+      if (t < h) sm[t] += sm[t + h];
+      __syncthreads();
     }
+    if (t == 0) loss_part[blockIdx.x] = sm[0];
   }
 }
 

@@ -145,6 +145,16 @@ def test_matrix_vector_both_layouts(shape, spec, bspec):
     assert np.array_equal(out, 2.0 * ref - 1.0)
 
 
+@pytest.mark.parametrize("M,K", [(32, 31), (70, 300), (129, 33), (1000, 64)])
+def test_matrix_vector_bits_do_not_depend_on_the_layout(M, K):
+    rng = np.random.default_rng(M + K)
+    A, x = rng.standard_normal((M, K)), rng.standard_normal(K)
+    rc, rows = _run(PIPE, "mk,k->m", A, x, np.zeros(M))
+    rc2, cols = _run(PIPE, "km,k->m", np.ascontiguousarray(A.T), x, np.zeros(M))
+    assert rc == 0 and rc2 == 0
+    assert np.array_equal(rows, cols)
+
+
 def test_results_repeat_bit_for_bit():
     rng = np.random.default_rng(2)
     for M, N, K in ((40, 30, 20000), (300, 300, 300)):
