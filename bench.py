@@ -56,8 +56,8 @@ DE_BUDGET = 1e-6            # |dE_total| of the mixed form against the FP64 form
 # arm and scales the one-iteration CPU sample by that; the reference arm,
 # which has no GPU, uses this value.
 FP64_ITERATIONS = 17
-FP64_PEAK_TFLOPS = 1.05     # measured DMMA / DFMA peak of this GB300 pool (own probe)
-# MEASURED_PEAKS.json values of this pool, used when the file is not present
+FP64_PEAK_TFLOPS = 1.05     # measured DMMA / DFMA peak of a GB300 (own probe)
+# MEASURED_PEAKS.json values, used when the file is not present
 PEAKS_FALLBACK = {"hbm_gbs": 6778.3, "bf16_tflops": 1908.9, "bf16_tflops_sustained": 1714.6}
 # DRAM traffic per algorithmic flop of the DMMA kernel, from one ncu capture of
 # its largest launch (the o^3 v^3 ring contraction at (H2O)8, M = N = K = 4864:
@@ -66,7 +66,8 @@ DMMA_DRAM_BYTES_PER_FLOP = (7.114e9 + 0.186e9) / (2.0 * 4864.0 ** 3)
 # the same for the exact-slice kernel per executed BF16 flop, from one ncu
 # capture (dram__bytes_read.sum + dram__bytes_write.sum, one pass) of all 541
 # gemm_oz_kernel launches of one (H2O)8 mixed solve: 359.8e9 + 78.6e9 B for
-# 541 launches of 8.989e11 executed flop on average
+# 541 launches of 8.989e11 executed flop on average (single CTAs on 128 x 128 tiles;
+# the pairs on 256 x 128 tiles read each B panel half as often)
 OZ_DRAM_BYTES_PER_FLOP = (359.8e9 + 78.6e9) / (541 * 8.989e11)
 
 
@@ -180,13 +181,14 @@ def rhf_fock_part(args):
         t = (time.perf_counter() - t0) / k
         lib.fcc_prof_enable(0)
         lib.fcc_prof_read(prof, 6)
-        return t, prof[1] / k, prof[2] / k          # wall s, DMMA ms, DMMA flop per build
+        c = 5 if prof[21] > prof[1] else 0          # the products: exact-slice or FP64 pipe
+        return t, prof[4 * c + 1] / k, prof[4 * c + 2] / k, c   # wall s, ms and flop of the products per build
 
     k = max(args.steps, 5)
     l0 = lib.fcc_stat_launches()
-    t_d, ms_d, fl_d = timed(lambda: f.build(p.H, D), k)
+    t_d, ms_d, fl_d, cls_d = timed(lambda: f.build(p.H, D), k)
     launches_d = (lib.fcc_stat_launches() - l0) // (k + args.warmup)
-    t_o, ms_o, fl_o = timed(lambda: f.build_occ(p.H, Co), k)
+    t_o, ms_o, fl_o, _ = timed(lambda: f.build_occ(p.H, Co), k)
     F_dev, _ = f.build(p.H, D)
     t0 = time.perf_counter()
     F_ref = orhf.build_fock_df(p.H, D, p.b)
@@ -200,6 +202,7 @@ def rhf_fock_part(args):
     t_rhf_cpu = time.perf_counter() - t0
     f.close()
     ach = fl_d / (ms_d * 1e9) if ms_d else None
+    peak = measured_peaks()[0]["bf16_tflops_sustained"] if cls_d == 5 else FP64_PEAK_TFLOPS
     out = {"metric": f"DF-RHF Fock build time (H2O){args.waters}", "value": t_d * 1e3, "unit": "ms",
            "higher_is_better": False, "n_gpus": 1, "steps": k, "warmup": args.warmup, "dtype": "f64",
            "data": "synthetic (seeded water cluster, stand-in basis)",
@@ -208,11 +211,11 @@ def rhf_fock_part(args):
            "e2e_note": "value and occ_form_ms are host wall time per call through the C ABI (H, D / Co in, "
                        "F and the energy out)",
            "occ_form_ms": t_o * 1e3, "max_abs_dF_vs_oracle": err, "gpu_launches": launches_d,
-           "roofline": {"bound": "tensor", "kernel": "contract_f64_kernel (DMMA FP64), density form",
-                        "achieved": ach, "peak": FP64_PEAK_TFLOPS, "unit": "TFLOP/s",
-                        "frac": ach / FP64_PEAK_TFLOPS if ach else None,
-                        "dmma_ms_per_build": ms_d, "dmma_flop_per_build": fl_d,
-                        "occ_form_dmma_ms": ms_o, "occ_form_dmma_flop": fl_o},
+           "roofline": {"bound": "tensor", "kernel": ("gemm_oz_kernel (tcgen05 exact-slice BF16)" if cls_d == 5
+                                                  else "contract_f64 kernels (FP64 pipe)") + ", density form",
+                        "achieved": ach, "peak": peak, "unit": "TFLOP/s", "frac": ach / peak if ach else None,
+                        "product_ms_per_build": ms_d, "product_flop_per_build": fl_d,
+                        "occ_form_product_ms": ms_o, "occ_form_product_flop": fl_o},
            "cpu_baseline": {"value": t_cpu * 1e3, "unit": "ms", "kind": "port", "cores": os.cpu_count(),
                             "sample": "one restated build_fock! (numpy einsum, all host threads)"},
            "rhf": {"device_fock_s": t_rhf, "iterations": r.iterations, "energy": r.energy,
@@ -229,14 +232,14 @@ def dist_info():
 
 
 def measured_peaks():
-    """MEASURED_PEAKS.json of this pool (HBM copy GB/s, cuBLAS BF16 TFLOP/s)."""
+    """MEASURED_PEAKS.json (HBM copy GB/s, cuBLAS BF16 TFLOP/s)."""
     p = os.path.join(ROOT, "MEASURED_PEAKS.json")
     try:
         with open(p) as f:
             d = json.load(f)
         return {k: float(d[k]) for k in PEAKS_FALLBACK}, "MEASURED_PEAKS.json"
     except (OSError, KeyError, ValueError):
-        return dict(PEAKS_FALLBACK), "MEASURED_PEAKS.json values of this pool (file absent at run time)"
+        return dict(PEAKS_FALLBACK), "MEASURED_PEAKS.json values (file absent at run time)"
 
 
 def algorithmic_flops(o, v, Q):
@@ -475,7 +478,7 @@ def main():
     f_it, f_t = algorithmic_flops(inp.o, inp.v, inp.naux)
     # per-class kernel timing over the profiled step (CUDA events on the
     # library's stream): launches, ms, algorithmic work, longest launch
-    cls = {0: "contract_f64_kernel (DMMA FP64)", 1: "gemm_bf16_tc_kernel + gemm_t3_kernel (tcgen05 split-BF16)",
+    cls = {0: "contract_f64 kernels (FP64 pipe)", 1: "gemm_bf16_tc_kernel + gemm_t3_kernel (tcgen05 split-BF16)",
            2: "pack kernels (split + gather)", 5: "gemm_oz_kernel (tcgen05 exact-slice BF16)"}
     bf = peaks["bf16_tflops_sustained"]
     pk = {0: (FP64_PEAK_TFLOPS, "TFLOP/s"), 1: (bf, "TFLOP/s"), 2: (peaks["hbm_gbs"], "GB/s"), 5: (bf, "TFLOP/s")}

@@ -130,9 +130,10 @@ struct ErrSlots {
 // The FP64 pipe (two lanes per clk and SM) bounds this pass, not HBM, so it is
 // kept short: the quotient by D takes a reciprocal seed in single precision and
 // three Newton steps (Markstein, IBM J. Res. Dev. 34, 111 (1990): the remainder
-// r - q D by one fma, rounded as a division is) instead of the compiler's division, the stored errors are widened by integer arithmetic, and the dot of
-// the error with itself comes from this pass.  (H2O)8: 0.90 + 0.19 ms with a
-// division and a second pass over the errors, see the launch list.
+// r - q D by one fma, rounded as a division is) instead of the compiler's
+// division, and the stored errors are widened by integer arithmetic: 0.7 ms at
+// (H2O)8, 0.90 with divisions.  The order of the sums, and the dot of the error
+// with itself as a pass of its own, are kept: they enter the DIIS coefficients.
 // a float as a double, exactly, without the FP64 pipe (subnormals become 0)
 __device__ __forceinline__ double widen(float f) {
   const uint32_t b = __float_as_uint(f);

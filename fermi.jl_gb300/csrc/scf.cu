@@ -12,8 +12,8 @@
 //                                        is a broadcast; partial sums per row
 //                                        chunk, summed in a fixed order.
 //   J = 2 b^T gamma                     warp-per-row FP64 GEMV (rows contiguous).
-//   Y[Q,m,s] = sum_r b[Q,m,r] D[r,s]    FP64 DMMA contraction, M = (Q,m) fused.
-//   K[m,n] = sum_{Q,s} Y[Q,m,s] b[Q,n,s] FP64 DMMA contraction, split over K.
+//   Y[Q,m,s] = sum_r b[Q,m,r] D[r,s]    FP64 contraction, M = (Q,m) fused.
+//   K[m,n] = sum_{Q,s} Y[Q,m,s] b[Q,n,s] FP64 contraction, long in K = (Q,s).
 // The occupied-orbital form (D = Co Co^T, as every RHF iteration has) factors
 // K through X[Q,m,i] = sum_r b[Q,m,r] Co[r,i], K = X X^T: 4 naux nbf^2 nocc
 // flops instead of 4 naux nbf^3.

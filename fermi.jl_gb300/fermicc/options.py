@@ -18,7 +18,7 @@ keys the coupled-cluster path reads, plus the keys this backend adds:
 * ``cc_gpu_switch_rms`` -- residual at which the mixed form leaves the
   split-BF16 products.
 * ``cc_gpu_finish`` -- finish of the mixed form: "exact" (exact-slice products
-  at 9 weight groups, FP64-accurate) or "fp64" (DMMA).
+  at 9 weight groups, FP64-accurate) or "fp64".
 * ``cc_gpu_guess`` -- "mp2" or "mlp" (learned T2 initialiser).
 * ``pt_gpu_precision`` -- "fp64" or "mixed" for (T).
 * ``cc_gpu_checkpoint`` / ``cc_gpu_checkpoint_every`` -- checkpoint file of the

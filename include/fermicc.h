@@ -63,7 +63,7 @@ extern "C" {
 
 /* finish of the mixed form (fcc_opts.mixed_finish) */
 #define FCC_FINISH_EXACT 0 /* exact-slice products at 9 weight groups (default)   */
-#define FCC_FINISH_FP64 1  /* FP64 (DMMA) contractions                             */
+#define FCC_FINISH_FP64 1  /* FP64 contractions, as in the FP64 form               */
 
 typedef struct fcc_ctx fcc_ctx;
 
