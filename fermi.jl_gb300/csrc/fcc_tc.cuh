@@ -173,10 +173,13 @@ bool scratch_fits(double bytes);
 // products; pairs of one weight 2^(-b (s+t)) are summed on the tensor cores in
 // FP32 while |sum| <= 2^24, so every partial sum is an exact integer, and
 // those are added in double-FP32 (~2^-48 relative).  BF16 carries 8-bit digits
-// exactly, and fewer, wider digits need fewer products for the same bits: 48
-// bits take S = 6 and 21 products instead of the 36 of eight 6-bit digits.
-// The reduced levels of the mixed form stay at 6-bit digits: its iterates, and
-// so its converged amplitudes, depend on what those levels drop.
+// exactly, and fewer, wider digits need fewer products for the same bits (48
+// bits: S = 6 and 21 products instead of the 36 of eight 6-bit digits), which
+// the FP64 level uses.  The levels of the mixed and exact forms keep 6-bit
+// digits, the finish too: its iterates, and so its converged T1, depend on what
+// a level drops.  (At (H2O)8 a finish of six 8-bit digits, as many bits, moved T1
+// by 1.3e-9 of its norm and T2 by 4e-12, where repeated solves agree to 1e-12;
+// 6-bit digits agree to 1e-11.)
 // `cut` > 0: the first `cut` bands of groups get a running sum of their own
 // (the FP64 level, see gemm_oz.cu).  guard: the digits are cut from x 2^-guard,
 // |d_1| <= 2^(b - guard), so that sums reach 2^24 later.
@@ -198,8 +201,7 @@ constexpr OzLevel OZ_F64{8, 9, 1, 8, 2};
 constexpr int OZ_MAXS = 8;
 constexpr int OZ_G_DEFAULT = 8;
 // the level of `groups` weight groups of 6-bit digits, the unit the phases of
-// the mixed form are counted in: those digits themselves up to 7 groups, 8-bit
-// digits with at least their 6 (groups - 1) bits above
+// the mixed form are counted in
 OzLevel oz_level(int groups);
 // slice pairs (BF16 products) of a level
 inline double oz_pairs(OzLevel lv) {

@@ -23,16 +23,15 @@
 // and roles in threads the compiler could not tell from warps, fcc_tcgen05.cuh
 // elect_one).
 //
-// When an accumulator could reach 2^24 (a chunk: 1-4 k-blocks of 8-bit digits,
-// 25-64 of 6-bit ones) the eight epilogue warps add it, times its weight (a
+// When an accumulator could reach 2^24 (a chunk: 2-16 k-blocks at the FP64 level,
+// 25-64 of 6-bit digits) the eight epilogue warps add it, times its weight (a
 // power of two), into a running double-FP32 sum (hi + lo, ~2^-48 relative)
 // held in registers, 64 columns per thread.  Registers instead of TMEM leave
 // TMEM for two sets of two chunk accumulators, so the MMA thread fills one set
 // while the other is drained, and a drain reads 4 bytes per element from TMEM
 // instead of moving 20.  The additions run two per instruction (fma.rn.f32x2).
-// With 8-bit digits the chunks are short and the drains show: 1325 TFLOP/s at
-// 4864, 3.65 ms for the 48 bits that took 10.2 ms with 36 products of 6-bit
-// digits.
+// The FP64 level's 8-bit digits close a chunk every 2-16 k-blocks and its drains
+// show.
 //
 // Batches: products of the same shape whose rows lie apart by fixed steps in A,
 // B and C run in one launch (EpiMap batch, ba, bb, bc), which fills the chip
@@ -697,13 +696,7 @@ std::once_flag g_oz_attr;
 
 }  // namespace
 
-OzLevel oz_level(int groups) {
-  // up to 7 groups: 6-bit digits; above: the same 6 (groups - 1) bits or more
-  // in 8-bit digits
-  if (groups <= 7) return OzLevel{groups - 1, groups, 0, 6, 0};
-  const int S = (6 * (groups - 1) + 7) / 8;
-  return OzLevel{S, S + 1, 0, 8, 0};
-}
+OzLevel oz_level(int groups) { return OzLevel{groups - 1, groups, 0, 6, 0}; }
 
 void gemm_oz(const __nv_bfloat16* A, int64_t a_rows, const int* exA, const __nv_bfloat16* B, int64_t b_rows,
              const int* exB, int64_t Kpad, OzLevel lv, const EpiMap& ep0, DBuf<double>& ws, int* err, cudaStream_t s) {

@@ -7,6 +7,7 @@ import struct
 import numpy as np
 import pytest
 
+from oracle import ozaki
 from test_gpu_contract import _run
 
 pytestmark = pytest.mark.gpu
@@ -107,3 +108,19 @@ def test_infinities_and_nans_reach_their_rows_and_columns_only():
     bad = np.zeros((40, 50), dtype=bool)
     bad[3, :], bad[:, 7] = True, True
     assert np.array_equal(~np.isfinite(out), bad)
+
+
+def test_nine_groups_cut_what_the_integer_model_cuts():
+    # Sums that cancel to 2^-40 of their terms, where what a level drops (2^-48 of
+    # the row scales) is 2^-8 of the result: the finish of the mixed form has to
+    # drop what eight 6-bit digits drop.  The leading digits cancel exactly, so
+    # the running sums stay near the size of the result and add 8 2^-47 of it.
+    rng = np.random.default_rng(11)
+    M, N, K = 20, 17, 64
+    a, b = rng.standard_normal((M, K // 2)), rng.standard_normal((N, K // 2))
+    A = np.concatenate([a, -a * (1 + 2.0 ** -40 * rng.standard_normal(a.shape))], 1)
+    B = np.concatenate([b, b], 1)
+    rc, out = _run(19, "mk,nk->mn", A, B, np.zeros((M, N)))
+    assert rc == 0
+    want = ozaki.product(A, B, 9)
+    assert np.abs(out - want).max() <= 2.0 ** -30 * np.abs(want).max()
