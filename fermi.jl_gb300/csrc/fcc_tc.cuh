@@ -172,7 +172,7 @@ bool scratch_fits(double bytes);
 // A.B^T is the sum over slice pairs (s, t) with s + t <= G of the digit
 // products; pairs of one weight 2^(-b (s+t)) are summed on the tensor cores in
 // FP32 while |sum| <= 2^24, so every partial sum is an exact integer, and
-// those are added in double-FP32 (~2^-48 relative).  BF16 carries 8-bit digits
+// those are added in double-FP32 (2^-47 to 2^-48).  BF16 carries 8-bit digits
 // exactly, and fewer, wider digits need fewer products for the same bits (48
 // bits: S = 6 and 21 products instead of the 36 of eight 6-bit digits), which
 // the FP64 level uses.  The levels of the mixed and exact forms keep 6-bit
@@ -189,7 +189,7 @@ struct OzLevel {
 // FP64 level: 62 bits below the row maximum (two guard bits, so that sums of
 // first digits stay below 2^24 over 16 k-blocks), the first 36 pairs, the first
 // band summed apart.  Dropped pairs and cut digits are about 2^-62 of max|A_r|
-// max|B_c| per term and the sums carry ~2^-60 of the result, where an FP64
+// max|B_c| per term and the sums carry ~2^-59 of the result, where an FP64
 // product accumulates roundings of 2^-53 of its partial sums.  Error against
 // quadruple precision on the operands of (H2O)4 (2-norm of the difference over
 // that of the result), this level / FP64 pipe: DF fit over J^-1/2 1.6e-15 /

@@ -25,7 +25,7 @@
 //
 // When an accumulator could reach 2^24 (a chunk: 2-16 k-blocks at the FP64 level,
 // 25-64 of 6-bit digits) the eight epilogue warps add it, times its weight (a
-// power of two), into a running double-FP32 sum (hi + lo, ~2^-48 relative)
+// power of two), into a running double-FP32 sum (hi + lo, 2^-47 over K = 11628)
 // held in registers, 64 columns per thread.  Registers instead of TMEM leave
 // TMEM for two sets of two chunk accumulators, so the MMA thread fills one set
 // while the other is drained, and a drain reads 4 bytes per element from TMEM
@@ -157,16 +157,25 @@ __device__ __forceinline__ void unpack2(uint64_t d, uint32_t& x, uint32_t& y) {
 }
 
 // two independent (hi + lo) += v * w: TwoSum of hi and v * w (the product by a
-// power of two is exact inside the fma), the error into lo.  lo is left to grow
-// to a few last places of hi (n chunks: sqrt(n) / 2, n / 2 at most) and
-// renormalised once at the end: seven packed operations a chunk instead of ten,
-// and the FP32 pipe is what a drain takes (two clk per packed instruction).
+// power of two is exact inside the fma), the error into lo.  lo grows by half a
+// last place of hi an addition and ff_norm2 takes it back every second drain: 8.5
+// packed operations an addition instead of ten with every one, and the FP32 pipe
+// is what a drain takes (two clk per packed instruction).  Without it lo, and the
+// last place it is rounded to, grew over all of a product: at K = 11628 the sums
+// carried 2^-45.8 at nine groups and 2^-44.7 in the FP64 level's lower bands, now
+// 2^-47.2 and 2^-47.5 (an FP64 step at (H2O)8 75.1 ms, 75.2 with it).
 __device__ __forceinline__ void ff_add2(uint64_t& hi, uint64_t& lo, uint64_t v, uint64_t w, uint64_t m1) {
   const uint64_t s = fma2(v, w, hi);
   const uint64_t nbb = fma2(s, m1, hi);       // -(s - hi)
   const uint64_t t = add2(s, nbb);
   lo = add2(lo, add2(fma2(t, m1, hi), fma2(v, w, nbb)));
   hi = s;
+}
+
+__device__ __forceinline__ void ff_norm2(uint64_t& hi, uint64_t& lo, uint64_t m1) {
+  const uint64_t h = add2(hi, lo);
+  lo = fma2(fma2(hi, m1, h), m1, lo);   // lo - (h - hi)
+  hi = h;
 }
 
 __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
@@ -483,7 +492,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
           const int64_t n = (int64_t)nt * OZ_BN + half * 64 + 32 * c + lane;
           ecl[c] = n < ep.N ? oz_scale_exp(exB[bq * ep.bb + n]) : 0;
         }
-        int last = -1;
+        int last = -1, drains = 0;
         uint64_t hi[32], lo[32];
 #pragma unroll
         for (int c = 0; c < 32; ++c) hi[c] = lo[c] = 0ull;
@@ -529,6 +538,10 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
               asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
               __syncwarp();
               if (lane == 0) drained(set);
+              if ((++drains & 1) == 0) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) ff_norm2(hi[j], lo[j], m1);
+              }
             }
           }
         }

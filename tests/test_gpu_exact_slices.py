@@ -124,3 +124,67 @@ def test_nine_groups_cut_what_the_integer_model_cuts():
     assert rc == 0
     want = ozaki.product(A, B, 9)
     assert np.abs(out - want).max() <= 2.0 ** -30 * np.abs(want).max()
+
+
+def _base(x, bits, S):
+    """Balanced digits of the integers x, those of |x| with its sign, most
+    significant first."""
+    sign, x, d = np.sign(x), np.abs(x), []
+    for _ in range(S - 1):
+        r = ((x + (1 << (bits - 1))) & ((1 << bits) - 1)) - (1 << (bits - 1))
+        x = (x - r) >> bits
+        d.append(r)
+    return [(t * sign).astype(float) for t in [x] + d[::-1]]
+
+
+def _group_sum(DA, DB, g, bits):
+    """The pairs of weight 2^(-bits g), exact (integers below 2^53, then a power of two)."""
+    S = len(DA)
+    return sum(DA[s - 1] @ DB[g - s - 1].T for s in range(max(1, g - S), min(S, g - 1) + 1)).astype(np.longdouble) \
+        * np.longdouble(2.0) ** (-bits * g)
+
+
+# Running sums over the longest product of an (H2O)8 iteration (K = 11628, the
+# ladder), in one job: the number of outputs leaves no room for partial results,
+# so 130 copies of 32 rows and columns.  An addition rounds the error word, of the
+# size of a last place of the sum's (24 bits), to 24 bits of itself, twice:
+# sqrt(2 / 12) 2^-48 of the sum at most, 2^-49.5 in the mean over a binade, and n
+# of them add up to sqrt(n) that.
+_REP, _K = 130, 11628
+
+
+def test_nine_group_sums_over_a_long_product():
+    rng = np.random.default_rng(21)
+    A = np.rint(np.clip(0.15 * rng.standard_normal((32, _K)), -0.7, 0.7) * 2.0 ** 48)
+    B = np.rint(np.clip(0.15 * rng.standard_normal((32, _K)), -0.7, 0.7) * 2.0 ** 48)
+    A[:, 0] = B[:, 0] = 0.75 * 2.0 ** 48                      # row scales 1
+    DA, DB = _base(A.astype(np.int64), 6, 8), _base(B.astype(np.int64), 6, 8)
+    want = sum(_group_sum(DA, DB, g, 6) for g in range(2, 10))
+    M = 32 * _REP
+    rc, out = _run(19, "mk,nk->mn", np.tile(A * 2.0 ** -48, (_REP, 1)), np.tile(B * 2.0 ** -48, (_REP, 1)), np.zeros((M, M)))
+    assert rc == 0
+    assert np.array_equal(out, np.tile(out[:32, :32], (_REP, _REP)))
+    err = np.sqrt(np.mean((out[:32, :32] - want) ** 2) / np.mean(want ** 2))
+    # 16 blocks of up to 12 k-blocks, a chunk for each of four bands of two groups
+    assert err <= np.sqrt(16 * 4 * 2) * 2.0 ** -49.5, np.log2(float(err))
+
+
+def test_lower_bands_of_the_fp64_level_over_a_long_product():
+    # 30-bit operands (four digits: nothing is dropped), neighbouring columns
+    # opposite to 2^-17, so that the first band (all but carries of a digit) cancels
+    # chunk by chunk and the error of the others' sums shows in the result
+    rng = np.random.default_rng(22)
+    a = np.rint(np.clip(0.15 * rng.standard_normal((32, _K // 2)), -0.7, 0.7) * 2.0 ** 30)
+    b = np.rint(np.clip(0.15 * rng.standard_normal((32, _K // 2)), -0.7, 0.7) * 2.0 ** 30)
+    a[:, 0] = b[:, 0] = 0.75 * 2.0 ** 30
+    A, B = np.repeat(a, 2, axis=1), np.repeat(b, 2, axis=1)
+    A[:, 1::2] = -a + np.rint(0.2 * rng.standard_normal(a.shape) * 2.0 ** 13)
+    DA, DB = _base(A.astype(np.int64), 8, 4), _base(B.astype(np.int64), 8, 4)   # of x 2^-2: 32 bits
+    band = [_group_sum(DA, DB, g, 8) * 16 for g in range(2, 9)]
+    want, lower = sum(band), sum(band[2:])
+    M = 32 * _REP
+    rc, out = _run(20, "mk,nk->mn", np.tile(A * 2.0 ** -30, (_REP, 1)), np.tile(B * 2.0 ** -30, (_REP, 1)), np.zeros((M, M)))
+    assert rc == 0
+    err = np.sqrt(np.mean((out[:32, :32] - want) ** 2) / np.mean(lower ** 2))
+    # in each block chunks of 5, 3 and 2 k-blocks: 3 + 4 + 6 of them, two groups each
+    assert err <= np.sqrt(16 * 13 * 2) * 2.0 ** -49.5, np.log2(float(err))
