@@ -1,6 +1,7 @@
 // Shared definitions for the GB300 coupled-cluster library (libfermicc).
 #pragma once
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstdint>
 #include <cstdio>
 #include <string>
@@ -35,6 +36,22 @@ void note_launch();
     ::fcc::note_launch();           \
     FCC_CUDA(cudaGetLastError());   \
   } while (0)
+
+// The dynamic shared-memory limit of a kernel, one object for each.  A limit
+// holds for the device that is current when it is set, and contexts may sit on
+// several, so what was set is kept by device.
+struct SmemLimit {
+  std::atomic<uint64_t> done{0};
+  template <class K>
+  void raise(K* kernel, int bytes) {
+    int dev = 0;
+    FCC_CUDA(cudaGetDevice(&dev));
+    const uint64_t bit = dev < 64 ? uint64_t(1) << dev : 0;
+    if (done.load() & bit) return;
+    FCC_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    done.fetch_or(bit);
+  }
+};
 
 // Opt-in kernel timing (csrc/prof.cu): classes of work.
 enum { PROF_F64 = 0, PROF_TC = 1, PROF_PACK = 2, PROF_UPDATE = 3, PROF_TRIPLES = 4, PROF_OZ = 5, PROF_NCLS = 6 };

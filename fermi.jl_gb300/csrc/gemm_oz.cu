@@ -55,7 +55,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <mutex>
 
 #include "fcc_tc.cuh"
 #include "fcc_tcgen05.cuh"
@@ -705,8 +704,6 @@ __global__ void __launch_bounds__(256) oz_reduce_kernel(const double* __restrict
   }
 }
 
-std::once_flag g_oz_attr;
-
 }  // namespace
 
 OzLevel oz_level(int groups) { return OzLevel{groups - 1, groups, 0, 6, 0}; }
@@ -743,12 +740,10 @@ void gemm_oz(const __nv_bfloat16* A, int64_t a_rows, const int* exA, const __nv_
     std::swap(ep.ba, ep.bb);
   }
   const bool pair = pairs(ep.M);
-  std::call_once(g_oz_attr, []() {
-    cudaFuncSetAttribute(gemm_oz_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM);
-    cudaFuncSetAttribute(gemm_oz_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM);
-    cudaFuncSetAttribute(gemm_oz_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM);
-    cudaFuncSetAttribute(gemm_oz_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM);
-  });
+  auto* const kernel = lv.cut ? (pair ? gemm_oz_kernel<true, true> : gemm_oz_kernel<true, false>)
+                              : (pair ? gemm_oz_kernel<false, true> : gemm_oz_kernel<false, false>);
+  static SmemLimit smem[2][2];
+  smem[lv.cut != 0][pair].raise(kernel, OZ_SMEM);
   OzParams P;
   std::memset(&P, 0, sizeof(P));
   const int nb = make_bands(lv, P.band);
@@ -864,8 +859,7 @@ void gemm_oz(const __nv_bfloat16* A, int64_t a_rows, const int* exA, const __nv_
   cfg.attrs = at;
   cfg.numAttrs = 1;
   const int pidx = prof_begin(s);
-  if (lv.cut) FCC_CUDA(cudaLaunchKernelEx(&cfg, pair ? gemm_oz_kernel<true, true> : gemm_oz_kernel<true, false>, ta, tb, P, exA, exB, ep, err));
-  else FCC_CUDA(cudaLaunchKernelEx(&cfg, pair ? gemm_oz_kernel<false, true> : gemm_oz_kernel<false, false>, ta, tb, P, exA, exB, ep, err));
+  FCC_CUDA(cudaLaunchKernelEx(&cfg, kernel, ta, tb, P, exA, exB, ep, err));
   FCC_CHECK_LAUNCH();
   if (P.njobs > 1) {
     const int64_t MN = ep.M * ep.N;

@@ -18,7 +18,6 @@
 
 #include <algorithm>
 #include <cstring>
-#include <mutex>
 
 #include "fcc_t3.cuh"
 #include "fcc_tcgen05.cuh"
@@ -261,10 +260,8 @@ __global__ void __launch_bounds__(T3_THREADS, 1) gemm_t3_kernel(const __grid_con
 template <int BN>
 void launch_t3(const T3Params& P, cudaStream_t s) {
   using Cfg = T3Cfg<BN>;
-  static std::once_flag once;
-  std::call_once(once, []() {
-    cudaFuncSetAttribute(gemm_t3_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
-  });
+  static SmemLimit smem;
+  smem.raise(gemm_t3_kernel<BN>, Cfg::SMEM);
   const int64_t tm = ((int64_t)P.v * P.v + 2 * T3_BM - 1) / (2 * T3_BM);
   const int64_t tn = (P.v + BN - 1) / BN;
   const int64_t ntiles = tm * tn * 3 * P.nk;

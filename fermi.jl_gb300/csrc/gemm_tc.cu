@@ -548,10 +548,8 @@ template <int BN>
 void launch_tc(const __nv_bfloat16* A, int64_t a_rows, int64_t a_row0, const __nv_bfloat16* B, int64_t b_rows,
                int64_t b_row0, int64_t Kp, const EpiMap& ep, int* err, cudaStream_t s) {
   using Cfg = TcCfg<BN>;
-  static std::once_flag attr_once;
-  std::call_once(attr_once, []() {
-    cudaFuncSetAttribute(gemm_bf16_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
-  });
+  static SmemLimit smem;
+  smem.raise(gemm_bf16_tc_kernel<BN>, Cfg::SMEM);
   CUtensorMap ta = make_map(A, a_rows, Kp, BM);
   CUtensorMap tb = make_map(B, b_rows, Kp, BN);
   const int64_t tm = (ep.M + BM - 1) / BM, tn = (ep.N + BN - 1) / BN;

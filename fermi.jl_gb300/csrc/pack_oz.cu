@@ -13,7 +13,6 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
-#include <mutex>
 
 #include "fcc_tc.cuh"
 #include "fcc_tcgen05.cuh"
@@ -519,11 +518,8 @@ void pack(const double* src, const PackSpec& ps, int guard, __nv_bfloat16* dst, 
   if (tiles && Kpad <= 8 * TILE_KW) {
     const int nc = (int)((Kpad + TILE_KW - 1) / TILE_KW);
     const int kw = (int)((Kpad / 64 + nc - 1) / nc * 64);
-    static std::once_flag once;
-    std::call_once(once, []() {
-      cudaFuncSetAttribute(oz_pack_tiles_cluster_kernel<S, BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           TILE_KW * 33 * 8);
-    });
+    static SmemLimit smem;
+    smem.raise(oz_pack_tiles_cluster_kernel<S, BITS>, TILE_KW * 33 * 8);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(std::min<int64_t>(ntr, 152 * 4) * nc));
     cfg.blockDim = dim3(256);
@@ -540,10 +536,8 @@ void pack(const double* src, const PackSpec& ps, int guard, __nv_bfloat16* dst, 
     return;
   }
   if (!tiles && Kpad > 4096 && Kpad <= ROW_KMAX && ps.R >= 304) {
-    static std::once_flag once;
-    std::call_once(once, []() {
-      cudaFuncSetAttribute(oz_pack_rows_smem_kernel<S, BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROW_KMAX * 8);
-    });
+    static SmemLimit smem;
+    smem.raise(oz_pack_rows_smem_kernel<S, BITS>, ROW_KMAX * 8);
     oz_pack_rows_smem_kernel<S, BITS><<<(unsigned)std::min<int64_t>(ps.R, 152 * 8), 512, (size_t)Kpad * 8, s>>>(
         src, ps, Kpad, guard, ex, dst);
     FCC_CHECK_LAUNCH();
