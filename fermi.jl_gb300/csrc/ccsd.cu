@@ -820,8 +820,14 @@ void residual(fcc_ctx* c) {
     const bool exact = tc && (tc->exact || !tc->enabled);
     const OzLevel lv = tc && tc->enabled ? tc->oz : OZ_F64;
     const int64_t R = v * v;
-    const bool tcw = tc && (tc->enabled || (2.0 * v * v * v * (double)v * Q >= tc->f64_min_flops &&
-                                            scratch_fits(2.0 * ((double)R * lv.S * oz_kpad(Q) - (double)c->bvvA.n))));
+    bool tcw = tc && (tc->enabled || 2.0 * v * v * v * (double)v * Q >= tc->f64_min_flops);
+    if (tcw && !tc->enabled) {   // FP64: on the FP64 pipe where the slices cannot be had
+      const int64_t need = R * lv.S * oz_kpad(Q);
+      tcw = tc->scratch_fits(std::max(0.0, 2.0 * ((double)need - (double)tc->bvvA.n)) +
+                             std::max(0.0, 4.0 * ((double)R - (double)tc->bvvEx.n))) &&
+            ((int64_t)tc->bvvA.n >= need || tc->bvvA.try_alloc(need)) &&
+            ((int64_t)tc->bvvEx.n >= R || tc->bvvEx.try_alloc(R));
+    }
     int64_t Wk = 0;   // packed row length
     if (tcw) {
       PackSpec ps{};
@@ -832,19 +838,19 @@ void residual(fcc_ctx* c) {
         const int S = lv.S;
         Wk = S * oz_kpad(Q);
         ps.Kp = Wk;
-        if ((int64_t)c->bvvA.n < R * Wk) c->bvvA.alloc(R * Wk);
-        if ((int64_t)c->bvvEx.n < R) c->bvvEx.alloc(R);
-        pack_oz(Btvv.p, ps, S, lv.bits, lv.guard, c->bvvA.p, c->bvvEx.p, s);
+        if ((int64_t)tc->bvvA.n < R * Wk) tc->bvvA.alloc(R * Wk);
+        if ((int64_t)tc->bvvEx.n < R) tc->bvvEx.alloc(R);
+        pack_oz(Btvv.p, ps, S, lv.bits, lv.guard, tc->bvvA.p, tc->bvvEx.p, s);
       } else {
         Wk = packed_kp(Q, tc->scheme.P);
         ps.Kp = Wk;
         ps.P = tc->scheme.P;
-        if ((int64_t)c->bvvA.n < R * Wk) c->bvvA.alloc(R * Wk);
-        if ((int64_t)c->bvvB.n < R * Wk) c->bvvB.alloc(R * Wk);
+        if ((int64_t)tc->bvvA.n < R * Wk) tc->bvvA.alloc(R * Wk);
+        if ((int64_t)tc->bvvB.n < R * Wk) tc->bvvB.alloc(R * Wk);
         ps.code = tc->scheme.code_a;
-        pack_split(Btvv.p, ps, c->bvvA.p, s);
+        pack_split(Btvv.p, ps, tc->bvvA.p, s);
         ps.code = tc->scheme.code_b;
-        pack_split(Btvv.p, ps, c->bvvB.p, s);
+        pack_split(Btvv.p, ps, tc->bvvB.p, s);
       }
     }
     for (int64_t a0 = 0; a0 < v; a0 += c->ladder_block) {
@@ -861,13 +867,13 @@ void residual(fcc_ctx* c) {
         const int64_t r0 = a0 * v;
         if (exact) {
           ep.work = 2.0 * (double)ep.M * (double)ep.N * (double)Q * oz_pairs(lv);
-          gemm_oz(c->bvvA.p + r0 * Wk, ep.M, c->bvvEx.p + r0, c->bvvA.p + r0 * Wk, ep.N, c->bvvEx.p + r0,
+          gemm_oz(tc->bvvA.p + r0 * Wk, ep.M, tc->bvvEx.p + r0, tc->bvvA.p + r0 * Wk, ep.N, tc->bvvEx.p + r0,
                   Wk / lv.S, lv, ep, tc->ozws, tc->err, s);
         } else {
           ep.work = 2.0 * (double)ep.M * (double)ep.N * (double)Q * tc->scheme.P;
           ep.no_loads = tc->no_loads_once;
           tc->no_loads_once = 0;
-          gemm_bf16x3(c->bvvA.p, R, r0, c->bvvB.p, R, r0, Wk, ep, tc->err, s);
+          gemm_bf16x3(tc->bvvA.p, R, r0, tc->bvvB.p, R, r0, Wk, ep, tc->err, s);
         }
         tc->tc_calls++;
         tc->tc_flops += ep.work;

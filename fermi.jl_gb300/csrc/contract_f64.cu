@@ -778,7 +778,8 @@ TcEngine::KeptPack* kept_a(TcEngine* tc, const double* src, const PackSpec& ps, 
 
 // Tensor-core evaluation of C = alpha * A.B + beta * C (no batch index): by
 // exact-slice products of level lv, or (lv.S = 0) by the engine's split scheme.
-void run_tc(TcEngine* tc, OzLevel lv, double alpha, const TView& A, const TView& B, double beta, const TView& C,
+// `optional`: false, with nothing done, where scratch cannot be had.
+bool run_tc(TcEngine* tc, bool optional, OzLevel lv, double alpha, const TView& A, const TView& B, double beta, const TView& C,
             std::vector<Ix> gm, std::vector<Ix> gn, std::vector<Ix> gk, cudaStream_t s) {
   // fastest-moving member last: the one with the smallest stride in the operand that is read along it
   auto order = [](std::vector<Ix>& g, int op) {
@@ -789,14 +790,17 @@ void run_tc(TcEngine* tc, OzLevel lv, double alpha, const TView& A, const TView&
   order(gk, 0);
   pad3(gm); pad3(gn); pad3(gk);
   const int64_t M = gdim(gm), N = gdim(gn), K = gdim(gk);
+  auto grow = [&](auto& buf, int64_t n) {
+    if ((int64_t)buf.n >= n) return true;
+    if (optional) return buf.try_alloc(n);
+    buf.alloc(n);
+    return true;
+  };
   if (lv.S > 0) {
     // exact-slice products: S digit slices of each operand, FP64 output
     const int S = lv.S;
     const int64_t Kpad = oz_kpad(K), W = S * Kpad;
-    if ((int64_t)tc->bufA.n < M * W) tc->bufA.alloc(M * W);
-    if ((int64_t)tc->bufB.n < N * W) tc->bufB.alloc(N * W);
-    if ((int64_t)tc->exA.n < M) tc->exA.alloc(M);
-    if ((int64_t)tc->exB.n < N) tc->exB.alloc(N);
+    if (!grow(tc->bufA, M * W) || !grow(tc->bufB, N * W) || !grow(tc->exA, M) || !grow(tc->exB, N)) return false;
     PackSpec pa{M, K, W, gm[1].dim, gm[2].dim, gm[0].s[0], gm[1].s[0], gm[2].s[0],
                 gk[1].dim, gk[2].dim, gk[0].s[0], gk[1].s[0], gk[2].s[0], S, 0};
     PackSpec pb{N, K, W, gn[1].dim, gn[2].dim, gn[0].s[1], gn[1].s[1], gn[2].s[1],
@@ -807,8 +811,10 @@ void run_tc(TcEngine* tc, OzLevel lv, double alpha, const TView& A, const TView&
     int* eA = tc->exA.p;
     if (ka) {
       if (fresh) {
-        if ((int64_t)ka->buf.n < M * W) ka->buf.alloc(M * W);
-        if ((int64_t)ka->ex.n < M) ka->ex.alloc(M);
+        if (!grow(ka->buf, M * W) || !grow(ka->ex, M)) {
+          ka->valid = false;
+          return false;
+        }
         pack_oz(A.p, pa, S, lv.bits, lv.guard, ka->buf.p, ka->ex.p, s);
       }
       pA = ka->buf.p;
@@ -826,7 +832,7 @@ void run_tc(TcEngine* tc, OzLevel lv, double alpha, const TView& A, const TView&
     gemm_oz(pA, M, eA, tc->bufB.p, N, tc->exB.p, Kpad, lv, ep, tc->ozws, tc->err, s);
     tc->tc_calls++;
     tc->tc_flops += ep.work;
-    return;
+    return true;
   }
   const SplitScheme sc = tc->scheme;
   const int64_t Kp = packed_kp(K, sc.P);
@@ -860,16 +866,16 @@ void run_tc(TcEngine* tc, OzLevel lv, double alpha, const TView& A, const TView&
   gemm_bf16x3(pA, M, 0, tc->bufB.p, N, 0, Kp, ep, tc->err, s);
   tc->tc_calls++;
   tc->tc_flops += 2.0 * (double)M * (double)N * (double)K * sc.P;
+  return true;
 }
 
 }  // namespace
 
-// The slices take twice the memory of an FP64 operand.  Large ones are taken
-// only while they leave half of the free memory; the FP64 pipe needs none.
-bool scratch_fits(double bytes) {
-  if (bytes < 4e9) return true;
+bool TcEngine::scratch_fits(double growth) const {
+  if (growth <= 0) return true;
+  if (scratch_held() + growth > scratch_max) return false;
   size_t f = 0, t = 0;
-  return cudaMemGetInfo(&f, &t) == cudaSuccess && bytes <= 0.5 * (double)f;
+  return cudaMemGetInfo(&f, &t) == cudaSuccess && growth <= 0.5 * (double)f;
 }
 
 static std::atomic<int64_t> g_launches{0};
@@ -889,7 +895,8 @@ DBuf<double>*& f64_workspace() {
 // bytes by which run_tc would grow the engine's buffers for a product
 static double pack_growth(const TcEngine* tc, const OzLevel& lv, int64_t M, int64_t N, int64_t K) {
   const double w = (double)lv.S * (double)oz_kpad(K);
-  return 2.0 * (std::max(0.0, (double)M * w - (double)tc->bufA.n) + std::max(0.0, (double)N * w - (double)tc->bufB.n));
+  auto more = [](double need, size_t have) { return std::max(0.0, need - (double)have); };
+  return 2.0 * (more(M * w, tc->bufA.n) + more(N * w, tc->bufB.n)) + 4.0 * (more(M, tc->exA.n) + more(N, tc->exB.n));
 }
 
 void einsum(double alpha, const char* spec, const TView& A, const TView& B, double beta, const TView& C,
@@ -925,7 +932,7 @@ void einsum(double alpha, const char* spec, const TView& A, const TView& B, doub
     std::vector<Ix> m3 = gm, n3 = gn, k3 = gk;
     if (flops >= tc->min_flops && gdim(gm) >= tc->min_dim && gdim(gn) >= tc->min_dim && try_fuse(m3, 3) && try_fuse(n3, 3) &&
         try_fuse(k3, 3)) {
-      run_tc(tc, tc->exact ? tc->oz : OzLevel{0, 0, 0, 0, 0}, alpha, A, B, beta, C, m3, n3, k3, s);
+      run_tc(tc, false, tc->exact ? tc->oz : OzLevel{0, 0, 0, 0, 0}, alpha, A, B, beta, C, m3, n3, k3, s);
       return;
     }
   }
@@ -934,11 +941,11 @@ void einsum(double alpha, const char* spec, const TView& A, const TView& B, doub
   if (tc && gb.empty() && !tc->f64_wide) {
     const double flops = 2.0 * (double)gdim(gm) * (double)gdim(gn) * (double)gdim(gk);
     std::vector<Ix> m3 = gm, n3 = gn, k3 = gk;
-    if (flops >= tc->f64_min_flops && gdim(gm) > 1 && gdim(gn) > 1 && try_fuse(m3, 3) && try_fuse(n3, 3) && try_fuse(k3, 3) &&
-        scratch_fits(pack_growth(tc, OZ_F64, gdim(gm), gdim(gn), gdim(gk)))) {
-      run_tc(tc, OZ_F64, alpha, A, B, beta, C, m3, n3, k3, s);
+    if (flops >= tc->f64_min_flops && gdim(gm) > 1 && gdim(gn) > 1 && oz_takes(gdim(gm), gdim(gn), gdim(gk)) &&
+        try_fuse(m3, 3) && try_fuse(n3, 3) && try_fuse(k3, 3) &&
+        tc->scratch_fits(pack_growth(tc, OZ_F64, gdim(gm), gdim(gn), gdim(gk))) &&
+        run_tc(tc, true, OZ_F64, alpha, A, B, beta, C, m3, n3, k3, s))
       return;
-    }
   }
   fuse(gb, 1, spec);
   fuse(gm, 3, spec);

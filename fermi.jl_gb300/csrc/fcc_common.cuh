@@ -78,6 +78,21 @@ struct DBuf {
     FCC_CUDA(cudaMalloc(&p, count * sizeof(T)));
     n = count;
   }
+  // the same for memory that can be done without: false (and empty) where there is too little
+  bool try_alloc(size_t count) {
+    release();
+    if (count == 0) return true;
+    const cudaError_t e = cudaMalloc(&p, count * sizeof(T));
+    if (e == cudaErrorMemoryAllocation) {
+      (void)cudaGetLastError();
+      p = nullptr;
+      return false;
+    }
+    FCC_CUDA(e);
+    n = count;
+    return true;
+  }
+  size_t bytes() const { return n * sizeof(T); }
   void zero(cudaStream_t s) { if (p) FCC_CUDA(cudaMemsetAsync(p, 0, n * sizeof(T), s)); }
   void release() {
     if (p) cudaFree(p);

@@ -161,9 +161,6 @@ void gemm_bf16x3(const __nv_bfloat16* A, int64_t a_rows, int64_t a_row0, const _
 // (one 128-byte swizzle atom) x box_rows rows; cols must be a multiple of 64.
 CUtensorMap tma_map_bf16(const __nv_bfloat16* base, int64_t rows, int64_t cols, int box_rows);
 
-// whether scratch of that many bytes is small or leaves half of the free memory
-bool scratch_fits(double bytes);
-
 // Exact-slice products (the Ozaki scheme: Ozaki, Ogita, Oishi & Rump, Numer.
 // Algorithms 59, 95 (2012); on tensor cores: Mukunoki et al., ISC 2020).
 // Each row r of an operand is scaled by 2^e_r (|x| < 2^e_r over the row) and
@@ -213,6 +210,11 @@ inline double oz_pairs(OzLevel lv) {
 // to (s+1)*Kpad; ex[r] = biased FP64 exponent of max_k |x_rk| (0: all zero,
 // 2047: the row holds an infinity or NaN, and so will its products)
 int64_t oz_kpad(int64_t K);
+// the extents pack_oz and gemm_oz take
+constexpr int64_t OZ_KMAX = int64_t(1) << 27;
+inline bool oz_takes(int64_t M, int64_t N, int64_t K) {
+  return M < (int64_t(1) << 31) && N < (int64_t(1) << 31) && K <= OZ_KMAX;
+}
 void pack_oz(const double* src, const PackSpec& ps, int S, int bits, int guard, __nv_bfloat16* dst, int* ex,
              cudaStream_t s);
 // exact-slice product over packed operands, written to ep;
@@ -256,6 +258,21 @@ struct TcEngine {
   };
   const double* keep_src[2] = {nullptr, nullptr};
   KeptPack kept[2];
+  // The ladder's dressed factors Bt[Q][x][y] (x, y virtual) packed once per
+  // residual for every block's (ac|bd) product (rows (x, y), K = Q): digit
+  // slices and row exponents, or the split pieces in the A and in the B order
+  DBuf<__nv_bfloat16> bvvA, bvvB;
+  DBuf<int> bvvEx;
+  // Digit slices take twice the memory of an FP64 operand, and FP64 contractions
+  // can do without: they take more scratch only while that leaves half of the
+  // free memory, and run on the FP64 pipe otherwise.
+  double scratch_max = 1e300;   // test hook: bytes of packed operands in all
+  double scratch_held() const {
+    double b = (double)(bufA.bytes() + bufB.bytes() + exA.bytes() + exB.bytes() + bvvA.bytes() + bvvB.bytes() + bvvEx.bytes());
+    for (const KeptPack& k : kept) b += (double)(k.buf.bytes() + k.ex.bytes());
+    return b;
+  }
+  bool scratch_fits(double growth) const;
   int64_t tc_calls = 0, f64_calls = 0;
   double tc_flops = 0, f64_flops = 0;
 };

@@ -43,6 +43,16 @@ extern "C" int fcc_test_set_t3_kc(fcc_ctx* c, int32_t kc) {
   return FCC_OK;
 }
 
+extern "C" int fcc_test_set_scratch(fcc_ctx* c, int64_t bytes) {
+  if (!c) return FCC_ERR_BAD_ARG;
+  c->tc.scratch_max = bytes < 0 ? 1e300 : (double)bytes;
+  return FCC_OK;
+}
+
+extern "C" int64_t fcc_test_scratch_held(const fcc_ctx* c) { return c ? (int64_t)c->tc.scratch_held() : -1; }
+
+extern "C" int64_t fcc_test_products(const fcc_ctx* c) { return c ? c->tc.tc_calls : -1; }
+
 extern "C" int fcc_test_inject(fcc_ctx* c, int32_t kind) {
   if (!c || !(kind == 0 || kind == FCC_TEST_FAULT_NO_LOADS || kind == FCC_TEST_FAULT_NAN)) return FCC_ERR_BAD_ARG;
   c->test_fault = kind;

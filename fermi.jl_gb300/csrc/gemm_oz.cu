@@ -714,7 +714,7 @@ void gemm_oz(const __nv_bfloat16* A, int64_t a_rows, const int* exA, const __nv_
   if (ep.M <= 0 || ep.N <= 0) return;
   if (lv.S < 1 || lv.S > OZ_MAXS || lv.G < 2 || lv.G > lv.S + 2 || (lv.bits != 6 && lv.bits != 8) || lv.guard < 0 || lv.guard > 2)
     fail(FCC_ERR_BAD_ARG, "bad exact-slice level");
-  if (Kpad <= 0 || Kpad % OZ_BK || Kpad > (1 << 27)) fail(FCC_ERR_BAD_ARG, "bad padded K");
+  if (Kpad <= 0 || Kpad % OZ_BK || Kpad > OZ_KMAX) fail(FCC_ERR_BAD_ARG, "bad padded K");
   if (ep.batch < 1 || ep.batch > 65535 || a_rows < ep.M + (ep.batch - 1) * ep.ba || b_rows < ep.N + (ep.batch - 1) * ep.bb)
     fail(FCC_ERR_BAD_ARG, "packed operands smaller than the output");
   if (ep.M >= (int64_t(1) << 31) || ep.N >= (int64_t(1) << 31)) fail(FCC_ERR_BAD_ARG, "output extent too large");
@@ -832,8 +832,12 @@ void gemm_oz(const __nv_bfloat16* A, int64_t a_rows, const int* exA, const __nv_
   P.units = (uint32_t)(tiles * P.njobs * ep.batch);
   if (P.njobs > 1) {
     const size_t need = (size_t)P.njobs * ep.batch * ep.M * ep.N;
-    if (ws.n < need) ws.alloc(need);
-    P.part = ws.p;
+    if (ws.n >= need || ws.try_alloc(need)) {
+      P.part = ws.p;
+    } else {   // no room for partial results: one job a tile
+      P.njobs = (uint32_t)build(0.0);
+      P.units = (uint32_t)(tiles * P.njobs * ep.batch);
+    }
   }
   // One job and one chunk in the first band: the other bands go first, and the
   // store stage adds the first band's two accumulators to their sums, so the

@@ -40,7 +40,8 @@ EXPORTS = ("fcc_default_opts", "fcc_create", "fcc_upload_df", "fcc_upload_conv",
            "fcc_scf_last_error", "fcc_scf_upload_b", "fcc_scf_fit", "fcc_scf_build_fock", "fcc_scf_build_fock_occ")
 TEST_EXPORTS = ("fcc_test_contract", "fcc_stat_launches", "fcc_stream", "fcc_prof_enable", "fcc_prof_read",
                 "fcc_test_set_t3_bn", "fcc_test_split3", "fcc_test_pack_oz", "fcc_test_inject",
-                "fcc_test_triples_subset", "fcc_test_set_t3_kc")
+                "fcc_test_triples_subset", "fcc_test_set_t3_kc", "fcc_test_set_scratch", "fcc_test_scratch_held",
+                "fcc_test_products")
 
 
 class FccOpts(ctypes.Structure):
@@ -136,6 +137,12 @@ def load():
     lib.fcc_test_pack_oz.restype = ctypes.c_int
     lib.fcc_test_set_t3_kc.argtypes = [vp, i32]
     lib.fcc_test_set_t3_kc.restype = ctypes.c_int
+    lib.fcc_test_set_scratch.argtypes = [vp, i64]
+    lib.fcc_test_set_scratch.restype = ctypes.c_int
+    lib.fcc_test_scratch_held.argtypes = [vp]
+    lib.fcc_test_scratch_held.restype = i64
+    lib.fcc_test_products.argtypes = [vp]
+    lib.fcc_test_products.restype = i64
     lib.fcc_test_inject.argtypes = [vp, i32]
     lib.fcc_test_inject.restype = ctypes.c_int
     lib.fcc_test_triples_subset.argtypes = [vp, ctypes.POINTER(ctypes.c_int32), i32, dp]

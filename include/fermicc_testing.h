@@ -59,6 +59,14 @@ int fcc_test_set_t3_bn(fcc_ctx* ctx, int32_t bn);
  * number the FP64 form also packs its operands run by run. */
 int fcc_test_set_t3_kc(fcc_ctx* ctx, int32_t kc);
 
+/* The most bytes of packed operands that the FP64 contractions of ctx may hold
+ * (negative: no such limit, as by default); those that need more run on the
+ * FP64 pipe, as they do where memory is short.  fcc_test_scratch_held: the bytes
+ * held now.  fcc_test_products: contractions run on the tensor cores so far. */
+int fcc_test_set_scratch(fcc_ctx* ctx, int64_t bytes);
+int64_t fcc_test_scratch_held(const fcc_ctx* ctx);
+int64_t fcc_test_products(const fcc_ctx* ctx);
+
 /* One-shot failure injection on ctx for the error-path tests; nothing here
  * faults the GPU.  FCC_TEST_FAULT_NO_LOADS: the first split-BF16 tensor-core
  * GEMM of the next mixed-form fcc_ccsd_run issues no TMA loads, so its MMA
