@@ -758,22 +758,24 @@ bool same_spec(const PackSpec& a, const PackSpec& b) {
          a.ks3 == b.ks3 && a.P == b.P && a.code == b.code && a.scale == b.scale;
 }
 
-// The kept pack of operand A for (src, ps, S) when src is one of the
-// engine's kept sources (nullptr otherwise); `fresh` is set when it has to be
-// packed now.
-TcEngine::KeptPack* kept_a(TcEngine* tc, const double* src, const PackSpec& ps, int S, bool& fresh) {
-  fresh = false;
-  for (int i = 0; i < 2; ++i) {
-    if (!src || tc->keep_src[i] != src) continue;
-    TcEngine::KeptPack& k = tc->kept[i];
-    if (k.valid && k.S == S && same_spec(k.ps, ps)) return &k;
-    k.ps = ps;
-    k.S = S;
-    k.valid = true;
-    fresh = true;
-    return &k;
-  }
+// The entry of the engine's kept operands that belongs to the source `src` of
+// operand A (nullptr: not one of the kept sources).
+TcEngine::KeptPack* kept_of(TcEngine* tc, const double* src) {
+  for (int i = 0; i < 2; ++i)
+    if (src && tc->keep_src[i] == src) return &tc->kept[i];
   return nullptr;
+}
+
+// Whether a kept operand has to be packed now: (ps, lv) is not what it holds.
+// lv.S = 0: the split scheme.
+bool kept_stale(TcEngine::KeptPack* k, const PackSpec& ps, const OzLevel& lv) {
+  if (k->valid && k->S == lv.S && k->bits == lv.bits && k->guard == lv.guard && same_spec(k->ps, ps)) return false;
+  k->ps = ps;
+  k->S = lv.S;
+  k->bits = lv.bits;
+  k->guard = lv.guard;
+  k->valid = true;
+  return true;
 }
 
 // Tensor-core evaluation of C = alpha * A.B + beta * C (no batch index): by
@@ -800,28 +802,16 @@ bool run_tc(TcEngine* tc, bool optional, OzLevel lv, double alpha, const TView& 
     // exact-slice products: S digit slices of each operand, FP64 output
     const int S = lv.S;
     const int64_t Kpad = oz_kpad(K), W = S * Kpad;
-    if (!grow(tc->bufA, M * W) || !grow(tc->bufB, N * W) || !grow(tc->exA, M) || !grow(tc->exB, N)) return false;
+    TcEngine::KeptPack* ka = kept_of(tc, A.p);
+    auto& bufA = ka ? ka->buf : tc->bufA;
+    auto& exA = ka ? ka->ex : tc->exA;
+    if (ka && ((int64_t)bufA.n < M * W || (int64_t)exA.n < M)) ka->valid = false;
+    if (!grow(bufA, M * W) || !grow(tc->bufB, N * W) || !grow(exA, M) || !grow(tc->exB, N)) return false;
     PackSpec pa{M, K, W, gm[1].dim, gm[2].dim, gm[0].s[0], gm[1].s[0], gm[2].s[0],
                 gk[1].dim, gk[2].dim, gk[0].s[0], gk[1].s[0], gk[2].s[0], S, 0};
     PackSpec pb{N, K, W, gn[1].dim, gn[2].dim, gn[0].s[1], gn[1].s[1], gn[2].s[1],
                 gk[1].dim, gk[2].dim, gk[0].s[1], gk[1].s[1], gk[2].s[1], S, 0};
-    bool fresh;
-    TcEngine::KeptPack* ka = kept_a(tc, A.p, pa, 10 * lv.bits + S, fresh);
-    __nv_bfloat16* pA = tc->bufA.p;
-    int* eA = tc->exA.p;
-    if (ka) {
-      if (fresh) {
-        if (!grow(ka->buf, M * W) || !grow(ka->ex, M)) {
-          ka->valid = false;
-          return false;
-        }
-        pack_oz(A.p, pa, S, lv.bits, lv.guard, ka->buf.p, ka->ex.p, s);
-      }
-      pA = ka->buf.p;
-      eA = ka->ex.p;
-    } else {
-      pack_oz(A.p, pa, S, lv.bits, lv.guard, pA, eA, s);
-    }
+    if (!ka || kept_stale(ka, pa, lv)) pack_oz(A.p, pa, S, lv.bits, lv.guard, bufA.p, exA.p, s);
     pack_oz(B.p, pb, S, lv.bits, lv.guard, tc->bufB.p, tc->exB.p, s);
     EpiMap ep;
     ep.M = M; ep.N = N;
@@ -829,31 +819,22 @@ bool run_tc(TcEngine* tc, bool optional, OzLevel lv, double alpha, const TView& 
     ep.nd2 = gn[1].dim; ep.nd3 = gn[2].dim; ep.ns1 = gn[0].s[2]; ep.ns2 = gn[1].s[2]; ep.ns3 = gn[2].s[2];
     ep.alpha = alpha; ep.beta = beta; ep.C = C.p;
     ep.work = 2.0 * (double)M * (double)N * (double)K * oz_pairs(lv);
-    gemm_oz(pA, M, eA, tc->bufB.p, N, tc->exB.p, Kpad, lv, ep, tc->ozws, tc->err, s);
+    gemm_oz(bufA.p, M, exA.p, tc->bufB.p, N, tc->exB.p, Kpad, lv, ep, tc->ozws, tc->err, s);
     tc->tc_calls++;
     tc->tc_flops += ep.work;
     return true;
   }
   const SplitScheme sc = tc->scheme;
   const int64_t Kp = packed_kp(K, sc.P);
-  if ((int64_t)tc->bufA.n < M * Kp) tc->bufA.alloc(M * Kp);
-  if ((int64_t)tc->bufB.n < N * Kp) tc->bufB.alloc(N * Kp);
+  TcEngine::KeptPack* ka = kept_of(tc, A.p);
+  auto& bufA = ka ? ka->buf : tc->bufA;
+  if (ka && (int64_t)bufA.n < M * Kp) ka->valid = false;
+  if (!grow(bufA, M * Kp) || !grow(tc->bufB, N * Kp)) return false;
   PackSpec pa{M, K, Kp, gm[1].dim, gm[2].dim, gm[0].s[0], gm[1].s[0], gm[2].s[0],
               gk[1].dim, gk[2].dim, gk[0].s[0], gk[1].s[0], gk[2].s[0], sc.P, sc.code_a};
   PackSpec pb{N, K, Kp, gn[1].dim, gn[2].dim, gn[0].s[1], gn[1].s[1], gn[2].s[1],
               gk[1].dim, gk[2].dim, gk[0].s[1], gk[1].s[1], gk[2].s[1], sc.P, sc.code_b};
-  bool fresh;
-  TcEngine::KeptPack* ka = kept_a(tc, A.p, pa, 0, fresh);
-  __nv_bfloat16* pA = tc->bufA.p;
-  if (ka) {
-    if (fresh) {
-      if ((int64_t)ka->buf.n < M * Kp) ka->buf.alloc(M * Kp);
-      pack_split(A.p, pa, ka->buf.p, s);
-    }
-    pA = ka->buf.p;
-  } else {
-    pack_split(A.p, pa, pA, s);
-  }
+  if (!ka || kept_stale(ka, pa, lv)) pack_split(A.p, pa, bufA.p, s);
   pack_split(B.p, pb, tc->bufB.p, s);
   EpiMap ep;
   ep.M = M; ep.N = N;
@@ -863,7 +844,7 @@ bool run_tc(TcEngine* tc, bool optional, OzLevel lv, double alpha, const TView& 
   ep.work = 2.0 * (double)M * (double)N * (double)K * sc.P;
   ep.no_loads = tc->no_loads_once;
   tc->no_loads_once = 0;
-  gemm_bf16x3(pA, M, 0, tc->bufB.p, N, 0, Kp, ep, tc->err, s);
+  gemm_bf16x3(bufA.p, M, 0, tc->bufB.p, N, 0, Kp, ep, tc->err, s);
   tc->tc_calls++;
   tc->tc_flops += 2.0 * (double)M * (double)N * (double)K * sc.P;
   return true;
@@ -893,10 +874,12 @@ DBuf<double>*& f64_workspace() {
 }
 
 // bytes by which run_tc would grow the engine's buffers for a product
-static double pack_growth(const TcEngine* tc, const OzLevel& lv, int64_t M, int64_t N, int64_t K) {
+static double pack_growth(TcEngine* tc, const OzLevel& lv, const double* a, int64_t M, int64_t N, int64_t K) {
   const double w = (double)lv.S * (double)oz_kpad(K);
+  const TcEngine::KeptPack* ka = kept_of(tc, a);
+  const size_t na = ka ? ka->buf.n : tc->bufA.n, ne = ka ? ka->ex.n : tc->exA.n;
   auto more = [](double need, size_t have) { return std::max(0.0, need - (double)have); };
-  return 2.0 * (more(M * w, tc->bufA.n) + more(N * w, tc->bufB.n)) + 4.0 * (more(M, tc->exA.n) + more(N, tc->exB.n));
+  return 2.0 * (more(M * w, na) + more(N * w, tc->bufB.n)) + 4.0 * (more(M, ne) + more(N, tc->exB.n));
 }
 
 void einsum(double alpha, const char* spec, const TView& A, const TView& B, double beta, const TView& C,
@@ -943,7 +926,7 @@ void einsum(double alpha, const char* spec, const TView& A, const TView& B, doub
     std::vector<Ix> m3 = gm, n3 = gn, k3 = gk;
     if (flops >= tc->f64_min_flops && gdim(gm) > 1 && gdim(gn) > 1 && oz_takes(gdim(gm), gdim(gn), gdim(gk)) &&
         try_fuse(m3, 3) && try_fuse(n3, 3) && try_fuse(k3, 3) &&
-        tc->scratch_fits(pack_growth(tc, OZ_F64, gdim(gm), gdim(gn), gdim(gk))) &&
+        tc->scratch_fits(pack_growth(tc, OZ_F64, A.p, gdim(gm), gdim(gn), gdim(gk))) &&
         run_tc(tc, true, OZ_F64, alpha, A, B, beta, C, m3, n3, k3, s))
       return;
   }

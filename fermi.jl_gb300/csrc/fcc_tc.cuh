@@ -247,11 +247,11 @@ struct TcEngine {
   // Packed A operands kept across calls: an A operand whose source is one of
   // keep_src (set by a KeepPackedA scope, whose caller guarantees that those
   // sources do not change meanwhile) is packed into its own entry and packed
-  // again only when its layout or slice count changes, so an operand used by
+  // again only when its layout or level changes, so an operand used by
   // every block of a loop is packed once.
   struct KeptPack {
     PackSpec ps{};
-    int S = 0;
+    int S = 0, bits = 0, guard = 0;
     bool valid = false;
     DBuf<__nv_bfloat16> buf;
     DBuf<int> ex;

@@ -35,3 +35,24 @@ def test_contractions_keep_to_the_scratch_there_is():
         # both routes are at the level of one FP64 rounding of sums of a few thousand terms
         assert np.abs(r.T1 - ref.T1).max() < 1e-13 and np.abs(r.T2 - ref.T2).max() < 1e-13
         assert abs(r.correlation - ref.correlation) < 1e-12
+
+
+def test_kept_operands_count():
+    # the ladder's A operands are packed once and kept beside the other packed
+    # operands: limits all over the range, some of which only they exceed
+    from fermicc import Options, RCCSD, _lib
+    from fermicc.rccsd import Context
+    lib = _lib.load()
+    Options.reset()
+    Options.set("cc_max_iter", 1)
+    held, energies = [], []
+    for step in range(-1, 48):
+        ctx = Context(inputs(4))
+        limit = -1 if step < 0 else held[0] * step // 48
+        assert lib.fcc_test_set_scratch(ctx.h, limit) == 0
+        energies.append(RCCSD.compute(inputs(4), context=ctx).correlation)
+        held.append(lib.fcc_test_scratch_held(ctx.h))
+        ctx.close()
+        assert limit < 0 or held[-1] <= limit, (limit, held[-1])
+    Options.reset()
+    assert np.ptp(energies) < 1e-12
