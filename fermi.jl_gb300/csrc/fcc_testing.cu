@@ -43,6 +43,12 @@ extern "C" int fcc_test_set_t3_kc(fcc_ctx* c, int32_t kc) {
   return FCC_OK;
 }
 
+extern "C" int fcc_test_set_t3_form(fcc_ctx* c, int32_t form) {
+  if (!c || form < 0 || form > 3) return FCC_ERR_BAD_ARG;
+  c->t3_form = form;
+  return FCC_OK;
+}
+
 extern "C" int fcc_test_set_scratch(fcc_ctx* c, int64_t bytes) {
   if (!c) return FCC_ERR_BAD_ARG;
   c->tc.scratch_max = bytes < 0 ? 1e300 : (double)bytes;

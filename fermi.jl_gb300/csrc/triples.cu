@@ -202,18 +202,42 @@ double triples_fp64(fcc_ctx* c, const std::vector<int3>* subset, std::vector<dou
     DBuf<int> e;
     void alloc(int64_t rows, int64_t rowlen) { p.alloc(rows * rowlen); e.alloc(rows); }
   };
-  // rows of a packed operand from one on, and the same rows in FP64: three
-  // levels of strides and that of a product of a batch, in rows
-  struct Rows { const __nv_bfloat16* p; const int* e; int64_t n; const double* f; int64_t s1, s2, s3, sb; };
+  // Rows of F or H for a product: packed from one on (p, e, n of them), or in
+  // FP64, row (x, y, z) of segment q at p + x sx + y sy + z sz with K columns ks
+  // apart, times a.  The columns [d, l] are one segment, or two that read the
+  // integrals and amplitudes where they are; r gives the indices of a product's
+  // three row levels and of its batch as (x, y, z) = (0, 1, 2).
+  struct Seg { const double* p; int64_t sx, sy, sz, ks, K; double a; };
+  struct Rows { const __nv_bfloat16* p; const int* e; int64_t n; int64_t x, y, z; int r1, r2, r3, rb; };
   Packed pF, pF2, pHx, pHy, pFj;
-  auto rows = [&](const Packed& x, int64_t r0, const double* f, int64_t s1, int64_t s2, int64_t s3, int64_t sb) {
-    return Rows{x.p.p + r0 * rowlen, x.e.p + r0, (int64_t)x.e.n - r0, f, s1, s2, s3, sb};
+  auto rows = [&](const Packed& pk, int64_t r0, int64_t x, int64_t y, int64_t z, int r1, int r2, int r3, int rb) {
+    return Rows{pk.p.p + r0 * rowlen, pk.e.p + r0, (int64_t)pk.e.n - r0, x, y, z, r1, r2, r3, rb};
   };
+  // W for a run of i and of k: at most ~2 GB
+  const int64_t slots_max = std::max<int64_t>(1, (int64_t)(2ll << 30) / (8 * v3));
+  int64_t slots = 0;   // the largest run of any j
+  for (int64_t j = 0; j < o; ++j) slots = std::max(slots, (o - j) * (j + 1));
+  slots = subset ? 1 : std::min(slots, c->t3_kc_override > 0 ? (int64_t)c->t3_kc_override : slots_max);
+  const int64_t run = std::min(slots, o);
   // Small systems on the FP64 pipe: an exact-slice product takes 33 us however
   // short, a few us on the pipe while it has little to do (at (H2O)1 1.2 ms for
   // the 30 products, 0.2 on the pipe; at (H2O)2 the pipe would need 6 ms where
-  // the slices take 2).  The line is 0.2 ms of the pipe's time.
-  const bool pipe = (double)o * o * o * (double)v3 * Kc < 1e8;
+  // the slices take 2).  The line is 0.2 ms of the pipe's time.  Others too where
+  // the slices of H and of a run of F, beside F and W, leave too little memory:
+  // then without F and H, whose parts [d] and [l] are two products each.
+  bool small = (double)o * o * o * (double)v3 * Kc < 1e8, split = false;
+  size_t mfree = 0, mtotal = 0;
+  if (!small) {
+    FCC_CUDA(cudaMemGetInfo(&mfree, &mtotal));
+    const double slices = (2.0 * rowlen + 4.0) * (2.0 * RH + (double)(2 * run + 1) * v2);
+    split = slices > c->tc.scratch_max ||
+            slices + 8.0 * ((double)std::max(RF, RH) * Kc + (double)slots * v3) + 2e9 > (double)mfree;
+  }
+  if (c->t3_form) {
+    small = c->t3_form == 1;
+    split = c->t3_form == 3;
+  }
+  const bool pipe = small || split;
   auto pack = [&](const double* src, int64_t d1, int64_t d2, int64_t d3, int64_t s1, int64_t s2, int64_t s3, Packed& dst) {
     PackSpec ps{};
     ps.R = d1 * d2 * d3;
@@ -223,11 +247,18 @@ double triples_fp64(fcc_ctx* c, const std::vector<int3>* subset, std::vector<dou
     ps.kd2 = 1; ps.kd3 = Kc; ps.ks3 = 1;
     pack_oz(src, ps, lv.S, lv.bits, lv.guard, dst.p.p, dst.e.p, s);
   };
-  DBuf<double> H;
-  H.alloc(RH * Kc);
-  TView Hv = rm(H.p, {o, o, v, Kc});
-  einsum1(1.0, "xyzd->xyzd", t2v, 0.0, slice(Hv, 3, 0, v), s);
-  einsum(1.0, "Qly,Qxz->xyzl", Boo, Bov, 0.0, slice(Hv, 3, v, o), s);             // (ly|xz)
+  DBuf<double> H, F;
+  // with split: (xy|zd) [x][y][z][d] and (ly|xz) [l][y][x][z]
+  const int64_t Fk = split ? v : Kc;
+  if (split) {
+    H.alloc(o * o * o * v);
+    einsum(1.0, "Qly,Qxz->lyxz", Boo, Bov, 0.0, rm(H.p, {o, o, o, v}), s);
+  } else {
+    H.alloc(RH * Kc);
+    TView Hv = rm(H.p, {o, o, v, Kc});
+    einsum1(1.0, "xyzd->xyzd", t2v, 0.0, slice(Hv, 3, 0, v), s);
+    einsum(1.0, "Qly,Qxz->xyzl", Boo, Bov, 0.0, slice(Hv, 3, v, o), s);             // (ly|xz)
+  }
   if (!pipe) {
     pHx.alloc(RH, rowlen);
     pHy.alloc(RH, rowlen);
@@ -236,16 +267,22 @@ double triples_fp64(fcc_ctx* c, const std::vector<int3>* subset, std::vector<dou
     FCC_CUDA(cudaStreamSynchronize(s));
     H.release();
   }
-  DBuf<double> F;
-  F.alloc(RF * Kc);
-  TView Fv = rm(F.p, {o, v, v, Kc});
+  F.alloc(RF * Fk);
+  TView Fv = rm(F.p, {o, v, v, Fk});
   einsum(1.0, "Qia,Qbd->iabd", Bov, Bvv, 0.0, slice(Fv, 3, 0, v), s);             // (xy|zd)
-  einsum1(-1.0, "xlyz->xyzl", t2v, 0.0, slice(Fv, 3, v, o), s);
+  if (!split) einsum1(-1.0, "xlyz->xyzl", t2v, 0.0, slice(Fv, 3, v, o), s);
+  std::vector<Seg> segF, segH;
+  if (split) {
+    segF = {Seg{F.p, v3, v2, v, 1, v, 1.0}, Seg{c->t2.p, o * v2, v, 1, v2, o, -1.0}};
+    segH = {Seg{c->t2.p, o * v2, v2, v, 1, v, 1.0}, Seg{H.p, v, o * v, 1, o * o * v, o, 1.0}};
+  } else if (pipe) {
+    segF = {Seg{F.p, v2 * Kc, v * Kc, Kc, 1, Kc, 1.0}};
+    segH = {Seg{H.p, o * v * Kc, v * Kc, Kc, 1, Kc, 1.0}};
+  }
   // The slices of F take four times the memory of F, twice that of the FP64
   // array in either order.  Where they do not fit beside the rest, F stays in
   // FP64 and the rows of a run are packed for each pair of runs (hook: t3_kc).
-  size_t mfree = 0, mtotal = 0;
-  FCC_CUDA(cudaMemGetInfo(&mfree, &mtotal));
+  if (!pipe) FCC_CUDA(cudaMemGetInfo(&mfree, &mtotal));
   const bool whole = !pipe && c->t3_kc_override <= 0 && 4.0 * (double)RF * (double)rowlen + 6e9 < (double)mfree;
   if (whole) {
     pF.alloc(RF, rowlen);
@@ -255,14 +292,8 @@ double triples_fp64(fcc_ctx* c, const std::vector<int3>* subset, std::vector<dou
     FCC_CUDA(cudaStreamSynchronize(s));
     F.release();
   }
-  // W for a run of i and of k: at most ~2 GB
-  const int64_t slots_max = std::max<int64_t>(1, (int64_t)(2ll << 30) / (8 * v3));
-  int64_t slots = 0;   // the largest run of any j
-  for (int64_t j = 0; j < o; ++j) slots = std::max(slots, (o - j) * (j + 1));
-  slots = subset ? 1 : std::min(slots, c->t3_kc_override > 0 ? (int64_t)c->t3_kc_override : slots_max);
   c->Wt.alloc(slots * v3);
   if (!whole && !pipe) {
-    const int64_t run = std::min(slots, o);
     pF.alloc(run * v2, rowlen);
     pFj.alloc(v2, rowlen);
     pF2.alloc(run * v2, rowlen);
@@ -284,8 +315,8 @@ double triples_fp64(fcc_ctx* c, const std::vector<int3>* subset, std::vector<dou
   // One product: rows m of A (packed rows ar0..), columns n of B (br0..), each a
   // three-level index with the given strides in W
   struct Ix3 { int64_t d2, d3, s1, s2, s3; };
-  auto product = [&](Rows a, int64_t M, Ix3 m, Rows b, int64_t N, Ix3 nn, double beta, int64_t batch, int64_t ba,
-                     int64_t bb, int64_t bc) {
+  auto product = [&](bool a_is_f, Rows a, int64_t M, Ix3 m, Rows b, int64_t N, Ix3 nn, double beta, int64_t batch,
+                     int64_t ba, int64_t bb, int64_t bc) {
     EpiMap ep;
     ep.M = M; ep.N = N;
     ep.md2 = m.d2; ep.md3 = m.d3; ep.ms1 = m.s1; ep.ms2 = m.s2; ep.ms3 = m.s3;
@@ -294,16 +325,22 @@ double triples_fp64(fcc_ctx* c, const std::vector<int3>* subset, std::vector<dou
     ep.C = c->Wt.p;
     ep.batch = (int)batch; ep.ba = ba; ep.bb = bb; ep.bc = bc;
     if (pipe) {
-      CtrDesc d{};
-      d.M = M; d.M2 = m.d2; d.M3 = m.d3; d.N = N; d.N2 = nn.d2; d.N3 = nn.d3; d.K = d.K2 = Kc; d.batch = batch;
-      d.a_m1 = a.s1 * Kc; d.a_m2 = a.s2 * Kc; d.a_m3 = a.s3 * Kc; d.a_k2 = 1;
-      d.b_n1 = b.s1 * Kc; d.b_n2 = b.s2 * Kc; d.b_n3 = b.s3 * Kc; d.b_k2 = 1;
-      d.c_m1 = m.s1; d.c_m2 = m.s2; d.c_m3 = m.s3; d.c_n1 = nn.s1; d.c_n2 = nn.s2; d.c_n3 = nn.s3;
-      d.a_b = batch > 1 && ba ? a.sb * Kc : 0;
-      d.b_b = batch > 1 && bb ? b.sb * Kc : 0;
-      d.c_b = bc;
-      d.alpha = 1.0; d.beta = beta;
-      contract_f64_launch(a.f, b.f, c->Wt.p, d, s);
+      for (size_t q = 0; q < segF.size(); ++q) {
+        const Seg &sa = a_is_f ? segF[q] : segH[q], &sb = a_is_f ? segH[q] : segF[q];
+        auto at = [](const Seg& g, const Rows& r) { return g.p + r.x * g.sx + r.y * g.sy + r.z * g.sz; };
+        auto stride = [](const Seg& g, int r) { return r == 0 ? g.sx : (r == 1 ? g.sy : (r == 2 ? g.sz : 0)); };
+        CtrDesc d{};
+        d.M = M; d.M2 = m.d2; d.M3 = m.d3; d.N = N; d.N2 = nn.d2; d.N3 = nn.d3; d.K = d.K2 = sa.K; d.batch = batch;
+        d.a_m1 = stride(sa, a.r1); d.a_m2 = stride(sa, a.r2); d.a_m3 = stride(sa, a.r3); d.a_k2 = sa.ks;
+        d.b_n1 = stride(sb, b.r1); d.b_n2 = stride(sb, b.r2); d.b_n3 = stride(sb, b.r3); d.b_k2 = sb.ks;
+        d.c_m1 = m.s1; d.c_m2 = m.s2; d.c_m3 = m.s3; d.c_n1 = nn.s1; d.c_n2 = nn.s2; d.c_n3 = nn.s3;
+        d.a_b = batch > 1 && ba ? stride(sa, a.rb) : 0;
+        d.b_b = batch > 1 && bb ? stride(sb, b.rb) : 0;
+        d.c_b = bc;
+        d.alpha = sa.a * sb.a;
+        d.beta = q == 0 ? beta : 1.0;
+        contract_f64_launch(at(sa, a), at(sb, b), c->Wt.p, d, s);
+      }
       return;
     }
     ep.work = 2.0 * (double)batch * (double)M * (double)N * (double)Kc * oz_pairs(lv);
@@ -318,30 +355,29 @@ double triples_fp64(fcc_ctx* c, const std::vector<int3>* subset, std::vector<dou
       pack(F.p + k0 * v2 * Kc, nk, v, v, v2, 1, v, pF2);
     }
     // F[i] and F[j] by (x, y, z), F[k] by (x, z, y)
-    const double* Fp = F.p;
-    const double* Hp = H.p;
-    const Rows fi = rows(pF, whole ? i0 * v2 : 0, Fp + i0 * v2 * Kc, v2, v, 1, 0);
-    const Rows fj = rows(whole || pipe ? pF : pFj, whole ? j * v2 : 0, Fp + j * v2 * Kc, v2, v, 1, 0);
-    const Rows fk = rows(pF2, whole ? k0 * v2 : 0, Fp + k0 * v2 * Kc, v2, 1, v, 0);
-    auto h = [&](const Packed& ph, int64_t first, int64_t x, int64_t y, int64_t s2, int64_t sb) {
-      return rows(ph, first * v, Hp + (x * o + y) * v * Kc, 0, s2, 1, sb);
+    const Rows fi = rows(pF, whole ? i0 * v2 : 0, i0, 0, 0, 0, 1, 2, -1);
+    const Rows fj = rows(whole || pipe ? pF : pFj, whole ? j * v2 : 0, j, 0, 0, 0, 1, 2, -1);
+    const Rows fk = rows(pF2, whole ? k0 * v2 : 0, k0, 0, 0, 0, 2, 1, -1);
+    // H[x][y] over a run of x or of y (the second row level) and z
+    auto h = [&](const Packed& ph, int64_t first, int64_t x, int64_t y, int r2, int rb) {
+      return rows(ph, first * v, x, y, 0, -1, r2, 2, rb);
     };
-    const Rows hk = h(pHy, j * o + k0, k0, j, o * v, 0);         // H[k..][j]
-    const Rows hki = h(pHy, i0 * o + k0, k0, i0, o * v, v);      // H[k..][i]
-    const Rows hji = h(pHx, j * o + i0, j, i0, v, 0), hjk = h(pHx, j * o + k0, j, k0, v, 0);
-    const Rows hij = h(pHy, j * o + i0, i0, j, o * v, 0), hik = h(pHx, i0 * o + k0, i0, k0, v, o * v);
+    const Rows hk = h(pHy, j * o + k0, k0, j, 0, -1);          // H[k..][j]
+    const Rows hki = h(pHy, i0 * o + k0, k0, i0, 0, 1);        // H[k..][i]
+    const Rows hji = h(pHx, j * o + i0, j, i0, 1, -1), hjk = h(pHx, j * o + k0, j, k0, 1, -1);
+    const Rows hij = h(pHy, j * o + i0, i0, j, 0, -1), hik = h(pHx, i0 * o + k0, i0, k0, 1, 0);
     // F[i](a,b) H[k][j](c): rows (i,a,b), columns (k,c)
-    product(fi, ni * v2, {v, v, ws, v2, v}, hk, nk * v, {nk, v, 0, v3, 1}, 0.0, 1, 0, 0, 0);
+    product(true, fi, ni * v2, {v, v, ws, v2, v}, hk, nk * v, {nk, v, 0, v3, 1}, 0.0, 1, 0, 0, 0);
     // F[j](b,a) H[k][i](c): rows (b,a), columns (k,c), a product per i
-    product(fj, v2, {v, v, 0, v, v2}, hki, nk * v, {nk, v, 0, v3, 1}, 1.0, ni, 0, o * v, ws);
+    product(true, fj, v2, {v, v, 0, v, v2}, hki, nk * v, {nk, v, 0, v3, 1}, 1.0, ni, 0, o * v, ws);
     // H[j][i](b) F[k](c,a): rows (i,b), columns (k,a,c)
-    product(hji, ni * v, {ni, v, 0, ws, v}, fk, nk * v2, {v, v, v3, v2, 1}, 1.0, 1, 0, 0, 0);
+    product(false, hji, ni * v, {ni, v, 0, ws, v}, fk, nk * v2, {v, v, v3, v2, 1}, 1.0, 1, 0, 0, 0);
     // H[j][k](b) F[i](a,c): rows (k,b), columns (i,a,c)
-    product(hjk, nk * v, {nk, v, 0, v3, v}, fi, ni * v2, {v, v, ws, v2, 1}, 1.0, 1, 0, 0, 0);
+    product(false, hjk, nk * v, {nk, v, 0, v3, v}, fi, ni * v2, {v, v, ws, v2, 1}, 1.0, 1, 0, 0, 0);
     // H[i][j](a) F[k](c,b): rows (i,a), columns (k,b,c)
-    product(hij, ni * v, {ni, v, 0, ws, v2}, fk, nk * v2, {v, v, v3, v, 1}, 1.0, 1, 0, 0, 0);
+    product(false, hij, ni * v, {ni, v, 0, ws, v2}, fk, nk * v2, {v, v, v3, v, 1}, 1.0, 1, 0, 0, 0);
     // H[i][k](a) F[j](b,c): rows (k,a), columns (b,c), a product per i
-    product(hik, nk * v, {nk, v, 0, v3, v2}, fj, v2, {v, v, 0, v, 1}, 1.0, ni, o * v, 0, ws);
+    product(false, hik, nk * v, {nk, v, 0, v3, v2}, fj, v2, {v, v, 0, v, 1}, 1.0, ni, o * v, 0, ws);
   };
   auto energy = [&](int64_t i0, int64_t ni, int64_t j, int64_t k0, int64_t nk) {
     const int pe = prof_begin(s);

@@ -59,6 +59,11 @@ int fcc_test_set_t3_bn(fcc_ctx* ctx, int32_t bn);
  * number the FP64 form also packs its operands run by run. */
 int fcc_test_set_t3_kc(fcc_ctx* ctx, int32_t kc);
 
+/* Form of the FP64 (T) whatever the size: 1 contractions on the FP64 pipe, 2
+ * exact-slice products, 3 contractions on the pipe that read the integrals and
+ * amplitudes where they are (the form for little memory); 0 chosen by size. */
+int fcc_test_set_t3_form(fcc_ctx* ctx, int32_t form);
+
 /* The most bytes of packed operands that the FP64 contractions of ctx may hold
  * (negative: no such limit, as by default); those that need more run on the
  * FP64 pipe, as they do where memory is short.  fcc_test_scratch_held: the bytes

@@ -56,3 +56,60 @@ def test_kept_operands_count():
         assert limit < 0 or held[-1] <= limit, (limit, held[-1])
     Options.reset()
     assert np.ptp(energies) < 1e-12
+
+
+@pytest.mark.parametrize("waters", [1, 2])
+def test_triples_forms_agree(waters):
+    # the contractions of the joined operands, their slices (whole and by runs) and
+    # the contractions that read the operands where they are, on one system; (T) is
+    # a sum of about 1e5 to 1e7 terms with cancellations of a decade
+    import ctypes
+    from fermicc import Options, RCCSD, _lib
+    from fermicc.rccsd import Context
+    inp = inputs(waters)
+    lib = _lib.load()
+    Options.reset()
+    Options.set("cc_max_iter", 2)
+    ctx = Context(inp)
+    RCCSD.compute(inp, context=ctx)
+    ijk = np.array([(i, j, k) for i in range(inp.o) for j in range(i + 1) for k in range(j + 1) if not i == j == k][:7], np.int32)
+    whole, each = {}, {}
+    for form, kc in ((1, 0), (1, 3), (2, 0), (2, 3), (3, 0), (3, 3)):
+        assert lib.fcc_test_set_t3_form(ctx.h, form) == 0 and lib.fcc_test_set_t3_kc(ctx.h, kc) == 0
+        n0 = lib.fcc_stat_launches()
+        whole[form, kc] = ctx.triples(_lib.FCC_PREC_FP64)
+        e = np.zeros(len(ijk))
+        assert lib.fcc_test_triples_subset(ctx.h, ijk.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)), len(ijk),
+                                           e.ctypes.data_as(ctypes.POINTER(ctypes.c_double))) == 0
+        each[form, kc] = e
+        assert lib.fcc_stat_launches() > n0
+    # without a hook a system that may hold no slices takes the third form
+    assert lib.fcc_test_set_t3_form(ctx.h, 0) == 0 and lib.fcc_test_set_t3_kc(ctx.h, 0) == 0
+    assert lib.fcc_test_set_scratch(ctx.h, 0) == 0
+    whole["limit"] = ctx.triples(_lib.FCC_PREC_FP64)
+    ctx.close()
+    Options.reset()
+    ref = whole[2, 0]
+    assert all(abs(w - ref) < 1e-12 * abs(ref) for w in whole.values()), whole
+    assert all(np.abs(e - each[2, 0]).max() < 1e-12 * abs(ref) for e in each.values()), each
+
+
+def test_a_triples_without_room_for_slices_takes_none():
+    from fermicc import Options, RCCSD, _lib
+    from fermicc.rccsd import Context
+    inp = inputs(2)
+    lib = _lib.load()
+    Options.reset()
+    Options.set("cc_max_iter", 1)
+    ctx = Context(inp)
+    assert lib.fcc_test_set_scratch(ctx.h, 0) == 0
+    RCCSD.compute(inp, context=ctx)
+    prof = np.zeros(24)
+    import ctypes
+    lib.fcc_prof_enable(1)
+    ctx.triples(_lib.FCC_PREC_FP64)
+    lib.fcc_prof_enable(0)
+    assert lib.fcc_prof_read(prof.ctypes.data_as(ctypes.POINTER(ctypes.c_double)), 6) == 0
+    ctx.close()
+    Options.reset()
+    assert prof[4 * 5] == 0 and prof[4 * 2] == 0 and prof[4 * 0] > 0   # no exact-slice product, no packing
