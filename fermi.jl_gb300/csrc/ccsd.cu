@@ -828,6 +828,7 @@ void residual(fcc_ctx* c) {
             ((int64_t)tc->bvvA.n >= need || tc->bvvA.try_alloc(need)) &&
             ((int64_t)tc->bvvEx.n >= R || tc->bvvEx.try_alloc(R));
     }
+    ScratchInUse in_use(tc);
     int64_t Wk = 0;   // packed row length
     if (tcw) {
       PackSpec ps{};

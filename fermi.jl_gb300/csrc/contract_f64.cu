@@ -792,6 +792,7 @@ bool run_tc(TcEngine* tc, bool optional, OzLevel lv, double alpha, const TView& 
   order(gk, 0);
   pad3(gm); pad3(gn); pad3(gk);
   const int64_t M = gdim(gm), N = gdim(gn), K = gdim(gk);
+  ScratchInUse in_use(tc);
   auto grow = [&](auto& buf, int64_t n) {
     if ((int64_t)buf.n >= n) return true;
     if (optional) return buf.try_alloc(n);
@@ -857,6 +858,24 @@ bool TcEngine::scratch_fits(double growth) const {
   if (scratch_held() + growth > scratch_max) return false;
   size_t f = 0, t = 0;
   return cudaMemGetInfo(&f, &t) == cudaSuccess && growth <= 0.5 * (double)f;
+}
+
+void TcEngine::release_scratch() {
+  for (auto* b : {&bufA, &bufB, &bvvA, &bvvB}) b->release();
+  for (auto* b : {&exA, &exB, &bvvEx}) b->release();
+  ozws.release();
+  for (KeptPack& k : kept) {
+    k.valid = false;
+    k.buf.release();
+    k.ex.release();
+  }
+}
+
+bool reclaim_scratch() {
+  TcEngine* tc = tc_engine();
+  if (!tc || tc->busy || tc->scratch_held() + (double)tc->ozws.bytes() == 0) return false;
+  tc->release_scratch();
+  return true;
 }
 
 static std::atomic<int64_t> g_launches{0};

@@ -23,6 +23,7 @@ int guarded(fcc_ctx* c, F&& f) {
       if (e != cudaSuccess) { c->last_error = cudaGetErrorString(e); return FCC_ERR_CUDA; }
     }
     fcc::WorkspaceScope ws(c ? &c->f64ws : nullptr);
+    fcc::ScratchBound bound(c ? &c->tc : nullptr);
     fcc::TcScope tc(c ? &c->tc : nullptr);   // large FP64 contractions run on the tensor cores
     if (c) c->tc.enabled = false;
     return f();
@@ -179,7 +180,12 @@ int fcc_create(fcc_ctx** out, int32_t o, int32_t v, int32_t naux, int32_t device
     fcc::reset_device_error(c);
     return FCC_OK;
   });
-  if (rc != FCC_OK) { delete c; return rc; }
+  if (rc != FCC_OK) {
+    cudaStream_t s = c->stream;
+    delete c;
+    if (s) cudaStreamDestroy(s);
+    return rc;
+  }
   *out = c;
   return FCC_OK;
 }

@@ -58,6 +58,10 @@ enum { PROF_F64 = 0, PROF_TC = 1, PROF_PACK = 2, PROF_UPDATE = 3, PROF_TRIPLES =
 int prof_begin(cudaStream_t s);
 void prof_end(cudaStream_t s, int idx, int cls, double work);
 
+// Gives back the scratch of the engine that this thread's call uses, if there is
+// any and nothing is using it (contract_f64.cu).
+bool reclaim_scratch();
+
 // Device buffer owned by a context.
 template <class T>
 struct DBuf {
@@ -73,10 +77,8 @@ struct DBuf {
   }
   ~DBuf() { release(); }
   void alloc(size_t count) {
-    release();
-    if (count == 0) return;
-    FCC_CUDA(cudaMalloc(&p, count * sizeof(T)));
-    n = count;
+    if (!try_alloc(count) && !(reclaim_scratch() && try_alloc(count)))
+      fail(FCC_ERR_OOM, "cudaMalloc of " + std::to_string(count * sizeof(T)) + " bytes: out of memory");
   }
   // the same for memory that can be done without: false (and empty) where there is too little
   bool try_alloc(size_t count) {

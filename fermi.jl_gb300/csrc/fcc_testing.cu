@@ -55,6 +55,20 @@ extern "C" int fcc_test_set_scratch(fcc_ctx* c, int64_t bytes) {
   return FCC_OK;
 }
 
+extern "C" int fcc_test_set_scratch_keep(fcc_ctx* c, int64_t bytes) {
+  if (!c) return FCC_ERR_BAD_ARG;
+  c->tc.scratch_keep = bytes < 0 ? fcc::TcEngine::KEEP : (double)bytes;
+  return FCC_OK;
+}
+
+extern "C" int fcc_test_reclaim(fcc_ctx* c, int32_t in_use) {
+  if (!c) return FCC_ERR_BAD_ARG;
+  fcc::TcScope scope(&c->tc);
+  if (!in_use) return fcc::reclaim_scratch() ? 1 : 0;
+  fcc::ScratchInUse hold(&c->tc);
+  return fcc::reclaim_scratch() ? 1 : 0;
+}
+
 extern "C" int64_t fcc_test_scratch_held(const fcc_ctx* c) { return c ? (int64_t)c->tc.scratch_held() : -1; }
 
 extern "C" int64_t fcc_test_products(const fcc_ctx* c) { return c ? c->tc.tc_calls : -1; }

@@ -101,6 +101,7 @@ int guarded(fcc_scf* s, Fn&& f) {
       cudaError_t e = cudaSetDevice(s->device);
       if (e != cudaSuccess) { s->last_error = cudaGetErrorString(e); return FCC_ERR_CUDA; }
     }
+    fcc::ScratchBound bound(s ? &s->tc : nullptr);
     fcc::TcScope tc(s ? &s->tc : nullptr);   // every contraction here is FP64
     fcc::WorkspaceScope ws(s ? &s->f64ws : nullptr);
     return f();

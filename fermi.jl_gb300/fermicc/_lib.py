@@ -41,7 +41,7 @@ EXPORTS = ("fcc_default_opts", "fcc_create", "fcc_upload_df", "fcc_upload_conv",
 TEST_EXPORTS = ("fcc_test_contract", "fcc_stat_launches", "fcc_stream", "fcc_prof_enable", "fcc_prof_read",
                 "fcc_test_set_t3_bn", "fcc_test_split3", "fcc_test_pack_oz", "fcc_test_inject",
                 "fcc_test_triples_subset", "fcc_test_set_t3_kc", "fcc_test_set_scratch", "fcc_test_scratch_held",
-                "fcc_test_products", "fcc_test_set_t3_form")
+                "fcc_test_products", "fcc_test_set_t3_form", "fcc_test_set_scratch_keep", "fcc_test_reclaim")
 
 
 class FccOpts(ctypes.Structure):
@@ -141,6 +141,10 @@ def load():
     lib.fcc_test_set_t3_form.restype = ctypes.c_int
     lib.fcc_test_set_scratch.argtypes = [vp, i64]
     lib.fcc_test_set_scratch.restype = ctypes.c_int
+    lib.fcc_test_set_scratch_keep.argtypes = [vp, i64]
+    lib.fcc_test_set_scratch_keep.restype = ctypes.c_int
+    lib.fcc_test_reclaim.argtypes = [vp, i32]
+    lib.fcc_test_reclaim.restype = ctypes.c_int
     lib.fcc_test_scratch_held.argtypes = [vp]
     lib.fcc_test_scratch_held.restype = i64
     lib.fcc_test_products.argtypes = [vp]

@@ -69,6 +69,12 @@ int fcc_test_set_t3_form(fcc_ctx* ctx, int32_t form);
  * FP64 pipe, as they do where memory is short.  fcc_test_scratch_held: the bytes
  * held now.  fcc_test_products: contractions run on the tensor cores so far. */
 int fcc_test_set_scratch(fcc_ctx* ctx, int64_t bytes);
+
+/* The bytes that a call may leave held for the next one (negative: the default,
+ * 4 GB), and what an allocation that finds no memory does: 1 if the held bytes
+ * were given back, 0 if there are none or (in_use) a product is using them. */
+int fcc_test_set_scratch_keep(fcc_ctx* ctx, int64_t bytes);
+int fcc_test_reclaim(fcc_ctx* ctx, int32_t in_use);
 int64_t fcc_test_scratch_held(const fcc_ctx* ctx);
 int64_t fcc_test_products(const fcc_ctx* ctx);
 

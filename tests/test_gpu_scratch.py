@@ -113,3 +113,33 @@ def test_a_triples_without_room_for_slices_takes_none():
     ctx.close()
     Options.reset()
     assert prof[4 * 5] == 0 and prof[4 * 2] == 0 and prof[4 * 0] > 0   # no exact-slice product, no packing
+
+
+@pytest.mark.parametrize("precision", ["fp64", "exact", "mixed"])
+def test_what_a_call_leaves_is_bounded_and_given_back(precision):
+    from fermicc import Options, RCCSD, _lib
+    from fermicc.rccsd import Context
+    inp = inputs(4)
+    lib = _lib.load()
+    Options.reset()
+    Options.set("cc_max_iter", 2)
+    Options.set("cc_gpu_precision", precision)
+    ctx = Context(inp)
+
+    def steps():
+        assert lib.fcc_set_guess(ctx.h, None, None) == 0
+        return RCCSD.compute(inp, context=ctx).correlation, lib.fcc_test_scratch_held(ctx.h)
+    e, held = steps()
+    assert held > 0
+    # an allocation that finds no memory gets it, but not from under a product
+    assert lib.fcc_test_reclaim(ctx.h, 1) == 0 and lib.fcc_test_scratch_held(ctx.h) == held
+    assert lib.fcc_test_reclaim(ctx.h, 0) == 1 and lib.fcc_test_scratch_held(ctx.h) == 0
+    assert lib.fcc_test_reclaim(ctx.h, 0) == 0
+    for keep in (0, held - 1, held):
+        assert lib.fcc_test_set_scratch_keep(ctx.h, keep) == 0
+        for _ in range(2):
+            e2, now = steps()
+            assert now <= keep and abs(e2 - e) < 1e-10
+    assert lib.fcc_test_set_scratch_keep(ctx.h, -1) == 0
+    ctx.close()
+    Options.reset()
