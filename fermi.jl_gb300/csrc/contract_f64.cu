@@ -820,6 +820,8 @@ bool run_tc(TcEngine* tc, bool optional, OzLevel lv, double alpha, const TView& 
     ep.nd2 = gn[1].dim; ep.nd3 = gn[2].dim; ep.ns1 = gn[0].s[2]; ep.ns2 = gn[1].s[2]; ep.ns3 = gn[2].s[2];
     ep.alpha = alpha; ep.beta = beta; ep.C = C.p;
     ep.work = 2.0 * (double)M * (double)N * (double)K * oz_pairs(lv);
+    ep.no_loads = tc->no_loads_once;
+    tc->no_loads_once = 0;
     gemm_oz(bufA.p, M, exA.p, tc->bufB.p, N, tc->exB.p, Kpad, lv, ep, tc->ozws, tc->err, s);
     tc->tc_calls++;
     tc->tc_flops += ep.work;

@@ -24,6 +24,7 @@ struct T3Params {
   int bn;      // B tile width: 128, 160, 192 or 256 (t3_bn(v) unless set for a test)
   float* G;    // G[g][k - k0] FP32 in 8 x 8 x 8 sub-cubes (t3_cube, t3_pos)
   int* err;    // set to 1 if a bounded wait gave up
+  int no_loads;   // test hook: no TMA loads, so the bounded waits give up
 };
 
 // Layout of one G_g[k] slab over (pair first index x, pair second index y,

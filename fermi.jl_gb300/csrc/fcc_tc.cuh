@@ -243,7 +243,7 @@ struct TcEngine {
   bool f64_sym = false;   // and the next ones' results are symmetric in (m, n)
   DBuf<__nv_bfloat16> bufA, bufB;
   int* err = nullptr;
-  int no_loads_once = 0;   // test hook: the next split-BF16 GEMM runs with EpiMap::no_loads
+  int no_loads_once = 0;   // test hook: the next tensor-core GEMM runs with EpiMap::no_loads
   // Packed A operands kept across calls: an A operand whose source is one of
   // keep_src (set by a KeepPackedA scope, whose caller guarantees that those
   // sources do not change meanwhile) is packed into its own entry and packed

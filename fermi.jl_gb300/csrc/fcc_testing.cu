@@ -74,7 +74,7 @@ extern "C" int64_t fcc_test_scratch_held(const fcc_ctx* c) { return c ? (int64_t
 extern "C" int64_t fcc_test_products(const fcc_ctx* c) { return c ? c->tc.tc_calls : -1; }
 
 extern "C" int fcc_test_inject(fcc_ctx* c, int32_t kind) {
-  if (!c || !(kind == 0 || kind == FCC_TEST_FAULT_NO_LOADS || kind == FCC_TEST_FAULT_NAN)) return FCC_ERR_BAD_ARG;
+  if (!c || kind < 0 || kind > FCC_TEST_FAULT_NO_LOADS_ENERGY) return FCC_ERR_BAD_ARG;
   c->test_fault = kind;
   return FCC_OK;
 }
@@ -126,6 +126,11 @@ extern "C" int fcc_test_contract(int32_t precision, const char* spec, const doub
     FCC_CUDA(cudaMemcpyAsync(dB.p, B, nb * 8, cudaMemcpyHostToDevice, s));
     FCC_CUDA(cudaMemcpyAsync(dC.p, C, nc * 8, cudaMemcpyHostToDevice, s));
     fcc::TcEngine eng;
+    // 30, 31: the exact-slice kernel at 9 groups and at the FP64 level without loads
+    if (precision == 30 || precision == 31) {
+      eng.no_loads_once = 1;
+      precision = precision == 30 ? 19 : 20;
+    }
     const bool fp64 = precision == FCC_PREC_FP64 || precision == 20 || precision == 21;
     eng.enabled = !fp64;
     if (precision == 20) eng.f64_min_flops = 0.0;

@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       int s = 0;                   // ring slot of the chain's first tile, and its phase
       uint32_t ph = 0;
       uint32_t issued = 0, parity = 0;   // slots loaded by this thread, phase parity of the last load of each
-      bool stop = false;
+      bool stop = ep.no_loads != 0;
       for (uint32_t u = wid; u < P.units && !stop; u += nwork) {
         uint32_t mt, nt;
         grouped_tile(u % tiles, P.tm, P.tn, mt, nt);

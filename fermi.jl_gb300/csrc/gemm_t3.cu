@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(T3_THREADS, 1) gemm_t3_kernel(const __grid_con
    if (elect_one()) {
     // ---------------- TMA producer over the tiles' K segments
     int it = 0;
-    bool stop = false;
+    bool stop = P.no_loads != 0;
     for (int t = wid; t < ntiles && !stop; t += nwork) {
       const T3Tile tl = t3_tile(t, tm, tn, P.nk);
       const int kk = P.k0 + tl.kq;

@@ -28,6 +28,8 @@ FCC_FINISH_EXACT = 0
 FCC_FINISH_FP64 = 1
 FCC_TEST_FAULT_NO_LOADS = 1
 FCC_TEST_FAULT_NAN = 2
+FCC_TEST_FAULT_NO_LOADS_T3 = 3
+FCC_TEST_FAULT_NO_LOADS_ENERGY = 4
 
 # every symbol include/fermicc.h declares, and the test hooks of include/fermicc_testing.h
 EXPORTS = ("fcc_default_opts", "fcc_create", "fcc_upload_df", "fcc_upload_conv", "fcc_set_guess",

@@ -22,7 +22,9 @@ extern "C" {
  * 2 the six-product one, 3 the exact-slice (Ozaki) kernel with 8 weight
  * groups and 10 + G the exact-slice kernel with G groups (2 <= G <= 9),
  * 20 the exact-slice kernel at the FP64 level whatever the size and 21 the
- * FP64 pipe whatever the size (error if the contraction cannot be expressed for it).  Returns an fcc
+ * FP64 pipe whatever the size (error if the contraction cannot be expressed for it);
+ * 30 and 31 are 19 and 20 without loads, whose bounded waits give up
+ * (FCC_ERR_TIMEOUT).  Returns an fcc
  * status code. */
 int fcc_test_contract(int32_t precision, const char* spec, const double* A, const int64_t* adims, int32_t arank,
                       const double* B, const int64_t* bdims, int32_t brank, double* C, const int64_t* cdims,
@@ -84,9 +86,13 @@ int64_t fcc_test_products(const fcc_ctx* ctx);
  * thread's bounded mbarrier wait (2 s) gives up with nothing in flight, the
  * kernel frees its TMEM and returns, and the run reports FCC_ERR_TIMEOUT.
  * FCC_TEST_FAULT_NAN: a NaN is written into the doubles residual of the next
- * iteration before the device update, which then reports FCC_ERR_NAN. */
+ * iteration before the device update, which then reports FCC_ERR_NAN.
+ * FCC_TEST_FAULT_NO_LOADS_T3 and _ENERGY: the first grouped GEMM, or the first
+ * energy launch, of the next mixed fcc_triples issues no loads, likewise. */
 #define FCC_TEST_FAULT_NO_LOADS 1
 #define FCC_TEST_FAULT_NAN 2
+#define FCC_TEST_FAULT_NO_LOADS_T3 3
+#define FCC_TEST_FAULT_NO_LOADS_ENERGY 4
 int fcc_test_inject(fcc_ctx* ctx, int32_t kind);
 
 /* FP64 (T) energy contributions of n single triplets ijk[3q..3q+2] = (i, j, k)
