@@ -19,6 +19,7 @@
 
 #include "../../include/fermicc_testing.h"
 #include "fcc_ctx.cuh"
+#include "fcc_quotient.cuh"
 
 namespace fcc {
 
@@ -134,22 +135,6 @@ struct ErrSlots {
 // division, and the stored errors are widened by integer arithmetic: 0.7 ms at
 // (H2O)8, 0.90 with divisions.  The order of the sums, and the dot of the error
 // with itself as a pass of its own, are kept: they enter the DIIS coefficients.
-// a float as a double, exactly, without the FP64 pipe (subnormals become 0)
-__device__ __forceinline__ double widen(float f) {
-  const uint32_t b = __float_as_uint(f);
-  const uint32_t hi = ((b & 0x7FFFFFFFu) >> 3) + (896u << 20);
-  if ((b & 0x7F800000u) == 0u) return 0.0;
-  if ((b & 0x7F800000u) == 0x7F800000u) return (double)f;
-  return __hiloint2double((int)(hi | (b & 0x80000000u)), (int)(b << 29));
-}
-__device__ __forceinline__ double quotient(double r, double D) {
-  // |D| is an orbital-energy difference: far inside the single-precision range
-  double y = widen(__frcp_rn((float)D));
-  y = fma(y, fma(-D, y, 1.0), y);        // 2^-24 -> 2^-47
-  y = fma(y, fma(-D, y, 1.0), y);        // the reciprocal, rounded
-  const double q = r * y;
-  return fma(y, fma(-D, q, r), q);       // remainder in full precision
-}
 __device__ __forceinline__ void update_one(int64_t e, double t, double r, double D, double t1ab, bool energy, double lt,
                                            float* err_s, double* err_d, const ErrSlots& others, double& tn,
                                            double (&vals)[NPART]) {

@@ -3,6 +3,7 @@
 
 #include "../../include/fermicc_testing.h"
 #include "fcc_ctx.cuh"
+#include "fcc_quotient.cuh"
 
 static cudaStream_t fcc_stream_of(const fcc_ctx* c) { return c->stream; }
 
@@ -15,6 +16,11 @@ fcc::TView view_of(double* p, const int64_t* dims, int rank) {
   int64_t s = 1;
   for (int k = rank - 1; k >= 0; --k) { t.dim[k] = dims[k]; t.str[k] = s; s *= dims[k]; }
   return t;
+}
+
+__global__ void quotient_kernel(const double* x, const double* d, int64_t n, bool f32, double* out) {
+  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x)
+    out[e] = f32 ? (double)fcc::quotient_f((float)x[e], (float)d[e]) : fcc::quotient(x[e], d[e]);
 }
 
 int64_t count(const int64_t* dims, int rank) {
@@ -192,6 +198,29 @@ extern "C" int fcc_test_split3(const double* x, int64_t R, int64_t K, int32_t ro
     fcc::pack_split(dx.p, ps, dy.p, s);
     FCC_CUDA(cudaMemcpyAsync(out, dy.p, sizeof(uint16_t) * R * 3 * K, cudaMemcpyDeviceToHost, s));
     FCC_CUDA(cudaStreamSynchronize(s));
+    return FCC_OK;
+  } catch (const fcc::Error& e) {
+    return e.code;
+  } catch (...) {
+    return FCC_ERR_CUDA;
+  }
+}
+
+extern "C" int fcc_test_quotient(const double* x, const double* d, int64_t n, int32_t f32, double* out) {
+  try {
+    if (!x || !d || !out || n < 1) return FCC_ERR_BAD_ARG;
+    int ndev = 0;
+    if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev < 1) return FCC_ERR_NO_DEVICE;
+    FCC_CUDA(cudaSetDevice(0));
+    fcc::DBuf<double> dx, dd, dy;
+    dx.alloc(n);
+    dd.alloc(n);
+    dy.alloc(n);
+    FCC_CUDA(cudaMemcpy(dx.p, x, sizeof(double) * n, cudaMemcpyHostToDevice));
+    FCC_CUDA(cudaMemcpy(dd.p, d, sizeof(double) * n, cudaMemcpyHostToDevice));
+    quotient_kernel<<<152, 256>>>(dx.p, dd.p, n, f32 != 0, dy.p);
+    FCC_CHECK_LAUNCH();
+    FCC_CUDA(cudaMemcpy(out, dy.p, sizeof(double) * n, cudaMemcpyDeviceToHost));
     return FCC_OK;
   } catch (const fcc::Error& e) {
     return e.code;

@@ -43,7 +43,7 @@ EXPORTS = ("fcc_default_opts", "fcc_create", "fcc_upload_df", "fcc_upload_conv",
 TEST_EXPORTS = ("fcc_test_contract", "fcc_stat_launches", "fcc_stream", "fcc_prof_enable", "fcc_prof_read",
                 "fcc_test_set_t3_bn", "fcc_test_split3", "fcc_test_pack_oz", "fcc_test_inject",
                 "fcc_test_triples_subset", "fcc_test_set_t3_kc", "fcc_test_set_scratch", "fcc_test_scratch_held",
-                "fcc_test_products", "fcc_test_set_t3_form", "fcc_test_set_scratch_keep", "fcc_test_reclaim")
+                "fcc_test_products", "fcc_test_set_t3_form", "fcc_test_set_scratch_keep", "fcc_test_reclaim", "fcc_test_quotient")
 
 
 class FccOpts(ctypes.Structure):
@@ -139,6 +139,8 @@ def load():
     lib.fcc_test_pack_oz.restype = ctypes.c_int
     lib.fcc_test_set_t3_kc.argtypes = [vp, i32]
     lib.fcc_test_set_t3_kc.restype = ctypes.c_int
+    lib.fcc_test_quotient.argtypes = [dp, dp, i64, i32, dp]
+    lib.fcc_test_quotient.restype = ctypes.c_int
     lib.fcc_test_set_t3_form.argtypes = [vp, i32]
     lib.fcc_test_set_t3_form.restype = ctypes.c_int
     lib.fcc_test_set_scratch.argtypes = [vp, i64]

@@ -48,6 +48,10 @@ int fcc_test_pack_oz(const double* x, int64_t R, int64_t K, int32_t row_fastest,
 /* Number of kernels this library has launched in the process so far. */
 int64_t fcc_stat_launches(void);
 
+/* out[q] = x[q] / d[q] on device 0 as the amplitude update (f32 = 0) and the mixed
+ * (T) energy (f32 != 0, x and d rounded to single) form it. */
+int fcc_test_quotient(const double* x, const double* d, int64_t n, int32_t f32, double* out);
+
 /* The CUDA stream (cudaStream_t) every call on ctx runs on, so a caller can
  * bracket library work with its own events. */
 void* fcc_stream(const fcc_ctx* ctx);
