@@ -207,3 +207,40 @@ def test_triples_small_and_sliced_forms_agree():
     ctx.close()
     Options.reset()
     assert abs(each.sum() - whole) < 1e-12 * abs(whole), (each.sum(), whole)
+
+
+# the longest sums of an (H2O)8 iteration: the ladder's (columns c <= d) and the
+# singles' (Q, d)
+@pytest.mark.parametrize("M,N,K", [(130, 20, 11628), (40, 24, 102144)])
+@pytest.mark.parametrize("spread", [0.0, 8.0])
+def test_no_less_accurate_than_the_fp64_pipe_over_long_sums(M, N, K, spread):
+    rng = np.random.default_rng(M + K)
+    A = rng.standard_normal((M, K)) * 10.0 ** rng.uniform(-spread, 0, (M, K))
+    B = rng.standard_normal((N, K)) * 10.0 ** rng.uniform(-spread, 0, (N, K))
+    ref = _quad(A, B)
+    err = {}
+    for prec in (TC, PIPE):
+        rc, out = _run(prec, "mk,nk->mn", A, B, np.zeros((M, N)))
+        assert rc == 0
+        err[prec] = np.linalg.norm(out - ref) / np.linalg.norm(ref)
+    assert err[TC] <= max(err[PIPE], 2.0 ** -53), err
+
+
+# Elements of rows that span decades.  An operand is cut 2^-62 below its row's
+# scale (up to twice the maximum), and pairs of weight 2^-76 of the scales are
+# dropped, seven of 2^14 at most per term: 2^-56 K of the product of the maxima at
+# most, whatever an element's own terms are.  (An FP64 product is within K 2^-53 of
+# the sum of an element's own |a| |b|: nearer where that sum is below 2^-3 of the
+# product of the maxima, as here.)
+@pytest.mark.parametrize("M,N,K", [(300, 257, 64), (200, 300, 700), (130, 40, 5000)])
+def test_elements_of_wide_rows(M, N, K):
+    rng = np.random.default_rng(K)
+    A = rng.standard_normal((M, K)) * 10.0 ** rng.uniform(-12, 0, (M, K))
+    B = rng.standard_normal((N, K)) * 10.0 ** rng.uniform(-12, 0, (N, K))
+    A[:, 0], B[:, 0] = 1.0, 0.0        # the row maxima do not meet
+    A[:, 1], B[:, 1] = 0.0, 1.0
+    rc, out = _run(TC, "mk,nk->mn", A, B, np.zeros((M, N)))
+    assert rc == 0
+    ref = _quad(A, B)
+    scale = np.abs(A).max(1)[:, None] * np.abs(B).max(1)[None, :]
+    assert np.all(np.abs(out - ref) <= K * 2.0 ** -56 * scale + 2.0 ** -53 * np.abs(ref))
