@@ -313,8 +313,9 @@ __global__ void __launch_bounds__(32 * SM_WARPS) contract_f64_small_kernel(const
   // z: K range of a partial product, or (batch, block of the cluster)
   const uint32_t zb = partial ? 0 : blockIdx.z / (uint32_t)cl;
   const int zk = partial ? (int)blockIdx.z : (int)(blockIdx.z - zb * (uint32_t)cl);
-  const int kbeg = zk * k_chunk;
-  const int kend = min((int)d.K, kbeg + k_chunk);
+  // unsigned: K is below 2^31, a loop's last step may not be
+  const uint32_t kbeg = (uint32_t)zk * (uint32_t)k_chunk;
+  const uint32_t kend = min((uint32_t)d.K, kbeg + (uint32_t)k_chunk);
   A += (int64_t)zb * d.a_b;
   B += (int64_t)zb * d.b_b;
   C += (int64_t)zb * d.c_b;
@@ -324,14 +325,14 @@ __global__ void __launch_bounds__(32 * SM_WARPS) contract_f64_small_kernel(const
   const int64_t cb = cok ? off3(n, d.N2, d.N3, d.b_n1, d.b_n2, d.b_n3) : 0;
   double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
   constexpr int U = 8;   // k-steps in flight
-  for (int k0 = kbeg + 4 * warp; k0 < kend; k0 += 4 * SM_WARPS * U) {
+  for (uint32_t k0 = kbeg + 4 * warp; k0 < kend; k0 += 4 * SM_WARPS * U) {
     double a[U], b[U];
 #pragma unroll
     for (int q = 0; q < U; ++q) {
-      const int k = k0 + 4 * SM_WARPS * q + (lane & 3);
+      const uint32_t k = k0 + 4 * SM_WARPS * q + (lane & 3);
       a[q] = b[q] = 0.0;
       if (k < kend) {
-        const uint32_t k1 = (uint32_t)k / (uint32_t)d.K2, k2 = (uint32_t)k - k1 * (uint32_t)d.K2;
+        const uint32_t k1 = k / (uint32_t)d.K2, k2 = k - k1 * (uint32_t)d.K2;
         if (rok) a[q] = A[ra + (int64_t)k1 * d.a_k1 + (int64_t)k2 * d.a_k2];
         if (cok) b[q] = B[cb + (int64_t)k1 * d.b_k1 + (int64_t)k2 * d.b_k2];
       }
