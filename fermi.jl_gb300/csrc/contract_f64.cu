@@ -859,6 +859,7 @@ bool run_tc(TcEngine* tc, bool optional, OzLevel lv, double alpha, const TView& 
 bool TcEngine::scratch_fits(double growth) const {
   if (growth <= 0) return true;
   if (scratch_held() + growth > scratch_max) return false;
+  if (growth < 2.5e8) return true;   // try_alloc sees to it, and it can be reclaimed: no need to ask the driver
   size_t f = 0, t = 0;
   return cudaMemGetInfo(&f, &t) == cudaSuccess && growth <= 0.5 * (double)f;
 }

@@ -264,8 +264,9 @@ struct TcEngine {
   DBuf<__nv_bfloat16> bvvA, bvvB;
   DBuf<int> bvvEx;
   // Digit slices take twice the memory of an FP64 operand, and FP64 contractions
-  // can do without: they take more scratch only while that leaves half of the
-  // free memory, and run on the FP64 pipe otherwise.
+  // can do without: they take more scratch (from 250 MB on) only while that leaves
+  // half of the free memory, and run on the FP64 pipe otherwise or where the
+  // allocation fails.
   double scratch_max = 1e300;   // test hook: bytes of packed operands in all
   double scratch_held() const {
     double b = (double)(bufA.bytes() + bufB.bytes() + exA.bytes() + exB.bytes() + bvvA.bytes() + bvvB.bytes() + bvvEx.bytes());
