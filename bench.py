@@ -59,16 +59,11 @@ FP64_ITERATIONS = 17
 FP64_PEAK_TFLOPS = 1.05     # measured DMMA / DFMA peak of a GB300 (own probe)
 # MEASURED_PEAKS.json values, used when the file is not present
 PEAKS_FALLBACK = {"hbm_gbs": 6778.3, "bf16_tflops": 1908.9, "bf16_tflops_sustained": 1714.6}
-# DRAM traffic per algorithmic flop of the DMMA kernel, from one ncu capture of
-# its largest launch (the o^3 v^3 ring contraction at (H2O)8, M = N = K = 4864:
-# dram__bytes_read + dram__bytes_write = 7.114e9 + 0.186e9 B for 2 * 4864^3 flop)
-DMMA_DRAM_BYTES_PER_FLOP = (7.114e9 + 0.186e9) / (2.0 * 4864.0 ** 3)
-# the same for the exact-slice kernel per executed BF16 flop, from one ncu
-# capture (dram__bytes_read.sum + dram__bytes_write.sum, one pass) of all 541
-# gemm_oz_kernel launches of one (H2O)8 mixed solve: 359.8e9 + 78.6e9 B for
-# 541 launches of 8.989e11 executed flop on average (single CTAs on 128 x 128 tiles;
-# the pairs on 256 x 128 tiles read each B panel half as often)
-OZ_DRAM_BYTES_PER_FLOP = (359.8e9 + 78.6e9) / (541 * 8.989e11)
+# DRAM traffic of the exact-slice kernel per executed BF16 flop, from one ncu
+# capture (dram__bytes_read.sum + dram__bytes_write.sum, one pass) of all 443
+# gemm_oz_kernel launches of one (H2O)8 mixed solve: 260.7e9 + 45.7e9 B for 443
+# launches of 8.265e11 executed flop on average
+OZ_DRAM_BYTES_PER_FLOP = (260.7e9 + 45.7e9) / (443 * 8.265e11)
 
 
 def parse():
@@ -498,17 +493,13 @@ def main():
     dom = max(((c, prof[4 * c + 1]) for c in cls), key=lambda x: x[1])[0]
     n, ms, work = prof[4 * dom], prof[4 * dom + 1], prof[4 * dom + 2]
     ach = work / ms / (1e9 if dom != 2 else 1e6) if ms else None
-    traffic = None
-    if dom == 0 and n:
-        traffic = DMMA_DRAM_BYTES_PER_FLOP * work / n
-    elif dom == 5 and n:
-        traffic = OZ_DRAM_BYTES_PER_FLOP * work / n
+    # measured for the mixed solve of (H2O)8 only
+    traffic = OZ_DRAM_BYTES_PER_FLOP * work / n if dom == 5 and n and args.waters == 8 and args.form == "mixed" else None
     roof = {"bound": "hbm" if dom == 2 else "tensor", "kernel": cls[dom], "achieved": ach,
             "peak": pk[dom][0], "unit": pk[dom][1], "frac": (ach / pk[dom][0]) if ach else None,
             "traffic": traffic,
-            "traffic_note": ("bytes per average launch: ncu-measured DRAM bytes per executed flop (all launches of "
-                             "one solve for the exact-slice kernel, the largest launch for the DMMA kernel) times "
-                             "the average launch's flops" if traffic is not None else None),
+            "traffic_note": ("bytes per average launch: ncu-measured DRAM bytes per executed flop over all launches "
+                             "of one solve, times the average launch's flops" if traffic is not None else None),
             "launches": int(n), "work_per_launch": (work / n) if n else None,
             "peak_source": ("own measurement (DMMA probe; MEASURED_PEAKS.json has no FP64 figure)" if dom == 0
                             else peaks_src + (" (sustained BF16)" if dom != 2 else " (HBM copy)")),

@@ -1087,9 +1087,9 @@ int ccsd_run(fcc_ctx* c, const fcc_opts* opt, fcc_iter_stats* log, int32_t log_c
   int status = FCC_OK;
   bool conv_final = false;
   // Iteration kinds: FP64 residual; split-BF16 residual with three
-  // products (mixed form, first phase); exact-slice BF16 residual at 6-8
+  // products (mixed form, first phase); exact-slice BF16 residual at 6-7
   // weight groups (mixed form, second phase: Ozaki-scheme products whose
-  // error, ~1e-11 absolute in the residual, is far below the convergence
+  // error, ~1e-10 in the Jacobi step, is far below the convergence
   // criteria); exact-slice residual at 9 weight groups, whose truncation
   // (below 2^-47 of max|A_r| max|B_c| per term) and exact accumulation give
   // FP64-class contractions.  A run ends only on an iteration of its finish

@@ -168,7 +168,7 @@ struct CtrDesc {
   double alpha, beta;
   int64_t M3 = 1, N3 = 1;
   int64_t a_m3 = 0, c_m3 = 0, b_n3 = 0, c_n3 = 0;
-  bool wide = false;   // 64 x 64 tiles whatever the size
+  bool wide = false;   // 64 x 64 tiles also where small ones would be faster (einsum: from 1e7 flop on)
   bool sym = false;    // C(m, n) = C(n, m): tiles below the diagonal may be copied (beta = 0)
 };
 

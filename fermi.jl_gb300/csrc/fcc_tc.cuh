@@ -237,7 +237,7 @@ struct TcEngine {
   // FP64 contractions of this size and more run as exact-slice products at the
   // FP64 level, whether `enabled` or not
   double f64_min_flops = 4e7;
-  // FP64 contractions on 64 x 64 tiles of the FP64 pipe whatever their size: the
+  // FP64 contractions on the FP64 pipe, from 1e7 flop on in 64 x 64 tiles: the
   // integrals that every form starts from (setup_integrals)
   bool f64_wide = false;
   bool f64_sym = false;   // and the next ones' results are symmetric in (m, n)

@@ -20,7 +20,8 @@
 // where their rows are not adjacent), with c or its run the columns so that
 // stores coalesce.  (Twelve FP64-pipe contractions per pair and run of k took
 // 0.54 s at (H2O)4 where this takes 0.04, of which the products' store stages
-// are the larger part: K = v + o is short.)  The energy kernel then works on 8 x
+// are the larger part: K = v + o is short.)  Small systems, and those whose slices
+// do not fit in memory, run the terms on the FP64 pipe.  The energy kernel then works on 8 x
 // 8 x 8 sub-cubes (blocks A >= B >= C): it stages the six permutations of a
 // sub-cube of W in shared memory with loads along W's stride-1 index, forms V
 // from T1 and (ia|jb) blocks staged beside them, and reduces in FP64 into
